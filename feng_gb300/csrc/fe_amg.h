@@ -27,6 +27,7 @@ struct HostCSR {
 
 struct AMGLevel {
   HostCSR A, P, R;
+  HostCSR AP;             // A P (the Galerkin product's first half)
   std::vector<double> dinv;
   double lmax = 0;  // spectral radius estimate of D^-1 A
 };
@@ -62,24 +63,24 @@ struct AMGParams {
 };
 
 int amg_build(const HostCSR &A, const AMGParams &p, AMGHierarchy &H);
-
-template <typename V>
-struct DevLevelT;
+HostCSR amg_transpose(const HostCSR &A);
 
 // Device hierarchy and V-cycle, in FP64 or FP32.
 class AMGDevice {
  public:
   ~AMGDevice();
-  int upload(const AMGHierarchy &H, const AMGParams &p, int fp32, cudaStream_t s);
+  // keepA: keep the finest operator for spmv64 / spmv32.
+  int upload(const AMGHierarchy &H, const AMGParams &p, int fp32, cudaStream_t s, bool keepA);
   // x = V-cycle(b) for the finest operator (x overwritten).
   void vcycle64(const double *b, double *x);
   void vcycle32(const float *b, float *x);
   // The same V-cycle on two right-hand sides stored interleaved
   // (b[2 i + c], component c of row i): one pass over each operator.
-  // The caller's vector for the result of a paired V-cycle: component c of
-  // finest row i goes, times *scale, to z[dofX[i]] (c = 0) or z[dofY[i]].
+  // The caller's vector for the result of a V-cycle: component c of finest
+  // row i goes, times *scale, to z[dofC[NV i + c]] when dofC is set, else to
+  // z[dofX[i]] (c = 0) or z[dofY[i]].
   struct OutMap {
-    const int32_t *dofX = nullptr, *dofY = nullptr;
+    const int32_t *dofX = nullptr, *dofY = nullptr, *dofC = nullptr;
     const double *scale = nullptr;
     void *z = nullptr;
     // Optional pressure fold of the steady saddle-point preconditioner
@@ -96,27 +97,27 @@ class AMGDevice {
     const double *pMass = nullptr, *consts = nullptr;
     const void *r = nullptr;
   };
-  // Whether the finest level runs on its sliced-ELL copy (then a paired
-  // V-cycle with an OutMap always writes through it).
-  bool fineSell() const { return !lv_.empty() && lv_[0].sellPtr != nullptr; }
-  // Both components at once (x, b interleaved).  With om, the finest
-  // post-smoothing pass writes the result through om when it can (then
-  // returns true; x does not hold the result), otherwise x holds it.
+  // Whether a cycle with an OutMap writes its result through it (the finest
+  // level's pass on the way up; not the Chebyshev path, nor a single level).
+  bool writesOut() const { return lv_.size() > 1 && p_.chebyDegree == 1; }
+  // Both components at once (x, b interleaved).  With om, the finest level's
+  // last pass writes the result through om when it can (then returns true; x
+  // does not hold the result), otherwise x holds it.
   bool vcycle2_64(const double *b, double *x, const OutMap *om = nullptr);
   bool vcycle2_32(const float *b, float *x, const OutMap *om = nullptr);
   // Three interleaved components (b[3 i + c]): the velocity of tetrahedral
-  // Taylor-Hood systems, one pass over each level operator; x holds the result.
-  void vcycle3_64(const double *b, double *x);
-  void vcycle3_32(const float *b, float *x);
+  // Taylor-Hood systems, one pass over each level operator; om as above.
+  bool vcycle3_64(const double *b, double *x, const OutMap *om = nullptr);
+  bool vcycle3_32(const float *b, float *x, const OutMap *om = nullptr);
   // y = A x with the finest operator.
   void spmv64(const double *x, double *y);
   void spmv32(const float *x, float *y);
-  // The finest-level pre-smoothing pass (zero start + first Chebyshev step
-  // in one kernel) on two interleaved components, on the level's own work
-  // vectors: one of the two finest-level kernels of every V-cycle.
+  // The finest level's pass of a V-cycle on the way down (both products with
+  // its right-hand side in one kernel) on two interleaved components, on the
+  // level's own work vectors.
   void fineStep2();
-  // Algorithmic bytes of fineStep2: the level operator once (values,
-  // columns, row pointers) and every vector entry it reads or writes once.
+  // Algorithmic bytes of fineStep2: its operators once (values, columns, row
+  // pointers) and every vector entry it reads or writes once.
   int64_t fineStep2Bytes() const;
   int64_t n() const { return n0_; }
   int levels() const { return (int)lv_.size(); }
@@ -133,13 +134,31 @@ class AMGDevice {
     // Sliced-ELL copy of A (slices of 32 rows, each padded to its longest
     // row with a valid column and value 0, entries column-major in the
     // slice): one thread per row, every load a full line.  Built for the
-    // finest level only, for A and for the prolongation P.
+    // finest level only.
     int32_t *sellPtr = nullptr;  // [nSlices + 1] first entry of each slice
     int32_t *sellCol = nullptr;
     void *sellVal = nullptr;
-    int32_t *sellPPtr = nullptr, *sellPCol = nullptr;  // the same for P
-    void *sellPVal = nullptr;
+    // Combined operators of the degree-1 cycle (w = D^-1 / theta):
+    // T = 2 w - w A w, Q = (I - w A) P and Q^T, so that the level is
+    // b_c = Q^T b, s = T b on the way down (one kernel: both read b) and
+    // x = s + Q x_c on the way up, instead of pre-smoothing, restriction,
+    // prolongation and post-smoothing, four kernels that also pass x, y and
+    // the residual through memory.  Q has 7 to 18 entries per row where A has
+    // 11 to 26 and P 2 to 4, so T, Q and Q^T together are as large as A
+    // twice, P and R.  T and Q in sliced ELL on a large finest level, else
+    // CSR; Q^T in CSR (30 to 250 entries per row).  tRow / qRow: the row of
+    // each thread of the sliced-ELL copies (rows sorted by length).
+    int32_t *tPtr = nullptr, *tCol = nullptr, *qPtr = nullptr, *qCol = nullptr, *rPtr = nullptr, *rCol = nullptr;
+    void *tVal = nullptr, *qVal = nullptr, *rVal = nullptr;
+    int32_t *tRow = nullptr, *qRow = nullptr;
+    int lanesT = 4, lanesQ = 4;  // lanes per row of T and Q in CSR (Q^T: lanesR)
+    int64_t nnzT = 0, nnzR = 0;
+    bool sellTQ = false;
   };
+  int upload_combined(const AMGLevel &h, Lev &L, bool fine, double theta);
+  // bc = Q^T b, s = T b; x = s + Q xc (through out_ when out)
+  template <typename V, int NV> void down(const Lev &L, const V *b, V *bc, V *s);
+  template <typename V, int NV> void up(const Lev &L, const V *xc, const V *s, V *x, bool out);
   template <typename V, int NV> void vcycle_t(int l, const V *b, V *x);
   OutMap out_;
   bool outWritten_ = false;

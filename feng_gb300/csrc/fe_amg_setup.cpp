@@ -176,6 +176,8 @@ int64_t aggregate(const HostCSR &A, double theta, std::vector<int32_t> &agg)
 
 }  // namespace
 
+HostCSR amg_transpose(const HostCSR &A) { return transpose(A); }
+
 int amg_build(const HostCSR &A0, const AMGParams &p, AMGHierarchy &H)
 {
   H = AMGHierarchy();
@@ -230,8 +232,8 @@ int amg_build(const HostCSR &A0, const AMGParams &p, AMGHierarchy &H)
       // plain aggregation: P = T
       L.P = T;
       L.R = transpose(T);
-      HostCSR AT = spgemm(A, T);
-      A = spgemm(L.R, AT);
+      L.AP = spgemm(A, T);
+      A = spgemm(L.R, L.AP);
       H.levels.push_back(std::move(L));
       continue;
     }
@@ -305,8 +307,8 @@ int amg_build(const HostCSR &A0, const AMGParams &p, AMGHierarchy &H)
     }
     L.P = P;
     L.R = transpose(P);
-    HostCSR AP = spgemm(A, P);
-    A = spgemm(L.R, AP);
+    L.AP = spgemm(A, P);
+    A = spgemm(L.R, L.AP);
     H.levels.push_back(std::move(L));
   }
   // Dense inverse of the coarsest operator (Gauss-Jordan, partial pivoting).

@@ -221,7 +221,7 @@ class Krylov {
   // Schur complement approximation mu M_p^-1.  c0 = 0 restores the steady
   // preconditioner.  Replayed cycle graphs are rebuilt.
   int setTransientShift(double c0, double mu);
-  // The multigrid's finest-level smoother step alone (benchmarking); bytes:
+  // The multigrid's finest-level pass on the way down alone (benchmarking); bytes:
   // its algorithmic bytes, 0 when there is no multigrid.
   int smootherStep(int64_t *bytes);
   // One pass of the mixed FGMRES Gram-Schmidt on the current FP32 basis with

@@ -650,7 +650,7 @@ int Krylov::setup_mg(const PrecondInfo &pi)
   }
   AMGHierarchy H;
   FE_TRY(amg_build(*pi.lap, ap, H));
-  FE_TRY(M.amg->upload(H, ap, M.fp32, s_));
+  FE_TRY(M.amg->upload(H, ap, M.fp32, s_, M.inner > 0));
   M.lapDiagSum = M.amg->finestDiagSum();
   FE_TRY(up(&M.dofX, pi.nodeDofX));
   if(M.kind == 4) FE_TRY(up(&M.dofY, pi.nodeDofY));
@@ -830,13 +830,13 @@ int Krylov::factor_mg(const double *values64, const float *values32)
   M.hconst[3] = M.cc;
   CKM(cudaMemcpyAsync(M.consts, M.hconst, sizeof(double) * 4, cudaMemcpyHostToDevice, s_));
   // The pressure fold: the steady two-component preconditioner with one
-  // V-cycle on a sliced-ELL finest level (the fold's output goes through
-  // that level's post-smoothing pass).
+  // V-cycle whose last pass writes the caller's vector (the fold's output
+  // goes through that pass).
   static const bool foldOn = [] {
     const char *e = std::getenv("FENG_PFOLD");
     return !(e && std::strcmp(e, "0") == 0);
   }();
-  M.fold = foldOn && M.kind == 4 && M.nc == 2 && M.inner <= 0 && !M.amgP && M.amg->fineSell();
+  M.fold = foldOn && M.kind == 4 && M.nc == 2 && M.inner <= 0 && !M.amgP && M.amg->writesOut();
   if(M.kind == 4) {
     // the pressure scale (FP64 and FP32) and, for the fold, u on the device
     const double coef = -SCHUR_FACTOR * M.s, den = M.vfac * M.sigma * M.divu;
@@ -881,7 +881,7 @@ int Krylov::setTransientShift(double c0, double mu)
   AMGHierarchy H;
   FE_TRY(amg_build(L, vp, H));
   auto amg = std::make_unique<AMGDevice>();
-  FE_TRY(amg->upload(H, vp, M.fp32, s_));
+  FE_TRY(amg->upload(H, vp, M.fp32, s_, M.inner > 0));
   M.amg = std::move(amg);
   M.lapDiagSum = M.amg->finestDiagSum();
   // Pressure Laplacian multigrid (built once) and the Cahouet-Chabard weight.
@@ -910,7 +910,7 @@ int Krylov::setTransientShift(double c0, double mu)
     AMGHierarchy HP;
     FE_TRY(amg_build(Lp, M.params, HP));
     auto ap = std::make_unique<AMGDevice>();
-    FE_TRY(ap->upload(HP, M.params, M.fp32, s_));
+    FE_TRY(ap->upload(HP, M.params, M.fp32, s_, false));
     M.amgP = std::move(ap);
     const size_t vs = M.fp32 ? sizeof(float) : sizeof(double);
     CKM(cudaMalloc(&M.pr, vs * std::max<int64_t>(1, M.nP)));
@@ -975,7 +975,7 @@ void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
     bool written;
     if constexpr(sizeof(V) == 8) written = M.amg->vcycle2_64((const double *)M.bxy, (double *)M.zxy, &om);
     else written = M.amg->vcycle2_32((const float *)M.bxy, (float *)M.zxy, &om);
-    if(!written) set_error("pressure fold: the finest post-smoothing pass did not write the result");
+    if(!written) set_error("pressure fold: the V-cycle did not write the result");
     return;
   } else {
     const int gp = (int)std::min<int64_t>(NPART, std::max<int64_t>(1, (M.nP + 255) / 256));
@@ -1001,9 +1001,14 @@ void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
       const int64_t nq = 3 * M.nNodes;
       ::feng::launch_k(k_vel_rhs_nc<V>, grid(nq), 256, 0, s_, nq, M.dofC, M.upIa, M.upCol, (const V *)M.gVals, r, z, (V *)M.bxy,
                                                  skip);
-      if constexpr(sizeof(V) == 8) M.amg->vcycle3_64((const double *)M.bxy, (double *)M.zxy);
-      else M.amg->vcycle3_32((const float *)M.bxy, (float *)M.zxy);
-      ::feng::launch_k(k_vel_out_nc<V>, grid(nq), 256, 0, s_, nq, M.dofC, (const V *)M.zxy, M.consts, z, skip);
+      AMGDevice::OutMap om;
+      om.dofC = M.dofC;
+      om.scale = M.consts;
+      om.z = z;
+      bool written;
+      if constexpr(sizeof(V) == 8) written = M.amg->vcycle3_64((const double *)M.bxy, (double *)M.zxy, &om);
+      else written = M.amg->vcycle3_32((const float *)M.bxy, (float *)M.zxy, &om);
+      if(!written) ::feng::launch_k(k_vel_out_nc<V>, grid(nq), 256, 0, s_, nq, M.dofC, (const V *)M.zxy, M.consts, z, skip);
       return;
     }
     if(M.inner <= 0) {
@@ -1011,7 +1016,7 @@ void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
       // each level operator for the two right-hand sides).
       ::feng::launch_k(k_vel_rhs_pair<V>, grid(2 * M.nNodes), 256, 0, s_, M.nNodes, M.dofX, M.dofY, M.upIa, nullptr, M.upCol,
                                                                (const V *)M.gVals, r, z, (V *)M.bxy, skip);
-      // the finest post-smoothing pass writes z_u (times 1/s) itself when
+      // the V-cycle's last pass writes z_u (times 1/s) itself when
       // it can; otherwise the interleaved result is scattered here
       AMGDevice::OutMap om;
       om.dofX = M.dofX;

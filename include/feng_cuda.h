@@ -390,8 +390,9 @@ int fe_cuda_reset_times(fe_cuda_system *s);
  * events on the system stream, each run preceded by an L2 flush (a write, then a read, of
  * flush_bytes): which = 0 residual assembly (all colors), 1 Jacobian assembly
  * (a zeroed matrix, then the Jacobian), 2 SpMV with the system matrix, 3 one preconditioner
- * application, 4 one finest-level multigrid pre-smoothing pass (zero start
- * fused with the first Chebyshev step, both velocity components), 5 one
+ * application, 4 the finest level's multigrid pass on the way down (smoother
+ * degree 1: restriction and smoothing in one kernel; above: the pre-smoothing
+ * pass; both velocity components), 5 one
  * Gram-Schmidt dot pass of the mixed FGMRES over restart/2 basis vectors,
  * 6 one Gram-Schmidt update + norm pass over restart/2 basis vectors;
  * 7 and 8 the passes of 5 and 6 launched 10 * reps times back to back, with
@@ -409,7 +410,7 @@ int fe_cuda_reset_times(fe_cuda_system *s);
  * Phases 5 to 9 need a mixed-precision system that has solved once, 11 and 12 a system that has solved
  * once (12: FGMRES).  Uses the current solution state. */
 int fe_cuda_bench_phase(fe_cuda_system *s, int which, int reps, int64_t flush_bytes, double *avg_ms);
-/* Algorithmic bytes of one run of phase 4 (finest multigrid operator read
+/* Algorithmic bytes of one run of phase 4 (its finest-level operators read
  * once, each vector entry read or written once). */
 int fe_cuda_smoother_bytes(fe_cuda_system *s, int64_t *bytes);
 /* Algorithmic bytes of one run of phase 4 to 10 (every operand read or
