@@ -1233,9 +1233,10 @@ __global__ void k_cg_p(int64_t n, CGState *cs, const RedState *st, const double 
   if(cs->done) return;
   const double rzNew = st->result[0];
   const double beta = first ? 0. : rzNew / cs->rz;
+  // the first p is z alone: p is not initialised then (0 * NaN is NaN)
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = z[i] + beta * p[i];
+    p[i] = first ? z[i] : z[i] + beta * p[i];
   __syncthreads();
   // the scalar update happens in k_cg_rz once every block is done
 }

@@ -155,7 +155,8 @@ __global__ void k_pcg_xr(int64_t n, const double *__restrict__ scal, const V *__
   }
 }
 
-// p = z + beta p with beta = rz_new / rz (scal[2] / scal[0]); then rz = rz_new.
+// p = z + beta p with beta = rz_new / rz (scal[2] / scal[0]); then rz =
+// rz_new.  The first p is z alone (p is not initialised then: 0 * NaN is NaN).
 template <typename V>
 __global__ void k_pcg_p(int64_t n, const double *__restrict__ scal, const V *__restrict__ z, V *__restrict__ p,
                         int first)
@@ -163,7 +164,7 @@ __global__ void k_pcg_p(int64_t n, const double *__restrict__ scal, const V *__r
   FE_PDL_ENTRY();
   const double beta = (first || scal[0] == 0.) ? 0. : scal[2] / scal[0];
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = z[i] + (V)beta * p[i];
+    p[i] = first ? z[i] : z[i] + (V)beta * p[i];
 }
 
 __global__ void k_pcg_shift(double *scal) {
