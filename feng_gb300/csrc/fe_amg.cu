@@ -895,6 +895,9 @@ int AMGDevice::upload(const AMGHierarchy &H, const AMGParams &p, int fp32, cudaS
   nCoarse_ = lv_.empty() ? 0 : lv_.back().n;
   nnz0_ = H.levels.empty() ? 0 : H.levels[0].A.nnz();
   FE_TRY(fp32 ? upload_vec<float>(&coarseInv_, H.coarseInv) : upload_vec<double>(&coarseInv_, H.coarseInv));
+  // the copies ran on the legacy stream, with which s (non-blocking) is not
+  // ordered, and one may return before it has reached the device
+  CKA(cudaStreamSynchronize(cudaStreamLegacy));
   return FE_OK;
 }
 

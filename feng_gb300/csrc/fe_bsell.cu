@@ -2,6 +2,7 @@
 #include "fe_bsell.h"
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "fe_common.h"
@@ -82,12 +83,12 @@ __device__ __forceinline__ void madd(dfl &s, float a, float2 x)
   s = df_add(s, df_fast2(p, e));
 }
 
-// Adds the entries of steps [k0, k1) of one lane (NR rows, NC columns each)
-// to acc, in steps of UNR entries, the next step's columns and values loaded
-// before this step's gathers of x (one memory latency per step).
+// Adds the entries k0, k0 + st, ... below k1 of one lane (NR rows, NC columns
+// each) to acc, UNR entries at a time, the next ones' columns and values
+// loaded before the gathers of x of these (one memory latency per UNR).
 template <int NR, int NC, int UNR, bool VEC, typename VA, typename X, typename S>
 __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *__restrict__ val, int32_t k0,
-                                     int32_t k1, int lane, const X *__restrict__ x, S (&acc)[NR])
+                                     int32_t k1, int st, int lane, const X *__restrict__ x, S (&acc)[NR])
 {
   constexpr int NV = NR * NC, W = vec_width<VA, NV>(), PL = NV / W;
   int32_t c[UNR];
@@ -96,16 +97,16 @@ __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *
 #pragma unroll
     for(int u = 0; u < UNR; ++u) {
       c[u] = -1;
-      if(k + u < k1) {
-        c[u] = __ldcs(col + ((int64_t)(k + u) << 5) + lane);
+      if(k + u * st < k1) {
+        c[u] = __ldcs(col + ((int64_t)(k + u * st) << 5) + lane);
 #pragma unroll
         for(int p = 0; p < PL; ++p)
-          load_vec<VA, W>(val + ((((int64_t)(k + u) * PL + p) << 5) + lane) * W, &v[u][p * W]);
+          load_vec<VA, W>(val + ((((int64_t)(k + u * st) * PL + p) << 5) + lane) * W, &v[u][p * W]);
       }
     }
   };
   load(k0);
-  for(int32_t k = k0; k < k1; k += UNR) {
+  for(int32_t k = k0; k < k1; k += UNR * st) {
     int32_t cc[UNR];
     VA vc[UNR][NV];
 #pragma unroll
@@ -114,7 +115,7 @@ __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *
 #pragma unroll
       for(int q = 0; q < NV; ++q) vc[u][q] = v[u][q];
     }
-    load(k + UNR);
+    load(k + UNR * st);
 #pragma unroll
     for(int u = 0; u < UNR; ++u)
       if(cc[u] >= 0) {
@@ -128,6 +129,19 @@ __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *
   }
 }
 
+__device__ __forceinline__ float add(float a, float b) { return a + b; }
+__device__ __forceinline__ double add(double a, double b) { return a + b; }
+__device__ __forceinline__ dfl add(dfl a, dfl b) { return df_add(a, b); }
+__device__ __forceinline__ float from_lane(float a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ double from_lane(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ dfl from_lane(dfl a, int o)
+{
+  dfl r;
+  r.hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
+  r.lo = __shfl_xor_sync(0xffffffffu, a.lo, o);
+  return r;
+}
+
 // Entries in flight per thread: about 20 registers of them.
 template <typename VA, int NV>
 constexpr int unroll()
@@ -137,14 +151,19 @@ constexpr int unroll()
 }
 
 template <int NR, int D, bool VEC, typename VA, typename X, typename S>
-__device__ __forceinline__ void group_sum(const BlockSell::Part &P, int64_t g, const X *__restrict__ x, S (&acc)[NR])
+__device__ __forceinline__ void group_sum(const BlockSell::Part &P, int64_t g, int sub, int lanes,
+                                          const X *__restrict__ x, S (&acc)[NR])
 {
   const int64_t sl = g >> 5;
   const int lane = (int)(g & 31);
   if constexpr(D > 1)
-    walk<NR, D, unroll<VA, NR * D>(), VEC, VA, X, S>(P.pCol, (const VA *)P.pVal, P.pPtr[sl], P.pPtr[sl + 1], lane, x,
-                                                     acc);
-  walk<NR, 1, unroll<VA, NR>(), false, VA, X, S>(P.sCol, (const VA *)P.sVal, P.sPtr[sl], P.sPtr[sl + 1], lane, x, acc);
+    walk<NR, D, unroll<VA, NR * D>(), VEC, VA, X, S>(P.pCol, (const VA *)P.pVal, P.pPtr[sl] + sub, P.pPtr[sl + 1],
+                                                     lanes, lane, x, acc);
+  walk<NR, 1, unroll<VA, NR>(), false, VA, X, S>(P.sCol, (const VA *)P.sVal, P.sPtr[sl] + sub, P.sPtr[sl + 1], lanes,
+                                                 lane, x, acc);
+  for(int o = lanes >> 1; o > 0; o >>= 1)
+#pragma unroll
+    for(int i = 0; i < NR; ++i) acc[i] = add(acc[i], from_lane(acc[i], o));
 }
 
 template <typename S>
@@ -154,14 +173,18 @@ __device__ __forceinline__ S zero_of()
   else return (S)0;
 }
 
-// y = A x or b - A x, one thread per row group; the single rows' blocks come
+// y = A x or b - A x, `lanes` (a power of two) threads per row group, each
+// taking every lanes-th entry; the single rows' blocks come
 // first (pressure rows, whose groups are as long as a vertex node's).
 // Bound: HBM, the layout's bytes (88 MB for the FP32 Jacobian of the 256 x
-// 256 Kovasznay case against 143 MB with a column per entry); in FP64 the
-// FP64 pipe (one product per entry) and the bytes about equally.
+// 256 Kovasznay case against 143 MB with a column per entry, 21.8 us cold
+// against 26.3 us; 32^3 cube 65 us against 116 us); in FP64 the FP64 pipe (one
+// product per entry, no lane sums) and the bytes about equally: 41 us against
+// 82 us with eight lanes per CSR row.
 template <int MODE, int D, bool VEC, typename VA, typename X, typename Y>
-__global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::Part one, const X *__restrict__ x,
-                                               const double *__restrict__ b, Y *__restrict__ y,
+__global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::Part one, int lanes,
+                                               const X *__restrict__ x, const double *__restrict__ b,
+                                               Y *__restrict__ y,
                                                const int *__restrict__ done)
 {
   FE_PDL_ENTRY();
@@ -172,22 +195,24 @@ __global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::P
     else if constexpr(MODE == RESID32_DF) y[row] = b[row] - df_to(s);
     else y[row] = b[row] - s;
   };
-  const int64_t ob = (one.n + 255) >> 8;
+  const int64_t ob = (one.n * lanes + 255) >> 8;
+  const int sub = threadIdx.x & (lanes - 1);
+  // groups past the end repeat the last one, so that the lane sums run with
+  // full warps
   if((int64_t)blockIdx.x < ob) {
-    const int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if(g >= one.n) return;
+    const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / lanes, g = t < one.n ? t : one.n - 1;
     S acc[1] = {zero_of<S>()};
-    group_sum<1, D, VEC, VA, X, S>(one, g, x, acc);
-    put(one.row[g], acc[0]);
+    group_sum<1, D, VEC, VA, X, S>(one, g, sub, lanes, x, acc);
+    if(t == g && sub == 0) put(one.row[g], acc[0]);
     return;
   }
   if constexpr(D > 1) {
-    const int64_t g = ((int64_t)blockIdx.x - ob) * 256 + threadIdx.x;
-    if(g >= grp.n) return;
+    const int64_t t = (((int64_t)blockIdx.x - ob) * 256 + threadIdx.x) / lanes, g = t < grp.n ? t : grp.n - 1;
     S acc[D];
 #pragma unroll
     for(int i = 0; i < D; ++i) acc[i] = zero_of<S>();
-    group_sum<D, D, VEC, VA, X, S>(grp, g, x, acc);
+    group_sum<D, D, VEC, VA, X, S>(grp, g, sub, lanes, x, acc);
+    if(t != g || sub != 0) return;
     const int64_t row = grp.row[g];
 #pragma unroll
     for(int i = 0; i < D; ++i) put(row + i, acc[i]);
@@ -429,6 +454,13 @@ int BlockSell::build(const DeviceCSR &A, bool fp32, cudaStream_t s)
   CKB(cudaMemcpyAsync(d, start.data(), (size_t)n, cudaMemcpyHostToDevice, s));
   FE_TRY(fill(grp_, grp, d));
   FE_TRY(fill(one_, one, d));
+  // threads per group: at least a quarter of the 311 k resident threads of
+  // the GPU (20^3 cube, 69 k groups: 27.0 ms per two time steps with two
+  // threads against 28.1 ms with one; four times as many threads are no
+  // faster)
+  const int64_t groups = (int64_t)(grp.size() + one.size());
+  lanes_ = 1;
+  while(lanes_ < (fp32 ? 8 : 4) && groups * lanes_ < 75000) lanes_ *= 2;
   built_ = true;
   return FE_OK;
 }
@@ -454,12 +486,12 @@ void BlockSell::gather(const void *vals)
 template <int MODE, typename VA, typename X, typename Y>
 void BlockSell::launch(const X *x, const double *b, Y *y, const int *done) const
 {
-  const unsigned g = (unsigned)std::max<int64_t>(1, (one_.n + 255) / 256 + (grp_.n + 255) / 256);
+  const unsigned g = (unsigned)((one_.n * lanes_ + 255) / 256 + (grp_.n * lanes_ + 255) / 256);
   auto k = D_ == 3   ? k_bsell<MODE, 3, false, VA, X, Y>
            : D_ == 1 ? k_bsell<MODE, 1, false, VA, X, Y>
            : even_   ? k_bsell<MODE, 2, true, VA, X, Y>
                      : k_bsell<MODE, 2, false, VA, X, Y>;
-  ::feng::launch_k(k, g, 256, 0, s_, grp_, one_, x, b, y, done);
+  if(g > 0) ::feng::launch_k(k, g, 256, 0, s_, grp_, one_, lanes_, x, b, y, done);
 }
 
 void BlockSell::mul32(const float *x, float *y, const int *done) const

@@ -5,7 +5,7 @@
 // columns and those columns come in runs of one node's unknowns, so a node's
 // D x D entries need one column index: 5 (D = 2) or 4.4 (D = 3) bytes per
 // FP32 entry instead of 8, one gather of D consecutive entries of x for D^2
-// products, and one thread holds the D row sums.  The blocks are found in the
+// products, and the threads of a node hold its D row sums.  The blocks are found in the
 // pattern itself (rows with equal columns; runs of columns), not in the
 // numbering, so any pattern is accepted: rows and columns that do not pair
 // up stay single.
@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "fe_krylov.h"
 
@@ -44,7 +45,7 @@ class BlockSell {
   int64_t bytes() const;
 
   // A set of row groups (NR = D rows each, or single rows): groups in slices
-  // of 32, one thread per group; a slice's entries are padded to its longest
+  // of 32, one or more threads per group; a slice's entries are padded to its longest
   // group and stored step by step (entry k of the 32 groups together).
   struct Part {
     int64_t n = 0;                                   // groups
@@ -64,6 +65,7 @@ class BlockSell {
   cudaStream_t s_ = 0;
   Part grp_, one_;  // groups of D rows; single rows
   int D_ = 1;
+  int lanes_ = 1;      // threads per row group
   bool even_ = false;  // D = 2: every block starts at an even column
   bool fp32_ = false, built_ = false;
 };

@@ -6,6 +6,7 @@
 #include <cstring>
 #include <vector>
 
+#include "fe_bsell.h"
 #include "fe_common.h"
 #include "fe_df.h"
 #include "fe_launch.h"
@@ -172,7 +173,7 @@ __global__ void k_absmax(int64_t n, const double *__restrict__ x, double *partia
 }
 
 // h[c] (+)= V_c . w for c < ncols; grid (parts, ncols).  Partials per column.
-__global__ void k_mdot_partial(int64_t n, const double *__restrict__ V, int ncols,
+__global__ void k_mdot_partial(int64_t n, int64_t ld, const double *__restrict__ V, int ncols,
                                const double *__restrict__ w, double *partials,
                                const int *__restrict__ done)
 {
@@ -180,7 +181,7 @@ __global__ void k_mdot_partial(int64_t n, const double *__restrict__ V, int ncol
   if(*done) return;
   __shared__ double sh[RB / 32];
   const int c = blockIdx.y;
-  const double *vc = V + (int64_t)c * n;
+  const double *vc = V + (int64_t)c * ld;
   double v = 0.;
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x)
@@ -207,7 +208,7 @@ __global__ void k_mdot_final(int nparts, double *partials, double *hcur, double 
 }
 
 // w -= sum_c h[c] V_c
-__global__ void k_mupdate(int64_t n, const double *__restrict__ V, int ncols,
+__global__ void k_mupdate(int64_t n, int64_t ld, const double *__restrict__ V, int ncols,
                           const double *__restrict__ h, double *__restrict__ w,
                           const int *__restrict__ done)
 {
@@ -219,7 +220,7 @@ __global__ void k_mupdate(int64_t n, const double *__restrict__ V, int ncols,
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x) {
     double acc = w[i];
-    for(int c = 0; c < ncols; ++c) acc -= sh[c] * V[(int64_t)c * n + i];
+    for(int c = 0; c < ncols; ++c) acc -= sh[c] * V[(int64_t)c * ld + i];
     w[i] = acc;
   }
 }
@@ -1309,7 +1310,7 @@ Krylov::~Krylov()
 {
   cudaFree(V_); cudaFree(Z_); cudaFree(Z32_); cudaFree(V32_); cudaFree(vc32_); cudaFree(xs2_); cudaFree(v32_); cudaFree(w32_);
   cudaFree(zeroFlag_);
-  cudaFree(sellPtr_); cudaFree(sellCol_); cudaFree(sellSrc_); cudaFree(sellVal_);
+  delete bs_;
   cudaFree(w_); cudaFree(r_); cudaFree(t_); cudaFree(p_); cudaFree(q_);
   cudaFree(diag_); cudaFree(diag32_); cudaFree(red_); cudaFree(dsum_);
   cudaFreeHost(hred_);
@@ -1384,11 +1385,20 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
       CK(cudaMemset(V32_, 0, sizeof(float) * ld32_ * (m + 1)));
       CK(cudaMemset(Z32_, 0, sizeof(float) * ld32_ * m));
       CK(cudaMemset(vc32_, 0, sizeof(float) * ld32_));
-      if(n_ >= 32 * 152) FE_TRY(build_sell());
     } else {
-      CK(cudaMalloc(&V_, sizeof(double) * n_ * (m + 1)));
-      CK(cudaMalloc(&Z_, sizeof(double) * n_ * m));
+      ld64_ = (n_ + 31) / 32 * 32;
+      CK(cudaMalloc(&V_, sizeof(double) * ld64_ * (m + 1)));
+      CK(cudaMalloc(&Z_, sizeof(double) * ld64_ * m));
     }
+  }
+  // The block copy pays from about 75 k rows on; below, the CSR kernel's
+  // lanes per row are as fast or faster (ms per solve, block copy / CSR:
+  // Kovasznay FP64 9 k rows 60.2 / 58.1, 36 k 94.6 / 92.0, 84 k 146.6 / 150.0;
+  // mixed 36 k 20.7 / 20.5, 229 k 36.7 / 39.4; P2 diffusion 102 k 4.7 / 4.7,
+  // 408 k 24.3 / 26.2; cube 62 k 21.7 / 21.4, 187 k 27.0 / 28.4).
+  if(n_ >= 75000) {
+    bs_ = new BlockSell();
+    FE_TRY(bs_->build(A_, opt.mixed != 0, s_));
   }
   // one group of 4 rows per thread: the whole pass is one wave of loads
   {
@@ -1601,105 +1611,7 @@ void Krylov::ilu_solve_levels(const VV *r, VV *z, const int *done)
 }
 
 namespace {
-// y = A x on the sliced-ELL copy, FP32, thread = row (rows of a warp are one
-// slice, so every column and value load is one full line).  Steps of UNR
-// entries, software-pipelined: the next step's columns and values are
-// loaded before this step's gathers of x, so a step waits for one memory
-// latency instead of two (29.4 us against 35.0 us with plain unrolled steps
-// of 4 on the 256 x 256 Kovasznay Jacobian).
-template <int UNR>
-__global__ void __launch_bounds__(256) k_spmv_sell(int64_t n, const int32_t *__restrict__ sp,
-                                                   const int32_t *__restrict__ sc, const float *__restrict__ sv,
-                                                   const float *__restrict__ x, float *__restrict__ y,
-                                                   const int *__restrict__ done)
-{
-  FE_PDL_ENTRY();
-  if(done && *done) return;
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if(row >= n) return;
-  const int64_t sl = row >> 5;
-  const int lane = (int)(row & 31);
-  const int32_t base = sp[sl], len = (sp[sl + 1] - base) >> 5;
-  float acc = 0.f;
-  int32_t c[UNR];
-  float a[UNR];
-#pragma unroll
-  for(int u = 0; u < UNR; ++u) {
-    const bool ok = u < len;
-    const int32_t e = base + (u << 5) + lane;
-    c[u] = ok ? __ldcs(sc + e) : -1;
-    a[u] = ok ? __ldcs(sv + e) : 0.f;
-  }
-  for(int32_t k = 0; k < len; k += UNR) {
-    int32_t cn[UNR];
-    float an[UNR];
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      const bool ok = k + UNR + u < len;
-      const int32_t e = base + ((k + UNR + u) << 5) + lane;
-      cn[u] = ok ? __ldcs(sc + e) : -1;
-      an[u] = ok ? __ldcs(sv + e) : 0.f;
-    }
-#pragma unroll
-    for(int u = 0; u < UNR; ++u)
-      if(c[u] >= 0) acc = fmaf(a[u], x[c[u]], acc);
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      c[u] = cn[u];
-      a[u] = an[u];
-    }
-  }
-  y[row] = acc;
-}
-
-// r = b - A x on the sliced-ELL copy of the FP32 matrix with FP64 x and
-// FP64 accumulation (the mixed FGMRES's restart residual: iterative
-// refinement), thread = row, the pipelined walk of k_spmv_sell.
-template <int UNR>
-__global__ void __launch_bounds__(256) k_resid_sell(int64_t n, const int32_t *__restrict__ sp,
-                                                    const int32_t *__restrict__ sc, const float *__restrict__ sv,
-                                                    const double *__restrict__ x, const double *__restrict__ b,
-                                                    double *__restrict__ y)
-{
-  FE_PDL_ENTRY();
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if(row >= n) return;
-  const int64_t sl = row >> 5;
-  const int lane = (int)(row & 31);
-  const int32_t base = sp[sl], len = (sp[sl + 1] - base) >> 5;
-  double acc = 0.;
-  int32_t c[UNR];
-  float a[UNR];
-#pragma unroll
-  for(int u = 0; u < UNR; ++u) {
-    const bool ok = u < len;
-    const int32_t e = base + (u << 5) + lane;
-    c[u] = ok ? __ldcs(sc + e) : -1;
-    a[u] = ok ? __ldcs(sv + e) : 0.f;
-  }
-  for(int32_t k = 0; k < len; k += UNR) {
-    int32_t cn[UNR];
-    float an[UNR];
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      const bool ok = k + UNR + u < len;
-      const int32_t e = base + ((k + UNR + u) << 5) + lane;
-      cn[u] = ok ? __ldcs(sc + e) : -1;
-      an[u] = ok ? __ldcs(sv + e) : 0.f;
-    }
-#pragma unroll
-    for(int u = 0; u < UNR; ++u)
-      if(c[u] >= 0) acc = fma((double)a[u], x[c[u]], acc);
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      c[u] = cn[u];
-      a[u] = an[u];
-    }
-  }
-  y[row] = b[row] - acc;
-}
-
-// x split into two floats, x ~ hi + lo (the operand of k_resid_sell_df)
+// x split into two floats, x ~ hi + lo (the operand of BlockSell::resid32_df)
 __global__ void k_split_x(int64_t n, const double *__restrict__ x, float2 *__restrict__ xs)
 {
   FE_PDL_ENTRY();
@@ -1709,113 +1621,12 @@ __global__ void k_split_x(int64_t n, const double *__restrict__ x, float2 *__res
   }
 }
 
-// r = b - A x as k_resid_sell, the products a (x_hi + x_lo) and their sum in
-// double-float on the FP32 pipes (a x_hi exact by a fused multiply-add), the
-// result subtracted from b in FP64: ~2^-44 relative to sum |a x| against
-// FP64's 2^-53, far below the refinement's stops, and the FP64 pipe of the
-// GB300 (one FP64 product per entry would take ~27 us at 588 k rows) left
-// out.
-template <int UNR>
-__global__ void __launch_bounds__(256) k_resid_sell_df(int64_t n, const int32_t *__restrict__ sp,
-                                                       const int32_t *__restrict__ sc, const float *__restrict__ sv,
-                                                       const float2 *__restrict__ xs, const double *__restrict__ b,
-                                                       double *__restrict__ y)
-{
-  FE_PDL_ENTRY();
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if(row >= n) return;
-  const int64_t sl = row >> 5;
-  const int lane = (int)(row & 31);
-  const int32_t base = sp[sl], len = (sp[sl + 1] - base) >> 5;
-  dfl acc = df_zero();
-  int32_t c[UNR];
-  float a[UNR];
-#pragma unroll
-  for(int u = 0; u < UNR; ++u) {
-    const bool ok = u < len;
-    const int32_t e = base + (u << 5) + lane;
-    c[u] = ok ? __ldcs(sc + e) : -1;
-    a[u] = ok ? __ldcs(sv + e) : 0.f;
-  }
-  for(int32_t k = 0; k < len; k += UNR) {
-    int32_t cn[UNR];
-    float an[UNR];
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      const bool ok = k + UNR + u < len;
-      const int32_t e = base + ((k + UNR + u) << 5) + lane;
-      cn[u] = ok ? __ldcs(sc + e) : -1;
-      an[u] = ok ? __ldcs(sv + e) : 0.f;
-    }
-#pragma unroll
-    for(int u = 0; u < UNR; ++u)
-      if(c[u] >= 0) {
-        const float2 xv = xs[c[u]];
-        const float p = __fmul_rn(a[u], xv.x);
-        float e = __fmaf_rn(a[u], xv.x, -p);
-        e = __fmaf_rn(a[u], xv.y, e);
-        acc = df_add(acc, df_fast2(p, e));
-      }
-#pragma unroll
-    for(int u = 0; u < UNR; ++u) {
-      c[u] = cn[u];
-      a[u] = an[u];
-    }
-  }
-  y[row] = b[row] - df_to(acc);
-}
-
-// sliced-ELL values from the CSR values (padding: 0)
-__global__ void k_sell_gather(int64_t m, const int32_t *__restrict__ src, const float *__restrict__ a,
-                              float *__restrict__ out)
-{
-  FE_PDL_ENTRY();
-  for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t k = src[e];
-    out[e] = k >= 0 ? a[k] : 0.f;
-  }
-}
 }  // namespace
 
-int Krylov::build_sell()
+void Krylov::refreshMatrix(const double *values64, const float *values32)
 {
-  std::vector<int32_t> ia(n_ + 1), ja(A_.nnz);
-  CK(cudaMemcpy(ia.data(), A_.ia, sizeof(int32_t) * (n_ + 1), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(ja.data(), A_.ja, sizeof(int32_t) * A_.nnz, cudaMemcpyDeviceToHost));
-  const int64_t ns = (n_ + 31) / 32;
-  std::vector<int32_t> ptr(ns + 1, 0);
-  for(int64_t sl = 0; sl < ns; ++sl) {
-    int64_t len = 0;
-    for(int64_t r = sl * 32; r < std::min<int64_t>(n_, sl * 32 + 32); ++r) len = std::max<int64_t>(len, ia[r + 1] - ia[r]);
-    if(ptr[sl] + 32 * len >= (int64_t)INT32_MAX) return FE_OK;  // CSR only
-    ptr[sl + 1] = (int32_t)(ptr[sl] + 32 * len);
-  }
-  sellN_ = ptr[ns];
-  std::vector<int32_t> col(std::max<int64_t>(sellN_, 1)), src(col.size(), -1);
-  for(int64_t sl = 0; sl < ns; ++sl) {
-    const int32_t len = (ptr[sl + 1] - ptr[sl]) / 32;
-    for(int lane = 0; lane < 32; ++lane) {
-      const int64_t r = sl * 32 + lane;
-      for(int32_t k = 0; k < len; ++k) {
-        const int64_t e = ptr[sl] + (int64_t)k * 32 + lane;
-        if(r < n_ && ia[r] + k < ia[r + 1]) {
-          col[e] = ja[ia[r] + k];
-          src[e] = ia[r] + k;
-        } else {
-          col[e] = (int32_t)std::min<int64_t>(r, n_ - 1);  // padding: value 0 on an existing column
-        }
-      }
-    }
-  }
-  CK(cudaMalloc(&sellPtr_, sizeof(int32_t) * ptr.size()));
-  CK(cudaMalloc(&sellCol_, sizeof(int32_t) * col.size()));
-  CK(cudaMalloc(&sellSrc_, sizeof(int32_t) * src.size()));
-  CK(cudaMalloc(&sellVal_, sizeof(float) * col.size()));
-  CK(cudaMemcpy(sellPtr_, ptr.data(), sizeof(int32_t) * ptr.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(sellCol_, col.data(), sizeof(int32_t) * col.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(sellSrc_, src.data(), sizeof(int32_t) * src.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemset(sellVal_, 0, sizeof(float) * col.size()));
-  return FE_OK;
+  const void *v = opt.mixed ? (const void *)values32 : (const void *)values64;
+  if(bs_ && v) bs_->gather(v);
 }
 
 int Krylov::factor(const double *values64, const float *values32)
@@ -1823,8 +1634,7 @@ int Krylov::factor(const double *values64, const float *values32)
   factoredOk_ = false;
   cur64_ = values64;
   cur32_ = values32;
-  if(opt.mixed && sellVal_ && values32)
-    ::feng::launch_k(k_sell_gather, grid_for(sellN_, 256, 4096), 256, 0, s_, sellN_, sellSrc_, values32, sellVal_);
+  refreshMatrix(values64, values32);
   if(opt.precond == 0) { factoredOk_ = true; return FE_OK; }
   if(opt.precond == 3 || opt.precond == 4) {
     FE_TRY(factor_mg(values64, values32));
@@ -1912,7 +1722,7 @@ int Krylov::spmvHot()
     set_error("no mixed-precision FGMRES");
     return FE_INVALID_ARG;
   }
-  if(sellVal_) spmv_sell(Z32_, w32_, nullptr);
+  if(bs_) bs_->mul32(Z32_, w32_, nullptr);
   else if(cur32_) spmv_launch<float, float, float, float, false>(lanes_, n_, A_, cur32_, Z32_, nullptr, w32_, nullptr, s_);
   return FE_OK;
 }
@@ -1985,25 +1795,29 @@ int Krylov::cycleGraph(bool mixed, const void *vals, const double *b, double *x,
   return st;
 }
 
-// r = b - A x for the FP32 matrix with FP64 x and accumulation: the sliced
+// r = b - A x for the FP32 matrix with FP64 x and accumulation: the block
 // copy when it is built (it holds the same values), else the CSR kernel.
 void Krylov::resid32(const float *vals, const double *x, const double *b, double *r)
 {
-  if(sellVal_ && xs2_ && dfResid_) {
+  if(bs_ && xs2_ && dfResid_) {
     ::feng::launch_k(k_split_x, grid_for(n_, 256, 4096), 256, 0, s_, n_, x, (float2 *)xs2_);
-    ::feng::launch_k(k_resid_sell_df<8>, grid_for(n_, 256, 1 << 20), 256, 0, s_, n_, sellPtr_, sellCol_, sellVal_,
-                     (const float2 *)xs2_, b, r);
-  } else if(sellVal_)
-    ::feng::launch_k(k_resid_sell<8>, grid_for(n_, 256, 1 << 20), 256, 0, s_, n_, sellPtr_, sellCol_, sellVal_, x, b,
-                     r);
+    bs_->resid32_df((const float2 *)xs2_, b, r);
+  } else if(bs_)
+    bs_->resid32(x, b, r);
   else
     spmv_launch<float, double, double, double, true>(lanes_, n_, A_, vals, x, b, r, nullptr, s_);
 }
 
-void Krylov::spmv_sell(const float *x, float *y, const int *done)
+void Krylov::mul64(const double *vals, const double *x, double *y, const int *done)
 {
-  ::feng::launch_k(k_spmv_sell<8>, grid_for(n_, 256, 1 << 20), 256, 0, s_, n_, sellPtr_, sellCol_, sellVal_, x, y,
-                   done);
+  if(bs_) bs_->mul64(x, y, done);
+  else spmv_launch<double, double, double, double, false>(lanes_, n_, A_, vals, x, nullptr, y, done, s_);
+}
+
+void Krylov::resid64(const double *vals, const double *x, const double *b, double *r)
+{
+  if(bs_) bs_->resid64(x, b, r);
+  else spmv_launch<double, double, double, double, true>(lanes_, n_, A_, vals, x, b, r, nullptr, s_);
 }
 
 __global__ void k_f32_to_f64(int64_t n, const float *__restrict__ x, double *__restrict__ y)
@@ -2193,33 +2007,32 @@ void Krylov::launch_cycle(bool mixed, const void *vals, const double *b, double 
     launch_cycle_mixed((const float *)vals, b, x, jmax, poll);
     return;
   }
-  spmv_launch<double, double, double, double, true>(lanes_, n_, A_, (const double *)vals, x, b, w_, nullptr, s_);
+  resid64((const double *)vals, x, b, w_);
   cudaMemsetAsync(&w.gs->done, 0, sizeof(int), s_);
   cudaMemcpyAsync(&w.gs->tol, htol_, sizeof(double), cudaMemcpyHostToDevice, s_);
   ::feng::launch_k(k_norm_to, nParts_, RB, 0, s_, n_, w_, red_, w.st, &w.gs->done);
   ::feng::launch_k(k_gmres_init, 1, 1, 0, s_, w.gs, w.st);
   ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_, w.st, &w.gs->beta, &w.gs->done);
   for(int j = 0; j < jmax; ++j) {
-    double *vj = V_ + (int64_t)j * n_;
+    double *vj = V_ + (int64_t)j * ld64_;
     {
-      double *zj = Z_ + (int64_t)j * n_;
+      double *zj = Z_ + (int64_t)j * ld64_;
       precond64(vj, zj, &w.gs->done);
-      spmv_launch<double, double, double, double, false>(lanes_, n_, A_, (const double *)vals, zj, nullptr,
-                                                         w_, &w.gs->done, s_);
+      mul64((const double *)vals, zj, w_, &w.gs->done);
     }
     double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
     for(int pass = 0; pass < 2; ++pass) {
-      ::feng::launch_k(k_mdot_partial, dim3(nParts_, j + 1), RB, 0, s_, n_, V_, j + 1, w_, red_, &w.gs->done);
+      ::feng::launch_k(k_mdot_partial, dim3(nParts_, j + 1), RB, 0, s_, n_, ld64_, V_, j + 1, w_, red_, &w.gs->done);
       ::feng::launch_k(k_mdot_final, j + 1, RB, 0, s_, nParts_, red_, w.gs->hcur, Hcol, pass, &w.gs->done);
-      ::feng::launch_k(k_mupdate, gv, 256, 0, s_, n_, V_, j + 1, w.gs->hcur, w_, &w.gs->done);
+      ::feng::launch_k(k_mupdate, gv, 256, 0, s_, n_, ld64_, V_, j + 1, w.gs->hcur, w_, &w.gs->done);
     }
     ::feng::launch_k(k_norm_to, nParts_, RB, 0, s_, n_, w_, red_, w.st, &w.gs->done);
-    ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_ + (int64_t)(j + 1) * n_, w.st, Hcol + j + 1, &w.gs->done);
+    ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_ + (int64_t)(j + 1) * ld64_, w.st, Hcol + j + 1, &w.gs->done);
     ::feng::launch_k(k_givens, 1, 32, 0, s_, w.gs, j);
     if(poll && poll_done(&w.gs->done, j)) break;
   }
   ::feng::launch_k(k_backsolve, 1, 256, backsolveSmem(opt.restart), s_, w.gs);
-  ::feng::launch_k(k_xupdate<double>, gv, 256, 0, s_, n_, n_, Z_, w.gs, x);
+  ::feng::launch_k(k_xupdate<double>, gv, 256, 0, s_, n_, ld64_, Z_, w.gs, x);
   cudaMemcpyAsync(h_gmres_, w.gs, sizeof(GmresHead), cudaMemcpyDeviceToHost, s_);
 }
 
@@ -2257,8 +2070,8 @@ void Krylov::mixed_part(const float *vals, const double *b, double *x, int j0, i
     float *zj = Z32_ + (int64_t)j * ld32_;
     precond32(vj, zj, &w.gs->done);
     double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
-    if(sellVal_)
-      spmv_sell(zj, w32_, &w.gs->done);
+    if(bs_)
+      bs_->mul32(zj, w32_, &w.gs->done);
     else
       spmv_launch<float, float, float, float, false>(lanes_, n_, A_, vals, zj, nullptr, w32_, &w.gs->done, s_);
     if(opt.gsPasses == 2) {
@@ -2454,7 +2267,7 @@ int Krylov::solve_fgmres64(const double *vals, const double *b, double *x, doubl
   // Converged on the Arnoldi estimate (as PETSc's default test); report the
   // true residual alongside.
   const bool conv = hd->est <= tolAbs;
-  spmv_launch<double, double, double, double, true>(lanes_, n_, A_, vals, x, b, w_, nullptr, s_);
+  resid64(vals, x, b, w_);
   st.rnorm = norm2(w_);
   return conv ? FE_OK : FE_NOT_CONVERGED;
 }
@@ -2508,8 +2321,7 @@ int Krylov::solve_cg64(const double *vals, const double *b, double *x, double to
   while(it < maxIt) {
     const int batch = std::min(8, maxIt - it);
     for(int k = 0; k < batch; ++k) {
-      spmv_launch<double, double, double, double, false>(lanes_, n_, A_, vals, p_, nullptr, q_,
-                                                         &w.cg->done, s_);
+      mul64(vals, p_, q_, &w.cg->done);
       ::feng::launch_k(k_dot_if, nParts_, RB, 0, s_, n_, p_, q_, red_, w.st, w.cg);
       ::feng::launch_k(k_cg_pq, 1, 1, 0, s_, w.cg, w.st);
       ::feng::launch_k(k_cg_xr, nParts_, RB, 0, s_, n_, w.cg, p_, q_, x, r_, red_, w.st);

@@ -100,6 +100,8 @@ struct KrylovStats {
   double rnorm0 = 0, rnorm = 0;
 };
 
+class BlockSell;
+
 class Krylov {
  public:
   ~Krylov();
@@ -108,11 +110,16 @@ class Krylov {
             const KrylovOptions &opt, cudaStream_t s, const PrecondInfo *pinfo = nullptr);
   // Factors the preconditioner from the current matrix values.
   int factor(const double *values64, const float *values32);
+  // Takes over changed matrix values (part of factor()).
+  void refreshMatrix(const double *values64, const float *values32);
   // Solves A x = b (x initial guess is zero).  Returns a Status.
   int solve(const double *values64, const float *values32, const double *b, double *x,
             KrylovStats &st);
   // y = A x (FP64 values, FP64 vectors) on this object's stream.
   void spmv64(const double *values, const double *x, double *y);
+  // The same on the copy that the solves use (values of the last factor();
+  // x 16-byte aligned).
+  void mul64(const double *vals, const double *x, double *y, const int *done);
   // The inner-loop FP32 product: x rounded to FP32, FP32 accumulation.
   void spmv32(const float *values, const double *x, double *y);
   // One preconditioner application z = M^-1 r (the FP32 path rounds r).
@@ -151,18 +158,15 @@ class Krylov {
                           // rows (column c of row block k at (k (m+1) + c) 1024)
   float *vc32_ = nullptr;  // the newest basis vector, contiguous (the preconditioner's input)
   void *xs2_ = nullptr;     // float2 split of the FP64 iterate (the mixed restart residual)
-  // The mixed restart residual in double-float (k_resid_sell_df) when the
+  // The mixed restart residual in double-float (BlockSell::resid32_df) when the
   // solve's tolerance is at least 1e-9 relative (its error, ~1e-13 of
   // sum |a x| per row, stays far below the stop), else in FP64.
   bool dfResid_ = false;
-  // Sliced-ELL copy of the FP32 matrix for the Arnoldi SpMV of the mixed
-  // path (slices of 32 rows padded to the longest row, entries column-major
-  // in the slice; padding: the row's own column, value 0), refreshed from the
-  // CSR values at each factor().
-  int32_t *sellPtr_ = nullptr, *sellCol_ = nullptr, *sellSrc_ = nullptr;  // sellSrc_: CSR position or -1
-  float *sellVal_ = nullptr;
-  int64_t sellN_ = 0;  // entries with padding
-  int build_sell();
+  // Block-column sliced-ELL copy of the matrix (FP32 or FP64, as it is
+  // solved), refreshed from the CSR values at each factor().
+  BlockSell *bs_ = nullptr;
+  int64_t ld64_ = 0;  // rows of V_ / Z_ (n rounded up to whole 256-byte lines)
+  void resid64(const double *vals, const double *x, const double *b, double *r);
   bool allDots_ = true;       // dot pass k_gs_dots_all (else k_gs_dots)
   int *zeroFlag_ = nullptr;  // a device 0 ("not done") for gsStep
   int gsParts_ = 0;       // blocks of the FP32 Gram-Schmidt update passes
@@ -233,10 +237,9 @@ class Krylov {
   // reads data evicted by the others), timed as a batch with CUDA events:
   // the average time of a pass as it runs inside the Arnoldi loop.
   int gsStepStream(int mode, int ncols, int reps, double *avgMs);
-  // The Arnoldi SpMV of the mixed path on the current FP32 matrix (sliced
-  // ELL when built, else CSR), FP32 vectors (benchmark phase).
+  // The Arnoldi SpMV of the mixed path on the current FP32 matrix (the block
+  // copy when built, else CSR), FP32 vectors (benchmark phase).
   int spmvHot();
-  void spmv_sell(const float *x, float *y, const int *done);
   void resid32(const float *vals, const double *x, const double *b, double *r);
   // The preconditioner application of an Arnoldi step (the mixed path: the
   // FP32 basis column 0 into Z column 0; FP64 otherwise), reps of them

@@ -1082,6 +1082,7 @@ int SystemCUDA::ensureMatrixZeroed() const
   if(vals64_) CK(cudaMemsetAsync(vals64_, 0, sizeof(double) * pat_.nnz(), s_));
   if(vals32_) CK(cudaMemsetAsync(vals32_, 0, sizeof(float) * pat_.nnz(), s_));
   zeroPending_ = false;
+  zeroedOut_ = true;
   return FE_OK;
 }
 
@@ -1385,6 +1386,7 @@ int SystemCUDA::factorIfPending()
   int s = kry_.factor(vals64_, vals32_);
   times.factor_ms += end_phase();
   if(s == FE_OK) factorPending_ = false;
+  zeroedOut_ = false;
   return s;
 }
 
@@ -1538,6 +1540,8 @@ int SystemCUDA::solve(double *normDx, double *normRHS, double *normAxb, int *nIt
 {
   FE_TRY(ensureMatrixZeroed());
   FE_TRY(factorIfPending());
+  if(zeroedOut_) kry_.refreshMatrix(vals64_, vals32_);  // zeroed and not assembled again
+  zeroedOut_ = false;
   begin_phase();
   KrylovStats st;
   int s = kry_.solve(vals64_, vals32_, rhs_, du_, st);
@@ -1691,7 +1695,7 @@ int SystemCUDA::benchPhase(int which, int reps, size_t flushBytes, double *avgMs
       case 2:
         // the Krylov loop's SpMV: FP64 (plain), or the mixed Arnoldi SpMV
         // on FP32 vectors
-        if(vals64_) kry_.spmv64(vals64_, x, y);
+        if(vals64_) kry_.mul64(vals64_, x, y, nullptr);
         else status = kry_.spmvHot();
         break;
       case 3:

@@ -177,6 +177,7 @@ class SystemCUDA {
   // values instead of adding to them; any other use of the values zeroes
   // them first.
   mutable bool zeroPending_ = false;
+  mutable bool zeroedOut_ = false;   // the values were zeroed after the last factor()
   int ensureMatrixZeroed() const;
   // The mixed path assembles the Taylor-Hood residual in double-float on
   // the FP32 pipes (FP64-class accuracy, the 7-node rule); otherwise FP64.
