@@ -81,6 +81,7 @@ struct RedState {
   unsigned int counter;
   float finv;   // 1 / ||w|| of the last FP32 Gram-Schmidt norm pass
   int reorth;   // the last Gram-Schmidt pass asks for a second one
+  unsigned int slices[MAXM / 8];  // blocks done of each column slice (k_gs64)
   double result[4];
 };
 
@@ -172,59 +173,6 @@ __global__ void k_absmax(int64_t n, const double *__restrict__ x, double *partia
   finish_reduction<1, true>(v, partials, st, out);
 }
 
-// h[c] (+)= V_c . w for c < ncols; grid (parts, ncols).  Partials per column.
-__global__ void k_mdot_partial(int64_t n, int64_t ld, const double *__restrict__ V, int ncols,
-                               const double *__restrict__ w, double *partials,
-                               const int *__restrict__ done)
-{
-  FE_PDL_ENTRY();
-  if(*done) return;
-  __shared__ double sh[RB / 32];
-  const int c = blockIdx.y;
-  const double *vc = V + (int64_t)c * ld;
-  double v = 0.;
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (int64_t)gridDim.x * blockDim.x)
-    v += vc[i] * w[i];
-  v = block_sum(v, sh);
-  if(threadIdx.x == 0) partials[(int64_t)c * MAXRED + blockIdx.x] = v;
-}
-
-// Sums the partials of each column c (block c) into hcol[c] (and H column).
-__global__ void k_mdot_final(int nparts, double *partials, double *hcur, double *Hcol, int accum,
-                             const int *__restrict__ done)
-{
-  FE_PDL_ENTRY();
-  if(*done) return;
-  __shared__ double sh[RB / 32];
-  const int c = blockIdx.x;
-  double s = 0.;
-  for(int i = threadIdx.x; i < nparts; i += blockDim.x) s += partials[(int64_t)c * MAXRED + i];
-  s = block_sum(s, sh);
-  if(threadIdx.x == 0) {
-    hcur[c] = s;
-    Hcol[c] = accum ? Hcol[c] + s : s;
-  }
-}
-
-// w -= sum_c h[c] V_c
-__global__ void k_mupdate(int64_t n, int64_t ld, const double *__restrict__ V, int ncols,
-                          const double *__restrict__ h, double *__restrict__ w,
-                          const int *__restrict__ done)
-{
-  FE_PDL_ENTRY();
-  if(*done) return;
-  __shared__ double sh[MAXM + 1];
-  for(int c = threadIdx.x; c < ncols; c += blockDim.x) sh[c] = h[c];
-  __syncthreads();
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (int64_t)gridDim.x * blockDim.x) {
-    double acc = w[i];
-    for(int c = 0; c < ncols; ++c) acc -= sh[c] * V[(int64_t)c * ld + i];
-    w[i] = acc;
-  }
-}
-
 // Sum of squares of w into st->result[0] (k_scale_from takes the root).
 __global__ void k_norm_to(int64_t n, const double *__restrict__ w, double *partials, RedState *st,
                           const int *__restrict__ done)
@@ -285,7 +233,7 @@ struct GmresHead {
 struct GmresState : GmresHead {
   double H[MAXM * (MAXM + 1)];
   double cs[MAXM], sn[MAXM], g[MAXM + 1], y[MAXM];
-  double hcur[MAXM + 1];
+  double hcur[MAXM + 1], hcur2[MAXM + 1];
 };
 
 // One warp: the column and the previous rotations are staged in shared
@@ -1001,6 +949,212 @@ __global__ void k_scale32(int64_t n4, const float *__restrict__ w, float *__rest
     V4[vidx4(g, col, m1)] = t;
     c4[g] = t;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Classical Gram-Schmidt on the FP64 basis (plain path), applied twice, in
+// passes over the columns c < ncols (column-major, leading dimension ld):
+// DOT h = V^T w; UPD_DOT wo = w - V hprev, then h = V^T wo with the columns of
+// a row chunk read again from the L2; UPD only the update; UPD_NORM wo =
+// w - V hprev, then ||wo||^2.  Large systems take DOT, UPD_DOT, UPD_NORM (one
+// pass over the basis less), small ones DOT, UPD, DOT, UPD_NORM.
+// Bound: the FP64 pipe (two lanes per cycle and SM: one product per basis
+// entry and pass, 24 us for 25 columns of 588 k rows) and the bytes about
+// equally.  So every addition beside the products counts: a thread holds R
+// rows per chunk (R products per column before any lane sum), and B columns
+// are summed over the lanes by a reduce-scatter (B - 1 + 5 - log2 B additions
+// per warp instead of 5 B).  Small systems are bound by the chain of loads,
+// lane sums and last block instead, the latter again FP64 additions of one SM:
+// their dots split the columns over grid y, each slice with its own last
+// block, and the next B columns are loaded ahead.
+// Partials are summed in a fixed order (deterministic).
+// ---------------------------------------------------------------------------
+enum GsMode { GS_DOT = 0, GS_UPD_DOT = 1, GS_UPD_NORM = 2, GS_UPD = 3 };
+
+// Sums v[0..B) over the lanes of a warp; lane l returns the total of v[l % B].
+template <int B>
+__device__ __forceinline__ double lane_sum_n(double (&v)[B], int lane)
+{
+#pragma unroll
+  for(int h = B / 2; h > 0; h >>= 1) {
+    const bool hi = lane & h;
+#pragma unroll
+    for(int i = 0; i < h; ++i) {
+      const double keep = hi ? v[i + h] : v[i];
+      const double send = hi ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
+#pragma unroll
+  for(int o = B; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// hcur: the coefficients of this pass; Hcol: the Hessenberg column (second:
+// adds to it); UPD_NORM: Hcol is the subdiagonal entry.  wo may be w.  Grid y
+// (DOT only): slices of `slice` columns.
+template <int MODE, int TB, int R, int B>
+__global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
+    int64_t n, int64_t ld, const double *__restrict__ V, int ncols, int slice, const double *hprev,
+    const double *w, double *wo, double *partials, RedState *st, double *hcur, double *Hcol,
+    const int *__restrict__ done, int second)
+{
+  FE_PDL_ENTRY();
+  if(*done) return;
+  constexpr int NW = TB / 32;
+  constexpr bool AHEAD = R * B <= 16;
+  __shared__ double hs[MAXM];
+  __shared__ double red[NW][MAXM];  // per warp and column (UPD_NORM: column 0)
+  __shared__ bool last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cb = MODE == GS_DOT ? (int)blockIdx.y * slice : 0;
+  const int ce = MODE == GS_UPD_NORM ? 1 : MODE == GS_DOT ? min(ncols, cb + slice) : ncols;
+  for(int c = tid; MODE != GS_DOT && c < ncols; c += TB) hs[c] = hprev[c];
+  for(int c = cb + lane; c < ce; c += 32) red[warp][c] = 0.;
+  __syncthreads();
+  double q = 0.;
+  for(int64_t r0 = (int64_t)blockIdx.x * (TB * R); r0 < n; r0 += (int64_t)gridDim.x * (TB * R)) {
+    double x[R], v[B][R], nx[AHEAD ? B : 1][R];
+    // columns c0 .. c0 + B - 1 (below `end`) of this thread's rows
+    auto load = [&](int c0, int end, double (*d)[R]) {
+#pragma unroll
+      for(int u = 0; u < B; ++u)
+#pragma unroll
+        for(int k = 0; k < R; ++k) {
+          const int64_t i = r0 + k * TB + tid;
+          d[u][k] = c0 + u < end && i < n ? V[(int64_t)(c0 + u) * ld + i] : 0.;
+        }
+    };
+    // f(c0) for every batch of columns of [c0, end), the next batch's loads
+    // issued first when there is room for them
+    auto batches = [&](int begin, int end, auto &&f) {
+      if constexpr(AHEAD) load(begin, end, v);
+      for(int c0 = begin; c0 < end; c0 += B) {
+        if constexpr(AHEAD) load(c0 + B, end, nx);
+        else load(c0, end, v);
+        f(c0);
+        if constexpr(AHEAD)
+#pragma unroll
+          for(int u = 0; u < B; ++u)
+#pragma unroll
+            for(int k = 0; k < R; ++k) v[u][k] = nx[u][k];
+      }
+    };
+#pragma unroll
+    for(int k = 0; k < R; ++k) {
+      const int64_t i = r0 + k * TB + tid;
+      x[k] = i < n ? w[i] : 0.;
+    }
+    if constexpr(MODE != GS_DOT) {
+      batches(0, ncols, [&](int c0) {
+#pragma unroll
+        for(int u = 0; u < B; ++u) {
+          const double h = c0 + u < ncols ? hs[c0 + u] : 0.;
+#pragma unroll
+          for(int k = 0; k < R; ++k) x[k] -= h * v[u][k];
+        }
+      });
+#pragma unroll
+      for(int k = 0; k < R; ++k) {
+        const int64_t i = r0 + k * TB + tid;
+        if(i < n) wo[i] = x[k];
+      }
+    }
+    if constexpr(MODE == GS_UPD_NORM) {
+#pragma unroll
+      for(int k = 0; k < R; ++k) q += x[k] * x[k];
+    } else if constexpr(MODE != GS_UPD) {
+      batches(cb, ce, [&](int c0) {
+        double t[B];
+#pragma unroll
+        for(int u = 0; u < B; ++u) {
+          t[u] = v[u][0] * x[0];
+#pragma unroll
+          for(int k = 1; k < R; ++k) t[u] += v[u][k] * x[k];
+        }
+        const double sum = lane_sum_n<B>(t, lane);
+        if(lane < B && c0 + lane < ce) red[warp][c0 + lane] += sum;
+      });
+    }
+  }
+  if constexpr(MODE == GS_UPD) return;
+  if constexpr(MODE == GS_UPD_NORM) {
+    for(int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if(lane == 0) red[warp][0] = q;
+  }
+  __syncthreads();
+  for(int c = cb + tid; c < ce; c += TB) {
+    double sum = 0.;
+#pragma unroll
+    for(int k = 0; k < NW; ++k) sum += red[k][c];
+    partials[(int64_t)c * MAXRED + blockIdx.x] = sum;
+    // only the threads that wrote partials order them before the counter
+    __threadfence();
+  }
+  __syncthreads();
+  unsigned int *counter = &st->slices[blockIdx.y];
+  if(tid == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if(!last) return;
+  __threadfence();
+  const int nb = (int)gridDim.x, sub = lane & 7;
+  if constexpr(MODE == GS_UPD_NORM) {
+    // one sum: every thread of the block, then lanes and warps in order
+    double sum = 0.;
+    for(int b = tid; b < nb; b += TB) sum += __ldcg(partials + b);
+    for(int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if(lane == 0) red[warp][0] = sum;
+    __syncthreads();
+    if(tid == 0) {
+      sum = red[0][0];
+      for(int k = 1; k < NW; ++k) sum += red[k][0];
+      st->result[0] = sum;
+      *Hcol = sqrt(sum);
+      *counter = 0;
+    }
+    return;
+  }
+  // eight lanes per column, four columns per warp
+  for(int c0 = cb + warp * 4; c0 < ce; c0 += NW * 4) {
+    const int c = c0 + (lane >> 3);
+    double sum = 0.;
+    if(c < ce) {
+      const double *pc = partials + (int64_t)c * MAXRED;
+      for(int b0 = sub; b0 < nb; b0 += 64) {
+        double p[8];
+#pragma unroll
+        for(int k = 0; k < 8; ++k) p[k] = __ldcg(pc + (b0 + 8 * k < nb ? b0 + 8 * k : 0));
+#pragma unroll
+        for(int k = 0; k < 8; ++k)
+          if(b0 + 8 * k < nb) sum += p[k];
+      }
+    }
+#pragma unroll
+    for(int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if(c < ce && sub == 0) {
+      hcur[c] = sum;
+      Hcol[c] = second ? Hcol[c] + sum : sum;
+    }
+  }
+  if(tid == 0) *counter = 0;
+}
+
+// v = w / ||w|| (||w||^2 in st->result[0]); the last block applies the Givens
+// rotations of step j meanwhile.
+__global__ void k_scale64(int64_t n, const double *__restrict__ w, double *__restrict__ v, const RedState *st,
+                          const int *__restrict__ done, GmresState *gs, int j)
+{
+  FE_PDL_ENTRY();
+  __shared__ double sh[MAXM + 1], scs[MAXM], ssn[MAXM];
+  if(*done) return;
+  if(blockIdx.x == gridDim.x - 1) {
+    if(threadIdx.x < 32) givens_warp(gs, j, threadIdx.x, sh, scs, ssn);
+    return;
+  }
+  const double nrm = sqrt(st->result[0]);
+  const double inv = nrm > 0 ? 1.0 / nrm : 0.0;
+  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)(gridDim.x - 1) * blockDim.x)
+    v[i] = w[i] * inv;
 }
 
 // V_0 = r / ||r|| rounded to FP32 (start of a mixed cycle; column 0 of the
@@ -1999,38 +2153,79 @@ void Krylov::gs32(int mode, int ncols, const double *hprev, double *hcur, double
 // classical Gram-Schmidt applied twice, Givens rotations on the device.
 // Every kernel after convergence is skipped through the device done flag,
 // so the same launch sequence can be replayed from a CUDA graph.
+// One pass of the FP64 Gram-Schmidt (k_gs64) on w_.
+void Krylov::gs64(int mode, int ncols, const double *hprev, double *hcur, double *Hcol, const int *done, int second)
+{
+  Ws w = Ws_INIT(this);
+  auto go = [&](auto kernel, int tb, int rows, int perSM) {
+    const int gx = grid_for(n_, tb * rows, std::min(perSM * nSM_, MAXRED));
+    int slice = ncols;
+    if(mode == GS_DOT) {
+      // column slices (multiples of 8) while the row chunks leave room
+      const int gy = std::max(1, std::min((ncols + 7) / 8, perSM * nSM_ / gx));
+      slice = ((ncols + gy - 1) / gy + 7) / 8 * 8;
+    }
+    ::feng::launch_k(kernel, dim3(gx, (ncols + slice - 1) / slice), tb, 0, s_, n_, ld64_, V_, ncols, slice, hprev, w_,
+                     w_, red_, w.st, hcur, Hcol, done, second);
+  };
+  // Kovasznay, ms per FP64 Newton solve: 256^2 (588 k rows) 511 with a dot
+  // kernel per column, an update and a norm kernel, each twice; 381 with the
+  // big passes.  290 k rows 262 with the small passes, 269 with the big ones;
+  // 84 k rows 147 -> 129, 36 k 92 -> 84, 9 k 58.5 -> 56.  Updates with 64
+  // threads per block instead of 256 at 3.5 k rows 49.6 against 51.9, at 9 k
+  // 56.9 against 56.1.
+  if(bigGs64()) {
+    if(mode == GS_DOT) go(k_gs64<GS_DOT, 256, 8, 4>, 256, 8, 2);
+    else if(mode == GS_UPD_DOT) go(k_gs64<GS_UPD_DOT, 256, 8, 4>, 256, 8, 2);
+    else go(k_gs64<GS_UPD_NORM, 256, 8, 4>, 256, 8, 2);
+  } else if(mode == GS_DOT) {
+    go(k_gs64<GS_DOT, 256, 2, 8>, 256, 2, 2);
+  } else if(n_ >= 8000) {
+    if(mode == GS_UPD) go(k_gs64<GS_UPD, 256, 1, 16>, 256, 1, 4);
+    else go(k_gs64<GS_UPD_NORM, 256, 1, 16>, 256, 1, 4);
+  } else {
+    if(mode == GS_UPD) go(k_gs64<GS_UPD, 64, 1, 16>, 64, 1, 4);
+    else go(k_gs64<GS_UPD_NORM, 64, 1, 16>, 64, 1, 4);
+  }
+}
+
 void Krylov::launch_cycle(bool mixed, const void *vals, const double *b, double *x, int jmax, bool poll)
+{
+  if(mixed) launch_cycle_mixed((const float *)vals, b, x, jmax, poll);
+  else fp64_part((const double *)vals, b, x, 0, jmax, poll, true, true);
+}
+
+// Part of an FP64 restart cycle (see mixed_part): classical Gram-Schmidt
+// applied twice (k_gs64), the rotations beside the scale pass.
+void Krylov::fp64_part(const double *vals, const double *b, double *x, int j0, int j1, bool poll, bool pro, bool epi)
 {
   Ws w = Ws_INIT(this);
   const int gv = grid_for(n_, 256, 2048);
-  if(mixed) {
-    launch_cycle_mixed((const float *)vals, b, x, jmax, poll);
-    return;
-  }
-  resid64((const double *)vals, x, b, w_);
-  cudaMemsetAsync(&w.gs->done, 0, sizeof(int), s_);
-  cudaMemcpyAsync(&w.gs->tol, htol_, sizeof(double), cudaMemcpyHostToDevice, s_);
-  ::feng::launch_k(k_norm_to, nParts_, RB, 0, s_, n_, w_, red_, w.st, &w.gs->done);
-  ::feng::launch_k(k_gmres_init, 1, 1, 0, s_, w.gs, w.st);
-  ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_, w.st, &w.gs->beta, &w.gs->done);
-  for(int j = 0; j < jmax; ++j) {
-    double *vj = V_ + (int64_t)j * ld64_;
-    {
-      double *zj = Z_ + (int64_t)j * ld64_;
-      precond64(vj, zj, &w.gs->done);
-      mul64((const double *)vals, zj, w_, &w.gs->done);
-    }
-    double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
-    for(int pass = 0; pass < 2; ++pass) {
-      ::feng::launch_k(k_mdot_partial, dim3(nParts_, j + 1), RB, 0, s_, n_, ld64_, V_, j + 1, w_, red_, &w.gs->done);
-      ::feng::launch_k(k_mdot_final, j + 1, RB, 0, s_, nParts_, red_, w.gs->hcur, Hcol, pass, &w.gs->done);
-      ::feng::launch_k(k_mupdate, gv, 256, 0, s_, n_, ld64_, V_, j + 1, w.gs->hcur, w_, &w.gs->done);
-    }
+  if(pro) {
+    resid64(vals, x, b, w_);
+    cudaMemsetAsync(&w.gs->done, 0, sizeof(int), s_);
+    cudaMemcpyAsync(&w.gs->tol, htol_, sizeof(double), cudaMemcpyHostToDevice, s_);
     ::feng::launch_k(k_norm_to, nParts_, RB, 0, s_, n_, w_, red_, w.st, &w.gs->done);
-    ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_ + (int64_t)(j + 1) * ld64_, w.st, Hcol + j + 1, &w.gs->done);
-    ::feng::launch_k(k_givens, 1, 32, 0, s_, w.gs, j);
+    ::feng::launch_k(k_gmres_init, 1, 1, 0, s_, w.gs, w.st);
+    ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_, w.st, &w.gs->beta, &w.gs->done);
+  }
+  for(int j = j0; j < j1; ++j) {
+    double *vj = V_ + (int64_t)j * ld64_, *zj = Z_ + (int64_t)j * ld64_;
+    precond64(vj, zj, &w.gs->done);
+    mul64(vals, zj, w_, &w.gs->done);
+    double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
+    gs64(GS_DOT, j + 1, nullptr, w.gs->hcur, Hcol, &w.gs->done, 0);
+    if(bigGs64()) {
+      gs64(GS_UPD_DOT, j + 1, w.gs->hcur, w.gs->hcur2, Hcol, &w.gs->done, 1);
+    } else {
+      gs64(GS_UPD, j + 1, w.gs->hcur, nullptr, nullptr, &w.gs->done, 1);
+      gs64(GS_DOT, j + 1, nullptr, w.gs->hcur2, Hcol, &w.gs->done, 1);
+    }
+    gs64(GS_UPD_NORM, j + 1, w.gs->hcur2, nullptr, Hcol + j + 1, &w.gs->done, 1);
+    ::feng::launch_k(k_scale64, gv + 1, 256, 0, s_, n_, w_, vj + ld64_, w.st, &w.gs->done, w.gs, j);
     if(poll && poll_done(&w.gs->done, j)) break;
   }
+  if(!epi) return;
   ::feng::launch_k(k_backsolve, 1, 256, backsolveSmem(opt.restart), s_, w.gs);
   ::feng::launch_k(k_xupdate<double>, gv, 256, 0, s_, n_, ld64_, Z_, w.gs, x);
   cudaMemcpyAsync(h_gmres_, w.gs, sizeof(GmresHead), cudaMemcpyDeviceToHost, s_);
@@ -2117,10 +2312,10 @@ void Krylov::mixed_part(const float *vals, const double *b, double *x, int j0, i
 
 // Runs one full restart cycle, from a CUDA graph when the cycle has its full
 // length (the graph is captured once per operand set and replayed).
-// A graph per part of the mixed cycle (part c: steps [cK, cK + K), the
+// A graph per part of a cycle (part c: steps [cK, cK + K), the
 // prologue with part 0, then a copy of the done flag to pinned memory;
 // part P: the epilogue), looked up or captured.
-int Krylov::part_graph(const GraphKey &key, int part, int P, int K, const float *vals, const double *b, double *x,
+int Krylov::part_graph(const GraphKey &key, int part, int P, int K, const void *vals, const double *b, double *x,
                        cudaGraphExec_t *out, size_t *nKernels)
 {
   for(size_t i = 0; i < graphs_.size(); ++i) {
@@ -2137,10 +2332,14 @@ int Krylov::part_graph(const GraphKey &key, int part, int P, int K, const float 
   cudaGraphExec_t exec = nullptr;
   CK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
   ++g_capturing;
+  auto steps = [&](int j0, int j1, bool pro, bool epi) {
+    if(key.mixed) mixed_part((const float *)vals, b, x, j0, j1, false, pro, epi);
+    else fp64_part((const double *)vals, b, x, j0, j1, false, pro, epi);
+  };
   if(part == P) {
-    mixed_part(vals, b, x, 0, 0, false, false, true);
+    steps(0, 0, false, true);
   } else {
-    mixed_part(vals, b, x, part * K, std::min(m, part * K + K), false, part == 0, false);
+    steps(part * K, std::min(m, part * K + K), part == 0, false);
     Ws w = Ws_INIT(this);
     cudaMemcpyAsync(hdone_ + part, &w.gs->done, sizeof(int), cudaMemcpyDeviceToHost, s_);
   }
@@ -2166,14 +2365,14 @@ int Krylov::part_graph(const GraphKey &key, int part, int P, int K, const float 
   return FE_OK;
 }
 
-// One full mixed restart cycle from part graphs of chunk_ Arnoldi steps:
+// One full restart cycle from part graphs of chunk_ Arnoldi steps:
 // part c + 1 is queued before the done flag of part c is read, so the GPU
 // always has work and a converged cycle stops within one part (instead of
 // replaying every remaining step's kernels, which return at once).
-int Krylov::run_cycle_chunked(const float *vals, const double *b, double *x)
+int Krylov::run_cycle_chunked(bool mixed, const void *vals, const double *b, double *x)
 {
   const int m = opt.restart, K = chunk_, P = (m + K - 1) / K;
-  GraphKey key{true, vals, b, x, dfResid_, -1};
+  GraphKey key{mixed, vals, b, x, mixed && dfResid_, -1};
   if(evs_.size() < (size_t)P) {
     for(size_t i = evs_.size(); i < (size_t)P; ++i) {
       cudaEvent_t e;
@@ -2205,7 +2404,7 @@ int Krylov::run_cycle_chunked(const float *vals, const double *b, double *x)
 int Krylov::run_cycle(bool mixed, const void *vals, const double *b, double *x, int jmax)
 {
   const int m = opt.restart;
-  if(useGraphs_ && jmax == m && mixed && chunk_ > 0 && chunk_ < m) return run_cycle_chunked((const float *)vals, b, x);
+  if(useGraphs_ && jmax == m && chunk_ > 0 && chunk_ < m) return run_cycle_chunked(mixed, vals, b, x);
   if(useGraphs_ && jmax == m) {
     GraphKey key{mixed, vals, b, x, mixed && dfResid_, -1};
     cudaGraphExec_t exec = nullptr;
