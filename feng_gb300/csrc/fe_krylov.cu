@@ -9,6 +9,7 @@
 #include "fe_bsell.h"
 #include "fe_common.h"
 #include "fe_df.h"
+#include "fe_ilu_stream.h"
 #include "fe_launch.h"
 #include "fe_krylov.h"
 
@@ -1465,6 +1466,7 @@ Krylov::~Krylov()
   cudaFree(V_); cudaFree(Z_); cudaFree(Z32_); cudaFree(V32_); cudaFree(vc32_); cudaFree(xs2_); cudaFree(v32_); cudaFree(w32_);
   cudaFree(zeroFlag_);
   delete bs_;
+  delete ilus_;
   cudaFree(w_); cudaFree(r_); cudaFree(t_); cudaFree(p_); cudaFree(q_);
   cudaFree(diag_); cudaFree(diag32_); cudaFree(red_); cudaFree(dsum_);
   cudaFreeHost(hred_);
@@ -1656,6 +1658,14 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
     CK(cudaMemcpy(ilu_.ldiag, ldiag.data(), sizeof(int32_t) * n_, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ilu_.srcPos, src.data(), sizeof(int32_t) * ilu_.lnnz, cudaMemcpyHostToDevice));
     FE_TRY(build_ilu_levels(lia, lja, ldiag));
+    // diagonal blocks whose vector fits in shared memory (about 20 k rows in FP64)
+    // are solved there; the level kernels stay for larger ones
+    ilus_ = new IluStream();
+    FE_TRY(ilus_->build(lia, lja, ldiag, perm, bstart, opt.mixed != 0, s_));
+    if(!ilus_->usable()) {
+      delete ilus_;
+      ilus_ = nullptr;
+    }
   }
   return FE_OK;
 }
@@ -1803,6 +1813,7 @@ int Krylov::factor(const double *values64, const float *values32)
   } else {
     if(opt.mixed) ilu_factor_levels<float>(nullptr, values32);
     else ilu_factor_levels<double>(values64, nullptr);
+    if(ilus_) ilus_->gather(ilu_.vals);
   }
   CK(cudaGetLastError());
   int hs = 0;
@@ -1825,7 +1836,8 @@ void Krylov::precond64(const double *r, double *z, const int *done)
   } else if(opt.precond == 2) {
     ::feng::launch_k(k_jacobi<double, double>, grid_for(n_, 256, 4096), 256, 0, s_, n_, diag_, r, z, done);
   } else {
-    ilu_solve_levels<double, double>(r, z, done);
+    if(ilus_) ilus_->solve(r, z, done);
+    else ilu_solve_levels<double, double>(r, z, done);
   }
 }
 
@@ -1838,7 +1850,8 @@ void Krylov::precond32(const float *r, float *z, const int *done)
   } else if(opt.precond == 2) {
     ::feng::launch_k(k_jacobi<float, float>, grid_for(n_, 256, 4096), 256, 0, s_, n_, diag32_, r, z, done);
   } else {
-    ilu_solve_levels<float, float>(r, z, done);
+    if(ilus_) ilus_->solve(r, z, done);
+    else ilu_solve_levels<float, float>(r, z, done);
   }
 }
 

@@ -101,6 +101,7 @@ struct KrylovStats {
 };
 
 class BlockSell;
+class IluStream;
 
 class Krylov {
  public:
@@ -165,6 +166,7 @@ class Krylov {
   // Block-column sliced-ELL copy of the matrix (FP32 or FP64, as it is
   // solved), refreshed from the CSR values at each factor().
   BlockSell *bs_ = nullptr;
+  IluStream *ilus_ = nullptr;  // triangular solves with the vector in shared memory, when the blocks fit
   int64_t ld64_ = 0;  // rows of V_ / Z_ (n rounded up to whole 256-byte lines)
   void resid64(const double *vals, const double *x, const double *b, double *r);
   bool allDots_ = true;       // dot pass k_gs_dots_all (else k_gs_dots)

@@ -58,3 +58,54 @@ def test_ilu0_block_jacobi_matches_serial():
     z = sys_.applyPreconditioner(r)
     zo = _oracle_ilu(g, sys_.getMatrix(), r, num.setup(64).blocks())
     assert np.max(np.abs(z - zo)) <= 1e-12 * np.max(np.abs(zo))
+
+
+def _ilu_reference(A, r, blocks):
+    """(LU)^-1 r of the ILU(0) of A restricted to the diagonal blocks (Saad,
+    Alg. 10.4), row by row in FP64."""
+    n = len(r)
+    rows = []
+    for i in range(n):
+        c, v = A.indices[A.indptr[i]:A.indptr[i + 1]], A.data[A.indptr[i]:A.indptr[i + 1]]
+        keep = blocks[c] == blocks[i]
+        rows.append(dict(zip(c[keep].tolist(), v[keep].tolist())))
+    for i in range(n):
+        for k in sorted(c for c in rows[i] if c < i):
+            rows[i][k] /= rows[k][k]
+            for j, u in rows[k].items():
+                if j > k and j in rows[i]:
+                    rows[i][j] -= rows[i][k] * u
+    z = r.copy()
+    for i in range(n):
+        z[i] -= sum(v * z[c] for c, v in rows[i].items() if c < i)
+    for i in range(n - 1, -1, -1):
+        z[i] = (z[i] - sum(v * z[c] for c, v in rows[i].items() if c > i)) / rows[i][i]
+    return z
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,rows", [(1, 0), (6, 0), (9, 1), (9, 40), (14, 0), (40, 256)])
+def test_ilu0_solves_match_serial_over_block_shapes(n, rows, precision):
+    """One block and many (the smallest partition up to 256 rows), levels of
+    one row and of more rows than a step, rows longer than a step's entries (the flow's
+    vertex rows): the solves with the vector in shared memory.  The flow's
+    pressure rows have no diagonal entry of their own: their pivots come from
+    the elimination.  Tolerances:
+    rounding times the growth of that elimination, taken as 1e4 for the
+    mass-dominated velocity block (1e-11 and 1e-2 of max |z|)."""
+    import scipy.sparse as sp
+    mesh = fe.Mesh2DP1.generate_square(n, jitter=0.1, seed=2)
+    num, forms = problem_spaces("ns_cavity_bdf2" if n < 40 else "diffusion", mesh, 40.0)
+    sys_ = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(
+        krylov="fgmres", precond="ilu0" if rows == 0 else "bjacobi-ilu0", pc_block_rows=max(rows, 1),
+        precision=precision))
+    sys_.setSolution(np.random.default_rng(1).uniform(-1, 1, sys_.nDofs))
+    sys_.setTime(0.0, 500.0)
+    sys_.setToZero()
+    sys_.assembleMatrices()
+    ia, ja = sys_.pattern()
+    A = sp.csr_matrix((sys_.getMatrix(), ja, ia))
+    blocks = np.zeros(sys_.nInc, int) if rows == 0 else num.setup(rows).blocks()
+    r = np.random.default_rng(4).uniform(-1, 1, sys_.nInc)
+    z, ref = sys_.applyPreconditioner(r), _ilu_reference(A, r, blocks)
+    assert np.max(np.abs(z - ref)) <= (1e-11 if precision == "fp64" else 1e-2) * np.max(np.abs(ref))
