@@ -114,10 +114,18 @@ __device__ double block_max(double v, double *sh)
   return v;
 }
 
-// Finishes a reduction of K values: writes partials, last block sums them.
-template <int K, bool MAX>
+struct NoTail {
+  __device__ void operator()(double) const {}
+};
+
+// Finishes a reduction of K values: writes partials, the last block sums
+// them; its thread 0 then calls tail(first sum).  (Scalars that the next
+// kernel needs are formed there, once: an FP64 division or root in every
+// thread of a vector kernel costs more on the FP64 pipe than the vector work:
+// 408 k threads, two divisions: 8 us.)
+template <int K, bool MAX, typename Tail = NoTail>
 __device__ void finish_reduction(const double (&v)[K], double *partials, RedState *st,
-                                 double *out)
+                                 double *out, Tail tail = Tail())
 {
   __shared__ double sh[RB / 32];
   __shared__ bool last;
@@ -147,6 +155,7 @@ __device__ void finish_reduction(const double (&v)[K], double *partials, RedStat
     if(threadIdx.x == 0) {
       st->result[k] = s;
       if(out) out[k] = s;
+      if(k == 0) tail(s);
     }
   }
   if(threadIdx.x == 0) st->counter = 0;
@@ -174,7 +183,7 @@ __global__ void k_absmax(int64_t n, const double *__restrict__ x, double *partia
   finish_reduction<1, true>(v, partials, st, out);
 }
 
-// Sum of squares of w into st->result[0] (k_scale_from takes the root).
+// ||w||^2 into st->result[0], 1 / ||w|| (0 for a zero w) into st->result[1].
 __global__ void k_norm_to(int64_t n, const double *__restrict__ w, double *partials, RedState *st,
                           const int *__restrict__ done)
 {
@@ -184,18 +193,18 @@ __global__ void k_norm_to(int64_t n, const double *__restrict__ w, double *parti
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x)
     v[0] += w[i] * w[i];
-  finish_reduction<1, false>(v, partials, st, nullptr);
+  finish_reduction<1, false>(v, partials, st, nullptr,
+                             [&](double ss) { st->result[1] = ss > 0 ? 1.0 / sqrt(ss) : 0.0; });
 }
 
-// v = w / sqrt(ss), and H[j+1][j] = sqrt(ss).  ss read from st->result[0].
+// v = w / ||w|| (st->result as k_norm_to leaves it), *Hsub = ||w||.
 __global__ void k_scale_from(int64_t n, const double *__restrict__ w, double *__restrict__ v,
                              const RedState *st, double *Hsub, const int *__restrict__ done)
 {
   FE_PDL_ENTRY();
   if(*done) return;
-  const double nrm = sqrt(st->result[0]);
-  if(blockIdx.x == 0 && threadIdx.x == 0) *Hsub = nrm;
-  const double inv = nrm > 0 ? 1.0 / nrm : 0.0;
+  if(blockIdx.x == 0 && threadIdx.x == 0) *Hsub = sqrt(st->result[0]);
+  const double inv = st->result[1];
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x)
     v[i] = w[i] * inv;
@@ -305,9 +314,20 @@ __device__ void givens_warp(GmresState *gs, int j, int lane, double *sh, double 
   for(int i = lane; i < j; i += 32) h[i] = sh[i];
   if(lane != 0) return;
   const double a = sh[j], b = sh[j + 1];
-  const double r = hypot(a, b);
-  double c = 1., s = 0.;
-  if(r > 0) { c = a / r; s = b / r; }
+  // one reciprocal root instead of hypot and two divisions (dependent FP64
+  // operations take about 110 cycles each); hypot where a^2 + b^2 leaves the
+  // normal range
+  double r, c = 1., s = 0.;
+  const double ss = a * a + b * b;
+  if(ss > 1e-280 && ss < 1e280) {
+    const double inv = rsqrt(ss);
+    r = ss * inv;
+    c = a * inv;
+    s = b * inv;
+  } else {
+    r = hypot(a, b);
+    if(r > 0) { c = a / r; s = b / r; }
+  }
   gs->cs[j] = c;
   gs->sn[j] = s;
   h[j] = r;
@@ -329,7 +349,8 @@ __global__ void k_givens(GmresState *gs, int j)
 
 // y = R^-1 g with R the upper triangle of H (k x k), by columns: the block
 // stages R in shared memory (all loads in flight at once), then one warp
-// sweeps c = k-1 .. 0: the lane holding row c divides, broadcasts y_c, and
+// sweeps c = k-1 .. 0: the lane holding row c multiplies by 1 / R_cc (all
+// formed at once beforehand), broadcasts y_c, and
 // every lane subtracts column c times y_c from its rows above c (lane l
 // holds rows l, l + 32, ...; fixed order, deterministic).
 __global__ void k_backsolve(GmresState *gs)
@@ -348,19 +369,26 @@ __global__ void k_backsolve(GmresState *gs)
   if(threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   constexpr int RPL = MAXM / 32;  // rows per lane
-  double s[RPL];
+  double s[RPL], inv[RPL];  // right-hand side and 1 / R_ii of the lane's rows (0: zero pivot)
 #pragma unroll
-  for(int t = 0; t < RPL; ++t) s[t] = lane + 32 * t < k ? gs->g[lane + 32 * t] : 0.;
+  for(int t = 0; t < RPL; ++t) {
+    const int i = lane + 32 * t;
+    s[t] = i < k ? gs->g[i] : 0.;
+    const double d = i < k ? sR[idx(i, i)] : 0.;
+    inv[t] = d != 0 ? 1.0 / d : 0.;
+  }
   for(int c = k - 1; c >= 0; --c) {
     const int owner = c & 31, tc = c >> 5;
-    double sc = 0.;
+    double sc = 0., ic = 0.;
 #pragma unroll
     for(int t = 0; t < RPL; ++t)
-      if(t == tc) sc = s[t];
+      if(t == tc) {
+        sc = s[t];
+        ic = inv[t];
+      }
     double yc = 0.;
     if(lane == owner) {
-      const double d = sR[idx(c, c)];
-      yc = d != 0 ? sc / d : 0.;
+      yc = sc * ic;
       gs->y[c] = yc;
     }
     yc = __shfl_sync(0xffffffffu, yc, owner);
@@ -1109,8 +1137,10 @@ __global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
     if(tid == 0) {
       sum = red[0][0];
       for(int k = 1; k < NW; ++k) sum += red[k][0];
+      const double nrm = sqrt(sum);
       st->result[0] = sum;
-      *Hcol = sqrt(sum);
+      st->result[1] = nrm > 0 ? 1.0 / nrm : 0.0;
+      *Hcol = nrm;
       *counter = 0;
     }
     return;
@@ -1140,7 +1170,7 @@ __global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
   if(tid == 0) *counter = 0;
 }
 
-// v = w / ||w|| (||w||^2 in st->result[0]); the last block applies the Givens
+// v = w / ||w|| (1 / ||w|| in st->result[1]); the last block applies the Givens
 // rotations of step j meanwhile.
 __global__ void k_scale64(int64_t n, const double *__restrict__ w, double *__restrict__ v, const RedState *st,
                           const int *__restrict__ done, GmresState *gs, int j)
@@ -1152,8 +1182,7 @@ __global__ void k_scale64(int64_t n, const double *__restrict__ w, double *__res
     if(threadIdx.x < 32) givens_warp(gs, j, threadIdx.x, sh, scs, ssn);
     return;
   }
-  const double nrm = sqrt(st->result[0]);
-  const double inv = nrm > 0 ? 1.0 / nrm : 0.0;
+  const double inv = st->result[1];
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)(gridDim.x - 1) * blockDim.x)
     v[i] = w[i] * inv;
 }
@@ -1165,9 +1194,8 @@ __global__ void k_scale_r32(int64_t n, const double *__restrict__ r, float *__re
 {
   FE_PDL_ENTRY();
   if(*done) return;
-  const double nrm = sqrt(st->result[0]);
-  if(blockIdx.x == 0 && threadIdx.x == 0) *beta = nrm;
-  const double inv = nrm > 0 ? 1.0 / nrm : 0.0;
+  if(blockIdx.x == 0 && threadIdx.x == 0) *beta = sqrt(st->result[0]);
+  const double inv = st->result[1];
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float v = (float)(r[i] * inv);
     V[(i / VBLK) * m1 * VBLK + (i % VBLK)] = v;
@@ -1348,80 +1376,74 @@ __global__ void k_inv_diag(int64_t n, const int32_t *__restrict__ diag, const VA
 // read back anything inside an iteration.
 struct CGState {
   double rz, rzOld, pq, rr;
+  double alpha, beta;
   double tol;
   int done;
   int it;
 };
 
+// pq = p.q and alpha = rz / pq (done when pq is zero or not finite).
+__global__ void k_cg_pq(int64_t n, const double *__restrict__ p, const double *__restrict__ q, double *partials,
+                        RedState *st, CGState *cs)
+{
+  FE_PDL_ENTRY();
+  if(cs->done) return;
+  double v[1] = {0.};
+  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v[0] += p[i] * q[i];
+  finish_reduction<1, false>(v, partials, st, nullptr, [&](double pq) {
+    cs->pq = pq;
+    cs->alpha = cs->rz / pq;
+    if(pq == 0.0 || !isfinite(pq)) cs->done = 1;
+  });
+}
+
+// x += alpha p ; r -= alpha q ; rr = r.r, the convergence test
 __global__ void k_cg_xr(int64_t n, CGState *cs, const double *__restrict__ p,
                         const double *__restrict__ q, double *__restrict__ x,
                         double *__restrict__ r, double *partials, RedState *st)
 {
   FE_PDL_ENTRY();
-  // alpha = rz / pq ; x += alpha p ; r -= alpha q ; accumulate rr
+  if(cs->done) return;
   double v[1] = {0.};
-  if(!cs->done) {
-    const double alpha = cs->rz / cs->pq;
-    for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-        i += (int64_t)gridDim.x * blockDim.x) {
-      x[i] += alpha * p[i];
-      const double ri = r[i] - alpha * q[i];
-      r[i] = ri;
-      v[0] += ri * ri;
-    }
+  const double alpha = cs->alpha;
+  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    x[i] += alpha * p[i];
+    const double ri = r[i] - alpha * q[i];
+    r[i] = ri;
+    v[0] += ri * ri;
   }
-  finish_reduction<1, false>(v, partials, st, nullptr);
+  finish_reduction<1, false>(v, partials, st, nullptr, [&](double rr) {
+    cs->rr = rr;
+    cs->it++;
+    if(!(sqrt(rr) > cs->tol) || !isfinite(rr)) cs->done = 1;
+  });
 }
 
-__global__ void k_cg_check(CGState *cs, const RedState *st)
+// rz = r.z, beta = rz / previous rz (first: 0)
+__global__ void k_cg_rz(int64_t n, const double *__restrict__ r, const double *__restrict__ z, double *partials,
+                        RedState *st, CGState *cs, int first)
 {
   FE_PDL_ENTRY();
   if(cs->done) return;
-  cs->rr = st->result[0];
-  cs->it++;
-  if(!(sqrt(cs->rr) > cs->tol) || !isfinite(cs->rr)) cs->done = 1;
-}
-
-__global__ void k_cg_p(int64_t n, CGState *cs, const RedState *st, const double *__restrict__ z,
-                       double *__restrict__ p, int first)
-{
-  FE_PDL_ENTRY();
-  if(cs->done) return;
-  const double rzNew = st->result[0];
-  const double beta = first ? 0. : rzNew / cs->rz;
-  // the first p is z alone: p is not initialised then (0 * NaN is NaN)
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = first ? z[i] : z[i] + beta * p[i];
-  __syncthreads();
-  // the scalar update happens in k_cg_rz once every block is done
-}
-
-__global__ void k_cg_rz(CGState *cs, const RedState *st)
-{
-  FE_PDL_ENTRY();
-  if(cs->done) return;
-  cs->rz = st->result[0];
-}
-
-__global__ void k_cg_pq(CGState *cs, const RedState *st)
-{
-  FE_PDL_ENTRY();
-  if(cs->done) return;
-  cs->pq = st->result[0];
-  if(cs->pq == 0.0 || !isfinite(cs->pq)) cs->done = 1;
-}
-
-__global__ void k_dot_if(int64_t n, const double *__restrict__ x, const double *__restrict__ y,
-                         double *partials, RedState *st, const CGState *cs)
-{
-  FE_PDL_ENTRY();
   double v[1] = {0.};
-  if(!cs->done)
-    for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-        i += (int64_t)gridDim.x * blockDim.x)
-      v[0] += x[i] * y[i];
-  finish_reduction<1, false>(v, partials, st, nullptr);
+  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v[0] += r[i] * z[i];
+  finish_reduction<1, false>(v, partials, st, nullptr, [&](double rz) {
+    cs->beta = first ? 0. : rz / cs->rz;
+    cs->rz = rz;
+  });
+}
+
+// p = z + beta p; the first p is z alone: p is not initialised then (0 * NaN
+// is NaN)
+__global__ void k_cg_p(int64_t n, const CGState *cs, const double *__restrict__ z, double *__restrict__ p, int first)
+{
+  FE_PDL_ENTRY();
+  if(cs->done) return;
+  const double beta = cs->beta;
+  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    p[i] = first ? z[i] : z[i] + beta * p[i];
 }
 
 __global__ void k_zero(int64_t n, double *x)
@@ -1516,7 +1538,15 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
   const double avg = n_ > 0 ? (double)A.nnz / n_ : 0;
   // 8 lanes per row beat 16 on the Taylor-Hood Jacobian (~29 entries per row)
   lanes_ = avg > 64 ? 16 : (avg > 12 ? 8 : 4);
-  nParts_ = grid_for(n_, RB, MAXRED);
+  {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    nSM_ = std::max(1, sms);
+  }
+  // reductions: two blocks per SM (each block's sum over its lanes and warps,
+  // and the last block's over the blocks, are FP64 additions)
+  nParts_ = grid_for(n_, RB, std::min(MAXRED, 2 * nSM_));
   const int m = opt.restart;
   CK(cudaMalloc(&red_, sizeof(double) * MAXRED * (MAXM + 2)));
   CK(cudaMalloc(&dsum_, sizeof(double) * 8));
@@ -1555,13 +1585,6 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
   if(n_ >= 75000) {
     bs_ = new BlockSell();
     FE_TRY(bs_->build(A_, opt.mixed != 0, s_));
-  }
-  // one group of 4 rows per thread: the whole pass is one wave of loads
-  {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    nSM_ = std::max(1, sms);
   }
   // whole waves of the update passes (three blocks per SM)
   gsParts_ = grid_for((n_ + 3) / 4, RB, std::min(MAXRED, 3 * nSM_));
@@ -2526,22 +2549,18 @@ int Krylov::solve_cg64(const double *vals, const double *b, double *x, double to
   cudaMemcpyAsync(w.cg, &init, sizeof(CGState), cudaMemcpyHostToDevice, s_);
   // z = M r ; rz = r.z ; p = z
   precond64(r_, t_, &w.cg->done);
-  ::feng::launch_k(k_dot_if, nParts_, RB, 0, s_, n_, r_, t_, red_, w.st, w.cg);
-  ::feng::launch_k(k_cg_p, gv, 256, 0, s_, n_, w.cg, w.st, t_, p_, 1);
-  ::feng::launch_k(k_cg_rz, 1, 1, 0, s_, w.cg, w.st);
+  ::feng::launch_k(k_cg_rz, nParts_, RB, 0, s_, n_, r_, t_, red_, w.st, w.cg, 1);
+  ::feng::launch_k(k_cg_p, gv, 256, 0, s_, n_, w.cg, t_, p_, 1);
   int it = 0;
   while(it < maxIt) {
     const int batch = std::min(8, maxIt - it);
     for(int k = 0; k < batch; ++k) {
       mul64(vals, p_, q_, &w.cg->done);
-      ::feng::launch_k(k_dot_if, nParts_, RB, 0, s_, n_, p_, q_, red_, w.st, w.cg);
-      ::feng::launch_k(k_cg_pq, 1, 1, 0, s_, w.cg, w.st);
+      ::feng::launch_k(k_cg_pq, nParts_, RB, 0, s_, n_, p_, q_, red_, w.st, w.cg);
       ::feng::launch_k(k_cg_xr, nParts_, RB, 0, s_, n_, w.cg, p_, q_, x, r_, red_, w.st);
-      ::feng::launch_k(k_cg_check, 1, 1, 0, s_, w.cg, w.st);
       precond64(r_, t_, &w.cg->done);
-      ::feng::launch_k(k_dot_if, nParts_, RB, 0, s_, n_, r_, t_, red_, w.st, w.cg);
-      ::feng::launch_k(k_cg_p, gv, 256, 0, s_, n_, w.cg, w.st, t_, p_, 0);
-      ::feng::launch_k(k_cg_rz, 1, 1, 0, s_, w.cg, w.st);
+      ::feng::launch_k(k_cg_rz, nParts_, RB, 0, s_, n_, r_, t_, red_, w.st, w.cg, 0);
+      ::feng::launch_k(k_cg_p, gv, 256, 0, s_, n_, w.cg, t_, p_, 0);
     }
     it += batch;
     cudaMemcpyAsync(w.hcg, w.cg, sizeof(CGState), cudaMemcpyDeviceToHost, s_);
