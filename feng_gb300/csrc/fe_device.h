@@ -50,17 +50,9 @@ struct RefTensorsTet {
   int nq;
   double qw[TET_MAXQ], qr[TET_MAXQ], qs[TET_MAXQ], qt[TET_MAXQ];
   double phi[TET_MAXQ][10];
-  // The rule as float pairs (hi + lo, lo = the double minus hi) for the
-  // double-float residual: weights, P2 values and reference gradients
-  // (dphi[q][r][a] = d phi_a / d r_r at node q), P1 values.
-  float qwh[TET_MAXQ], qwl[TET_MAXQ];
-  float phih[TET_MAXQ][10], phil[TET_MAXQ][10];
-  float dphih[TET_MAXQ][3][10], dphil[TET_MAXQ][3][10];
-  float psih[TET_MAXQ][4], psil[TET_MAXQ][4];
 };
-// The double-float tetrahedral residual keeps every node's terms in shared
-// memory: rules of up to this many nodes (degree 6; higher degrees use the
-// FP64 kernel).
+// Rules of up to this many nodes (degree 6) take the double-float residual on
+// tetrahedra, higher degrees the FP64 one.
 constexpr int TET_DF_MAXQ = 24;
 
 // Reference-element tensors of one quadrature rule (all sums over the rule's
@@ -78,15 +70,9 @@ struct RefTensors {
   int nq;
   double qw[16], qr[16], qs[16];  // the rule, for non-polynomial sources
   double phi[16][6];              // P2 functions at the nodes
-  // A 7-node rule exact to degree 5 (every polynomial integrand of the
-  // residual on affine triangles has degree <= 5).  Used when the rule above
-  // is itself exact to degree 5 (exact5), so both give the exact integrals.
+  // The rule is exact to degree 5 (every polynomial integrand of the residual
+  // on affine triangles has degree <= 5): a 7-node rule gives the same integrals.
   int exact5;
-  double w5[7], phi5[7][6], dr5[7][6], ds5[7][6], psi5[7][3];
-  // The same 7-node rule as float pairs (hi + lo, lo = the double minus hi
-  // rounded to float) for the double-float residual.
-  float w5h[7], w5l[7], phi5h[7][6], phi5l[7][6], dr5h[7][6], dr5l[7][6], ds5h[7][6], ds5l[7][6];
-  float psi5h[7][3], psi5l[7][3];
 };
 
 // Constant coefficients of the fused forms (0 = form absent).
@@ -102,9 +88,6 @@ struct FormCoeffs {
   int srcKind;      // SourceKind of SOURCE / VECTOR_SOURCE
   double srcParam[4];
   double srcCoeff;  // multiplies the source (1 when present)
-  // conv, mass, sigma, mu, divu as float pairs (hi, lo) for the
-  // double-float residual
-  float pair[5][2];
 };
 
 // Colors of an element coloring (tetrahedral meshes need more than triangles).
@@ -188,21 +171,12 @@ void launch_matrix_th_rows_f32(const RowAsm &ra, const FormCoeffs &fc, const Ref
 void launch_matrix_th_rows_f64(const RowAsm &ra, const FormCoeffs &fc, const RefTensors *dT, double c0,
                                double *values, int accumulate, cudaStream_t s);
 
-// Residual (FP64) of the fused forms on elements [begin,end) of the color
+// Residual (FP64) of the scalar P2 forms on elements [begin,end) of the color
 // order, accumulated into rhs with feNG's sign (rhs = sum of element Be).
-// exact5: the rule integrates degree 5 exactly (RefTensors::exact5), so the
-// Taylor-Hood residual may use the 7-node quadrature kernel.
-// dfloat: the Taylor-Hood 7-node kernel in double-float arithmetic (pairs of
-// floats, ~44-bit significands, on the FP32 pipes) instead of FP64.
+// Taylor-Hood: ResidualTH (fe_residual.h).
 void launch_assemble_residual(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                              const double *u, const double *udot, double t, int64_t nInc,
-                              double *rhs, int64_t begin, int64_t end, cudaStream_t s, int exact5);
-// The Taylor-Hood 7-node residual in double-float arithmetic (pairs of
-// floats, ~44-bit significands, on the FP32 pipes) from u and u-dot split
-// into float pairs (launch_split_pairs) and dm.geoPair.
-void launch_assemble_residual_df(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                                 const float2 *uPair, const float2 *udotPair, double t, int64_t nInc,
-                                 double *rhs, int64_t begin, int64_t end, cudaStream_t s);
+                              const double *u, double t, int64_t nInc, double *rhs, int64_t begin, int64_t end,
+                              cudaStream_t s);
 // out[i] = (hi, lo) of x[i]: hi = x rounded to float, lo = the rest rounded.
 void launch_split_pairs(int64_t n, const double *x, float2 *out, cudaStream_t s);
 // Jacobian of the fused forms, in double or float.
@@ -213,19 +187,14 @@ void launch_assemble_matrix_f32(const DeviceMesh &dm, const FormCoeffs &fc, cons
                                 const double *u, double c0, float *values, int64_t begin,
                                 int64_t end, cudaStream_t s);
 
-// Tetrahedra (fe_assembly_tet.cu): residual (FP64) and Jacobian (FP64 or
-// FP32) of the fused forms on elements [begin, end) of the color order, the
-// Jacobian scattered through the element-to-nonzero map (dm.map); scalar P2
-// (DIFFUSION + SOURCE) or Taylor-Hood P2-P1 (the vector forms).
+// Tetrahedra (fe_assembly_tet.cu): residual (FP64) of the scalar P2 forms
+// (DIFFUSION + SOURCE) and Jacobian (FP64 or FP32) of the scalar P2 or the
+// Taylor-Hood P2-P1 forms on elements [begin, end) of the color order, the
+// Jacobian scattered through the element-to-nonzero map (dm.map).
 void build_ref_tensors_tet(const QuadRule &q, RefTensorsTet &T);
 void launch_assemble_residual_tet(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensorsTet *dT,
-                                  const double *u, const double *udot, int64_t nInc, double *rhs,
-                                  int64_t begin, int64_t end, cudaStream_t s);
-// The Taylor-Hood residual in double-float from float pairs of u, u-dot and
-// the geometry (dm.geoPair), rules of at most TET_DF_MAXQ nodes (nq).
-void launch_assemble_residual_tet_df(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensorsTet *dT, int nq,
-                                     const float2 *up, const float2 *udp, int64_t nInc, double *rhs, int64_t begin,
-                                     int64_t end, cudaStream_t s);
+                                  const double *u, int64_t nInc, double *rhs, int64_t begin, int64_t end,
+                                  cudaStream_t s);
 void launch_assemble_matrix_tet_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensorsTet *dT,
                                     const double *u, double c0, double *values, int64_t begin, int64_t end,
                                     cudaStream_t s);

@@ -191,37 +191,6 @@ void build_ref_tensors(const QuadRule &q, RefTensors &T)
       const double exact = fact(i) * fact(j) / fact(i + j + 2);
       if(std::fabs(sum - exact) > 1e-13 * exact) T.exact5 = 0;
     }
-  QuadRule q5;
-  if(triangle_rule(5, q5) != FE_OK || q5.n() != 7) {
-    T.exact5 = 0;
-    return;
-  }
-  for(int k = 0; k < 7; ++k) {
-    double phi[6], d[2][6];
-    p2_basis(q5.r[k], q5.s[k], phi, d[0], d[1]);
-    T.w5[k] = q5.w[k];
-    for(int a = 0; a < 6; ++a) {
-      T.phi5[k][a] = phi[a];
-      T.dr5[k][a] = d[0][a];
-      T.ds5[k][a] = d[1][a];
-    }
-    T.psi5[k][0] = 1. - q5.r[k] - q5.s[k];
-    T.psi5[k][1] = q5.r[k];
-    T.psi5[k][2] = q5.s[k];
-  }
-  auto split = [](double x, float &h, float &l) {
-    h = (float)x;
-    l = (float)(x - (double)h);
-  };
-  for(int k = 0; k < 7; ++k) {
-    split(T.w5[k], T.w5h[k], T.w5l[k]);
-    for(int a = 0; a < 6; ++a) {
-      split(T.phi5[k][a], T.phi5h[k][a], T.phi5l[k][a]);
-      split(T.dr5[k][a], T.dr5h[k][a], T.dr5l[k][a]);
-      split(T.ds5[k][a], T.ds5h[k][a], T.ds5l[k][a]);
-    }
-    for(int j = 0; j < 3; ++j) split(T.psi5[k][j], T.psi5h[k][j], T.psi5l[k][j]);
-  }
 }
 
 SystemCUDA::~SystemCUDA()
@@ -322,14 +291,6 @@ int SystemCUDA::init(const SystemTables &t, const FormDesc *forms, int nforms,
                         : (k <= SRC_SIN_BODY);
     if(!ok) { set_error("source kind %d is not available on this element", k); return FE_INVALID_ARG; }
   }
-  {
-    const double cf[5] = {fc_.conv, fc_.mass, fc_.sigma, fc_.mu, fc_.divu};
-    for(int k = 0; k < 5; ++k) {
-      fc_.pair[k][0] = (float)cf[k];
-      fc_.pair[k][1] = (float)(cf[k] - (double)fc_.pair[k][0]);
-    }
-  }
-
   // Host tables: coloring, pattern, scatter map.
   ElementTables et;
   et.type = t.elemType; et.nloc = nloc_; et.nElm = nE;
@@ -473,6 +434,16 @@ int SystemCUDA::init(const SystemTables &t, const FormDesc *forms, int nforms,
   }
   CK(cudaMalloc(&dT_, sizeof(RefTensors)));
   CK(cudaMemcpy(dT_, &hT, sizeof(RefTensors), cudaMemcpyHostToDevice));
+
+  if(t.elemType == ELEM_TAYLOR_HOOD || t.elemType == ELEM_TET_TAYLOR_HOOD) {
+    // triangles: the 7-node rule for the polynomial terms when the form's own
+    // rule is exact to their degree, 5
+    QuadRule q5;
+    const bool seven = !tet && exact5_ && triangle_rule(5, q5) == FE_OK;
+    auto tab = std::make_unique<ResidualTables>();
+    build_residual_tables(seven ? q5 : t.quad, &t.quad, tet ? 3 : 2, *tab);
+    FE_TRY(resid_.build(dm_, tet ? 3 : 2, nInc_, *tab, s_));
+  }
 
   const int64_t nnz = pat_.nnz();
   std::vector<int32_t> ia32(nInc_ + 1);
@@ -1284,30 +1255,22 @@ int SystemCUDA::setResidualToZero()
 
 void SystemCUDA::launch_residual(double *out)
 {
-  if(tet()) {
-    if(dfResidual()) {
-      launch_split_pairs(nDofs_, u_, uPair_, s_);
-      if(fc_.hasMass) launch_split_pairs(nDofs_, udot_, udotPair_, s_);
-      for(int c = 0; c < dm_.nColors; ++c)
-        launch_assemble_residual_tet_df(dm_, fc_, dTt_, nq_, uPair_, udotPair_, nInc_, out, dm_.colorOff[c],
-                                        dm_.colorOff[c + 1], s_);
+  if(elemType_ == ELEM_TAYLOR_HOOD || elemType_ == ELEM_TET_TAYLOR_HOOD) {
+    if(!dfResidual()) {
+      resid_.add64(fc_, u_, udot_, out);
       return;
     }
-    for(int c = 0; c < dm_.nColors; ++c)
-      launch_assemble_residual_tet(dm_, fc_, dTt_, u_, udot_, nInc_, out, dm_.colorOff[c], dm_.colorOff[c + 1], s_);
-    return;
-  }
-  if(dfResidual()) {
     launch_split_pairs(nDofs_, u_, uPair_, s_);
     if(fc_.hasMass) launch_split_pairs(nDofs_, udot_, udotPair_, s_);
-    for(int c = 0; c < dm_.nColors; ++c)
-      launch_assemble_residual_df(dm_, fc_, dT_, uPair_, udotPair_, t_, nInc_, out, dm_.colorOff[c],
-                                  dm_.colorOff[c + 1], s_);
+    resid_.add_df(fc_, uPair_, udotPair_, out);
     return;
   }
-  for(int c = 0; c < dm_.nColors; ++c)
-    launch_assemble_residual(dm_, fc_, dT_, u_, udot_, t_, nInc_, out, dm_.colorOff[c], dm_.colorOff[c + 1], s_,
-                             exact5_);
+  for(int c = 0; c < dm_.nColors; ++c) {
+    if(tet())
+      launch_assemble_residual_tet(dm_, fc_, dTt_, u_, nInc_, out, dm_.colorOff[c], dm_.colorOff[c + 1], s_);
+    else
+      launch_assemble_residual(dm_, fc_, dT_, u_, t_, nInc_, out, dm_.colorOff[c], dm_.colorOff[c + 1], s_);
+  }
 }
 
 int SystemCUDA::assembleResiduals()

@@ -13,6 +13,7 @@
 
 #include "fe_amg.h"
 #include "fe_device.h"
+#include "fe_residual.h"
 #include "fe_krylov.h"
 #include "fe_setup.h"
 
@@ -164,6 +165,7 @@ class SystemCUDA {
   DeviceMesh dm_;
   FormCoeffs fc_{};
   RefTensors *dT_ = nullptr;
+  ResidualTH resid_;  // Taylor-Hood residuals
   int nq_ = 0;  // nodes of the system's quadrature rule
   // Row-owned Taylor-Hood FP32 Jacobian (used when every row is shorter
   // than 255).
