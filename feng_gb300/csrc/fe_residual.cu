@@ -2,7 +2,6 @@
 #include "fe_residual.h"
 
 #include <algorithm>
-#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -39,7 +38,6 @@ struct F64 {
   using T = double;
   using In = double;
   static __device__ __forceinline__ T zero() { return 0.; }
-  static __device__ __forceinline__ T from(double x) { return x; }
   static __device__ __forceinline__ T load(const double *p, int64_t i) { return p[i]; }
   static __device__ __forceinline__ T add(T a, T b) { return a + b; }
   static __device__ __forceinline__ T sub(T a, T b) { return a - b; }
@@ -53,7 +51,6 @@ struct DF {
   using T = dfl;
   using In = float2;
   static __device__ __forceinline__ T zero() { return df_zero(); }
-  static __device__ __forceinline__ T from(double x) { return df_from(x); }
   static __device__ __forceinline__ T load(const float2 *p, int64_t i)
   {
     const float2 v = p[i];
@@ -69,89 +66,129 @@ struct DF {
   static __device__ __forceinline__ double to(T a) { return df_to(a); }
 };
 
-template <typename A, int D>
-__host__ __device__ constexpr size_t table_bytes(int nq, int nqs)
+// The forms' coefficients in an arithmetic, formed on the host: conversions
+// from FP64 in every thread would be FP64 work.
+template <typename T>
+struct Coeffs {
+  T conv, mass, sigma, sigmaMu, divu;  // -conv, -mass, -sigma, sigma mu, -divu
+};
+template <typename T>
+Coeffs<T> coeffs(const FormCoeffs &fc)
 {
-  constexpr int NV = D + 1, N2 = D == 2 ? 6 : 10;
-  return sizeof(typename A::T) * (size_t)(nq * (2 * N2 + NV) + NV * NV + N2 * N2) +
-         sizeof(double) * (size_t)(nqs * (N2 + NV));
+  auto t = [](double x) {
+    if constexpr(std::is_same_v<T, double>) return x;
+    else return dfl{(float)x, (float)(x - (double)(float)x)};
+  };
+  return {t(-fc.conv), t(-fc.mass), t(-fc.sigma), t(fc.sigma * fc.mu), t(-fc.divu)};
 }
 
-// The element's residual vector be[local row][element].
+// Index of lambda_i lambda_j lambda_k among the cubic products, i <= j <= k
+// in lexicographic order: a closed form, so that unrolled loops index
+// registers.
+template <int D>
+__host__ __device__ constexpr int cubic(int i, int j, int k)
+{
+  const int x = i < j ? (i < k ? i : k) : (j < k ? j : k), z = i > j ? (i > k ? i : k) : (j > k ? j : k),
+            y = i + j + k - x - z;
+  // products before (x, ., .), before (x, y, .) and before (x, y, z)
+  const int m = D + 1 - x, n = D + 1 - y, all = (D + 1) * (D + 2) * (D + 3) / 6;
+  return all - m * (m + 1) * (m + 2) / 6 + (m * (m + 1) - n * (n + 1)) / 2 + z - y;
+}
+static_assert(cubic<3>(0, 0, 0) == 0 && cubic<3>(2, 1, 0) == 5 && cubic<3>(1, 1, 1) == 10 && cubic<3>(3, 3, 3) == 19 &&
+                  cubic<2>(0, 2, 1) == 4 && cubic<2>(1, 2, 2) == 8,
+              "lexicographic order");
+// Slot of lambda_i lambda_j among the quadratic products: the P2 node there.
+template <int D>
+__host__ __device__ constexpr int quadr(int i, int j)
+{
+  return i == j ? i : edge_node<D>(i, j);
+}
+
+// 8-byte words of shared memory: the rule's tables, the own rule's, an element.
+constexpr int n2_of(int D) { return D == 2 ? 6 : 10; }
+constexpr int n3_of(int D) { return D == 2 ? 10 : 20; }
+constexpr int table_words(int D) { return n2_of(D) * n3_of(D) + 3 * (D + 1) * (D + 1); }
+constexpr int own_words(int D, int nqs) { return nqs * (n2_of(D) + D + 1); }
+constexpr int elem_words(int D) { return 2 * D * n2_of(D) + (D + 1) * D * D; }
+
+// The element's residual vector be[local row][element]: thread (e, c) of a
+// block holds velocity component c of element e (one warp, one component).
 //
-// With p and the velocity gradient affine in the element (P1, P2 velocity on
-// a straight-sided element) the stress and divergence terms need no
-// quadrature nodes: the gradient is formed at the vertices (one
-// multiplication per vertex and function), the stress there, and its moments
-// with the P1 functions through the rule's P1 mass matrix, whose adjoint of
-// the same sparse map gives the rows.  Only the convective term runs over
-// the rule's nodes; the time derivative goes through the rule's P2 mass
-// matrix.  All are the rule's own sums regrouped.  Tetrahedra: about 2,400
-// products per element against 23,000 for the contraction of the reference
-// tensors with a warp per P2 function and 4,900 with every term at the
-// rule's 14 nodes.
-// Bound: the FP64 pipe, or the FP32 issue rate in double-float.  Residual
-// call with its host copies, before (colored scatter, one launch per color)
-// and now: 196,608 tetrahedra in FP64 7.29 -> 1.78 ms; 294,912 triangles in
-// double-float 534 -> 457 us.
+// A P2 function is a homogeneous quadratic in the barycentric coordinates l:
+// sum_i u_i l_i^2 + sum_(i<j) (4 u_ij - u_i - u_j) l_i l_j.  Its gradient at
+// the vertices is differences of those coefficients.  With p and the gradient
+// affine (straight-sided elements) no term needs a quadrature node: the
+// stress is formed at the vertices, and its moments and those of the
+// divergence go through the rule's P1 mass matrix; u . grad u is a cubic
+// whose 20 (triangles: 10) coefficients are products of the quadratic's and
+// the gradient's, u-dot joins them times sum l = 1, and the rule's moments of
+// the cubic products with the P2 functions give the rows.  All are the rule's
+// own sums regrouped, whatever its degree.  Tetrahedra: about 2,000 products
+// per element against 23,000 for the contraction of the reference tensors
+// with a warp per P2 function and 2,600 with the convective term at a rule's
+// 14 nodes.
+// Bound: the FP64 pipe (196,608 tetrahedra with a source, FP64: about 3,300
+// products, 1040 us of the pipe, 1064 measured; 1300 with node sums).  In
+// double-float the FP32 issue rate and, with a source, the FP64 pipe too: 675
+// us, of which the sources hold the FP64 pipe for 410; one thread for all
+// components held 255 registers, 8 warps an SM, and took 1113.  294,912
+// triangles in double-float: 95 us, 120 with node sums.
 template <int D, typename A>
-__global__ void __launch_bounds__(128, 2) k_residual_elem(int64_t nE, const int32_t *__restrict__ adr,
+__global__ void __launch_bounds__(D == 3 ? 96 : 128, D == 3 ? 5 : 4) k_residual_elem(int64_t nE, const int32_t *__restrict__ adr,
                                                          const double *__restrict__ geo,
                                                          const float2 *__restrict__ geoPair,
                                                          const double *__restrict__ xy,
-                                                         const ResidualTables *__restrict__ tab, FormCoeffs fc,
+                                                         const typename A::In *__restrict__ tab,
+                                                         const double *__restrict__ own, FormCoeffs fc,
+                                                         Coeffs<typename A::T> cf,
                                                          const typename A::In *__restrict__ u,
-                                                         const typename A::In *__restrict__ ud, int nq, int nqs,
+                                                         const typename A::In *__restrict__ ud, int nqs,
                                                          double *__restrict__ be)
 {
   using T = typename A::T;
-  constexpr int NV = D + 1, N2 = D == 2 ? 6 : 10;
+  constexpr int NV = D + 1, N2 = n2_of(D), N3 = n3_of(D);
   extern __shared__ __align__(16) unsigned char smem[];
-  T *sPhi = reinterpret_cast<T *>(smem), *sWphi = sPhi + nq * N2, *sLam = sWphi + nq * N2, *sm = sLam + nq * NV,
-    *sM = sm + NV * NV;
-  double *sSw = reinterpret_cast<double *>(sM + N2 * N2), *sSl = sSw + nqs * N2;
-  T *sU = reinterpret_cast<T *>(sSl + nqs * NV);  // [D N2][threads]
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for(int i = tid; i < nq * N2; i += nt) {
-    sPhi[i] = A::from(tab->phi[i / N2][i % N2]);
-    sWphi[i] = A::from(tab->wphi[i / N2][i % N2]);
-  }
-  for(int i = tid; i < nq * NV; i += nt) sLam[i] = A::from(tab->lam[i / NV][i % NV]);
-  for(int i = tid; i < NV * NV; i += nt) sm[i] = A::from(tab->m[i / NV][i % NV]);
-  for(int i = tid; i < N2 * N2; i += nt) sM[i] = A::from(tab->M[i / N2][i % N2]);
-  for(int i = tid; i < nqs * N2; i += nt) sSw[i] = tab->swphi[i / N2][i % N2];
-  for(int i = tid; i < nqs * NV; i += nt) sSl[i] = tab->slam[i / NV][i % NV];
-  const int64_t p = (int64_t)blockIdx.x * nt + tid;
-  const bool live = p < nE;
-  if(live) {
-#pragma unroll
-    for(int i = 0; i < D * N2; ++i) sU[i * nt + tid] = A::load(u, adr[(int64_t)i * nE + p]);
-  }
-  __syncthreads();
-  if(!live) return;
-  auto U = [&](int b, int c) { return sU[(D * b + c) * nt + tid]; };
+  T *sW = reinterpret_cast<T *>(smem), *sm = sW + N2 * N3, *sm4 = sm + NV * NV, *smv = sm4 + NV * NV;
+  double *sSw = reinterpret_cast<double *>(smv + NV * NV), *sSl = sSw + nqs * N2;
+  const int lane = threadIdx.x, c = threadIdx.y, EB = blockDim.x;
+  T *sU = reinterpret_cast<T *>(sSl + nqs * NV);  // [N2][D][EB] quadratic coefficients of u_c
+  T *sG = sU + N2 * D * EB;                       // [NV][D][D][EB]  d_k u_c at vertex v
+  T *sB = sG + NV * D * D * EB;                   // [N2][D][EB] rows of the convective term and u-dot
+  for(int i = c * EB + lane; i < table_words(D); i += EB * D) sW[i] = A::load(tab, i);
+  for(int i = c * EB + lane; i < own_words(D, nqs); i += EB * D) sSw[i] = own[i];
+  const int64_t p0 = (int64_t)blockIdx.x * EB + lane;
+  const bool live = p0 < nE;
+  const int64_t p = live ? p0 : nE - 1;
   auto geom = [&](int k) {
     if constexpr(std::is_same_v<T, double>) return geo[(int64_t)k * nE + p];
     else return DF::load(geoPair, (int64_t)k * nE + p);
+  };
+  // quadratic coefficients of a P2 function from its nodal values
+  auto quadratic = [&](const typename A::In *v, T *h) {
+#pragma unroll
+    for(int a = 0; a < N2; ++a) h[a] = A::load(v, adr[(int64_t)(D * a + c) * nE + p]);
+#pragma unroll
+    for(int i = 0; i < NV; ++i)
+#pragma unroll
+      for(int j = i + 1; j < NV; ++j)
+        h[quadr<D>(i, j)] = A::sub(A::scale(h[quadr<D>(i, j)], 4.f), A::add(h[i], h[j]));
   };
   T G[D][D];
 #pragma unroll
   for(int r = 0; r < D; ++r)
 #pragma unroll
     for(int k = 0; k < D; ++k) G[r][k] = geom(D * r + k);
-  const T J = geom(D * D);
-
-  // g[v][k][c] = d_k u_c at vertex v: the reference gradient there is
-  // sum_i grad lambda_i d_i with d_v = 3 u_v, d_i = 4 u_(v,i) - u_i
-  T g[NV][D][D];
+  T g[NV][D];  // d_k u_c at vertex v
+  {
+    T h[N2];
+    quadratic(u, h);
 #pragma unroll
-  for(int c = 0; c < D; ++c)
+    for(int a = 0; a < N2; ++a) sU[(a * D + c) * EB + lane] = h[a];
 #pragma unroll
     for(int v = 0; v < NV; ++v) {
       T d[NV];
 #pragma unroll
-      for(int i = 0; i < NV; ++i)
-        d[i] = i == v ? A::scale(U(v, c), 3.f) : A::sub(A::scale(U(edge_node<D>(v, i == v ? (v + 1) % NV : i), c), 4.f), U(i, c));
+      for(int i = 0; i < NV; ++i) d[i] = i == v ? A::add(h[v], h[v]) : h[quadr<D>(v, i)];
 #pragma unroll
       for(int r = 1; r < NV; ++r) d[r] = A::sub(d[r], d[0]);
 #pragma unroll
@@ -159,68 +196,118 @@ __global__ void __launch_bounds__(128, 2) k_residual_elem(int64_t nE, const int3
         T s = A::mul(G[0][k], d[1]);
 #pragma unroll
         for(int r = 1; r < D; ++r) s = A::fma(G[r][k], d[r + 1], s);
-        g[v][k][c] = s;
+        g[v][k] = s;
+        sG[((v * D + k) * D + c) * EB + lane] = s;
       }
     }
+  }
+  __syncthreads();
 
-  T b[N2][D];
+  // Be_(a,c) -= int phi_a (conv u . grad u + mass udot)_c
+  T b[N2];
+  if(fc.hasConv || fc.hasMass) {
+    T f[N3];
 #pragma unroll
-  for(int a = 0; a < N2; ++a)
+    for(int j = 0; j < N3; ++j) f[j] = A::zero();
+    if(fc.hasMass) {
+      T h[N2];
+      quadratic(ud, h);
 #pragma unroll
-    for(int c = 0; c < D; ++c) b[a][c] = A::zero();
+      for(int a = 0; a < N2; ++a) h[a] = A::mul(cf.mass, h[a]);
+#pragma unroll
+      for(int i = 0; i < NV; ++i)
+#pragma unroll
+        for(int j = i; j < NV; ++j)
+#pragma unroll
+          for(int v = 0; v < NV; ++v) f[cubic<D>(i, j, v)] = A::add(f[cubic<D>(i, j, v)], h[quadr<D>(i, j)]);
+    }
+    if(fc.hasConv) {
+#pragma unroll 1
+      for(int k = 0; k < D; ++k) {
+        T x[NV];
+#pragma unroll
+        for(int v = 0; v < NV; ++v) x[v] = A::mul(cf.conv, sG[((v * D + k) * D + c) * EB + lane]);
+#pragma unroll
+        for(int i = 0; i < NV; ++i)
+#pragma unroll
+          for(int j = i; j < NV; ++j) {
+            const T y = sU[(quadr<D>(i, j) * D + k) * EB + lane];
+#pragma unroll
+            for(int v = 0; v < NV; ++v) f[cubic<D>(i, j, v)] = A::fma(y, x[v], f[cubic<D>(i, j, v)]);
+          }
+      }
+    }
+#pragma unroll 1
+    for(int a = 0; a < N2; a += 2) {
+      T s0 = A::zero(), s1 = A::zero();
+#pragma unroll
+      for(int j = 0; j < N3; ++j) {
+        s0 = A::fma(sW[a * N3 + j], f[j], s0);
+        s1 = A::fma(sW[(a + 1) * N3 + j], f[j], s1);
+      }
+      sB[(a * D + c) * EB + lane] = s0;
+      sB[((a + 1) * D + c) * EB + lane] = s1;
+    }
+#pragma unroll
+    for(int a = 0; a < N2; ++a) b[a] = sB[(a * D + c) * EB + lane];
+  } else {
+#pragma unroll
+    for(int a = 0; a < N2; ++a) b[a] = A::zero();
+  }
 
   // Be_(a,c) += sigma (mu sum_m (d_m u_c + d_c u_m) d_m phi_a - p d_c phi_a)
   if(fc.hasSigma) {
-    const T sp = A::from(-fc.sigma), smu = A::mul(A::from(fc.sigma), A::from(fc.mu));
-    T P[NV];
+    T S[NV][D];  // sum_m G[r][m] stress_mc at the vertices
 #pragma unroll
-    for(int j = 0; j < NV; ++j) P[j] = A::mul(sp, A::load(u, adr[(int64_t)(D * N2 + j) * nE + p]));
+    for(int v = 0; v < NV; ++v) {
+      const T P = A::mul(cf.sigma, A::load(u, adr[(int64_t)(D * N2 + v) * nE + p]));
+      T st[D];
 #pragma unroll
-    for(int c = 0; c < D; ++c) {
-      T S[NV][D];  // sum_m G[r][m] stress_mc at the vertices
+      for(int m = 0; m < D; ++m) {
+        st[m] = A::mul(cf.sigmaMu, A::add(g[v][m], sG[((v * D + c) * D + m) * EB + lane]));
+        if(m == c) st[m] = A::add(st[m], P);
+      }
+#pragma unroll
+      for(int r = 0; r < D; ++r) {
+        T s = A::mul(G[r][0], st[0]);
+#pragma unroll
+        for(int m = 1; m < D; ++m) s = A::fma(G[r][m], st[m], s);
+        S[v][r] = s;
+      }
+    }
+    // edge (w, i): 4 (int lambda_w S_i + int lambda_i S_w), S_0 = -sum_r S_r;
+    // vertex w: int (4 lambda_w - 1) S_w
+#pragma unroll
+    for(int w = 0; w < NV; ++w) {
+      T e0 = A::zero();
+#pragma unroll
+      for(int r = 0; r < D; ++r) {
+        T h = A::mul(sm4[w * NV], S[0][r]);
+#pragma unroll
+        for(int v = 1; v < NV; ++v) h = A::fma(sm4[w * NV + v], S[v][r], h);
+        if(r + 1 != w) {
+          const int q = edge_node<D>(w, r + 1 == w ? (w + 1) % NV : r + 1);
+          b[q] = A::add(b[q], h);
+        }
+        e0 = A::sub(e0, h);
+      }
+      if(w) {
+        const int q = edge_node<D>(w == 0 ? 1 : w, 0);
+        b[q] = A::add(b[q], e0);
+      }
+      T x[NV];
 #pragma unroll
       for(int v = 0; v < NV; ++v) {
-        T st[D];
+        if(w) x[v] = S[v][w ? w - 1 : 0];
+        else {
+          x[v] = S[v][0];
 #pragma unroll
-        for(int m = 0; m < D; ++m) {
-          st[m] = A::mul(smu, A::add(g[v][m][c], g[v][c][m]));
-          if(m == c) st[m] = A::add(st[m], P[v]);
-        }
-#pragma unroll
-        for(int r = 0; r < D; ++r) {
-          T s = A::mul(G[r][0], st[0]);
-#pragma unroll
-          for(int m = 1; m < D; ++m) s = A::fma(G[r][m], st[m], s);
-          S[v][r] = s;
-        }
-      }
-      T tot[NV];  // sum over the vertices w of e_i(w), e_0 = -sum_r H_r, e_r = H_r
-#pragma unroll
-      for(int i = 0; i < NV; ++i) tot[i] = A::zero();
-#pragma unroll
-      for(int w = 0; w < NV; ++w) {
-        T e[NV];
-        e[0] = A::zero();
-#pragma unroll
-        for(int r = 0; r < D; ++r) {
-          T h = A::mul(sm[w * NV], S[0][r]);
-#pragma unroll
-          for(int v = 1; v < NV; ++v) h = A::fma(sm[w * NV + v], S[v][r], h);
-          e[r + 1] = h;
-          e[0] = A::sub(e[0], h);
-        }
-#pragma unroll
-        for(int i = 0; i < NV; ++i) {
-          tot[i] = A::add(tot[i], e[i]);
-          if(i == w) b[w][c] = A::add(b[w][c], A::scale(e[w], 4.f));
-          else {
-            const int q = edge_node<D>(w, i == w ? (w + 1) % NV : i);
-            b[q][c] = A::add(b[q][c], A::scale(e[i], 4.f));
-          }
+          for(int r = 1; r < D; ++r) x[v] = A::add(x[v], S[v][r]);
+          x[v] = A::neg(x[v]);
         }
       }
 #pragma unroll
-      for(int i = 0; i < NV; ++i) b[i][c] = A::sub(b[i][c], tot[i]);
+      for(int v = 0; v < NV; ++v) b[w] = A::fma(smv[w * NV + v], x[v], b[w]);
     }
   }
   // Be_pj -= divu int (div u) psi_j
@@ -228,113 +315,77 @@ __global__ void __launch_bounds__(128, 2) k_residual_elem(int64_t nE, const int3
     T dv[NV];
 #pragma unroll
     for(int v = 0; v < NV; ++v) {
-      T s = g[v][0][0];
+      T s = sG[v * D * D * EB + lane];
 #pragma unroll
-      for(int k = 1; k < D; ++k) s = A::add(s, g[v][k][k]);
+      for(int k = 1; k < D; ++k) s = A::add(s, sG[((v * D + k) * D + k) * EB + lane]);
       dv[v] = s;
     }
-    const T f = fc.hasDivu ? A::mul(A::from(-fc.divu), J) : A::zero();
-#pragma unroll
-    for(int j = 0; j < NV; ++j) {
+    const T f = fc.hasDivu ? A::mul(cf.divu, geom(D * D)) : A::zero();
+    for(int j = c; j < NV; j += D) {
       T s = A::mul(sm[j * NV], dv[0]);
 #pragma unroll
       for(int v = 1; v < NV; ++v) s = A::fma(sm[j * NV + v], dv[v], s);
-      be[(int64_t)(D * N2 + j) * nE + p] = fc.hasDivu ? A::to(A::mul(f, s)) : 0.;
+      if(live) be[(int64_t)(D * N2 + j) * nE + p] = fc.hasDivu ? A::to(A::mul(f, s)) : 0.;
     }
   }
-  // Be_(a,c) -= conv int phi_a (u . grad u)_c
-  if(fc.hasConv) {
-    const T cf = A::from(-fc.conv);
-#pragma unroll 1
-    for(int q = 0; q < nq; ++q) {
-      T uq[D], f[D];
+  const T J = geom(D * D);
+  double o[N2];
 #pragma unroll
-      for(int c = 0; c < D; ++c) {
-        T s = A::mul(sPhi[q * N2], U(0, c));
-#pragma unroll
-        for(int a = 1; a < N2; ++a) s = A::fma(sPhi[q * N2 + a], U(a, c), s);
-        uq[c] = s;
-      }
-#pragma unroll
-      for(int c = 0; c < D; ++c) {
-        f[c] = A::zero();
-#pragma unroll
-        for(int k = 0; k < D; ++k) {
-          T s = A::mul(sLam[q * NV], g[0][k][c]);
-#pragma unroll
-          for(int v = 1; v < NV; ++v) s = A::fma(sLam[q * NV + v], g[v][k][c], s);
-          f[c] = A::fma(uq[k], s, f[c]);
-        }
-        f[c] = A::mul(cf, f[c]);
-      }
-#pragma unroll
-      for(int a = 0; a < N2; ++a) {
-        const T w = sWphi[q * N2 + a];
-#pragma unroll
-        for(int c = 0; c < D; ++c) b[a][c] = A::fma(w, f[c], b[a][c]);
-      }
-    }
-  }
-  // Be_(a,c) -= mass int udot_c phi_a
-  if(fc.hasMass && ud) {
-    const T mf = A::from(-fc.mass);
-#pragma unroll 1
-    for(int d = 0; d < N2; ++d) {
-      T x[D];
-#pragma unroll
-      for(int c = 0; c < D; ++c) x[c] = A::mul(mf, A::load(ud, adr[(int64_t)(D * d + c) * nE + p]));
-#pragma unroll
-      for(int a = 0; a < N2; ++a) {
-        const T m = sM[d * N2 + a];
-#pragma unroll
-        for(int c = 0; c < D; ++c) b[a][c] = A::fma(m, x[c], b[a][c]);
-      }
-    }
-  }
-  double o[N2][D];
-#pragma unroll
-  for(int a = 0; a < N2; ++a)
-#pragma unroll
-    for(int c = 0; c < D; ++c) o[a][c] = A::to(A::mul(J, b[a][c]));
-  // Be_(a,c) -= int f_c phi_a with the form's own rule, in FP64
+  for(int a = 0; a < N2; ++a) o[a] = A::to(A::mul(J, b[a]));
+  // Be_(a,c) -= int f_c phi_a with the form's own rule, in FP64: the
+  // component threads share the nodes and add their sums
   if(nqs > 0) {
     const double sj = -fc.srcCoeff * geo[(int64_t)(D * D) * nE + p];
-    double X[NV][D];
-#pragma unroll
-    for(int v = 0; v < NV; ++v)
-#pragma unroll
-      for(int k = 0; k < D; ++k) X[v][k] = xy[(int64_t)(D * v + k) * nE + p];
+    if(D == 3 && fc.srcKind == SRC_CONST_VEC) {
+      const double f = sj * (c == 0 ? fc.srcParam[0] : c == 1 ? fc.srcParam[1] : fc.srcParam[2]);
 #pragma unroll 1
-    for(int q = 0; q < nqs; ++q) {
-      double x[D], f[D];
+      for(int q = 0; q < nqs; ++q)
 #pragma unroll
-      for(int k = 0; k < D; ++k) {
-        x[k] = sSl[q * NV] * X[0][k];
+        for(int a = 0; a < N2; ++a) o[a] += sSw[q * N2 + a] * f;
+    } else {
+      constexpr int NC = D == 2 ? 2 : 1;  // tetrahedral sources: the first component
+      double acc[N2][NC];
 #pragma unroll
-        for(int v = 1; v < NV; ++v) x[k] += sSl[q * NV + v] * X[v][k];
-        f[k] = 0.;
+      for(int a = 0; a < N2; ++a)
+#pragma unroll
+        for(int k = 0; k < NC; ++k) acc[a][k] = 0.;
+#pragma unroll 1
+      for(int q = c; q < nqs; q += D) {
+        double x[D], f[2];
+#pragma unroll
+        for(int k = 0; k < D; ++k) {
+          x[k] = sSl[q * NV] * xy[(int64_t)k * nE + p];
+#pragma unroll
+          for(int v = 1; v < NV; ++v) x[k] += sSl[q * NV + v] * xy[(int64_t)(D * v + k) * nE + p];
+        }
+        if constexpr(D == 2) source_value(fc.srcKind, fc.srcParam, x[0], x[1], f);
+        else f[0] = source_x(fc.srcKind, fc.srcParam, x[0], x[1], x[D - 1]);
+#pragma unroll
+        for(int a = 0; a < N2; ++a)
+#pragma unroll
+          for(int k = 0; k < NC; ++k) acc[a][k] += sSw[q * N2 + a] * f[k];
       }
-      if constexpr(D == 2) source_value(fc.srcKind, fc.srcParam, x[0], x[1], f);
-      else if(fc.srcKind == SRC_CONST_VEC) {
-        for(int k = 0; k < D; ++k) f[k] = fc.srcParam[k];
-      } else f[0] = source_x(fc.srcKind, fc.srcParam, x[0], x[1], x[D - 1]);
+      static_assert(D * N2 * NC <= elem_words(D), "the sums fit where the element was");
+      double *sX = reinterpret_cast<double *>(sU);  // [D][N2][NC][EB]
+      __syncthreads();
 #pragma unroll
-      for(int c = 0; c < D; ++c) f[c] *= sj;
-      const bool one = D == 3 && fc.srcKind != SRC_CONST_VEC;  // only the first component
+      for(int a = 0; a < N2; ++a)
 #pragma unroll
-      for(int a = 0; a < N2; ++a) {
-        const double w = sSw[q * N2 + a];
-        o[a][0] += w * f[0];
-        if(!one)
+        for(int k = 0; k < NC; ++k) sX[((c * N2 + a) * NC + k) * EB + lane] = acc[a][k];
+      __syncthreads();
+      if(c < NC)
 #pragma unroll
-          for(int c = 1; c < D; ++c) o[a][c] += w * f[c];
-      }
+        for(int a = 0; a < N2; ++a) {
+          double s = sX[(a * NC + c) * EB + lane];
+#pragma unroll
+          for(int t = 1; t < D; ++t) s += sX[((t * N2 + a) * NC + c) * EB + lane];
+          o[a] += sj * s;
+        }
     }
   }
+  if(!live) return;
 #pragma unroll
-  for(int a = 0; a < N2; ++a)
-#pragma unroll
-    for(int c = 0; c < D; ++c) be[(int64_t)(D * a + c) * nE + p] = o[a][c];
+  for(int a = 0; a < N2; ++a) be[(int64_t)(D * a + c) * nE + p] = o[a];
 }
 
 // rhs[r] += its elements' terms in color order (the colored scatter's sums).
@@ -385,9 +436,8 @@ __global__ void k_row_sort(int64_t n, int32_t nE, const int32_t *__restrict__ pt
 
 }  // namespace
 
-void build_residual_tables(const QuadRule &rule, const QuadRule *own, int dim, ResidualTables &T)
+void build_residual_tables(const QuadRule &rule, int dim, ResidualTables &T)
 {
-  std::memset(&T, 0, sizeof(T));
   const int nv = dim + 1, n2 = dim == 2 ? 6 : 10;
   auto basis = [&](const QuadRule &q, int k, double *lam, double *phi) {
     lam[1] = q.r[k];
@@ -399,29 +449,33 @@ void build_residual_tables(const QuadRule &rule, const QuadRule *own, int dim, R
     for(int i = 0; i < nv; ++i)
       for(int j = i + 1; j < nv; ++j) phi[dim == 2 ? edge_node<2>(i, j) : edge_node<3>(i, j)] = 4. * lam[i] * lam[j];
   };
-  T.nq = rule.n();
-  for(int k = 0; k < T.nq; ++k) {
-    basis(rule, k, T.lam[k], T.phi[k]);
-    const double w = rule.w[k];
-    for(int a = 0; a < n2; ++a) {
-      T.wphi[k][a] = w * T.phi[k][a];
-      for(int b = 0; b < n2; ++b) T.M[a][b] += w * T.phi[k][a] * T.phi[k][b];
-    }
+  const int n3 = n3_of(dim), nq = T.nq = rule.n();
+  T.rule.assign(table_words(dim), 0.);
+  T.own.assign(own_words(dim, nq), 0.);
+  double *W = T.rule.data(), *m = W + n2 * n3, *m4 = m + nv * nv, *mv = m4 + nv * nv;
+  for(int q = 0; q < nq; ++q) {
+    double *l = T.own.data() + nq * n2 + q * nv, f[10];
+    basis(rule, q, l, f);
+    const double w = rule.w[q];
+    for(int a = 0; a < n2; ++a) T.own[q * n2 + a] = w * f[a];
     for(int i = 0; i < nv; ++i)
-      for(int j = 0; j < nv; ++j) T.m[i][j] += w * T.lam[k][i] * T.lam[k][j];
-  }
-  if(!own) return;
-  T.nqs = own->n();
-  for(int k = 0; k < T.nqs; ++k) {
-    double phi[10];
-    basis(*own, k, T.slam[k], phi);
-    for(int a = 0; a < n2; ++a) T.swphi[k][a] = own->w[k] * phi[a];
+      for(int j = 0; j < nv; ++j) {
+        m[i * nv + j] += w * l[i] * l[j];
+        m4[i * nv + j] += 4. * w * l[i] * l[j];
+        mv[i * nv + j] += w * (4. * l[i] - 1.) * l[j];
+        for(int k = j; k < nv; ++k)
+          if(i <= j)
+            for(int a = 0; a < n2; ++a)
+              W[a * n3 + (dim == 2 ? cubic<2>(i, j, k) : cubic<3>(i, j, k))] += w * f[a] * l[i] * l[j] * l[k];
+      }
   }
 }
 
 ResidualTH::~ResidualTH()
 {
   cudaFree(tab_);
+  cudaFree(pairs_);
+  cudaFree(own_);
   cudaFree(be_);
   cudaFree(rowPtr_);
   cudaFree(rowEnt_);
@@ -432,7 +486,6 @@ int ResidualTH::build(const DeviceMesh &dm, int dim, int64_t nInc, const Residua
   dm_ = dm;
   dim_ = dim;
   nq_ = T.nq;
-  nqs_ = T.nqs;
   nInc_ = nInc;
   s_ = s;
   const int64_t m = dm.nElm * dm.nloc;
@@ -440,8 +493,17 @@ int ResidualTH::build(const DeviceMesh &dm, int dim, int64_t nInc, const Residua
     set_error("too many element DOFs for the residual's row tables");
     return FE_INVALID_ARG;
   }
-  CKR(cudaMalloc(&tab_, sizeof(ResidualTables)));
-  CKR(cudaMemcpy(tab_, &T, sizeof(ResidualTables), cudaMemcpyHostToDevice));
+  std::vector<float2> pairs(T.rule.size());
+  for(size_t i = 0; i < pairs.size(); ++i) {
+    const float h = (float)T.rule[i];
+    pairs[i] = make_float2(h, (float)(T.rule[i] - (double)h));
+  }
+  CKR(cudaMalloc(&tab_, sizeof(double) * T.rule.size()));
+  CKR(cudaMalloc(&pairs_, sizeof(float2) * pairs.size()));
+  CKR(cudaMalloc(&own_, sizeof(double) * T.own.size()));
+  CKR(cudaMemcpy(tab_, T.rule.data(), sizeof(double) * T.rule.size(), cudaMemcpyHostToDevice));
+  CKR(cudaMemcpy(pairs_, pairs.data(), sizeof(float2) * pairs.size(), cudaMemcpyHostToDevice));
+  CKR(cudaMemcpy(own_, T.own.data(), sizeof(double) * T.own.size(), cudaMemcpyHostToDevice));
   CKR(cudaMalloc(&be_, sizeof(double) * std::max<int64_t>(1, m)));
   CKR(cudaMalloc(&rowPtr_, sizeof(int32_t) * (nInc + 1)));
   // the mesh was copied on the legacy stream, with which s is not ordered
@@ -474,24 +536,24 @@ int ResidualTH::build(const DeviceMesh &dm, int dim, int64_t nInc, const Residua
 }
 
 template <int D, typename A, typename In>
-void ResidualTH::run(const FormCoeffs &fc, const In *u, const In *ud, double *rhs) const
+void ResidualTH::run(const FormCoeffs &fc, const In *tab, const In *u, const In *ud, double *rhs) const
 {
-  constexpr int N2 = D == 2 ? 6 : 10;
   const int64_t nE = dm_.nElm;
   if(nE <= 0 || nInc_ <= 0) return;
   // SRC_SIN3 is a scalar source: no vector form has it
-  const int nqs = fc.srcKind == SRC_NONE || fc.srcKind == SRC_SIN3 ? 0 : nqs_;
-  // smaller blocks while the elements do not give every SM one of 128
-  const int tb = nE >= 152 * 128 ? 128 : nE >= 152 * 64 ? 64 : 32;
-  const size_t sm = table_bytes<A, D>(nq_, nqs) + sizeof(typename A::T) * (size_t)(D * N2 * tb);
+  const int nqs = fc.srcKind == SRC_NONE || fc.srcKind == SRC_SIN3 ? 0 : nq_;
+  // tetrahedra: 3 warps a block, 15 an SM within 128 registers; triangles: 4,
+  // or 2 while the elements do not give every SM one block
+  const int eb = D == 2 && nE >= 152 * 64 ? 64 : 32;
+  auto bytes = [](int ns, int e) { return 8 * (size_t)(table_words(D) + own_words(D, ns) + elem_words(D) * e); };
   static bool set = false;
   if(!set) {
     cudaFuncSetAttribute(k_residual_elem<D, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(table_bytes<A, D>(RES_MAXQ, RES_MAXQ) + sizeof(typename A::T) * D * N2 * 128));
+                         (int)bytes(RES_MAXQ, 64));
     set = true;
   }
-  (k_residual_elem<D, A><<<(unsigned)((nE + tb - 1) / tb), tb, sm, s_>>>(nE, dm_.adr, dm_.geo, dm_.geoPair, dm_.xy, tab_,
-                                                                        fc, u, ud, nq_, nqs, be_),
+  (k_residual_elem<D, A><<<(unsigned)((nE + eb - 1) / eb), dim3(eb, D), bytes(nqs, eb), s_>>>(
+       nE, dm_.adr, dm_.geo, dm_.geoPair, dm_.xy, tab, own_, fc, coeffs<typename A::T>(fc), u, ud, nqs, be_),
    ::feng::count_launch());
   (k_residual_rows<<<(unsigned)((nInc_ + 255) / 256), 256, 0, s_>>>(nInc_, rowPtr_, rowEnt_, be_, rhs),
    ::feng::count_launch());
@@ -499,14 +561,14 @@ void ResidualTH::run(const FormCoeffs &fc, const In *u, const In *ud, double *rh
 
 void ResidualTH::add64(const FormCoeffs &fc, const double *u, const double *udot, double *rhs) const
 {
-  if(dim_ == 2) run<2, F64>(fc, u, udot, rhs);
-  else run<3, F64>(fc, u, udot, rhs);
+  if(dim_ == 2) run<2, F64>(fc, tab_, u, udot, rhs);
+  else run<3, F64>(fc, tab_, u, udot, rhs);
 }
 
 void ResidualTH::add_df(const FormCoeffs &fc, const float2 *up, const float2 *udp, double *rhs) const
 {
-  if(dim_ == 2) run<2, DF>(fc, up, udp, rhs);
-  else run<3, DF>(fc, up, udp, rhs);
+  if(dim_ == 2) run<2, DF>(fc, pairs_, up, udp, rhs);
+  else run<3, DF>(fc, pairs_, up, udp, rhs);
 }
 
 }  // namespace feng

@@ -1,11 +1,12 @@
 // Taylor-Hood P2-P1 residuals on triangles and tetrahedra: one thread per
-// element, element vectors in a buffer, one thread per row adding its
-// elements' terms in color order.
+// element and velocity component, element vectors in a buffer, one thread per
+// row adding its elements' terms in color order.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "fe_device.h"
 
@@ -14,18 +15,17 @@ namespace feng {
 constexpr int RES_MAXQ = 64;  // nodes of a rule
 
 // Tables of a rule on the reference element (D = 2: 3 + 3 functions, D = 3:
-// 4 + 6): nodes of the polynomial terms (phi, w phi, barycentric coordinates)
-// with the P1 and P2 mass matrices that the same nodes give, and the form's
-// own nodes for the sources.
+// 4 + 6), in the order in which a block keeps them; l: the barycentric
+// coordinates.
 struct ResidualTables {
-  int nq = 0, nqs = 0;
-  double phi[RES_MAXQ][10], wphi[RES_MAXQ][10], lam[RES_MAXQ][4];
-  double m[4][4], M[10][10];
-  double swphi[RES_MAXQ][10], slam[RES_MAXQ][4];
+  int nq = 0;
+  // sums over the nodes: w phi_a l_i l_j l_k (i <= j <= k), w l_i l_j, 4 times
+  // that, w (4 l_i - 1) l_j
+  std::vector<double> rule;
+  std::vector<double> own;  // per node, for the sources: w phi, l
 };
-// rule: the polynomial terms' rule; own: the form's rule, for the sources
-// (nqs = 0 without one).  Both on triangles (t empty) or tetrahedra.
-void build_residual_tables(const QuadRule &rule, const QuadRule *own, int dim, ResidualTables &T);
+// rule: on triangles (t empty) or tetrahedra.
+void build_residual_tables(const QuadRule &rule, int dim, ResidualTables &T);
 
 class ResidualTH {
  public:
@@ -41,12 +41,14 @@ class ResidualTH {
 
  private:
   template <int D, typename A, typename In>
-  void run(const FormCoeffs &fc, const In *u, const In *ud, double *rhs) const;
+  void run(const FormCoeffs &fc, const In *tab, const In *u, const In *ud, double *rhs) const;
   DeviceMesh dm_;
-  int dim_ = 0, nq_ = 0, nqs_ = 0;
+  int dim_ = 0, nq_ = 0;
   int64_t nInc_ = 0;
   cudaStream_t s_ = 0;
-  ResidualTables *tab_ = nullptr;
+  double *tab_ = nullptr;       // rule tables
+  float2 *pairs_ = nullptr;     // the same as float pairs
+  double *own_ = nullptr;
   double *be_ = nullptr;        // [nloc][nElm] element vectors
   int32_t *rowPtr_ = nullptr;   // [nInc + 1]
   int32_t *rowEnt_ = nullptr;   // local row * nElm + element, elements ascending (color order)

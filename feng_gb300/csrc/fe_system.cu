@@ -436,13 +436,9 @@ int SystemCUDA::init(const SystemTables &t, const FormDesc *forms, int nforms,
   CK(cudaMemcpy(dT_, &hT, sizeof(RefTensors), cudaMemcpyHostToDevice));
 
   if(t.elemType == ELEM_TAYLOR_HOOD || t.elemType == ELEM_TET_TAYLOR_HOOD) {
-    // triangles: the 7-node rule for the polynomial terms when the form's own
-    // rule is exact to their degree, 5
-    QuadRule q5;
-    const bool seven = !tet && exact5_ && triangle_rule(5, q5) == FE_OK;
-    auto tab = std::make_unique<ResidualTables>();
-    build_residual_tables(seven ? q5 : t.quad, &t.quad, tet ? 3 : 2, *tab);
-    FE_TRY(resid_.build(dm_, tet ? 3 : 2, nInc_, *tab, s_));
+    ResidualTables tab;
+    build_residual_tables(t.quad, tet ? 3 : 2, tab);
+    FE_TRY(resid_.build(dm_, tet ? 3 : 2, nInc_, tab, s_));
   }
 
   const int64_t nnz = pat_.nnz();

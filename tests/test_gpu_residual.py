@@ -3,8 +3,8 @@ sums (oracle.taylor_hood), every form present and each one alone, in FP64 and
 in the double-float arithmetic of the mixed path.
 
 Sizes: one square or cube of elements up to meshes whose elements leave a
-remainder in blocks of 32 and of 64, and one beyond the 152 x 64 elements from
-which blocks take 128.  Rules: exact to degree 5 and not (degrees 2 to 4), and
+remainder in blocks of 32 elements, and one beyond the 152 x 64 triangles from
+which blocks take 64.  Rules: exact to degree 5 and not (degrees 2 to 4), and
 the highest tetrahedral degree, whose mixed path is FP64.
 
 Tolerance: sums of at most about 200 terms of one row's elements, each with a
