@@ -12,6 +12,7 @@
 #include "fe_ilu_stream.h"
 #include "fe_launch.h"
 #include "fe_krylov.h"
+#include "fe_krylov_dev.h"
 
 namespace feng {
 
@@ -28,7 +29,6 @@ namespace {
 
 constexpr int RB = 256;        // threads per reduction block
 constexpr int MAXRED = 1024;   // maximum number of reduction blocks
-constexpr int MAXM = 128;      // maximum restart length
 
 // ---------------------------------------------------------------------------
 // SpMV: y = A x (or y = b - A x), LANES consecutive lanes per row.
@@ -78,14 +78,6 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int32_t *__restri
 // Reductions with in-kernel finalisation: every block writes a partial, the
 // last block to finish sums the partials in block order (deterministic).
 // ---------------------------------------------------------------------------
-struct RedState {
-  unsigned int counter;
-  float finv;   // 1 / ||w|| of the last FP32 Gram-Schmidt norm pass
-  int reorth;   // the last Gram-Schmidt pass asks for a second one
-  unsigned int slices[MAXM / 8];  // blocks done of each column slice (k_gs64)
-  double result[4];
-};
-
 __device__ double block_sum(double v, double *sh)
 {
   for(int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -231,114 +223,6 @@ __global__ void k_to_f32(int64_t n, const double *__restrict__ x, float *__restr
     y[i] = (float)x[i];
 }
 
-// Givens rotations on Hessenberg column j (device, one thread).  H is stored
-// column-major with leading dimension MAXM+1.
-struct GmresHead {
-  int done;       // set once the estimate reaches tol or on breakdown
-  int k;          // number of basis vectors in use
-  double est;     // |g[k]|: residual norm estimate
-  double tol;
-  double beta;    // ||r|| at the start of the cycle
-};
-struct GmresState : GmresHead {
-  double H[MAXM * (MAXM + 1)];
-  double cs[MAXM], sn[MAXM], g[MAXM + 1], y[MAXM];
-  double hcur[MAXM + 1], hcur2[MAXM + 1];
-};
-
-// One warp: the column and the previous rotations are staged in shared
-// memory, the (inherently sequential) rotation chain runs on lane 0 out of
-// registers and shared memory, and the column is written back by the warp.
-// Applies the previous rotations to Hessenberg column j, forms rotation j,
-// updates g and the residual estimate, sets done (one warp; sh, scs, ssn:
-// shared arrays of MAXM + 1, MAXM, MAXM doubles).
-__device__ void givens_warp(GmresState *gs, int j, int lane, double *sh, double *scs, double *ssn)
-{
-  double *h = gs->H + (int64_t)j * (MAXM + 1);
-  for(int i = lane; i <= j + 1; i += 32) sh[i] = h[i];
-  for(int i = lane; i < j; i += 32) {
-    scs[i] = gs->cs[i];
-    ssn[i] = gs->sn[i];
-  }
-  __syncwarp();
-  // The chain t_0 = h_0, t_{i+1} = -s_i t_i + c_i h_{i+1}, h_i <- c_i t_i +
-  // s_i h_{i+1}, h_j <- t_j is an affine recurrence: lane l composes the
-  // maps t -> -s_i t + c_i h_{i+1} of its GCH consecutive rotations, a warp
-  // scan composes the lanes' maps (Hillis-Steele, five shuffle rounds), and
-  // each lane replays its rotations from its start value: ~25 dependent FP64
-  // operations instead of two per rotation in sequence.
-  {
-    constexpr int GCH = (MAXM + 31) / 32;
-    const int i0 = lane * GCH;
-    const double h0 = sh[0];
-    double cv[GCH], sv[GCH], hv[GCH];
-    double A = 1., B = 0.;  // the lane's map t -> A t + B
-#pragma unroll
-    for(int u = 0; u < GCH; ++u) {
-      const bool ok = i0 + u < j;
-      cv[u] = ok ? scs[i0 + u] : 1.;
-      sv[u] = ok ? ssn[i0 + u] : 0.;
-      hv[u] = ok ? sh[i0 + u + 1] : 0.;
-      if(ok) {
-        const double al = -sv[u], be = cv[u] * hv[u];
-        A = al * A;
-        B = al * B + be;
-      }
-    }
-    // inclusive scan: (A, B) <- (A, B) o (lane - off's map)
-#pragma unroll
-    for(int off = 1; off < 32; off <<= 1) {
-      const double Ap = __shfl_up_sync(0xffffffffu, A, off), Bp = __shfl_up_sync(0xffffffffu, B, off);
-      if(lane >= off) {
-        B = A * Bp + B;
-        A = A * Ap;
-      }
-    }
-    // exclusive: the composition of the lanes before this one
-    double Ae = __shfl_up_sync(0xffffffffu, A, 1), Be = __shfl_up_sync(0xffffffffu, B, 1);
-    if(lane == 0) {
-      Ae = 1.;
-      Be = 0.;
-    }
-    __syncwarp();  // every read of sh before the writes below
-    double t = Ae * h0 + Be;
-#pragma unroll
-    for(int u = 0; u < GCH; ++u)
-      if(i0 + u < j) {
-        sh[i0 + u] = cv[u] * t + sv[u] * hv[u];
-        t = -sv[u] * t + cv[u] * hv[u];
-        if(i0 + u == j - 1) sh[j] = t;
-      }
-  }
-  __syncwarp();
-  for(int i = lane; i < j; i += 32) h[i] = sh[i];
-  if(lane != 0) return;
-  const double a = sh[j], b = sh[j + 1];
-  // one reciprocal root instead of hypot and two divisions (dependent FP64
-  // operations take about 110 cycles each); hypot where a^2 + b^2 leaves the
-  // normal range
-  double r, c = 1., s = 0.;
-  const double ss = a * a + b * b;
-  if(ss > 1e-280 && ss < 1e280) {
-    const double inv = rsqrt(ss);
-    r = ss * inv;
-    c = a * inv;
-    s = b * inv;
-  } else {
-    r = hypot(a, b);
-    if(r > 0) { c = a / r; s = b / r; }
-  }
-  gs->cs[j] = c;
-  gs->sn[j] = s;
-  h[j] = r;
-  h[j + 1] = 0.;
-  gs->g[j + 1] = -s * gs->g[j];
-  gs->g[j] = c * gs->g[j];
-  gs->k = j + 1;
-  gs->est = fabs(gs->g[j + 1]);
-  if(!(gs->est > gs->tol) || b == 0.0 || !isfinite(gs->est)) gs->done = 1;
-}
-
 __global__ void k_givens(GmresState *gs, int j)
 {
   FE_PDL_ENTRY();
@@ -458,17 +342,6 @@ __global__ void k_xupdate(int64_t n, int64_t ld, const VZ *__restrict__ Z, const
 // writes hcur / Hcol (MODE 0: Hcol = h, MODE 1: Hcol += h) or ss into
 // st->result[0].  The FP64 pipe of the GB300 is too slow for these loops.
 // ---------------------------------------------------------------------------
-
-// The FP32 Arnoldi basis of the mixed path is stored in row blocks of VBLK
-// rows: column c of row block k at V + (k m1 + c) VBLK (m1 = restart + 1
-// columns per block), so that a block of threads streaming several columns
-// over the same rows reads one contiguous region.  vidx4: the float4 index
-// of float4 row g (rows 4g..4g+3) of column c.
-constexpr int VBLK = 1024;
-__host__ __device__ __forceinline__ int64_t vidx4(int64_t g, int c, int m1)
-{
-  return ((g >> 8) * m1 + c) * (VBLK / 4) + (g & (VBLK / 4 - 1));
-}
 
 // A second read of a line this thread has just read (served by L1): a
 // separate load, so that the compiler does not keep the first read in
@@ -944,40 +817,15 @@ __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__r
   }
 }
 
-// v = w * (1 / ||w||) in FP32, 4 rows per thread; the scale comes from the
-// last update + norm pass (k_gs_upd<., true> or k_gs32<., 2>).
-// gated: only after a second Gram-Schmidt pass (otherwise k_gs_upd wrote v).
-// gs (ungated only): the last block does not scale; its warp 0 applies the
-// Givens rotations of step j meanwhile (k_givens folded in; a block that
-// starts after the step converged skips its share of v, which the cycle no
-// longer reads).
-// The result goes to column col of the row-blocked basis V and to its
-// contiguous copy vcopy (the preconditioner's next input).
-__global__ void k_scale32(int64_t n4, const float *__restrict__ w, float *__restrict__ V, int m1, int col,
-                          float *__restrict__ vcopy, const RedState *st, const int *__restrict__ done, int gated,
-                          GmresState *gs, int j)
+// Basis vector j + 1 and rotation j of an Arnoldi step (scale_blocks), where
+// the next preconditioner does not begin with them.  gated: only after a
+// second Gram-Schmidt pass (otherwise k_gs_upd wrote the vector).
+template <typename V>
+__global__ void k_scale(ScaleStep<V> sc, int gated)
 {
   FE_PDL_ENTRY();
-  __shared__ double sh[MAXM + 1], scs[MAXM], ssn[MAXM];
-  if(*done || (gated && !st->reorth)) return;
-  if(gs && blockIdx.x == gridDim.x - 1) {
-    if(threadIdx.x < 32) givens_warp(gs, j, threadIdx.x, sh, scs, ssn);
-    return;
-  }
-  const int nb = gs ? (int)gridDim.x - 1 : (int)gridDim.x;
-  const float inv = st->finv;
-  const float4 *w4 = reinterpret_cast<const float4 *>(w);
-  float4 *V4 = reinterpret_cast<float4 *>(V);
-  float4 *c4 = reinterpret_cast<float4 *>(vcopy);
-  for(int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n4; g += (int64_t)nb * blockDim.x) {
-    float4 t = w4[g];
-    t.x *= inv;
-    t.y *= inv;
-    t.z *= inv;
-    t.w *= inv;
-    V4[vidx4(g, col, m1)] = t;
-    c4[g] = t;
-  }
+  if(gated && !sc.st->reorth) return;
+  scale_blocks(sc, (int)blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1168,23 +1016,6 @@ __global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
     }
   }
   if(tid == 0) *counter = 0;
-}
-
-// v = w / ||w|| (1 / ||w|| in st->result[1]); the last block applies the Givens
-// rotations of step j meanwhile.
-__global__ void k_scale64(int64_t n, const double *__restrict__ w, double *__restrict__ v, const RedState *st,
-                          const int *__restrict__ done, GmresState *gs, int j)
-{
-  FE_PDL_ENTRY();
-  __shared__ double sh[MAXM + 1], scs[MAXM], ssn[MAXM];
-  if(*done) return;
-  if(blockIdx.x == gridDim.x - 1) {
-    if(threadIdx.x < 32) givens_warp(gs, j, threadIdx.x, sh, scs, ssn);
-    return;
-  }
-  const double inv = st->result[1];
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)(gridDim.x - 1) * blockDim.x)
-    v[i] = w[i] * inv;
 }
 
 // V_0 = r / ||r|| rounded to FP32 (start of a mixed cycle; column 0 of the
@@ -1850,12 +1681,12 @@ int Krylov::factor(const double *values64, const float *values32)
   return FE_OK;
 }
 
-void Krylov::precond64(const double *r, double *z, const int *done)
+void Krylov::precond64(const double *r, double *z, const int *done, const ScaleStep<double> *sc)
 {
   if(opt.precond == 0) {
     cudaMemcpyAsync(z, r, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s_);
   } else if(opt.precond >= 3) {
-    apply_mg<double>(cur64_, r, z, done);
+    apply_mg<double>(cur64_, r, z, done, sc);
   } else if(opt.precond == 2) {
     ::feng::launch_k(k_jacobi<double, double>, grid_for(n_, 256, 4096), 256, 0, s_, n_, diag_, r, z, done);
   } else {
@@ -1864,12 +1695,12 @@ void Krylov::precond64(const double *r, double *z, const int *done)
   }
 }
 
-void Krylov::precond32(const float *r, float *z, const int *done)
+void Krylov::precond32(const float *r, float *z, const int *done, const ScaleStep<float> *sc)
 {
   if(opt.precond == 0) {
     cudaMemcpyAsync(z, r, sizeof(float) * n_, cudaMemcpyDeviceToDevice, s_);
   } else if(opt.precond >= 3) {
-    apply_mg<float>(cur32_, r, z, done);
+    apply_mg<float>(cur32_, r, z, done, sc);
   } else if(opt.precond == 2) {
     ::feng::launch_k(k_jacobi<float, float>, grid_for(n_, 256, 4096), 256, 0, s_, n_, diag32_, r, z, done);
   } else {
@@ -2245,9 +2076,13 @@ void Krylov::fp64_part(const double *vals, const double *b, double *x, int j0, i
     ::feng::launch_k(k_gmres_init, 1, 1, 0, s_, w.gs, w.st);
     ::feng::launch_k(k_scale_from, gv, 256, 0, s_, n_, w_, V_, w.st, &w.gs->beta, &w.gs->done);
   }
+  // the scale pass of a step rides in the first kernel of the next step's
+  // preconditioner, not where the host looks at the estimate in between
+  const bool fuse = !poll && scaleInPrecond();
+  ScaleStep<double> sc{};
   for(int j = j0; j < j1; ++j) {
     double *vj = V_ + (int64_t)j * ld64_, *zj = Z_ + (int64_t)j * ld64_;
-    precond64(vj, zj, &w.gs->done);
+    precond64(vj, zj, &w.gs->done, fuse && j > j0 ? &sc : nullptr);
     mul64(vals, zj, w_, &w.gs->done);
     double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
     gs64(GS_DOT, j + 1, nullptr, w.gs->hcur, Hcol, &w.gs->done, 0);
@@ -2258,7 +2093,8 @@ void Krylov::fp64_part(const double *vals, const double *b, double *x, int j0, i
       gs64(GS_DOT, j + 1, nullptr, w.gs->hcur2, Hcol, &w.gs->done, 1);
     }
     gs64(GS_UPD_NORM, j + 1, w.gs->hcur2, nullptr, Hcol + j + 1, &w.gs->done, 1);
-    ::feng::launch_k(k_scale64, gv + 1, 256, 0, s_, n_, w_, vj + ld64_, w.st, &w.gs->done, w.gs, j);
+    sc = {w_, w.st, vj + ld64_, nullptr, n_, 0, 0, &w.gs->done, w.gs, j, gv};
+    if(!fuse || j + 1 == j1) ::feng::launch_k(k_scale<double>, gv + 1, 256, 0, s_, sc, 0);
     if(poll && poll_done(&w.gs->done, j)) break;
   }
   if(!epi) return;
@@ -2295,11 +2131,13 @@ void Krylov::mixed_part(const float *vals, const double *b, double *x, int j0, i
   ::feng::launch_k(k_scale_r32, gv, 256, 0, s_, n_, w_, V32_, m1, vc32_, w.st, &w.gs->beta, &w.gs->done);
   }
   const int g4 = grid_for(ld32_ / 4, 256, 4 * 152);
+  const bool fuse = !poll && opt.gsPasses != 3 && scaleInPrecond();  // see fp64_part
+  ScaleStep<float> sc{};
   for(int j = j0; j < j1; ++j) {
     // v_j: the contiguous copy written with basis column j
     const float *vj = vc32_;
     float *zj = Z32_ + (int64_t)j * ld32_;
-    precond32(vj, zj, &w.gs->done);
+    precond32(vj, zj, &w.gs->done, fuse && j > j0 ? &sc : nullptr);
     double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
     if(bs_)
       bs_->mul32(zj, w32_, &w.gs->done);
@@ -2329,14 +2167,14 @@ void Krylov::mixed_part(const float *vals, const double *b, double *x, int j0, i
       gs32(0, j + 1, nullptr, w.gs->hcur, Hcol, &w.gs->done, 1);
       gs32(4, j + 1, w.gs->hcur, nullptr, Hcol + j + 1, &w.gs->done, 1);
     }
+    sc = {w32_, w.st, vc32_, V32_, ld32_ / 4, m1, j + 1, &w.gs->done, w.gs, j, g4};
     if(opt.gsPasses == 3) {
       // gated scale (only after a second pass), then the rotations
-      ::feng::launch_k(k_scale32, g4, 256, 0, s_, ld32_ / 4, w32_, V32_, m1, j + 1, vc32_, w.st, &w.gs->done, 1,
-                       (GmresState *)nullptr, 0);
+      sc.gs = nullptr;
+      ::feng::launch_k(k_scale<float>, g4, 256, 0, s_, sc, 1);
       ::feng::launch_k(k_givens, 1, 32, 0, s_, w.gs, j);
-    } else {
-      ::feng::launch_k(k_scale32, g4 + 1, 256, 0, s_, ld32_ / 4, w32_, V32_, m1, j + 1, vc32_, w.st, &w.gs->done, 0,
-                       w.gs, j);
+    } else if(!fuse || j + 1 == j1) {
+      ::feng::launch_k(k_scale<float>, g4 + 1, 256, 0, s_, sc, 0);
     }
     if(poll && poll_done(&w.gs->done, j)) break;
   }

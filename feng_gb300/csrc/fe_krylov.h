@@ -19,6 +19,8 @@
 
 namespace feng {
 
+template <typename V> struct ScaleStep;
+
 struct DeviceCSR {
   int64_t n = 0, nnz = 0;
   int32_t *ia = nullptr;  // [n+1]
@@ -143,8 +145,11 @@ class Krylov {
   void ilu_factor_levels(const double *values64, const float *values32);
   template <typename VF, typename VV>
   void ilu_solve_levels(const VV *r, VV *z, const int *done);
-  void precond64(const double *r, double *z, const int *skip);
-  void precond32(const float *r, float *z, const int *skip);
+  // sc: r is to be formed first, as the scaled w of the step before, in the
+  // preconditioner's first kernel (scaleInPrecond())
+  void precond64(const double *r, double *z, const int *skip, const ScaleStep<double> *sc = nullptr);
+  void precond32(const float *r, float *z, const int *skip, const ScaleStep<float> *sc = nullptr);
+  bool scaleInPrecond() const;
 
   DeviceCSR A_;
   DeviceBlockILU ilu_;
@@ -257,7 +262,7 @@ class Krylov {
   // cycle's residual and update included (benchmark phase; x is scratch).
   int cycleGraph(bool mixed, const void *vals, const double *b, double *x, int reps, double *msPerStep);
   int factor_mg(const double *values64, const float *values32);
-  template <typename V> void apply_mg(const V *vals, const V *r, V *z, const int *skip);
+  template <typename V> void apply_mg(const V *vals, const V *r, V *z, const int *skip, const ScaleStep<V> *sc);
 };
 
 }  // namespace feng

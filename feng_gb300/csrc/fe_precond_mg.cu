@@ -18,6 +18,7 @@
 #include "fe_common.h"
 #include "fe_launch.h"
 #include "fe_krylov.h"
+#include "fe_krylov_dev.h"
 
 namespace feng {
 
@@ -289,13 +290,14 @@ __global__ void k_pressure(int64_t nP, const int32_t *__restrict__ rows, const S
 // of k_vel_rhs_fold).
 template <typename V>
 __device__ __forceinline__ void psum_blocks(int vb, int vg, int64_t nP, const int32_t *__restrict__ rows,
-                                            const V *__restrict__ r, double *part, unsigned *count, double *out)
+                                            const V *__restrict__ r, V f, double *part, unsigned *count,
+                                            double *out)
 {
   __shared__ double sh[256];
   __shared__ bool last;
   double s = 0.;
   for(int64_t k = (int64_t)vb * blockDim.x + threadIdx.x; k < nP; k += (int64_t)vg * blockDim.x)
-    s += (double)r[rows[k]];
+    s += (double)(r[rows[k]] * f);
   sh[threadIdx.x] = s;
   __syncthreads();
   for(int o = 128; o > 0; o >>= 1) {
@@ -329,7 +331,7 @@ __global__ void k_psum(int64_t nP, const int32_t *__restrict__ rows, const V *__
                        unsigned *count, double *out)
 {
   FE_PDL_ENTRY();
-  psum_blocks<V>(blockIdx.x, gridDim.x, nP, rows, r, part, count, out);
+  psum_blocks<V>(blockIdx.x, gridDim.x, nP, rows, r, (V)1, part, count, out);
 }
 
 // partial sums of a double array
@@ -464,27 +466,41 @@ __global__ void k_vel_rhs_pair(int64_t nN, const int32_t *__restrict__ dofX, con
 // (both components interleaved, one thread per slot), and in the leading
 // gp blocks (scheduled first, so that the sum's last-block reduction
 // overlaps the slots) the pressure sum c = sum of r over the pressure rows
-// (k_psum's partials and order) into *cr.
+// (k_psum's partials and order) into *cr.  With sc, r = w / ||w|| is not
+// there yet: the blocks read w and scale their sums, and the next sc.blocks
+// + 1 blocks write r, the basis column and the rotation of the step before
+// (the scale pass, a launch of its own otherwise).  Kovasznay solves: 32^2
+// FP64 54.6 -> 52.1 ms, 97^2 mixed 26.5 -> 25.4, 256^2 mixed 62.7 -> 61.4,
+// 256^2 FP64 365 -> 363.
 template <typename V>
 __global__ void k_vel_rhs_fold(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
                                const int32_t *__restrict__ upIa, const int32_t *__restrict__ upCol,
                                const V *__restrict__ gs, const V *__restrict__ r, V *__restrict__ bxy,
-                               int slotBlocks, int64_t nP, const int32_t *__restrict__ pRows, double *part,
-                               unsigned *count, double *cr, const int *__restrict__ skip)
+                               int gp, int64_t nP, const int32_t *__restrict__ pRows, double *part,
+                               unsigned *count, double *cr, ScaleStep<V> sc, const int *__restrict__ skip)
 {
   FE_PDL_ENTRY();
-  if(skip && *skip) return;
-  const int gp = (int)gridDim.x - slotBlocks;
+  const V *x = sc.w ? sc.w : r;
+  // with sc the rotation may set *skip meanwhile: the blocks that count one
+  // another must all run
   if((int)blockIdx.x < gp) {
-    psum_blocks<V>((int)blockIdx.x, gp, nP, pRows, r, part, count, cr);
+    if(!sc.w && skip && *skip) return;
+    psum_blocks<V>((int)blockIdx.x, gp, nP, pRows, x, sc.w ? scale_of(sc) : (V)1, part, count, cr);
     return;
   }
-  const int64_t q = (int64_t)((int)blockIdx.x - gp) * blockDim.x + threadIdx.x;
+  const int sb = sc.w ? sc.blocks + 1 : 0;
+  if((int)blockIdx.x < gp + sb) {
+    scale_blocks(sc, (int)blockIdx.x - gp);
+    return;
+  }
+  if(skip && *skip) return;
+  const int64_t q = (int64_t)((int)blockIdx.x - gp - sb) * blockDim.x + threadIdx.x;
   if(q >= 2 * nN) return;
+  const V f = sc.w ? scale_of(sc) : (V)1;
   const int64_t k = q >> 1;
-  V t = r[(q & 1) == 0 ? dofX[k] : dofY[k]];
-  for(int32_t e = upIa[q]; e < upIa[q + 1]; ++e) t -= gs[e] * r[upCol[e]];
-  bxy[q] = t;
+  V t = x[(q & 1) == 0 ? dofX[k] : dofY[k]];
+  for(int32_t e = upIa[q]; e < upIa[q + 1]; ++e) t -= gs[e] * x[upCol[e]];
+  bxy[q] = t * f;
 }
 
 // Per Jacobian: the pressure scale sc_k = coef / (den m_k) in FP64 and
@@ -941,7 +957,7 @@ int Krylov::smootherStep(int64_t *bytes)
 }
 
 template <typename V>
-void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
+void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip, const ScaleStep<V> *scale)
 {
   MG &M = *mg_;
   M.amg->setSkip(skip);
@@ -956,9 +972,11 @@ void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
     // kernel forms b0 and c, the V-cycle's last pass writes z_u and z_p.
     const int gp = (int)std::min<int64_t>(NPART, std::max<int64_t>(1, (M.nP + 255) / 256));
     const int slotBlocks = (int)((2 * M.nNodes + 255) / 256);
+    const ScaleStep<V> sc = scale ? *scale : ScaleStep<V>{};
+    const int sb = scale ? sc.blocks + 1 : 0;
     double *cr = M.scal + 3;
-    ::feng::launch_k(k_vel_rhs_fold<V>, slotBlocks + gp, 256, 0, s_, M.nNodes, M.dofX, M.dofY, M.upIa, M.upCol,
-                     (const V *)M.gScaled, r, (V *)M.bxy, slotBlocks, M.nP, M.pRows, M.part, M.count, cr, skip);
+    ::feng::launch_k(k_vel_rhs_fold<V>, gp + sb + slotBlocks, 256, 0, s_, M.nNodes, M.dofX, M.dofY, M.upIa,
+                     M.upCol, (const V *)M.gScaled, r, (V *)M.bxy, gp, M.nP, M.pRows, M.part, M.count, cr, sc, skip);
     AMGDevice::OutMap om;
     om.dofX = M.dofX;
     om.dofY = M.dofY;
@@ -1043,7 +1061,14 @@ void Krylov::apply_mg(const V *vals, const V *r, V *z, const int *skip)
                                                 (const V *)M.zx, (const V *)M.zy, M.consts, z, skip);
 }
 
-template void Krylov::apply_mg<double>(const double *, const double *, double *, const int *);
-template void Krylov::apply_mg<float>(const float *, const float *, float *, const int *);
+// With the pressure folded the first kernel needs no scaled vector: it carries
+// the scale pass.  (In front of the unfolded kernels, beside the pressure sum,
+// the pass gained nothing: cavity 384^2 44.4 and 44.5 ms, cube 32^3 44.0 and
+// 43.9.)
+bool Krylov::scaleInPrecond() const { return opt.precond >= 3 && mg_ && mg_->kind == 4 && mg_->fold; }
+
+template void Krylov::apply_mg<double>(const double *, const double *, double *, const int *,
+                                       const ScaleStep<double> *);
+template void Krylov::apply_mg<float>(const float *, const float *, float *, const int *, const ScaleStep<float> *);
 
 }  // namespace feng
