@@ -7,7 +7,10 @@
 // receives one contribution per color and the sums are the colored
 // read-modify-write's, in color order.
 //
-// Row-owned kernel (Taylor-Hood Jacobian, k_matrix_th_rows): one thread per
+// Taylor-Hood Jacobian in FP64: the element matrices of all elements to a
+// buffer, then the scatter a color at a time (k_jac_th, k_jac_scatter).
+//
+// Row-owned kernel (Taylor-Hood FP32 Jacobian, k_matrix_th_rows): one thread per
 // CSR row sums the element-matrix rows of the elements holding that DOF, in
 // color order, in shared memory; each block writes its contiguous range of
 // CSR values once (no atomics, no map, no separate zeroing pass).
@@ -184,159 +187,173 @@ __device__ __forceinline__ int th_map_index(int k, int m)
   return j < 15 ? i * 15 + j : (12 + j - 15) * 15 + i;
 }
 
-template <typename V>
-__device__ __forceinline__ void scatter_staged(const int32_t *__restrict__ map, int64_t nE, int64_t p0, int64_t end,
-                                               int hasSigma, int hasDivu, int m, const V (*sAdd)[EPB],
-                                               V *__restrict__ values)
-{
-  const int tid = threadIdx.y * EPB + threadIdx.x;
-  constexpr int NT = EPB * 6, TOTAL = 108 * EPB, BATCH = 6;
-  for(int base = tid; base < TOTAL; base += NT * BATCH) {
-    int32_t pos[BATCH];
-    V add[BATCH];
-#pragma unroll
-    for(int q = 0; q < BATCH; ++q) {
-      const int idx = base + q * NT;
-      pos[q] = -1;
-      add[q] = 0;
-      if(idx < TOTAL) {
-        const int e = idx % EPB, k = idx / EPB, j = k % 18;
-        const bool on = (j < 12) || (j < 15 ? hasSigma : hasDivu);
-        if(on && p0 + e < end) {
-          pos[q] = __ldg(map + (int64_t)th_map_index(k, m) * nE + p0 + e);
-          add[q] = sAdd[k][e];
-        }
-      }
-    }
-    // Within one color every CSR entry receives at most one contribution, so
-    // the reduction in L2 (no round trip to the SM) gives the same bits as
-    // a read-modify-write.
-#pragma unroll
-    for(int q = 0; q < BATCH; ++q)
-      if(pos[q] >= 0) atomicAdd(values + pos[q], add[q]);
-  }
-}
+// ---------------------------------------------------------------------------
+// Jacobian, Taylor-Hood P2-P1: element matrices, then the colored scatter.
+// ---------------------------------------------------------------------------
+constexpr int TH_ENT = 216;  // structurally nonzero entries: entry m * 108 + k (th_map_index)
 
-// ---------------------------------------------------------------------------
-// Jacobian, Taylor-Hood P2-P1.
-// ---------------------------------------------------------------------------
+// Entries of the elements [p0, end) to buf[entry][p - p0] (leading dimension
+// ld).  Thread (e, a), as above.
+//
+// A P2 function's gradient is affine, so u . grad u and its derivative need no
+// tensor over three P2 functions: with S[a][b][j] = int phi_a phi_b psi_j
+//   int phi_a phi_b d_n u_m     = J sum_v (d_n u_m)(vertex v) S[a][b][v],
+//   int phi_a psi_j u . grad l_i = J sum_c (u_c . grad l_i) S[a][c][j],
+// and grad phi_b is 4 l_i grad l_i - grad l_i or 4 (l_i grad l_j + l_j grad
+// l_i): the rule's own sums regrouped, 1,700 products an element for 3,300.
+// Bound: the FP64 pipe (32,768 elements: 91 us of it, 114 measured).  A color
+// at a time, with the scatter inside, the 128 x 128 Jacobian was six launches
+// of 170 blocks (the chip holds 600), 72 us each; now 114 us and the colors'
+// scatters of 12 (cold).  Call with its 28 MB copy to the host: 732 -> 455 us.
 template <typename V>
-__global__ void __launch_bounds__(EPB * 6) k_matrix_th(DeviceMesh dm, FormCoeffs fc,
-                                                      const RefTensors *__restrict__ gT,
-                                                      const double *__restrict__ u, double c0,
-                                                      V *__restrict__ values, int64_t begin,
-                                                      int64_t end)
+__global__ void __launch_bounds__(EPB * 6) k_jac_th(DeviceMesh dm, FormCoeffs fc, const RefTensors *__restrict__ gT,
+                                                   const double *__restrict__ u, double c0, V *__restrict__ buf,
+                                                   int64_t ld, int64_t p0, int64_t end)
 {
-  __shared__ SharedTensors<V> sT;
-  __shared__ V sU[12][EPB];
-  __shared__ V sG[5][EPB];
-  __shared__ V sAdd[108][EPB];
-  const int lane = threadIdx.x, a = threadIdx.y;
-  const int64_t p = begin + (int64_t)blockIdx.x * EPB + lane;
-  const bool live = p < end;
-  const int64_t nE = dm.nElm;
-  load_tensors(sT, gT);
-  if(live) {
-    if(fc.hasConv)
-      for(int i = a; i < 12; i += 6) sU[i][lane] = (V)u[dm.adr[(int64_t)i * nE + p]];
-    if(a < 5) sG[a][lane] = (V)dm.geo[(int64_t)a * nE + p];
-  } else {
-    // Past the end of the color: zero data, entries never scattered.
-    for(int i = a; i < 12; i += 6) sU[i][lane] = 0;
-    if(a < 5) sG[a][lane] = 0;
+  __shared__ V sK[2][2][6][6], sS[6][6][3], sD[2][3][6], sM[6][6];
+  __shared__ V sU[12][EPB], sA[2][6][EPB], sG[3][2][2][EPB];
+  const int lane = threadIdx.x, a = threadIdx.y, tid = a * EPB + lane;
+  for(int i = tid; i < 144; i += EPB * 6) (&sK[0][0][0][0])[i] = (V)(&gT->K[0][0][0][0])[i];
+  for(int i = tid; i < 108; i += EPB * 6) (&sS[0][0][0])[i] = (V)(&gT->S[0][0][0])[i];
+  for(int i = tid; i < 36; i += EPB * 6) {
+    (&sD[0][0][0])[i] = (V)(&gT->D[0][0][0])[i];
+    (&sM[0][0])[i] = (V)(&gT->M[0][0])[i];
+  }
+  const int64_t nE = dm.nElm, q = p0 + (int64_t)blockIdx.x * EPB + lane, p = q < end ? q : end - 1;
+  V G[2][2];
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int k = 0; k < 2; ++k) G[r][k] = (V)dm.geo[(int64_t)(2 * r + k) * nE + p];
+  const V J = (V)dm.geo[4 * nE + p], cc = (V)fc.conv * J;
+  if(fc.hasConv) {
+    const V x = (V)u[dm.adr[(int64_t)(2 * a) * nE + p]], y = (V)u[dm.adr[(int64_t)(2 * a + 1) * nE + p]];
+    sU[2 * a][lane] = x;
+    sU[2 * a + 1][lane] = y;
+#pragma unroll
+    for(int r = 0; r < 2; ++r) sA[r][a][lane] = cc * (G[r][0] * x + G[r][1] * y);
+    __syncthreads();
+    // cc d_n u_m at vertex v: differences of the quadratic's coefficients
+    // 2 u_v and 4 u_(v,i) - u_v - u_i
+    const int v = a % 3, m = a / 3;
+    V h[3];
+#pragma unroll
+    for(int i = 0; i < 3; ++i) {
+      const int e = v + i == 1 ? 3 : (v + i == 3 ? 4 : 5);  // edges (0,1) (1,2) (2,0)
+      const V uv = sU[2 * v + m][lane];
+      h[i] = i == v ? uv + uv : (V)4 * sU[2 * e + m][lane] - (uv + sU[2 * i + m][lane]);
+    }
+    const V d0 = cc * (h[1] - h[0]), d1 = cc * (h[2] - h[0]);
+#pragma unroll
+    for(int n = 0; n < 2; ++n) sG[v][n][m][lane] = G[0][n] * d0 + G[1][n] * d1;
   }
   __syncthreads();
-  const V G[2][2] = {{sG[0][lane], sG[1][lane]}, {sG[2][lane], sG[3][lane]}};
-  const V J = sG[4][lane];
+  if(q >= end) return;
+  V *out = buf + (q - p0) + (int64_t)(a * 18) * ld;
+  const int64_t ldm = 108 * ld;  // from row component 0 to 1
 
-  // Element rows (a,0) and (a,1): 12 velocity columns + 3 pressure columns.
-  V A[2][12];
-#pragma unroll
-  for(int m = 0; m < 2; ++m)
-#pragma unroll
-    for(int j = 0; j < 12; ++j) A[m][j] = 0;
-
+  V W[6] = {0, 0, 0, 0, 0, 0};  // cc int phi_a u . grad phi_b
+  V g[3][2][2];
   if(fc.hasConv) {
-    // A_(a,m),(b,n) += c [ delta_mn phi_a (u0 . grad phi_b) + phi_a phi_b d_n u0_m ]
-    // (vectorDotGradShapeDotShape + shapeDotTensorDotShape, feVectorSpace.cpp:202-290)
-    V V0[2][6];
-    for(int c = 0; c < 6; ++c)
-      for(int r = 0; r < 2; ++r) V0[r][c] = sU[2 * c][lane] * G[r][0] + sU[2 * c + 1][lane] * G[r][1];
-    const V cc = (V)fc.conv * J;
-    for(int b = 0; b < 6; ++b) {
-      V W = 0, Z[2][2] = {{0, 0}, {0, 0}};  // Z[r][m] = sum_c U_cm T[r][a][b][c]
-      for(int c = 0; c < 6; ++c) {
-        W += V0[0][c] * sT.T[0][a][c][b] + V0[1][c] * sT.T[1][a][c][b];
-        const V t0 = sT.T[0][a][b][c], t1 = sT.T[1][a][b][c];
-        const V uc0 = sU[2 * c][lane], uc1 = sU[2 * c + 1][lane];
-        Z[0][0] += uc0 * t0; Z[0][1] += uc1 * t0;
-        Z[1][0] += uc0 * t1; Z[1][1] += uc1 * t1;
+    V R[3][3];  // [i][j]: cc int phi_a psi_j u . grad l_i
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int j = 0; j < 3; ++j) {
+        V s = sA[r][0][lane] * sS[a][0][j];
+#pragma unroll
+        for(int c = 1; c < 6; ++c) s += sA[r][c][lane] * sS[a][c][j];
+        R[r + 1][j] = s;
       }
-      for(int m = 0; m < 2; ++m)
-        for(int n = 0; n < 2; ++n) {
-          V v = G[0][n] * Z[0][m] + G[1][n] * Z[1][m];
-          if(m == n) v += W;
-          A[m][2 * b + n] += cc * v;
-        }
+#pragma unroll
+    for(int j = 0; j < 3; ++j) R[0][j] = -(R[1][j] + R[2][j]);
+#pragma unroll
+    for(int i = 0; i < 3; ++i) {
+      W[i] = (V)4 * R[i][i] - (R[i][0] + R[i][1] + R[i][2]);
+      W[3 + i] = (V)4 * (R[(i + 1) % 3][i] + R[i][(i + 1) % 3]);
     }
+#pragma unroll
+    for(int v = 0; v < 3; ++v)
+#pragma unroll
+      for(int n = 0; n < 2; ++n)
+#pragma unroll
+        for(int m = 0; m < 2; ++m) g[v][n][m] = sG[v][n][m][lane];
   }
-  if(fc.hasSigma) {
+  const V cs = fc.hasSigma ? -(V)fc.sigma * (V)fc.mu * J : (V)0, cm = fc.hasMass ? (V)fc.mass * (V)c0 * J : (V)0;
+  V H[2][2];
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int k = 0; k < 2; ++k) H[r][k] = cs * G[r][k];
+#pragma unroll
+  for(int b = 0; b < 6; ++b) {
     // A_(a,m),(b,n) += -c mu [ delta_mn grad phi_a . grad phi_b + d_n phi_a d_m phi_b ]
     // (feVectorSysElm.cpp:1454-1492)
-    const V cs = -(V)fc.sigma * (V)fc.mu * J;
-    V GG[2][2][2][2];
-    for(int k = 0; k < 2; ++k)
-      for(int l = 0; l < 2; ++l)
-        for(int r = 0; r < 2; ++r)
-          for(int s2 = 0; s2 < 2; ++s2) GG[k][l][r][s2] = G[r][k] * G[s2][l];
-    for(int b = 0; b < 6; ++b) {
-      V S[2][2];
-      for(int k = 0; k < 2; ++k)
-        for(int l = 0; l < 2; ++l) {
-          V v = 0;
-          for(int r = 0; r < 2; ++r)
-            for(int s2 = 0; s2 < 2; ++s2) v += GG[k][l][r][s2] * sT.K[r][s2][a][b];
-          S[k][l] = v;
-        }
-      const V tr = S[0][0] + S[1][1];
-      for(int m = 0; m < 2; ++m)
-        for(int n = 0; n < 2; ++n) A[m][2 * b + n] += cs * ((m == n ? tr : (V)0) + S[n][m]);
+    V A[2][2] = {{0, 0}, {0, 0}}, d = W[b];  // A[m][n]; d: the delta_mn terms
+    if(fc.hasSigma) {
+#pragma unroll
+      for(int m = 0; m < 2; ++m) {
+        const V P0 = sK[0][0][a][b] * G[0][m] + sK[0][1][a][b] * G[1][m],
+                P1 = sK[1][0][a][b] * G[0][m] + sK[1][1][a][b] * G[1][m];
+#pragma unroll
+        for(int n = 0; n < 2; ++n) A[m][n] = H[0][n] * P0 + H[1][n] * P1;
+      }
+      d += A[0][0] + A[1][1];
     }
-  }
-  if(fc.hasMass) {
-    // A_(a,m),(b,n) += c c0 delta_mn phi_a phi_b   (feVectorSysElm.cpp:390-408)
-    const V cm = (V)fc.mass * (V)c0 * J;
-    for(int b = 0; b < 6; ++b) {
-      A[0][2 * b] += cm * sT.M[a][b];
-      A[1][2 * b + 1] += cm * sT.M[a][b];
-    }
+    // (feVectorSysElm.cpp:390-408)
+    if(fc.hasMass) d += cm * sM[a][b];
+    // A_(a,m),(b,n) += c [ delta_mn phi_a (u0 . grad phi_b) + phi_a phi_b d_n u0_m ]
+    // (vectorDotGradShapeDotShape + shapeDotTensorDotShape, feVectorSpace.cpp:202-290)
+    if(fc.hasConv)
+#pragma unroll
+      for(int v = 0; v < 3; ++v)
+#pragma unroll
+        for(int m = 0; m < 2; ++m)
+#pragma unroll
+          for(int n = 0; n < 2; ++n) A[m][n] += g[v][n][m] * sS[a][b][v];
+    A[0][0] += d;
+    A[1][1] += d;
+#pragma unroll
+    for(int m = 0; m < 2; ++m)
+#pragma unroll
+      for(int n = 0; n < 2; ++n) out[m * ldm + (int64_t)(2 * b + n) * ld] = A[m][n];
   }
   // Pressure columns of rows (a,m) and the column (a,m) of the pressure rows:
   // both are int psi_j d_m phi_a.
-  V Bp[2][3];
+  const V sj = (V)fc.sigma * J, dj = (V)fc.divu * J;
+#pragma unroll
   for(int m = 0; m < 2; ++m)
-    for(int j = 0; j < 3; ++j) Bp[m][j] = (G[0][m] * sT.D[0][j][a] + G[1][m] * sT.D[1][j][a]) * J;
-
-  // Stage the element's 216 structurally nonzero entries in shared memory
-  // (thread (e, a): rows 2a+m, velocity + pressure columns, and the
-  // pressure-row entries in columns 2a+m), then scatter them block-wide: consecutive
-  // threads take consecutive elements of one entry, so the map reads are
-  // coalesced and every thread keeps several read-modify-writes in flight.
-  // (two passes, one row component m at a time, to bound shared memory)
-#pragma unroll
-  for(int m = 0; m < 2; ++m) {
-    if(m) __syncthreads();
-#pragma unroll
-    for(int j = 0; j < 12; ++j) sAdd[a * 18 + j][lane] = A[m][j];
 #pragma unroll
     for(int j = 0; j < 3; ++j) {
-      sAdd[a * 18 + 12 + j][lane] = fc.hasSigma ? (V)fc.sigma * Bp[m][j] : (V)0;
-      sAdd[a * 18 + 15 + j][lane] = fc.hasDivu ? (V)fc.divu * Bp[m][j] : (V)0;
+      const V bp = G[0][m] * sD[0][j][a] + G[1][m] * sD[1][j][a];
+      if(fc.hasSigma) out[m * ldm + (int64_t)(12 + j) * ld] = sj * bp;
+      if(fc.hasDivu) out[m * ldm + (int64_t)(15 + j) * ld] = dj * bp;
     }
-    __syncthreads();
-    scatter_staged<V>(dm.map, nE, begin + (int64_t)blockIdx.x * EPB, end, fc.hasSigma, fc.hasDivu, m, sAdd,
-                      values);
+}
+
+// values += the entries of the elements [begin, end) of one color.  Within a
+// color every CSR entry receives at most one contribution, so the reduction
+// in L2 (no round trip to the SM) gives the bits of a read-modify-write.
+constexpr int JAC_BATCH = 6;
+template <typename V>
+__global__ void __launch_bounds__(256) k_jac_scatter(int64_t nE, const int32_t *__restrict__ map, int hasSigma,
+                                                    int hasDivu, const V *__restrict__ buf, int64_t ld, int64_t p0,
+                                                    int64_t begin, int64_t end, V *__restrict__ values)
+{
+  const int64_t p = begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if(p >= end) return;
+  int32_t pos[JAC_BATCH];
+  V add[JAC_BATCH];
+#pragma unroll
+  for(int t = 0; t < JAC_BATCH; ++t) {
+    const int e = (int)blockIdx.y * JAC_BATCH + t, m = e >= 108, k = m ? e - 108 : e, j = k % 18;
+    const bool on = j < 12 || (j < 15 ? hasSigma : hasDivu);
+    pos[t] = on ? __ldg(map + (int64_t)th_map_index(k, m) * nE + p) : -1;
+    add[t] = on ? buf[(int64_t)e * ld + p - p0] : (V)0;
   }
+#pragma unroll
+  for(int t = 0; t < JAC_BATCH; ++t)
+    if(pos[t] >= 0) atomicAdd(values + pos[t], add[t]);
 }
 
 int64_t nblocks(int64_t begin, int64_t end) { return (end - begin + EPB - 1) / EPB; }
@@ -608,24 +625,11 @@ void launch_pack_th_f32(const DeviceMesh &dm, const FormCoeffs &fc, const double
   (k_pack_th<float><<<pack_grid(dm.nElm), 256, 0, s>>>(dm, fc.hasConv, u, pack), ::feng::count_launch());
 }
 
-void launch_pack_th_f64(const DeviceMesh &dm, const FormCoeffs &fc, const double *u, double *pack, cudaStream_t s)
-{
-  (k_pack_th<double><<<pack_grid(dm.nElm), 256, 0, s>>>(dm, fc.hasConv, u, pack), ::feng::count_launch());
-}
-
 void launch_matrix_th_rows_f32(const RowAsm &ra, const FormCoeffs &fc, const RefTensors *dT, double c0,
                                float *values, int accumulate, cudaStream_t s)
 {
   if(ra.nBlocks < 1) return;
   (k_matrix_th_rows<float><<<ra.nBlocks, 256, ra.capBytes, s>>>(ra, fc, dT, c0, values, accumulate),
-   ::feng::count_launch());
-}
-
-void launch_matrix_th_rows_f64(const RowAsm &ra, const FormCoeffs &fc, const RefTensors *dT, double c0,
-                               double *values, int accumulate, cudaStream_t s)
-{
-  if(ra.nBlocks < 1) return;
-  (k_matrix_th_rows<double><<<ra.nBlocks, 256, ra.capBytes, s>>>(ra, fc, dT, c0, values, accumulate),
    ::feng::count_launch());
 }
 
@@ -644,28 +648,59 @@ void launch_assemble_residual(const DeviceMesh &dm, const FormCoeffs &fc, const 
   (k_residual_p2<<<nblocks(begin, end), block, 0, s>>>(dm, fc, dT, u, t, nInc, rhs, begin, end), ::feng::count_launch());
 }
 
-void launch_assemble_matrix_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                                const double *u, double c0, double *values, int64_t begin,
-                                int64_t end, cudaStream_t s)
+void launch_assemble_matrix_p2_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, double *values,
+                                   int64_t begin, int64_t end, cudaStream_t s)
 {
   if(end <= begin) return;
-  dim3 block(EPB, 6);
-  if(fc.elemType == 1)
-    (k_matrix_p2<double><<<nblocks(begin, end), block, 0, s>>>(dm, fc, dT, values, begin, end), ::feng::count_launch());
-  else
-    (k_matrix_th<double><<<nblocks(begin, end), block, 0, s>>>(dm, fc, dT, u, c0, values, begin, end), ::feng::count_launch());
+  (k_matrix_p2<double><<<nblocks(begin, end), dim3(EPB, 6), 0, s>>>(dm, fc, dT, values, begin, end),
+   ::feng::count_launch());
 }
 
-void launch_assemble_matrix_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                                const double *u, double c0, float *values, int64_t begin,
-                                int64_t end, cudaStream_t s)
+void launch_assemble_matrix_p2_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, float *values,
+                                   int64_t begin, int64_t end, cudaStream_t s)
 {
   if(end <= begin) return;
-  dim3 block(EPB, 6);
-  if(fc.elemType == 1)
-    (k_matrix_p2<float><<<nblocks(begin, end), block, 0, s>>>(dm, fc, dT, values, begin, end), ::feng::count_launch());
-  else
-    (k_matrix_th<float><<<nblocks(begin, end), block, 0, s>>>(dm, fc, dT, u, c0, values, begin, end), ::feng::count_launch());
+  (k_matrix_p2<float><<<nblocks(begin, end), dim3(EPB, 6), 0, s>>>(dm, fc, dT, values, begin, end),
+   ::feng::count_launch());
+}
+
+int64_t matrix_th_chunk(int64_t nElm) { return std::min<int64_t>(nElm, 1 << 18); }
+size_t matrix_th_buffer_bytes(int64_t nElm, int valueBytes)
+{
+  return (size_t)TH_ENT * (size_t)matrix_th_chunk(nElm) * valueBytes;
+}
+
+template <typename V>
+static void matrix_th(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, const double *u, double c0,
+                      V *buf, V *values, cudaStream_t s)
+{
+  const int64_t ch = matrix_th_chunk(dm.nElm);
+  int c = 0;
+  for(int64_t p0 = 0; p0 < dm.nElm; p0 += ch) {
+    const int64_t p1 = std::min(dm.nElm, p0 + ch);
+    (k_jac_th<V><<<(unsigned)nblocks(p0, p1), dim3(EPB, 6), 0, s>>>(dm, fc, dT, u, c0, buf, ch, p0, p1),
+     ::feng::count_launch());
+    for(int64_t b = p0; b < p1;) {
+      while(dm.colorOff[c + 1] <= b) ++c;
+      const int64_t e = std::min(p1, dm.colorOff[c + 1]);
+      (k_jac_scatter<V><<<dim3((unsigned)((e - b + 255) / 256), TH_ENT / JAC_BATCH), 256, 0, s>>>(
+           dm.nElm, dm.map, fc.hasSigma, fc.hasDivu, buf, ch, p0, b, e, values),
+       ::feng::count_launch());
+      b = e;
+    }
+  }
+}
+
+void launch_matrix_th_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, const double *u, double c0,
+                          double *buf, double *values, cudaStream_t s)
+{
+  matrix_th<double>(dm, fc, dT, u, c0, buf, values, s);
+}
+
+void launch_matrix_th_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, const double *u, double c0,
+                          float *buf, float *values, cudaStream_t s)
+{
+  matrix_th<float>(dm, fc, dT, u, c0, buf, values, s);
 }
 
 }  // namespace feng

@@ -67,6 +67,7 @@ struct RefTensors {
   double T[2][6][6][6];
   double D[2][3][6];
   double M[6][6];
+  double S[6][6][3];              // sum_q w phi_a phi_b psi_j
   int nq;
   double qw[16], qr[16], qs[16];  // the rule, for non-polynomial sources
   double phi[16][6];              // P2 functions at the nodes
@@ -163,13 +164,10 @@ void launch_matrix_tet_rows_f32(const RowAsmTet &ra, const FormCoeffs &fc, const
 
 // Per-element data of the row-owned assembly (RowAsm::pack), from u.
 void launch_pack_th_f32(const DeviceMesh &dm, const FormCoeffs &fc, const double *u, float *pack, cudaStream_t s);
-void launch_pack_th_f64(const DeviceMesh &dm, const FormCoeffs &fc, const double *u, double *pack, cudaStream_t s);
 // Row-owned Taylor-Hood Jacobian; accumulate = 0 overwrites the values
 // (the matrix was zeroed), 1 adds to them.
 void launch_matrix_th_rows_f32(const RowAsm &ra, const FormCoeffs &fc, const RefTensors *dT, double c0,
                                float *values, int accumulate, cudaStream_t s);
-void launch_matrix_th_rows_f64(const RowAsm &ra, const FormCoeffs &fc, const RefTensors *dT, double c0,
-                               double *values, int accumulate, cudaStream_t s);
 
 // Residual (FP64) of the scalar P2 forms on elements [begin,end) of the color
 // order, accumulated into rhs with feNG's sign (rhs = sum of element Be).
@@ -179,13 +177,19 @@ void launch_assemble_residual(const DeviceMesh &dm, const FormCoeffs &fc, const 
                               cudaStream_t s);
 // out[i] = (hi, lo) of x[i]: hi = x rounded to float, lo = the rest rounded.
 void launch_split_pairs(int64_t n, const double *x, float2 *out, cudaStream_t s);
-// Jacobian of the fused forms, in double or float.
-void launch_assemble_matrix_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                                const double *u, double c0, double *values, int64_t begin,
-                                int64_t end, cudaStream_t s);
-void launch_assemble_matrix_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT,
-                                const double *u, double c0, float *values, int64_t begin,
-                                int64_t end, cudaStream_t s);
+// Jacobian of the scalar P2 forms on elements [begin, end) of the color order.
+void launch_assemble_matrix_p2_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, double *values,
+                                   int64_t begin, int64_t end, cudaStream_t s);
+void launch_assemble_matrix_p2_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, float *values,
+                                   int64_t begin, int64_t end, cudaStream_t s);
+// Taylor-Hood Jacobian by element matrices, matrix_th_chunk(nElm) elements at
+// a time in buf (matrix_th_buffer_bytes), scattered a color at a time.
+int64_t matrix_th_chunk(int64_t nElm);
+size_t matrix_th_buffer_bytes(int64_t nElm, int valueBytes);
+void launch_matrix_th_f64(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, const double *u, double c0,
+                          double *buf, double *values, cudaStream_t s);
+void launch_matrix_th_f32(const DeviceMesh &dm, const FormCoeffs &fc, const RefTensors *dT, const double *u, double c0,
+                          float *buf, float *values, cudaStream_t s);
 
 // Tetrahedra (fe_assembly_tet.cu): residual (FP64) of the scalar P2 forms
 // (DIFFUSION + SOURCE) and Jacobian (FP64 or FP32) of the scalar P2 or the

@@ -174,7 +174,10 @@ void build_ref_tensors(const QuadRule &q, RefTensors &T)
       for(int j = 0; j < 3; ++j)
         for(int a = 0; a < 6; ++a) T.D[r][j][a] += w * psi[j] * d[r][a];
     for(int a = 0; a < 6; ++a)
-      for(int b = 0; b < 6; ++b) T.M[a][b] += w * phi[a] * phi[b];
+      for(int b = 0; b < 6; ++b) {
+        T.M[a][b] += w * phi[a] * phi[b];
+        for(int j = 0; j < 3; ++j) T.S[a][b][j] += w * phi[a] * phi[b] * psi[j];
+      }
   }
   // Is the rule exact to degree 5?  int_T r^i s^j = i! j! / (i + j + 2)!
   // on the reference triangle.
@@ -203,6 +206,7 @@ SystemCUDA::~SystemCUDA()
   cudaFree(ra_.blockUnits); cudaFree(ra_.unitRow); cudaFree(ra_.unitTwo); cudaFree(ra_.rowPtr); cudaFree(ra_.rowEnt);
   cudaFree(ra_.offs); cudaFree(ra_.pack);
   cudaFree(rat_.blockUnits); cudaFree(rat_.unitRow); cudaFree(rat_.unitKind); cudaFree(rat_.unitPtr);
+  cudaFree(jacBuf_);
   cudaFree(rat_.ent); cudaFree(rat_.offs); cudaFree(rat_.pack);
   cudaFree(dm_.geoPair); cudaFree(uPair_); cudaFree(udotPair_);
   if(ev0_) cudaEventDestroy(ev0_);
@@ -489,7 +493,9 @@ int SystemCUDA::init(const SystemTables &t, const FormDesc *forms, int nforms,
   ra_.ia = csr_.ia;
   rat_.ia = csr_.ia;
   if(useRowsTet_) CK(cudaMalloc(&rat_.pack, sizeof(float) * ROWTET_PACK * nE));
-  if(useRows_) CK(cudaMalloc(&ra_.pack, (opt.precision == 0 ? sizeof(double) : sizeof(float)) * ROWASM_PACK * nE));
+  if(useRows_) CK(cudaMalloc(&ra_.pack, sizeof(float) * ROWASM_PACK * nE));
+  if(t.elemType == ELEM_TAYLOR_HOOD && !useRows_)
+    CK(cudaMalloc(&jacBuf_, matrix_th_buffer_bytes(nE, opt.precision == 0 ? 8 : 4)));
   CK(cudaMalloc(&rhs_, sizeof(double) * nInc_));
   CK(cudaMalloc(&du_, sizeof(double) * nInc_));
   CK(cudaMalloc(&u_, sizeof(double) * nDofs_));
@@ -1063,8 +1069,9 @@ int SystemCUDA::build_row_assembly(const std::vector<int32_t> &adrP, const std::
   const int64_t nE = dm_.nElm;
   const int nl = nloc_;
   // FP32 Jacobians only: in FP64 the per-row recomputation of the shared
-  // element terms costs more on the FP64 pipe than the colored scatter
-  // (1.37 ms vs ~1.06 ms per Kovasznay 256 x 256 Jacobian)
+  // element terms costs more on the FP64 pipe than element matrices and a
+  // scatter (k_jac_th; by rows 1.37 ms per Kovasznay 256 x 256 Jacobian, by
+  // colors without the buffer 1.06)
   if(opt.precision != 1 || nl != 15 || nE >= (int64_t(1) << 27)) return FE_OK;
   for(int64_t r = 0; r < nInc_; ++r)
     if(pat_.ia[r + 1] - pat_.ia[r] >= 255) return FE_OK;  // offsets must fit a byte
@@ -1117,7 +1124,7 @@ int SystemCUDA::build_row_assembly(const std::vector<int32_t> &adrP, const std::
   }
   const int64_t nUnits = (int64_t)unitRow.size();
   unitRow.push_back((int32_t)nInc_);
-  const int vs = opt.precision == 0 ? 8 : 4;
+  const int vs = 4;
   const int cap = 40 * 1024 / vs;  // values per block in shared memory
   std::vector<int32_t> blockUnits{0};
   int64_t u0 = 0;
@@ -1284,13 +1291,8 @@ int SystemCUDA::launch_matrix()
   if(useRows_) {
     const int acc = zeroPending_ ? 0 : 1;
     zeroPending_ = false;
-    if(vals64_) {
-      launch_pack_th_f64(dm_, fc_, u_, (double *)ra_.pack, s_);
-      launch_matrix_th_rows_f64(ra_, fc_, dT_, c0_, vals64_, acc, s_);
-    } else {
-      launch_pack_th_f32(dm_, fc_, u_, (float *)ra_.pack, s_);
-      launch_matrix_th_rows_f32(ra_, fc_, dT_, c0_, vals32_, acc, s_);
-    }
+    launch_pack_th_f32(dm_, fc_, u_, (float *)ra_.pack, s_);
+    launch_matrix_th_rows_f32(ra_, fc_, dT_, c0_, vals32_, acc, s_);
     return FE_OK;
   }
   if(useRowsTet_) {
@@ -1310,13 +1312,14 @@ int SystemCUDA::launch_matrix()
     }
     return FE_OK;
   }
+  if(elemType_ == ELEM_TAYLOR_HOOD) {
+    if(vals64_) launch_matrix_th_f64(dm_, fc_, dT_, u_, c0_, (double *)jacBuf_, vals64_, s_);
+    else launch_matrix_th_f32(dm_, fc_, dT_, u_, c0_, (float *)jacBuf_, vals32_, s_);
+    return FE_OK;
+  }
   for(int c = 0; c < dm_.nColors; ++c) {
-    if(vals64_)
-      launch_assemble_matrix_f64(dm_, fc_, dT_, u_, c0_, vals64_, dm_.colorOff[c],
-                                 dm_.colorOff[c + 1], s_);
-    else
-      launch_assemble_matrix_f32(dm_, fc_, dT_, u_, c0_, vals32_, dm_.colorOff[c],
-                                 dm_.colorOff[c + 1], s_);
+    if(vals64_) launch_assemble_matrix_p2_f64(dm_, fc_, dT_, vals64_, dm_.colorOff[c], dm_.colorOff[c + 1], s_);
+    else launch_assemble_matrix_p2_f32(dm_, fc_, dT_, vals32_, dm_.colorOff[c], dm_.colorOff[c + 1], s_);
   }
   return FE_OK;
 }

@@ -171,6 +171,7 @@ class SystemCUDA {
   // than 255).
   RowAsm ra_;
   bool useRows_ = false;
+  void *jacBuf_ = nullptr;  // element matrices of the Taylor-Hood Jacobian otherwise
   // Row-owned FP32 Jacobian of tetrahedral Taylor-Hood systems.
   RowAsmTet rat_;
   bool useRowsTet_ = false;
