@@ -2,6 +2,7 @@
 #include "fe_ilu_stream.h"
 
 #include <algorithm>
+#include <cmath>
 
 #include "fe_common.h"
 #include "fe_launch.h"
@@ -20,53 +21,99 @@ namespace feng {
 namespace {
 
 constexpr int E = IluStream::E;
-constexpr int WORKERS = 256;       // threads that solve: 128 rows per step
-constexpr int THREADS = 512;       // the others copy the next steps' operands
+constexpr int WORKERS = 256;       // threads that solve
+constexpr int THREADS = WORKERS + 32;  // the last warp copies the coming steps' operands
 constexpr int STAGES = 3;
+constexpr int WARPS = WORKERS / 32;
+constexpr int LONG_ROW = 8;        // rows with more entries take LONG_SLOTS slots, the others two
+constexpr int LONG_SLOTS = 4;
+constexpr unsigned NO_ROW = 0xffffu;
 constexpr int MAX_STEPS = 4096;    // of one block (shared memory)
 constexpr size_t MAX_SMEM = 226 * 1024;
-enum : uint8_t { STEP_FIRST = 1, STEP_LAST = 2 };
+enum : uint8_t { STEP_FIRST = 1, STEP_LAST = 2, STEP_SCALE = 4 };
 
 // A step's operands in shared memory.
 template <typename V>
 struct Stage {
-  uint4 col[WORKERS];
+  uint4 col[WORKERS];  // 16 bits each: the E entries' local columns, then the row
   V val[E][WORKERS];
-  V scale[WORKERS];
-  int32_t row[WORKERS];
 };
 
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void *dst, const void *src)
+// A stage's barrier: one arrival and the bytes of its copies.
+__device__ __forceinline__ void bar_init(uint64_t *b)
 {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr(BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(b)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *b, unsigned bytes)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(b)),
+               "r"(bytes)
+               : "memory");
+}
+// False when the copies have not come (a few microseconds are usual).
+__device__ __forceinline__ bool bar_wait(uint64_t *b, unsigned parity)
+{
+  const unsigned a = (unsigned)__cvta_generic_to_shared(b);
+  for(int t = 0; t < 1 << 14; ++t) {
+    unsigned ok;
+    asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(a), "r"(parity)
+      : "memory");
+    if(ok) return true;
+  }
+  return false;
+}
+// Multiples of 16 bytes from and to 16-byte boundaries.
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, uint64_t *b)
+{
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                 (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(bytes), "r"((unsigned)__cvta_generic_to_shared(b))
+               : "memory");
 }
 
-// z = U^-1 L^-1 r on one diagonal block, z in shared memory.  Two slots
-// (neighbouring lanes) per row: the row's entries alternate between them, the
-// first starts from the row's right-hand side, and one exchange adds the two.
-// (More lanes per row would only queue at the FP64 pipe, which takes 64
-// cycles per warp; the rows of a step are sorted by length, so that a warp
-// runs no further than its own longest row.)  U's entries are scaled by the
-// inverse diagonal beforehand, so a row ends with an addition.  The upper
-// half of the threads copies the operands of the step after next while the
-// lower half solves; a block barrier ends every step.
-// Bound: the chain of levels (their products on one SM's FP64 pipe, an
-// exchange and a barrier).  64 x 64 P2 diffusion (16 k rows, 254 levels per
-// triangle): 0.42 ms per application against 3.75 ms with a warp per row and
-// the vector in global memory.
+// *p (shared memory) when on, without a branch (a conditional load in C++ is one, and branches
+// keep loads from overlapping).
+__device__ __forceinline__ void load_if(bool on, const float *p, float &v)
+{
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.shared.f32 %0, [%2];\n\t}"
+               : "+f"(v)
+               : "r"((unsigned)on), "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void load_if(bool on, const double *p, double &v)
+{
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.shared.f64 %0, [%2];\n\t}"
+               : "+d"(v)
+               : "r"((unsigned)on), "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+
+// z = U^-1 L^-1 r on one diagonal block, z in shared memory.  A row's entries
+// are dealt to two or four slots (neighbouring lanes; a warp holds rows of one
+// kind, of similar length), and the last slot starts from the row's right-hand
+// side.  The FP64 pipe takes 64 cycles per warp instruction and a dependent one
+// waits 110: two slots end rows of up to four products each soonest, four the
+// longer ones, more only queue (eight: 0.46 ms where four took 0.37, all rows
+// in four likewise).  Between the triangles the vector is scaled by U's inverse
+// diagonal, as U's entries are beforehand, so a row ends with additions.
+// One warp brings the operands of the steps ahead by bulk copies and waits for
+// them; the others take the next step's into registers before the barrier that
+// ends a step, with the right-hand sides, which no step but the row's own
+// writes.
+// Bound: the chain of levels (FP64 products and exchanges, about 700 cycles;
+// gathers, the next step's operands and the barrier, as many).  64 x 64 P2
+// diffusion (16 k rows, 254 levels per triangle): 0.34 ms per application; six
+// products in a chain and copies by half of the threads 0.42, a warp per row
+// and the vector in global memory 3.75.
 template <typename V>
 __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *__restrict__ steps,
                                                         const int32_t *__restrict__ stepStart,
                                                         const int32_t *__restrict__ start,
                                                         const int32_t *__restrict__ perm,
                                                         const uint4 *__restrict__ col, const V *__restrict__ val,
-                                                        const int32_t *__restrict__ row, const V *__restrict__ scale,
-                                                        const V *__restrict__ r, V *__restrict__ z,
+                                                        const V *__restrict__ scale, const V *__restrict__ r,
+                                                        V *__restrict__ z,
                                                         const int *__restrict__ done)
 {
   FE_PDL_ENTRY();
@@ -79,6 +126,13 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
   V *x = reinterpret_cast<V *>(smem + STAGES * sizeof(Stage<V>));
   IluStream::Step *st = reinterpret_cast<IluStream::Step *>(
       smem + STAGES * sizeof(Stage<V>) + (((size_t)n * sizeof(V) + 15) & ~(size_t)15));
+  __shared__ uint64_t full[STAGES];
+  __shared__ int late;  // a copy that did not come
+  if(tid == 0) {
+    late = 0;
+    for(int k = 0; k < STAGES; ++k) bar_init(full + k);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   for(int i = tid; i < ns; i += THREADS) st[i] = steps[s0 + i];
   for(int i0 = tid; i0 < n; i0 += 8 * THREADS) {
     V t[8];
@@ -89,74 +143,113 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
       if(i0 + u * THREADS < n) x[i0 + u * THREADS] = t[u];
   }
   __syncthreads();
-  // the copying threads: one commit group per step, empty past the end
-  const int h = tid - WORKERS;
+  const int warp = tid >> 5, lane = tid & 31;
+  // the copying warp: lane k < E brings the warps' entries k, lane E the columns
   auto copy = [&](int q) {
-    if(q < ns) {
-      const IluStream::Step s = st[q];
-      Stage<V> &g = stage[q % STAGES];
-      int64_t e = s.entry;
+    if(q >= ns) return;
+    const IluStream::Step s = st[q];
+    Stage<V> &g = stage[q % STAGES];
+    const int pre = lane <= E ? lane : E;
+    int before = 0, own = 0;  // warps with an entry j < pre, with entry lane
 #pragma unroll
-      for(int k = 0; k < E; ++k) {
-        if(h < 32 * s.groups[k]) copy_async<sizeof(V)>(&g.val[k][h], val + e + h);
-        e += 32 * s.groups[k];
-      }
-      if(h < s.n) {
-        copy_async<16>(&g.col[h], col + s.slot + h);
-        copy_async<sizeof(V)>(&g.scale[h], scale + s.slot + h);
-        copy_async<4>(&g.row[h], row + s.slot + h);
-      }
+    for(int w = 0; w < WARPS; ++w) {
+      const int chain = (s.chains >> (4 * w)) & 15;
+      before += min(chain, pre);
+      own += chain > lane;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    const void *src = val + s.entry + 32 * before;
+    void *dst = &g.val[lane < E ? lane : 0][0];
+    unsigned bytes = lane < E ? 32u * own * (unsigned)sizeof(V) : 0u;
+    if(lane == E) {
+      src = col + s.slot;
+      dst = &g.col[0];
+      bytes = 32u * s.warps * 16u;
+    }
+    const unsigned all = __reduce_add_sync(0xffffffffu, bytes);
+    if(lane == 0) bar_expect(full + q % STAGES, all);
+    __syncwarp();
+    if(bytes) bulk_copy(dst, src, bytes, full + q % STAGES);
   };
-  if(h >= 0) {
+  // until step q's operands are there; the barrier that follows tells the others
+  auto arrived = [&](int q) {
+    if(q < ns && !late && !bar_wait(full + q % STAGES, (unsigned)(q / STAGES) & 1u)) late = 1;
+  };
+  // the solving threads: the next step's operands, and what the slot starts from
+  uint4 c4 = make_uint4(0, 0, 0, 0);
+  V v[E], acc = 0, rhs = 0;
+  IluStream::Step s = {}, ahead = st[0];
+  auto fetch = [&](int q) {
+    s = ahead;
+    if(q >= ns) s.warps = s.flags = 0;
+    if(q + 1 < ns) ahead = st[q + 1];
+    if(warp >= s.warps) return;
+    const Stage<V> &g = stage[q % STAGES];
+    c4 = g.col[tid];
 #pragma unroll
-    for(int q = 0; q < STAGES - 1; ++q) copy(q);
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    for(int k = 0; k < E; ++k) load_if(k < (int)((s.chains >> (4 * warp)) & 15), &g.val[k][tid], v[k]);
+    const unsigned row = c4.w >> 16;
+    const int last = (s.wide >> warp) & 1 ? LONG_SLOTS - 1 : 1;
+    const V own = x[row != NO_ROW ? row : 0];
+    rhs = (tid & last) == last ? own : (V)0;
+  };
+  if(warp == WARPS) {
+#pragma unroll
+    for(int q = 0; q < STAGES; ++q) copy(q);
+    arrived(0);
+    arrived(1);
   }
   __syncthreads();
-  V acc = 0;
+  if(warp < WARPS) fetch(0);
+  __syncthreads();
   for(int q = 0; q < ns; ++q) {
-    if(h >= 0) {
-      // into the stage that the last step has left
-      copy(q + STAGES - 1);
-      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    } else {
-      const IluStream::Step &s = st[q];
-      if((tid & ~31) < s.n) {  // whole warps take part in the exchange
-        const Stage<V> &g = stage[q % STAGES];
-        const bool live = tid < s.n;
-        const int row = live ? g.row[tid] : 0;
-        const uint4 c4 = live ? g.col[tid] : make_uint4(0, 0, 0, 0);
-        if(s.flags & STEP_FIRST) acc = live && !(tid & 1) ? x[row] * g.scale[tid] : (V)0;
-        const unsigned cw[4] = {c4.x, c4.y, c4.z, c4.w};
-        V xv[E], v[E];
+    if(warp == WARPS) {
+      copy(q + STAGES);  // into the stage of this step, whose operands are in registers
+      arrived(q + 2);
+    } else if(warp < s.warps) {
+      const unsigned cw[4] = {c4.x, c4.y, c4.z, c4.w};
+      const unsigned row = c4.w >> 16;
+      const int chain = (s.chains >> (4 * warp)) & 15;
+      const bool wide = (s.wide >> warp) & 1, end = s.flags & STEP_LAST;
+      V xv[E];
 #pragma unroll
-        for(int k = 0; k < E; ++k) {
-          const bool on = (tid >> 5) < s.groups[k];
-          v[k] = on ? g.val[k][tid] : (V)0;
-          xv[k] = on ? x[(cw[k >> 1] >> (16 * (k & 1))) & 0xffffu] : (V)0;
-        }
+      for(int k = 0; k < E; ++k) load_if(k < chain, x + ((cw[k >> 1] >> (16 * (k & 1))) & 0xffffu), xv[k]);
+      if(s.flags & STEP_FIRST) acc = rhs;
 #pragma unroll
-        for(int k = 0; k < E; ++k)
-          if((tid >> 5) < s.groups[k]) acc -= v[k] * xv[k];
-        if(s.flags & STEP_LAST) {
-          const V other = __shfl_xor_sync(0xffffffffu, acc, 1);
-          if(live && !(tid & 1)) x[row] = acc + other;
-        }
+      for(int k = 0; k < E; ++k)
+        if(k < chain) acc -= v[k] * xv[k];
+      fetch(q + 1);
+      if(end) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        if(wide)
+#pragma unroll
+          for(int o = 2; o < LONG_SLOTS; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if(row != NO_ROW && !(tid & (wide ? LONG_SLOTS - 1 : 1))) x[row] = acc;
       }
+    } else {
+      if(s.flags & STEP_SCALE) {
+#pragma unroll 8
+        for(int i = tid; i < n; i += WORKERS) x[i] *= scale[p0 + i];
+        // the next step takes right-hand sides that others have scaled
+        asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");
+      }
+      fetch(q + 1);
     }
     __syncthreads();
+  }
+  if(late) {  // no result: the caller sees that it is not finite
+    for(int q = max(0, ns - STAGES); q < ns; ++q) bar_wait(full + q % STAGES, (unsigned)(q / STAGES) & 1u);
+    for(int i = tid; i < n; i += THREADS) z[perm[p0 + i]] = (V)NAN;
+    return;
   }
   for(int i = tid; i < n; i += THREADS) z[perm[p0 + i]] = x[i];
 }
 
 // The packed values: L as it is, U divided by its row's diagonal, and the
-// slots' scales (1 / diagonal for the first slot of a U row).
+// inverse diagonal by row.
 template <typename V>
 __global__ void k_ilu_pack(int64_t ne, const int32_t *__restrict__ pos, const int32_t *__restrict__ dpos,
-                           const V *__restrict__ f, V *__restrict__ val, int64_t nslots,
-                           const int32_t *__restrict__ slotDiag, V *__restrict__ scale)
+                           const V *__restrict__ f, V *__restrict__ val, int64_t nrows,
+                           const int32_t *__restrict__ rowDiag, V *__restrict__ scale)
 {
   FE_PDL_ENTRY();
   for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
@@ -164,8 +257,8 @@ __global__ void k_ilu_pack(int64_t ne, const int32_t *__restrict__ pos, const in
     if(pos[e] >= 0 && dpos[e] >= 0) v /= f[dpos[e]];
     val[e] = v;
   }
-  for(int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nslots; q += (int64_t)gridDim.x * blockDim.x)
-    scale[q] = slotDiag[q] >= 0 ? (V)1 / f[slotDiag[q]] : (V)1;
+  for(int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nrows; q += (int64_t)gridDim.x * blockDim.x)
+    scale[q] = (V)1 / f[rowDiag[q]];
 }
 
 template <typename T>
@@ -182,7 +275,7 @@ IluStream::~IluStream()
 {
   cudaFree(steps_); cudaFree(stepStart_); cudaFree(start_); cudaFree(perm_);
   cudaFree(col_); cudaFree(pos_); cudaFree(dpos_); cudaFree(val_);
-  cudaFree(row_); cudaFree(slotDiag_); cudaFree(scale_);
+  cudaFree(rowDiag_); cudaFree(scale_);
 }
 
 int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t> &lja,
@@ -197,17 +290,20 @@ int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t>
   const int64_t n = (int64_t)perm.size();
   for(int64_t b = 0; b < nBlocks_; ++b) {
     const int64_t rows = start[b + 1] - start[b];
-    if(rows > 65535 || stages + rows * vs > MAX_SMEM) return FE_OK;  // the level kernels
+    if(rows >= (int64_t)NO_ROW || stages + rows * vs > MAX_SMEM) return FE_OK;  // the level kernels
   }
-  std::vector<int32_t> local(n);
-  for(int64_t b = 0; b < nBlocks_; ++b)
-    for(int32_t q = start[b]; q < start[b + 1]; ++q) local[perm[q]] = q - start[b];
-
+  // the vector's order: a block's rows by levels of L, so that the rows of a
+  // warp read neighbouring entries (fewer bank conflicts)
+  std::vector<int32_t> local(n), order(n);
   std::vector<Step> steps;
-  std::vector<int32_t> stepStart(1, 0), pos, dpos, slotDiag, level(n, 0);
-  std::vector<int32_t> row;
+  std::vector<int32_t> stepStart(1, 0), pos, dpos, rowDiag(n), level(n, 0);
   std::vector<uint4> col;
   std::vector<int32_t> cnt, ord;
+  // a warp of a level: rows ord[first] .. ord[first + rows - 1], `slots` each
+  struct Warp {
+    int32_t first, rows, slots, chain;
+  };
+  std::vector<Warp> warps;
   for(int64_t b = 0; b < nBlocks_; ++b) {
     const int32_t p0 = start[b], p1 = start[b + 1];
     for(int lower = 1; lower >= 0; --lower) {
@@ -229,52 +325,79 @@ int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t>
         std::vector<int32_t> fill(cnt.begin(), cnt.end() - 1);
         for(int32_t q = p0; q < p1; ++q) ord[fill[level[perm[q]]]++] = perm[q];
       }
-      for(int32_t l = 0; l < nl; ++l) {
-        // rows of similar length together
-        auto len = [&](int32_t i) { return lower ? ldiag[i] - lia[i] : lia[i + 1] - ldiag[i] - 1; };
+      auto len = [&](int32_t i) { return lower ? ldiag[i] - lia[i] : lia[i + 1] - ldiag[i] - 1; };
+      for(int32_t l = 0; l < nl; ++l)  // rows of similar length together
         std::stable_sort(ord.begin() + cnt[l], ord.begin() + cnt[l + 1],
                          [&](int32_t x, int32_t y) { return len(x) > len(y); });
-        for(int32_t r0 = cnt[l]; r0 < cnt[l + 1]; r0 += WORKERS / 2) {
-          const int32_t nr = std::min<int32_t>(WORKERS / 2, cnt[l + 1] - r0);
-          const int per = (len(ord[r0]) + 1) / 2;  // entries per slot of the longest row
-          const int chunks = std::max(1, (per + E - 1) / E);
+      if(lower)
+        for(int32_t q = 0; q < p1 - p0; ++q) {
+          order[p0 + q] = ord[q];
+          local[ord[q]] = q;
+          rowDiag[p0 + q] = ldiag[ord[q]];
+        }
+      for(int32_t l = 0; l < nl; ++l) {
+        warps.clear();
+        for(int32_t r0 = cnt[l]; r0 < cnt[l + 1];) {
+          const int slots = len(ord[r0]) > LONG_ROW ? LONG_SLOTS : 2;
+          int32_t r1 = r0 + 1;
+          while(r1 < cnt[l + 1] && r1 - r0 < 32 / slots && (slots == 2 || len(ord[r1]) > LONG_ROW)) ++r1;
+          warps.push_back({r0, r1 - r0, slots, (len(ord[r0]) + slots - 1) / slots});
+          r0 = r1;
+        }
+        std::stable_sort(warps.begin(), warps.end(), [](const Warp &x, const Warp &y) { return x.chain > y.chain; });
+        for(size_t w0 = 0; w0 < warps.size(); w0 += WARPS) {
+          const int nw = (int)std::min<size_t>(WARPS, warps.size() - w0);
+          const int chunks = std::max(1, (warps[w0].chain + E - 1) / E);
           for(int c = 0; c < chunks; ++c) {
             Step st = {};
             st.entry = (int32_t)pos.size();
-            st.slot = (int32_t)row.size();
-            st.n = (uint16_t)(2 * nr);
+            st.slot = (int32_t)col.size();
+            st.warps = (uint8_t)nw;
             st.flags = (uint8_t)((c == 0 ? STEP_FIRST : 0) | (c + 1 == chunks ? STEP_LAST : 0));
+            for(int w = 0; w < nw; ++w)
+              if(warps[w0 + w].slots != 2) st.wide |= (uint8_t)(1u << w);
+            // row, first entry and end of lane t of warp w (row -1: none)
+            auto lane = [&](int w, int t, int32_t &i, int32_t &e, int32_t &end, int &slots) {
+              const Warp &W = warps[w0 + w];
+              slots = W.slots;
+              i = t / slots < W.rows ? ord[W.first + t / slots] : -1;
+              e = i < 0 ? 0 : (lower ? lia[i] : ldiag[i] + 1) + slots * c * E + t % slots;
+              end = i < 0 ? 0 : (lower ? ldiag[i] : lia[i + 1]);
+            };
+            for(int w = 0; w < nw; ++w)
+              st.chains |= (uint32_t)std::max(0, std::min<int>(E, warps[w0 + w].chain - c * E)) << (4 * w);
             for(int k = 0; k < E; ++k) {
-              // slots that hold an entry k: the leading ones, in whole warps
-              int32_t m = 0;
-              while(m < nr && len(ord[r0 + m]) > 2 * (c * E + k)) ++m;
-              st.groups[k] = (uint8_t)((2 * m + 31) / 32);
-              for(int32_t t = 0; t < 32 * st.groups[k]; ++t) {
-                const int32_t q = t / 2;
-                const int32_t i = q < nr ? ord[r0 + q] : -1;
-                const int32_t e = i < 0 ? 0 : (lower ? lia[i] : ldiag[i] + 1) + 2 * (c * E + k) + (t & 1);
-                const bool ok = i >= 0 && e < (lower ? ldiag[i] : lia[i + 1]);
-                pos.push_back(ok ? e : -1);
+              int g = 0;
+              while(g < nw && warps[w0 + g].chain > c * E + k) ++g;
+              for(int t = 0; t < 32 * g; ++t) {
+                int32_t i, e, end;
+                int slots;
+                lane(t / 32, t % 32, i, e, end, slots);
+                const bool ok = i >= 0 && e + slots * k < end;
+                pos.push_back(ok ? e + slots * k : -1);
                 dpos.push_back(ok && !lower ? ldiag[i] : -1);
               }
             }
-            for(int32_t q = 0; q < nr; ++q)
-              for(int h = 0; h < 2; ++h) {
-                const int32_t i = ord[r0 + q];
-                row.push_back(local[i]);
-                slotDiag.push_back(!lower && h == 0 ? ldiag[i] : -1);
-                uint32_t w[4] = {0, 0, 0, 0};
-                for(int k = 0; k < E; ++k) {
-                  const int32_t e = (lower ? lia[i] : ldiag[i] + 1) + 2 * (c * E + k) + h;
-                  // padding (value 0) reads the row's own entry of the vector
-                  const int32_t j = e < (lower ? ldiag[i] : lia[i + 1]) ? local[lja[e]] : local[i];
-                  w[k >> 1] |= (uint32_t)j << (16 * (k & 1));
-                }
-                col.push_back(make_uint4(w[0], w[1], w[2], w[3]));
+            for(int t = 0; t < 32 * nw; ++t) {
+              int32_t i, e, end;
+              int slots;
+              lane(t / 32, t % 32, i, e, end, slots);
+              uint32_t w[4] = {0, 0, 0, (i >= 0 ? (uint32_t)local[i] : NO_ROW) << 16};
+              for(int k = 0; k < E && i >= 0; ++k) {
+                // padding (value 0) reads the row's own entry of the vector
+                const int32_t j = e + slots * k < end ? local[lja[e + slots * k]] : local[i];
+                w[k >> 1] |= (uint32_t)j << (16 * (k & 1));
               }
+              col.push_back(make_uint4(w[0], w[1], w[2], w[3]));
+            }
             steps.push_back(st);
           }
         }
+      }
+      // between the triangles a step without rows, which scales the vector
+      if(lower) {
+        steps.push_back(Step{});
+        steps.back().flags = STEP_SCALE;
       }
     }
     stepStart.push_back((int32_t)steps.size());
@@ -284,18 +407,17 @@ int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t>
     smem_ = std::max(smem_, need);
   }
   nEntries_ = (int64_t)pos.size();
-  nSlots_ = (int64_t)row.size();
+  nRows_ = n;
   FE_TRY(to_device(&steps_, steps));
   FE_TRY(to_device(&stepStart_, stepStart));
   FE_TRY(to_device(&start_, start));
-  FE_TRY(to_device(&perm_, perm));
+  FE_TRY(to_device(&perm_, order));
   FE_TRY(to_device(&col_, col));
   FE_TRY(to_device(&pos_, pos));
   FE_TRY(to_device(&dpos_, dpos));
-  FE_TRY(to_device(&row_, row));
-  FE_TRY(to_device(&slotDiag_, slotDiag));
+  FE_TRY(to_device(&rowDiag_, rowDiag));
   CKI(cudaMalloc(&val_, vs * std::max<int64_t>(1, nEntries_)));
-  CKI(cudaMalloc(&scale_, vs * std::max<int64_t>(1, nSlots_)));
+  CKI(cudaMalloc(&scale_, vs * std::max<int64_t>(1, nRows_)));
   // the copies ran on the legacy stream, with which s is not ordered
   CKI(cudaStreamSynchronize(cudaStreamLegacy));
   if(fp32) CKI(cudaFuncSetAttribute(k_ilu_stream<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
@@ -308,18 +430,18 @@ void IluStream::gather(const void *f)
 {
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>((nEntries_ + 255) / 256, 4096));
   if(fp32_)
-    ::feng::launch_k(k_ilu_pack<float>, g, 256, 0, s_, nEntries_, pos_, dpos_, (const float *)f, (float *)val_, nSlots_,
-                     slotDiag_, (float *)scale_);
+    ::feng::launch_k(k_ilu_pack<float>, g, 256, 0, s_, nEntries_, pos_, dpos_, (const float *)f, (float *)val_, nRows_,
+                     rowDiag_, (float *)scale_);
   else
     ::feng::launch_k(k_ilu_pack<double>, g, 256, 0, s_, nEntries_, pos_, dpos_, (const double *)f, (double *)val_,
-                     nSlots_, slotDiag_, (double *)scale_);
+                     nRows_, rowDiag_, (double *)scale_);
 }
 
 template <typename V>
 void IluStream::launch(const V *r, V *z, const int *done) const
 {
   ::feng::launch_k(k_ilu_stream<V>, (int)nBlocks_, THREADS, smem_, s_, steps_, stepStart_, start_, perm_, col_,
-                   (const V *)val_, row_, (const V *)scale_, r, z, done);
+                   (const V *)val_, (const V *)scale_, r, z, done);
 }
 
 void IluStream::solve(const float *r, float *z, const int *done) const { launch<float>(r, z, done); }

@@ -1,8 +1,8 @@
 // Triangular solves of the block-Jacobi ILU(0) with the vector in shared
 // memory: one thread block per diagonal block, whose levels follow one
 // another with a block barrier between them, and the factor's entries packed
-// in the order in which the solve uses them, so that half of the threads copy
-// them into shared memory ahead of the dependences.
+// in the order in which the solve uses them, so that one warp copies them into
+// shared memory ahead of the dependences.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -30,35 +30,36 @@ class IluStream {
   void solve(const float *r, float *z, const int *done) const;
   void solve(const double *r, double *z, const int *done) const;
 
-  // One step of a block's stream: n slots (two per row), the longest first;
-  // entry k exists for the first 32 groups[k] slots (padded with zeros) and
-  // lies at entry + 32 (groups[0] + ... + groups[k - 1]) + slot.
-  static constexpr int E = 6;  // entries of a slot per step
+  // One step of a block's stream: `warps` warps of slots, the longest chains
+  // first; warp w holds rows of eight slots where bit w of wide is set, else of
+  // two, and in nibble w of chains the entries of its longest slot (the others
+  // padded with zeros).  Entry k of the warps that have one: from entry + 32
+  // (the warps with an entry 0, .. k - 1) on.
+  static constexpr int E = 5;  // entries of a slot per step
   struct Step {
     int32_t entry;      // first entry
-    int32_t slot;       // first slot (columns, row and scale arrays)
-    uint16_t n;         // slots
+    int32_t slot;       // first slot (columns)
+    uint32_t chains;
+    uint8_t warps, wide;
     uint8_t flags;      // STEP_*
-    uint8_t groups[E];  // warps that hold entry k
-    uint8_t pad[3];
+    uint8_t pad;
   };
 
  private:
   template <typename V> void launch(const V *r, V *z, const int *done) const;
   cudaStream_t s_ = 0;
   bool usable_ = false, fp32_ = false;
-  int64_t nBlocks_ = 0, nEntries_ = 0, nSlots_ = 0;
+  int64_t nBlocks_ = 0, nEntries_ = 0, nRows_ = 0;
   size_t smem_ = 0;
   Step *steps_ = nullptr;          // all blocks' steps
   int32_t *stepStart_ = nullptr;   // [nBlocks + 1]
   int32_t *start_ = nullptr, *perm_ = nullptr;
-  uint4 *col_ = nullptr;           // [slots] local indices of its E entries (16 bits each)
+  uint4 *col_ = nullptr;           // [slots] local indices of its E entries and its row (16 bits each)
   int32_t *pos_ = nullptr;         // [entries] position in the factor, -1: none
   int32_t *dpos_ = nullptr;        // [entries] position of the row's diagonal (U), -1 (L)
   void *val_ = nullptr;            // [entries]
-  int32_t *row_ = nullptr;         // [slots] local row
-  int32_t *slotDiag_ = nullptr;    // [slots] position of the row's diagonal (U, first slot), -1: scale 1
-  void *scale_ = nullptr;          // [slots]
+  int32_t *rowDiag_ = nullptr;     // [rows, as perm] position of the diagonal
+  void *scale_ = nullptr;          // [rows, as perm] inverse diagonal of U
 };
 
 }  // namespace feng
