@@ -305,9 +305,11 @@ __global__ void __launch_bounds__(256) k_cheb_first(int64_t n, const int32_t *__
 // of UNR entries, software-pipelined: the next step's columns and values are
 // loaded before this step's gathers, so a step waits for one memory latency
 // instead of two.
-template <int UNR, typename V, typename F>
-__device__ __forceinline__ void sell_walk(int32_t base, int32_t len, int lane, const int32_t *__restrict__ sc,
-                                          const V *__restrict__ sv, F &&f)
+// enter: called once the first step's columns and values are on their way
+// (early_entry); true ends the walk.
+template <int UNR, typename V, typename F, typename R>
+__device__ __forceinline__ bool sell_walk(int32_t base, int32_t len, int lane, const int32_t *__restrict__ sc,
+                                          const V *__restrict__ sv, F &&f, R &&enter)
 {
   int32_t c[UNR];
   V a[UNR];
@@ -318,6 +320,7 @@ __device__ __forceinline__ void sell_walk(int32_t base, int32_t len, int lane, c
     c[u] = ok ? __ldcs(sc + e) : -1;
     a[u] = ok ? __ldcs(sv + e) : (V)0;
   }
+  if(enter()) return false;
   for(int32_t k = 0; k < len; k += UNR) {
     int32_t cn[UNR];
     V an[UNR];
@@ -337,6 +340,23 @@ __device__ __forceinline__ void sell_walk(int32_t base, int32_t len, int lane, c
       a[u] = an[u];
     }
   }
+  return true;
+}
+template <int UNR, typename V, typename F>
+__device__ __forceinline__ void sell_walk(int32_t base, int32_t len, int lane, const int32_t *__restrict__ sc,
+                                          const V *__restrict__ sv, F &&f)
+{
+  sell_walk<UNR, V>(base, len, lane, sc, sv, f, [] { return false; });
+}
+
+// A kernel of an iteration (skip non-null: the kernel before it has not
+// written the operator) enters after its first operator loads, others at once.
+// True: the iteration has ended.
+__device__ __forceinline__ bool early_entry(const int *skip)
+{
+  if(!skip) return false;
+  FE_PDL_ENTRY();
+  return *skip != 0;
 }
 
 // k_cheb_first on the sliced-ELL copy of A: thread = row, both components.
@@ -406,9 +426,9 @@ __device__ __forceinline__ void lane_sum(int sub, int lanes, V (&acc)[NV])
 // read again by every cycle stay in the L2) and no such prefetch (most rows
 // take one step: 5.2 us against 5.8 us per pass over 28.6 k rows).
 template <typename V, int NV, bool FINE>
-__device__ __forceinline__ void row_part(int32_t beg, int32_t end, int sub, int lanes,
+__device__ __forceinline__ bool row_part(int32_t beg, int32_t end, int sub, int lanes,
                                          const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                         const V *__restrict__ x, V (&acc)[NV])
+                                         const V *x, V (&acc)[NV], const int *skip)
 {
   constexpr int UNR = 4;
   int32_t j[UNR];
@@ -433,9 +453,11 @@ __device__ __forceinline__ void row_part(int32_t beg, int32_t end, int sub, int 
   };
 #pragma unroll
   for(int c = 0; c < NV; ++c) acc[c] = 0;
+  int32_t k0 = beg + sub;
+  load(k0);
+  if(early_entry(skip)) return false;
   if constexpr(FINE) {
-    load(beg + sub);
-    for(int32_t k0 = beg + sub; k0 < end; k0 += lanes * UNR) {
+    for(; k0 < end; k0 += lanes * UNR) {
       int32_t jc[UNR];
       V ac[UNR];
 #pragma unroll
@@ -447,11 +469,13 @@ __device__ __forceinline__ void row_part(int32_t beg, int32_t end, int sub, int 
       use(jc, ac);
     }
   } else {
-    for(int32_t k0 = beg + sub; k0 < end; k0 += lanes * UNR) {
-      load(k0);
+    while(k0 < end) {
       use(j, av);
+      k0 += lanes * UNR;
+      if(k0 < end) load(k0);
     }
   }
+  return true;
 }
 
 // The component a lane writes after lane_sum, and its total; -1: none.
@@ -483,18 +507,16 @@ __global__ void __launch_bounds__(256) k_down(int lr, int lt, int64_t nc, const 
                                               const int32_t *__restrict__ rja, const V *__restrict__ ra, int64_t n,
                                               const int32_t *__restrict__ tia, const int32_t *__restrict__ tja,
                                               const V *__restrict__ ta, const int32_t *__restrict__ trow,
-                                              const V *__restrict__ b, V *__restrict__ bc, V *__restrict__ s,
-                                              const int *__restrict__ skip)
+                                              const V *b, V *__restrict__ bc, V *__restrict__ s, const int *skip)
 {
-  FE_PDL_ENTRY();
-  if(skip && *skip) return;
+  if(!skip) FE_PDL_ENTRY();
   const int64_t rBlocks = (nc * lr + 255) / 256;
   if((int64_t)blockIdx.x < rBlocks) {
     const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / lr;
     const int sub = threadIdx.x & (lr - 1);
     const bool live = row < nc;
     V acc[NV], v;
-    row_part<V, NV, SELL>(live ? ria[row] : 0, live ? ria[row + 1] : 0, sub, lr, rja, ra, b, acc);
+    if(!row_part<V, NV, SELL>(live ? ria[row] : 0, live ? ria[row + 1] : 0, sub, lr, rja, ra, b, acc, skip)) return;
     lane_sum<V, NV>(sub, lr, acc);
     const int c = lane_out<V, NV>(sub, acc, v);
     if(live && c >= 0) bc[row * NV + c] = v;
@@ -508,11 +530,15 @@ __global__ void __launch_bounds__(256) k_down(int lr, int lt, int64_t nc, const 
     V acc[NV];
 #pragma unroll
     for(int c = 0; c < NV; ++c) acc[c] = 0;
-    sell_walk<8, V>(base, len, (int)(t & 31), tja, ta, [&](int32_t j, V a) {
-      const Vals<V, NV> bv = ldv<V, NV>(b, j);
+    if(!sell_walk<8, V>(
+         base, len, (int)(t & 31), tja, ta,
+         [&](int32_t j, V a) {
+           const Vals<V, NV> bv = ldv<V, NV>(b, j);
 #pragma unroll
-      for(int c = 0; c < NV; ++c) acc[c] += a * bv.v[c];
-    });
+           for(int c = 0; c < NV; ++c) acc[c] += a * bv.v[c];
+         },
+         [&] { return early_entry(skip); }))
+      return;
 #pragma unroll
     for(int c = 0; c < NV; ++c) s[(int64_t)trow[t] * NV + c] = acc[c];
   } else {
@@ -520,7 +546,7 @@ __global__ void __launch_bounds__(256) k_down(int lr, int lt, int64_t nc, const 
     const int sub = threadIdx.x & (lt - 1);
     const bool live = row < n;
     V acc[NV], v;
-    row_part<V, NV, false>(live ? tia[row] : 0, live ? tia[row + 1] : 0, sub, lt, tja, ta, b, acc);
+    if(!row_part<V, NV, false>(live ? tia[row] : 0, live ? tia[row + 1] : 0, sub, lt, tja, ta, b, acc, skip)) return;
     lane_sum<V, NV>(sub, lt, acc);
     const int c = lane_out<V, NV>(sub, acc, v);
     if(live && c >= 0) s[row * NV + c] = v;
@@ -535,17 +561,16 @@ __global__ void __launch_bounds__(256) k_down(int lr, int lt, int64_t nc, const 
 template <typename V, int NV, bool SELL, bool OUT>
 __global__ void __launch_bounds__(256) k_up(int lu, int64_t n, const int32_t *__restrict__ qia,
                                             const int32_t *__restrict__ qja, const V *__restrict__ qa,
-                                            const int32_t *__restrict__ qrow, const V *__restrict__ xc, const V *__restrict__ s, V *__restrict__ x,
-                                            const int *__restrict__ skip, AMGDevice::OutMap om)
+                                            const int32_t *__restrict__ qrow, const V *xc, const V *s, V *x,
+                                            const int *skip, AMGDevice::OutMap om)
 {
-  FE_PDL_ENTRY();
-  if(skip && *skip) return;
+  if(!skip) FE_PDL_ENTRY();
   int64_t blk = blockIdx.x;
   if constexpr(OUT) {
     const int64_t pBlocks = om.bgu ? (om.nP + 255) / 256 : 0;
     if(blk < pBlocks) {
       const int64_t k = blk * 256 + threadIdx.x;
-      if(k >= om.nP) return;
+      if(early_entry(skip) || k >= om.nP) return;
       const double c = *om.cr, cSc = om.consts[1], cMc = om.consts[2];
       const double shift = cMc > 0 ? c / cMc : 0., lift = cSc != 0. ? c / cSc : 0.;
       const int32_t i = om.pRows[k];
@@ -575,11 +600,15 @@ __global__ void __launch_bounds__(256) k_up(int lu, int64_t n, const int32_t *__
     V acc[NV];
 #pragma unroll
     for(int c = 0; c < NV; ++c) acc[c] = 0;
-    sell_walk<8, V>(base, len, (int)(t & 31), qja, qa, [&](int32_t j, V a) {
-      const Vals<V, NV> xv = ldv<V, NV>(xc, j);
+    if(!sell_walk<8, V>(
+         base, len, (int)(t & 31), qja, qa,
+         [&](int32_t j, V a) {
+           const Vals<V, NV> xv = ldv<V, NV>(xc, j);
 #pragma unroll
-      for(int c = 0; c < NV; ++c) acc[c] += a * xv.v[c];
-    });
+           for(int c = 0; c < NV; ++c) acc[c] += a * xv.v[c];
+         },
+         [&] { return early_entry(skip); }))
+      return;
 #pragma unroll
     for(int c = 0; c < NV; ++c) put(qrow[t], c, acc[c]);
   } else {
@@ -587,7 +616,7 @@ __global__ void __launch_bounds__(256) k_up(int lu, int64_t n, const int32_t *__
     const int sub = threadIdx.x & (lu - 1);
     const bool live = row < n;
     V acc[NV], v;
-    row_part<V, NV, false>(live ? qia[row] : 0, live ? qia[row + 1] : 0, sub, lu, qja, qa, xc, acc);
+    if(!row_part<V, NV, false>(live ? qia[row] : 0, live ? qia[row + 1] : 0, sub, lu, qja, qa, xc, acc, skip)) return;
     lane_sum<V, NV>(sub, lu, acc);
     const int c = lane_out<V, NV>(sub, acc, v);
     if(live && c >= 0) put(row, c, v);
@@ -610,21 +639,32 @@ __global__ void k_cheb_last(int64_t m, const V *__restrict__ d, V *__restrict__ 
 // once; warp sums, then the warps' sums in order (deterministic).
 constexpr int DENSE_T = 128;
 template <typename V, int NV>
-__global__ void __launch_bounds__(DENSE_T) k_dense(int64_t n, const V *__restrict__ M, const V *__restrict__ b,
-                                                   V *__restrict__ x, const int *__restrict__ skip)
+__global__ void __launch_bounds__(DENSE_T) k_dense(int64_t n, const V *__restrict__ M, const V *b,
+                                                   V *__restrict__ x, const int *skip)
 {
-  FE_PDL_ENTRY();
-  if(skip && *skip) return;
+  if(!skip) FE_PDL_ENTRY();
   __shared__ V red[DENSE_T / 32][NV];
   const int64_t row = blockIdx.x;
   V acc[NV];
 #pragma unroll
   for(int c = 0; c < NV; ++c) acc[c] = 0;
-#pragma unroll 4
-  for(int64_t k = threadIdx.x; k < n; k += DENSE_T) {
-    const V m = M[row * n + k];
+  constexpr int UNR = 4;
+  V m[UNR];
+  auto load = [&](int64_t k0) {
 #pragma unroll
-    for(int c = 0; c < NV; ++c) acc[c] += m * b[k * NV + c];
+    for(int u = 0; u < UNR; ++u) m[u] = k0 + u * DENSE_T < n ? M[row * n + k0 + u * DENSE_T] : (V)0;
+  };
+  int64_t k0 = threadIdx.x;
+  load(k0);
+  if(early_entry(skip)) return;
+  while(k0 < n) {
+#pragma unroll
+    for(int u = 0; u < UNR; ++u)
+      if(k0 + u * DENSE_T < n)
+#pragma unroll
+        for(int c = 0; c < NV; ++c) acc[c] += m[u] * b[(k0 + u * DENSE_T) * NV + c];
+    k0 += UNR * DENSE_T;
+    if(k0 < n) load(k0);
   }
 #pragma unroll
   for(int c = 0; c < NV; ++c) {

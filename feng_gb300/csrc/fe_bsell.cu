@@ -86,9 +86,10 @@ __device__ __forceinline__ void madd(dfl &s, float a, float2 x)
 // Adds the entries k0, k0 + st, ... below k1 of one lane (NR rows, NC columns
 // each) to acc, UNR entries at a time, the next ones' columns and values
 // loaded before the gathers of x of these (one memory latency per UNR).
-template <int NR, int NC, int UNR, bool VEC, typename VA, typename X, typename S>
-__device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *__restrict__ val, int32_t k0,
-                                     int32_t k1, int st, int lane, const X *__restrict__ x, S (&acc)[NR])
+// enter: called once the first entries are on their way; true ends the walk.
+template <int NR, int NC, int UNR, bool VEC, typename VA, typename X, typename S, typename R>
+__device__ __forceinline__ bool walk(const int32_t *__restrict__ col, const VA *__restrict__ val, int32_t k0,
+                                     int32_t k1, int st, int lane, const X *x, S (&acc)[NR], R &&enter)
 {
   constexpr int NV = NR * NC, W = vec_width<VA, NV>(), PL = NV / W;
   int32_t c[UNR];
@@ -106,6 +107,7 @@ __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *
     }
   };
   load(k0);
+  if(enter()) return false;
   for(int32_t k = k0; k < k1; k += UNR * st) {
     int32_t cc[UNR];
     VA vc[UNR][NV];
@@ -127,6 +129,7 @@ __device__ __forceinline__ void walk(const int32_t *__restrict__ col, const VA *
           for(int j = 0; j < NC; ++j) madd(acc[i], vc[u][i * NC + j], xv[j]);
       }
   }
+  return true;
 }
 
 __device__ __forceinline__ float add(float a, float b) { return a + b; }
@@ -150,20 +153,28 @@ constexpr int unroll()
   return words <= 2 ? 8 : words <= 5 ? 4 : words <= 10 ? 2 : 1;
 }
 
-template <int NR, int D, bool VEC, typename VA, typename X, typename S>
-__device__ __forceinline__ void group_sum(const BlockSell::Part &P, int64_t g, int sub, int lanes,
-                                          const X *__restrict__ x, S (&acc)[NR])
+template <int NR, int D, bool VEC, typename VA, typename X, typename S, typename R>
+__device__ __forceinline__ bool group_sum(const BlockSell::Part &P, int64_t g, int sub, int lanes, const X *x,
+                                          S (&acc)[NR], R &&enter)
 {
   const int64_t sl = g >> 5;
   const int lane = (int)(g & 31);
-  if constexpr(D > 1)
-    walk<NR, D, unroll<VA, NR * D>(), VEC, VA, X, S>(P.pCol, (const VA *)P.pVal, P.pPtr[sl] + sub, P.pPtr[sl + 1],
-                                                     lanes, lane, x, acc);
-  walk<NR, 1, unroll<VA, NR>(), false, VA, X, S>(P.sCol, (const VA *)P.sVal, P.sPtr[sl] + sub, P.sPtr[sl + 1], lanes,
-                                                 lane, x, acc);
+  auto entered = [] { return false; };
+  if constexpr(D > 1) {
+    if(!walk<NR, D, unroll<VA, NR * D>(), VEC, VA, X, S>(P.pCol, (const VA *)P.pVal, P.pPtr[sl] + sub, P.pPtr[sl + 1],
+                                                         lanes, lane, x, acc, enter))
+      return false;
+    walk<NR, 1, unroll<VA, NR>(), false, VA, X, S>(P.sCol, (const VA *)P.sVal, P.sPtr[sl] + sub, P.sPtr[sl + 1], lanes,
+                                                   lane, x, acc, entered);
+  } else {
+    if(!walk<NR, 1, unroll<VA, NR>(), false, VA, X, S>(P.sCol, (const VA *)P.sVal, P.sPtr[sl] + sub, P.sPtr[sl + 1],
+                                                       lanes, lane, x, acc, enter))
+      return false;
+  }
   for(int o = lanes >> 1; o > 0; o >>= 1)
 #pragma unroll
     for(int i = 0; i < NR; ++i) acc[i] = add(acc[i], from_lane(acc[i], o));
+  return true;
 }
 
 template <typename S>
@@ -183,12 +194,16 @@ __device__ __forceinline__ S zero_of()
 // 82 us with eight lanes per CSR row.
 template <int MODE, int D, bool VEC, typename VA, typename X, typename Y>
 __global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::Part one, int lanes,
-                                               const X *__restrict__ x, const double *__restrict__ b,
-                                               Y *__restrict__ y,
-                                               const int *__restrict__ done)
+                                               const X *x, const double *b, Y *__restrict__ y, const int *done)
 {
-  FE_PDL_ENTRY();
-  if(done && *done) return;
+  // within an iteration (done non-null: the kernel before has not written the
+  // matrix) the first entries are read before the entry
+  if(!done) FE_PDL_ENTRY();
+  auto enter = [&] {
+    if(!done) return false;
+    FE_PDL_ENTRY();
+    return *done != 0;
+  };
   using S = std::conditional_t<MODE == MUL32, float, std::conditional_t<MODE == RESID32_DF, dfl, double>>;
   auto put = [&](int64_t row, S s) {
     if constexpr(MODE == MUL32 || MODE == MUL64) y[row] = s;
@@ -202,7 +217,7 @@ __global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::P
   if((int64_t)blockIdx.x < ob) {
     const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / lanes, g = t < one.n ? t : one.n - 1;
     S acc[1] = {zero_of<S>()};
-    group_sum<1, D, VEC, VA, X, S>(one, g, sub, lanes, x, acc);
+    if(!group_sum<1, D, VEC, VA, X, S>(one, g, sub, lanes, x, acc, enter)) return;
     if(t == g && sub == 0) put(one.row[g], acc[0]);
     return;
   }
@@ -211,7 +226,7 @@ __global__ void __launch_bounds__(256) k_bsell(BlockSell::Part grp, BlockSell::P
     S acc[D];
 #pragma unroll
     for(int i = 0; i < D; ++i) acc[i] = zero_of<S>();
-    group_sum<D, D, VEC, VA, X, S>(grp, g, sub, lanes, x, acc);
+    if(!group_sum<D, D, VEC, VA, X, S>(grp, g, sub, lanes, x, acc, enter)) return;
     if(t != g || sub != 0) return;
     const int64_t row = grp.row[g];
 #pragma unroll

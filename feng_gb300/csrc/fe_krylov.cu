@@ -36,12 +36,12 @@ constexpr int MAXRED = 1024;   // maximum number of reduction blocks
 template <typename VA, typename VX, typename VY, typename ACC, int LANES, bool RESID>
 __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int32_t *__restrict__ ia,
                                               const int32_t *__restrict__ ja,
-                                              const VA *__restrict__ a, const VX *__restrict__ x,
-                                              const double *__restrict__ b, VY *__restrict__ y,
-                                              const int *__restrict__ done)
+                                              const VA *__restrict__ a, const VX *x, const double *b,
+                                              VY *__restrict__ y, const int *done)
 {
-  FE_PDL_ENTRY();
-  if(done && *done) return;
+  // within an iteration (done non-null: the kernel before has not written the
+  // matrix) the first entries are read before the entry
+  if(!done) FE_PDL_ENTRY();
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
   const int sub = threadIdx.x % LANES;
   // Rows past n keep their lanes alive (zero work) so the shuffles below
@@ -51,10 +51,9 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int32_t *__restri
   // UNR segments of LANES entries per step: the column indices and values
   // (streamed, used once) are loaded before the gathers of x.
   constexpr int UNR = LANES >= 8 ? 4 : 2;
-  ACC acc = 0;
-  for(int32_t k0 = beg + sub; k0 < end; k0 += LANES * UNR) {
-    int32_t j[UNR];
-    VA av[UNR];
+  int32_t j[UNR];
+  VA av[UNR];
+  auto load = [&](int32_t k0) {
 #pragma unroll
     for(int u = 0; u < UNR; ++u) {
       const int32_t k = k0 + u * LANES;
@@ -62,9 +61,20 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int32_t *__restri
       j[u] = ok ? __ldcs(ja + k) : -1;
       av[u] = ok ? __ldcs(a + k) : (VA)0;
     }
+  };
+  int32_t k0 = beg + sub;
+  load(k0);
+  if(done) {
+    FE_PDL_ENTRY();
+    if(*done) return;
+  }
+  ACC acc = 0;
+  while(k0 < end) {
 #pragma unroll
     for(int u = 0; u < UNR; ++u)
       if(j[u] >= 0) acc += (ACC)av[u] * (ACC)x[j[u]];
+    k0 += LANES * UNR;
+    if(k0 < end) load(k0);
   }
 #pragma unroll
   for(int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LANES);
