@@ -277,28 +277,62 @@ __global__ void k_build_map(const int32_t *__restrict__ adr, int64_t nE, int nlo
 // ---------------------------------------------------------------------------
 constexpr int RT_WARPS = 8;
 
-// pack[p][0..29] = u at the velocity DOFs (local order 3 a + m), [30..38] =
-// G, [39] = J: 32 elements per block, read per local DOF (coalesced over
-// elements), written per element (coalesced) through shared memory.
+// Per element, in FP32: G (9), J, two unused, V0[c][q] = sum_k G[q][k] u_(c,k)
+// (10 x 4, the fourth unused) and g[m][n][v] = d_n u_m at vertex v (3 x 3 x 4,
+// from the differences of the quadratic's coefficients 2 u_v and
+// 4 u_(v,i) - u_v - u_i).  32 elements per block, read per local DOF (coalesced
+// over elements), written per element (coalesced) through shared memory.
+constexpr int PK_V0 = 12, PK_G = 52;
+static_assert(PK_G + 36 == ROWTET_PACK, "the packed element");
+
+// Local node of edge (i, j).
+__device__ __forceinline__ int tet_edge(int i, int j)
+{
+  const int a = min(i, j), b = max(i, j);  // (0,2) (2,1) (1,0) (1,3) (3,0) (3,2)
+  return a == 0 ? (b == 2 ? 4 : b == 1 ? 6 : 8) : a == 1 ? (b == 2 ? 5 : 7) : 9;
+}
+
 __global__ void __launch_bounds__(256) k_pack_tet(DeviceMesh dm, int hasConv, const double *__restrict__ u,
                                                   float *__restrict__ pack)
 {
-  __shared__ float sh[32][ROWTET_PACK + 1];
+  __shared__ float sh[32][41];  // u at the 30 velocity DOFs (3 c + k), G, J
+  __shared__ float out[32][ROWTET_PACK + 1];
   const int64_t nE = dm.nElm;
   for(int64_t p0 = (int64_t)blockIdx.x * 32; p0 < nE; p0 += (int64_t)gridDim.x * 32) {
     const int cnt = (int)(nE - p0 < 32 ? nE - p0 : 32);
-    for(int idx = threadIdx.x; idx < 32 * ROWTET_PACK; idx += blockDim.x) {
+    for(int idx = threadIdx.x; idx < 32 * 40; idx += blockDim.x) {
       const int i = idx >> 5, l = idx & 31;
-      if(l >= cnt) continue;
-      const int64_t p = p0 + l;
+      const int64_t p = p0 + (l < cnt ? l : 0);
       float v;
       if(i < 30) v = hasConv ? (float)u[dm.adr[(int64_t)i * nE + p]] : 0.f;
       else v = (float)dm.geo[(int64_t)(i - 30) * nE + p];
       sh[l][i] = v;
+      if(i >= 30) out[l][i - 30] = v;
+    }
+    __syncthreads();
+    // 40 values of V0 and two unused words, 12 pairs (vertex, component)
+    for(int idx = threadIdx.x; idx < 32 * 54; idx += blockDim.x) {
+      const int i = idx >> 5, l = idx & 31;
+      const float *E = sh[l], *G = E + 30;
+      if(i < 40) {
+        const int c = i >> 2, q = i & 3;
+        out[l][PK_V0 + i] = q < 3 ? G[3 * q] * E[3 * c] + G[3 * q + 1] * E[3 * c + 1] + G[3 * q + 2] * E[3 * c + 2] : 0.f;
+      } else if(i < 42) {
+        out[l][10 + i - 40] = 0.f;
+      } else {
+        const int v = (i - 42) & 3, m = (i - 42) >> 2;
+        float h[4];
+#pragma unroll
+        for(int r = 0; r < 4; ++r)
+          h[r] = r == v ? 2.f * E[3 * v + m] : 4.f * E[3 * tet_edge(v, r) + m] - (E[3 * v + m] + E[3 * r + m]);
+#pragma unroll
+        for(int n = 0; n < 3; ++n)
+          out[l][PK_G + (3 * m + n) * 4 + v] = G[n] * (h[1] - h[0]) + G[3 + n] * (h[2] - h[0]) + G[6 + n] * (h[3] - h[0]);
+      }
     }
     __syncthreads();
     for(int idx = threadIdx.x; idx < cnt * ROWTET_PACK; idx += blockDim.x)
-      pack[p0 * ROWTET_PACK + idx] = sh[idx / ROWTET_PACK][idx % ROWTET_PACK];
+      pack[p0 * ROWTET_PACK + idx] = out[idx / ROWTET_PACK][idx % ROWTET_PACK];
     __syncthreads();
   }
 }
@@ -323,26 +357,34 @@ __global__ void k_rowtet_offsets(int64_t nEnt, const int32_t *__restrict__ ent, 
   }
 }
 
-// One lane's share of entry k: pack words lane and 32 + lane, offset word
-// lane, and the entry's local DOF.
+// One lane's share of entry k: pack words lane, 32 + lane and 64 + lane (a
+// pressure row's entries: the first), offset word lane, and the entry's local
+// DOF.
 struct RowTetFetch {
-  float pa, pb;
+  float pa, pb, pc;
   uint32_t po;
   int li;
 };
 
 __device__ __forceinline__ RowTetFetch rowtet_fetch(const int32_t *__restrict__ ent, const float *__restrict__ pack,
-                                                    const uint8_t *__restrict__ offs, int32_t k, int lane)
+                                                    const uint8_t *__restrict__ offs, int32_t k, int lane, bool vel)
 {
-  RowTetFetch f{0.f, 0.f, 0u, 0};
+  RowTetFetch f{0.f, 0.f, 0.f, 0u, 0};
   const int32_t e = ent[k];
   const float *pk = pack + (int64_t)(e >> 6) * ROWTET_PACK;
   f.pa = pk[lane];
-  if(lane < ROWTET_PACK - 32) f.pb = pk[32 + lane];
+  if(vel) {
+    f.pb = pk[32 + lane];
+    if(lane < ROWTET_PACK - 64) f.pc = pk[64 + lane];
+  }
   if(lane < ROWTET_OFFS / 4) f.po = reinterpret_cast<const uint32_t *>(offs + (int64_t)k * ROWTET_OFFS)[lane];
   f.li = e & 63;
   return f;
 }
+
+// Tensors of the row-owned kernel in shared memory: K[a][b][q s] (9 of 12) and
+// S[a][b][j] for float4 reads, T, D, M as in TetTensors.
+constexpr int RT_K = 0, RT_S = 1200, RT_T = 1600, RT_D = 4600, RT_M = 4720, RT_TEN = 4820;
 
 // A persistent grid walks the row blocks; per block the CSR values of its
 // units live in shared memory.  Warp w takes units uA + w, uA + w + 8, ...
@@ -355,18 +397,31 @@ __device__ __forceinline__ RowTetFetch rowtet_fetch(const int32_t *__restrict__ 
 //   lane < 30: divu J sum_r G[r][m] D[r][j][a].
 // Every value gets one contribution per element, in the entries' (color)
 // order: the colored scatter's sum.
+// Bound: shared-memory reads.  int phi_a phi_b d_n u_m comes from the gradient
+// at the vertices (four products and two float4 reads a column, where the
+// tensor over three P2 functions took thirty of each) and the stress from nine
+// entries of K in three reads instead of shuffles: 196,608 tetrahedra
+// 1.17 -> 0.87 ms; cube 32^3 42.9 -> 41.9 ms per two steps.
 __global__ void __launch_bounds__(RT_WARPS * 32) k_matrix_tet_rows(RowAsmTet ra, FormCoeffs fc,
                                                                    const RefTensorsTet *__restrict__ gT, double c0,
                                                                    float *__restrict__ values, int accumulate)
 {
   extern __shared__ __align__(16) unsigned char rtsm[];
   float *sTen = reinterpret_cast<float *>(rtsm);
-  float *sv = sTen + NTEN;
-  __shared__ float sE[RT_WARPS][ROWTET_PACK];
-  __shared__ float sV0[RT_WARPS][30];
+  float *sv = sTen + RT_TEN;
+  __shared__ __align__(16) float sE[RT_WARPS][ROWTET_PACK];
   __shared__ __align__(16) uint8_t sOff[RT_WARPS][ROWTET_OFFS];
-  const TetTensors<float> Tt = load_tet_tensors(sTen, gT);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for(int i = tid; i < 1200; i += blockDim.x) {
+    const int ab = i / 12, qs = i % 12;
+    sTen[RT_K + i] = qs < 9 ? (float)(&gT->K[0][0][0][0])[qs * 100 + ab] : 0.f;
+  }
+  for(int i = tid; i < 400; i += blockDim.x) sTen[RT_S + i] = (float)(&gT->S[0][0][0])[i];
+  for(int i = tid; i < 3000; i += blockDim.x) sTen[RT_T + i] = (float)(&gT->T[0][0][0][0])[i];
+  for(int i = tid; i < 120; i += blockDim.x) sTen[RT_D + i] = (float)(&gT->D[0][0][0])[i];
+  for(int i = tid; i < 100; i += blockDim.x) sTen[RT_M + i] = (float)(&gT->M[0][0])[i];
+  const TetTensors<float> Tt{nullptr, sTen + RT_T, sTen + RT_D, sTen + RT_M};
+  const float4 *sK4 = reinterpret_cast<const float4 *>(sTen + RT_K), *sS4 = reinterpret_cast<const float4 *>(sTen + RT_S);
   const float fconv = (float)fc.conv, fcs = -(float)fc.sigma * (float)fc.mu, fcm = (float)fc.mass * (float)c0;
   const float fsig = (float)fc.sigma, fdiv = (float)fc.divu;
   for(int blk = blockIdx.x; blk < ra.nBlocks; blk += gridDim.x) {
@@ -383,88 +438,67 @@ __global__ void __launch_bounds__(RT_WARPS * 32) k_matrix_tet_rows(RowAsmTet ra,
       const int32_t kb = ra.unitPtr[un], ke = ra.unitPtr[un + 1];
       // the next entry's packed element data and column offsets are loaded
       // into registers while the current one is computed
-      RowTetFetch nx = kb < ke ? rowtet_fetch(ra.ent, ra.pack, ra.offs, kb, lane) : RowTetFetch{0.f, 0.f, 0u, 0};
+      RowTetFetch nx = kb < ke ? rowtet_fetch(ra.ent, ra.pack, ra.offs, kb, lane, vel) : RowTetFetch{0.f, 0.f, 0.f, 0u, 0};
       for(int32_t k = kb; k < ke; ++k) {
         const int li = nx.li;
         sE[warp][lane] = nx.pa;
-        if(lane < ROWTET_PACK - 32) sE[warp][32 + lane] = nx.pb;
+        if(vel) {
+          sE[warp][32 + lane] = nx.pb;
+          if(lane < ROWTET_PACK - 64) sE[warp][64 + lane] = nx.pc;
+        }
         if(lane < ROWTET_OFFS / 4) reinterpret_cast<uint32_t *>(sOff[warp])[lane] = nx.po;
         __syncwarp();
-        if(k + 1 < ke) nx = rowtet_fetch(ra.ent, ra.pack, ra.offs, k + 1, lane);
+        if(k + 1 < ke) nx = rowtet_fetch(ra.ent, ra.pack, ra.offs, k + 1, lane, vel);
         const float *E = sE[warp];
-        const float J = E[39];
-        float G[3][3];
-#pragma unroll
-        for(int q = 0; q < 3; ++q)
-#pragma unroll
-          for(int l = 0; l < 3; ++l) G[q][l] = E[30 + 3 * q + l];
+        const float4 *E4 = reinterpret_cast<const float4 *>(E);
+        const float J = E[9];
         if(vel) {
           const int a = li / 3;
-          if(fc.hasConv && lane < 30) {
-            // (runtime row index: G read from shared memory, not indexed in registers)
-            const int q = lane / 10, c = lane % 10;
-            sV0[warp][lane] = E[30 + 3 * q] * E[3 * c] + E[31 + 3 * q] * E[3 * c + 1] + E[32 + 3 * q] * E[3 * c + 2];
-          }
-          __syncwarp();
           if(lane < 30) {
             const int m = lane / 10, b = lane % 10;
-            // lanes b, b + 10, b + 20 hold the same column b: terms that do
-            // not depend on m are split among them and exchanged by shuffles
+            // lanes b, b + 10, b + 20 hold the same column b: the term that
+            // does not depend on m is split among them and exchanged by shuffles
             constexpr unsigned L30 = 0x3fffffffu;
             float A[3] = {0.f, 0.f, 0.f};
             if(fc.hasConv) {
-              // W = sum_c sum_r V0[r][c] T[r][a][c][b] (lane m sums c = m, m + 3, ...),
-              // Z_r = sum_c u_(c,m) T[r][a][b][c]
-              float Wp = 0.f, Z[3] = {0.f, 0.f, 0.f};
+              // W = sum_c sum_r V0[c][r] T[r][a][c][b] (lane m sums c = m, m + 3, ...)
+              float Wp = 0.f;
 #pragma unroll
               for(int cc = 0; cc < 4; ++cc) {
                 const int c = m + 3 * cc;
                 if(c < 10) {
-#pragma unroll
-                  for(int q = 0; q < 3; ++q) Wp += sV0[warp][q * 10 + c] * Tt.t(q, a, c, b);
+                  const float4 v0 = E4[PK_V0 / 4 + c];
+                  Wp += v0.x * Tt.t(0, a, c, b) + v0.y * Tt.t(1, a, c, b) + v0.z * Tt.t(2, a, c, b);
                 }
-              }
-#pragma unroll
-              for(int c = 0; c < 10; ++c) {
-                const float um = E[3 * c + m];
-#pragma unroll
-                for(int q = 0; q < 3; ++q) Z[q] += um * Tt.t(q, a, b, c);
               }
               const float W = __shfl_sync(L30, Wp, b) + __shfl_sync(L30, Wp, b + 10) + __shfl_sync(L30, Wp, b + 20);
               const float cc = fconv * J;
+              const float4 s4 = sS4[a * 10 + b];
 #pragma unroll
               for(int n = 0; n < 3; ++n) {
-                float v = G[0][n] * Z[0] + G[1][n] * Z[1] + G[2][n] * Z[2];
+                const float4 g = E4[PK_G / 4 + 3 * m + n];
+                float v = g.x * s4.x + g.y * s4.y + g.z * s4.z + g.w * s4.w;
                 if(n == m) v += W;
                 A[n] += cc * v;
               }
             }
             if(fc.hasSigma) {
-              // row q = m of P formed here, rows q != m from lanes q * 10 + b
-              float Pm3[3];
-              {
-                const float k0 = Tt.k(m, 0, a, b), k1 = Tt.k(m, 1, a, b), k2 = Tt.k(m, 2, a, b);
+              const float4 k0 = sK4[(a * 10 + b) * 3], k1 = sK4[(a * 10 + b) * 3 + 1], k2 = sK4[(a * 10 + b) * 3 + 2];
+              const float4 e0 = E4[0], e1 = E4[1];
+              const float G[3][3] = {{e0.x, e0.y, e0.z}, {e0.w, e1.x, e1.y}, {e1.z, e1.w, E[8]}};
+              // column m of P = K G
+              const float x0 = E[m], x1 = E[3 + m], x2 = E[6 + m];
+              const float P0 = k0.x * x0 + k0.y * x1 + k0.z * x2, P1 = k0.w * x0 + k1.x * x1 + k1.y * x2,
+                          P2 = k1.z * x0 + k1.w * x1 + k2.x * x2;
+              // S[n][m] of grad phi_a (x) grad phi_b; the trace from the three lanes' m = n
+              float sn[3];
 #pragma unroll
-                for(int l = 0; l < 3; ++l) Pm3[l] = k0 * G[0][l] + k1 * G[1][l] + k2 * G[2][l];
-              }
-              float P[3][3];
-#pragma unroll
-              for(int q = 0; q < 3; ++q)
-#pragma unroll
-                for(int l = 0; l < 3; ++l) P[q][l] = __shfl_sync(L30, Pm3[l], q * 10 + b);
-              float tr = 0.f;
-#pragma unroll
-              for(int kk = 0; kk < 3; ++kk) tr += G[0][kk] * P[0][kk] + G[1][kk] * P[1][kk] + G[2][kk] * P[2][kk];
+              for(int n = 0; n < 3; ++n) sn[n] = G[0][n] * P0 + G[1][n] * P1 + G[2][n] * P2;
+              const float own = m == 0 ? sn[0] : m == 1 ? sn[1] : sn[2];
+              const float tr = __shfl_sync(L30, own, b) + __shfl_sync(L30, own, b + 10) + __shfl_sync(L30, own, b + 20);
               const float cs = fcs * J;
-              // column m of P by selects (m is a runtime lane index)
-              float Pm[3];
 #pragma unroll
-              for(int qq = 0; qq < 3; ++qq) Pm[qq] = m == 0 ? P[qq][0] : (m == 1 ? P[qq][1] : P[qq][2]);
-#pragma unroll
-              for(int n = 0; n < 3; ++n) {
-                const float snm = G[0][n] * Pm[0] + G[1][n] * Pm[1] + G[2][n] * Pm[2];
-                A[n] += cs * ((n == m ? tr : 0.f) + snm);
-              }
+              for(int n = 0; n < 3; ++n) A[n] += cs * ((n == m ? tr : 0.f) + sn[n]);
             }
             if(fc.hasMass) {
               const float mv = fcm * J * Tt.m(a, b);
@@ -483,7 +517,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) k_matrix_tet_rows(RowAsmTet ra,
             const int m = lane >> 2, j = lane & 3;
             const uint8_t o = sOff[warp][30 + j];
             if(o != 255) {
-              const float bp = (E[30 + m] * Tt.d(0, j, a) + E[33 + m] * Tt.d(1, j, a) + E[36 + m] * Tt.d(2, j, a)) * J;
+              const float bp = (E[m] * Tt.d(0, j, a) + E[3 + m] * Tt.d(1, j, a) + E[6 + m] * Tt.d(2, j, a)) * J;
               row0[m * rl + o] += fsig * bp;
             }
           }
@@ -491,7 +525,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) k_matrix_tet_rows(RowAsmTet ra,
           const int j = li - 30, a = lane / 3, m = lane % 3;
           const uint8_t o = sOff[warp][lane];
           if(o != 255) {
-            const float bp = (E[30 + m] * Tt.d(0, j, a) + E[33 + m] * Tt.d(1, j, a) + E[36 + m] * Tt.d(2, j, a)) * J;
+            const float bp = (E[m] * Tt.d(0, j, a) + E[3 + m] * Tt.d(1, j, a) + E[6 + m] * Tt.d(2, j, a)) * J;
             row0[o] += fdiv * bp;
           }
         }
@@ -543,7 +577,10 @@ void build_ref_tensors_tet(const QuadRule &q, RefTensorsTet &T)
       for(int j = 0; j < 4; ++j)
         for(int a = 0; a < 10; ++a) T.D[rr][j][a] += w * l[j] * dphi[a][rr];
     for(int a = 0; a < 10; ++a)
-      for(int b = 0; b < 10; ++b) T.M[a][b] += w * phi[a] * phi[b];
+      for(int b = 0; b < 10; ++b) {
+        T.M[a][b] += w * phi[a] * phi[b];
+        for(int j = 0; j < 4; ++j) T.S[a][b][j] += w * phi[a] * phi[b] * l[j];
+      }
   }
 }
 
@@ -609,7 +646,7 @@ void launch_matrix_tet_rows_f32(const RowAsmTet &ra, const FormCoeffs &fc, const
                                 float *values, int accumulate, cudaStream_t s)
 {
   if(ra.nBlocks <= 0) return;
-  const size_t sm = sizeof(float) * NTEN + (size_t)ra.capBytes;
+  const size_t sm = sizeof(float) * RT_TEN + (size_t)ra.capBytes;
   static size_t set = 0;
   if(set != sm) {
     cudaFuncSetAttribute(k_matrix_tet_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -40,6 +40,7 @@ enum SourceKind : int {
 //   T[r][a][c][b] = sum_q w phi_a phi_c dphi_b/dr
 //   D[r][j][a]    = sum_q w psi_j dphi_a/dr
 //   M[a][b]       = sum_q w phi_a phi_b
+//   S[a][b][j]    = sum_q w phi_a phi_b psi_j
 // plus the rule itself and the P2 values at its nodes for the sources.
 constexpr int TET_MAXQ = 64;
 struct RefTensorsTet {
@@ -47,6 +48,7 @@ struct RefTensorsTet {
   double T[3][10][10][10];
   double D[3][4][10];
   double M[10][10];
+  double S[10][10][4];
   int nq;
   double qw[TET_MAXQ], qr[TET_MAXQ], qs[TET_MAXQ], qt[TET_MAXQ];
   double phi[TET_MAXQ][10];
@@ -148,10 +150,10 @@ struct RowAsmTet {
   int32_t *unitPtr = nullptr;     // [nUnits + 1] entries of each unit
   int32_t *ent = nullptr;         // [nEnt] p * 64 + local DOF of the unit's first row (3 a, or 30 + j)
   uint8_t *offs = nullptr;        // [nEnt][ROWTET_OFFS] offset of local column j in the row (255: none)
-  float *pack = nullptr;          // [nElm][ROWTET_PACK] u at the 30 velocity DOFs, G[3][3], J
+  float *pack = nullptr;          // [nElm][ROWTET_PACK], see k_pack_tet
   const int32_t *ia = nullptr;    // CSR row pointers
 };
-constexpr int ROWTET_PACK = 40;
+constexpr int ROWTET_PACK = 88;
 constexpr int ROWTET_OFFS = 40;
 
 void launch_pack_tet_f32(const DeviceMesh &dm, const FormCoeffs &fc, const double *u, float *pack, cudaStream_t s);
