@@ -219,13 +219,22 @@ def e2e_steps(sys_, nl, steps):
 def algorithmic_bytes(sys_, nvert, precision):
     """Per-launch algorithmic bytes (byte model of the assembly and SpMV roofline):
       assembly  nnz s_A + nElm n_loc 4 + nVert d 8 + nDofs 8 k_in + nInc 8
-      SpMV      nnz (s_A + 4) + (nInc + 1) 4 + nInc (s_x + s_y)"""
+      SpMV      nnz s_A + (column indices) 4 + (nInc + 1) 4 + nInc (s_x + s_y),
+                with an index per entry in CSR and, from 75,000 rows on, one
+                per 2 x 2, 2 x 1 or 1 x 2 block of a velocity node's unknowns"""
     sA = 4 if precision == "mixed" else 8
     nl = 15
     res = sys_.nElm * nl * 4 + nvert * 2 * 8 + sys_.nDofs * 8 + sys_.nInc * 8
     mat = sys_.nnz * sA + sys_.nElm * nl * 4 + nvert * 2 * 8 + sys_.nDofs * 8
     sx = 4 if precision == "mixed" else 8   # the Arnoldi SpMV: FP32 vectors (mixed), FP64 (plain)
-    spmv = sys_.nnz * (sA + 4) + (sys_.nInc + 1) * 4 + sys_.nInc * 2 * sx
+    idx = sys_.nnz
+    if sys_.nInc >= 75000:
+        ia, ja = sys_.pattern()
+        vel = np.asarray(sys_.dofInfo()[2])[:sys_.nInc] == 0
+        nv = np.add.reduceat(vel[ja].astype(np.int64), ia[:-1])
+        per = nv // 2 + (np.diff(ia) - nv)
+        idx = int(per[vel].sum()) // 2 + int(per[~vel].sum())
+    spmv = sys_.nnz * sA + idx * 4 + (sys_.nInc + 1) * 4 + sys_.nInc * 2 * sx
     from feng_gb300._lib import check
     out = {"residual_assembly": res, "matrix_assembly": mat, "spmv": spmv}
     for which, name in ((4, "smoother_step"), (5, "gs_dots"), (6, "gs_update"), (7, "gs_dots_stream"),
@@ -250,7 +259,7 @@ def ncu_traffic(kernel):
 
 def phase_bench(sys_, mixed, reps=20):
     """Device-timed phases (L2 flushed before each run): assembly, SpMV, one
-    preconditioner application, the finest-level pre-smoothing pass, and for
+    preconditioner application, the finest level's pass on the way down, and for
     the mixed path the two Gram-Schmidt passes at restart/2 = 25 columns
     (the mean column count of a 50-step cycle), each once alone (flushed,
     one launch between two events: the launch latency and the tail are in
@@ -593,8 +602,8 @@ def main():
               "preconditioner_build": ph["factor_ms"]}
     # The dominant kernel of the Newton step: the Krylov solve is ~97% of
     # it, and its largest kernel by device time is the Arnoldi SpMV
-    # (k_spmv_sell, one launch per FGMRES iteration; profiles/ holds the
-    # launch list with the shares).
+    # (k_bsell, one launch per FGMRES iteration; profiles/ holds the launch
+    # list with the shares).
     def roofline(key, kernel, traffic_key):
         # the streamed timing (launches back to back over cold data) where the
         # phase has one, with the single flushed launch beside it
@@ -608,13 +617,13 @@ def main():
         if ks:
             out["single_launch"] = {"ms": k["ms"], "achieved": k["gbs"], "frac": k["gbs"] / peak}
         return out
-    roof = roofline("spmv", "k_spmv_sell (FGMRES inner SpMV, sliced ELL, FP32)", "k_spmv_sell")
+    roof = roofline("spmv", "k_bsell<MUL32,2> (FGMRES inner SpMV, block-column sliced ELL, FP32)", "k_bsell<MUL32,2>")
     roof_gsd = roofline("gs_dots", "k_gs_dots_all<16> (FP32 Gram-Schmidt dot pass, one pass over w and every "
                         "column, 25 basis vectors)", "k_gs_dots_all@25")
     roof_gsu = roofline("gs_update", "k_gs_upd<32,true> (FP32 Gram-Schmidt update + norm, 25 basis vectors)",
                         "k_gs_upd<32,true>@25")
-    roof_sm = roofline("smoother_step", "k_cheb_first_sell<float,2> (finest AMG level, both velocity components)",
-                       "k_cheb_first_sell<float,2>")
+    roof_sm = roofline("smoother_step", "k_down<float,2> (finest AMG level on the way down: smoothing and restriction, both velocity "
+                       "components)", "k_down<float,2>")
     asm = kern["mixed"]["matrix_assembly"]
     roof_asm = {"kernel": "k_pack_th + k_matrix_th_rows<float> (row-owned Jacobian assembly)", "bound": "hbm",
                 "achieved": asm["gbs"], "peak": peak, "unit": "GB/s", "frac": asm["gbs"] / peak,

@@ -1,8 +1,8 @@
 // Element assembly kernels: residual (FP64) and Jacobian (FP64 or FP32) of
 // the fused weak forms.
 //
-// Colored kernels (residuals; scalar P2 Jacobian): one launch per element
-// color, entries scattered into CSR through the element-to-nonzero map as
+// Colored kernels (scalar P2 residual and Jacobian; Taylor-Hood residuals:
+// fe_residual.cu): one launch per element color, entries scattered into CSR through the element-to-nonzero map as
 // L2 reductions; no two elements of a color share a DOF, so every entry
 // receives one contribution per color and the sums are the colored
 // read-modify-write's, in color order.

@@ -73,8 +73,8 @@ struct RefTensors {
   int nq;
   double qw[16], qr[16], qs[16];  // the rule, for non-polynomial sources
   double phi[16][6];              // P2 functions at the nodes
-  // The rule is exact to degree 5 (every polynomial integrand of the residual
-  // on affine triangles has degree <= 5): a 7-node rule gives the same integrals.
+  // The rule is exact to degree 5, that of every polynomial integrand of the
+  // residual on affine triangles.
   int exact5;
 };
 

@@ -161,7 +161,7 @@ class SystemCUDA {
   std::vector<int64_t> adrHost_;      // element table, original element order
   std::vector<double> elemXYHost_;    // vertex coordinates per element
   int elemType_ = 0;
-  int exact5_ = 0;   // the rule integrates degree 5 exactly (quadrature residual kernel)
+  int exact5_ = 0;   // the rule integrates degree 5 exactly
   DeviceMesh dm_;
   FormCoeffs fc_{};
   RefTensors *dT_ = nullptr;
@@ -182,10 +182,9 @@ class SystemCUDA {
   mutable bool zeroPending_ = false;
   mutable bool zeroedOut_ = false;   // the values were zeroed after the last factor()
   int ensureMatrixZeroed() const;
-  // The mixed path assembles the Taylor-Hood residual in double-float on
-  // the FP32 pipes (FP64-class accuracy, the 7-node rule); otherwise FP64.
-  // the mixed path's residual in double-float (triangles: rules exact to
-  // degree 5; tetrahedra: Taylor-Hood with rules of at most TET_DF_MAXQ nodes)
+  // The mixed path assembles the Taylor-Hood residual in double-float on the
+  // FP32 pipes (FP64-class accuracy) on triangles with rules exact to degree 5
+  // and on tetrahedra with rules of at most TET_DF_MAXQ nodes; otherwise FP64.
   int dfResidual() const { return dm_.geoPair && (exact5_ || tet()) ? 1 : 0; }
   void launch_residual(double *out);  // the residual launches of assembleResiduals
   float2 *uPair_ = nullptr, *udotPair_ = nullptr;
