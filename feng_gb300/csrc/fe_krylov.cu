@@ -622,12 +622,10 @@ __global__ void __launch_bounds__(RB) k_gs_dots(int64_t n4, int m1, const float 
 // gridDim.x <= MAXRED.
 template <int CMAX>
 __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const float *__restrict__ V,
-                                                      int ncols, const float *__restrict__ w, double *partials,
+                                                      int ncols, const float *w, double *partials,
                                                       RedState *st, double *hcur, double *Hcol,
-                                                      const int *__restrict__ done, int second)
+                                                      const int *done, int second)
 {
-  FE_PDL_ENTRY();
-  if(*done || (second && !st->reorth)) return;
   __shared__ double red[RB / 32][CMAX + 1];
   __shared__ double flat[RB];
   __shared__ bool last;
@@ -636,21 +634,29 @@ __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const
   const bool wcol = blockIdx.y == 0;
   const float4 *w4 = reinterpret_cast<const float4 *>(w);
   const float4 *V4 = reinterpret_cast<const float4 *>(V);
+  const int64_t g0 = (int64_t)blockIdx.x * RB + tid;
+  // one batch of eight loads in flight (clamped columns, the extra products
+  // dropped by selects); the first ahead of the entry: the kernel before wrote
+  // w, not the basis (a second pass, which mostly returns at once, reads none)
+  float4 v[8];
+  auto load = [&](int64_t g, int c0) {
+#pragma unroll
+    for(int u = 0; u < 8; ++u) v[u] = __ldcs(V4 + vidx4(g, cb + (c0 + u < cn ? c0 + u : c0), m1));
+  };
+  if(!second && g0 < n4) load(g0, 0);
+  FE_PDL_ENTRY();
+  if(*done || (second && !st->reorth)) return;
   float acc[CMAX];
 #pragma unroll
   for(int c = 0; c < CMAX; ++c) acc[c] = 0.f;
   float wq = 0.f;
-  for(int64_t g = (int64_t)blockIdx.x * RB + tid; g < n4; g += (int64_t)gridDim.x * RB) {
+  for(int64_t g = g0; g < n4; g += (int64_t)gridDim.x * RB) {
     const float4 x = w4[g];
     if(wcol) wq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, wq))));
 #pragma unroll
     for(int c0 = 0; c0 < CMAX; c0 += 8) {
       if(c0 < cn) {
-        // one batch of eight loads in flight (clamped columns, the extra
-        // products dropped by selects)
-        float4 v[8];
-#pragma unroll
-        for(int u = 0; u < 8; ++u) v[u] = __ldcs(V4 + vidx4(g, cb + (c0 + u < cn ? c0 + u : c0), m1));
+        if(c0 || second || g != g0) load(g, c0);
 #pragma unroll
         for(int u = 0; u < 8; ++u) {
           const float t = fmaf(v[u].x, x.x, fmaf(v[u].y, x.y, fmaf(v[u].z, x.z, v[u].w * x.w)));
@@ -731,15 +737,31 @@ __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const
 // preconditioner's next input); otherwise it goes back to w.
 template <int CMAX, bool NORM>
 __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__restrict__ V, int ncols,
-                                                  const double *__restrict__ hprev, float *__restrict__ w,
+                                                  const double *hprev, float *w,
                                                   float *__restrict__ vcopy, RedState *st, double *partials,
-                                                  double *Hnext, const int *__restrict__ done, int second)
+                                                  double *Hnext, const int *done, int second)
 {
-  FE_PDL_ENTRY();
-  if(*done || (NORM && second && !st->reorth)) return;
   __shared__ float hs[CMAX];
   __shared__ double wred[RB / 32];
   __shared__ bool last;
+  // the first rows' first batch ahead of the entry: the kernel before formed
+  // the coefficients, not w or the basis
+  const bool ahead = NORM && !second;
+  const int64_t g0 = (int64_t)blockIdx.x * RB + threadIdx.x;
+  float4 v[8];
+  auto load = [&](int64_t g, int c0) {
+#pragma unroll
+    for(int u = 0; u < 8; ++u)
+      v[u] = c0 + u < ncols ? __ldcs(reinterpret_cast<const float4 *>(V) + vidx4(g, c0 + u, m1))
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if(ahead && g0 < n4) {
+    w0 = reinterpret_cast<const float4 *>(w)[g0];
+    load(g0, 0);
+  }
+  FE_PDL_ENTRY();
+  if(*done || (NORM && second && !st->reorth)) return;
   for(int c = threadIdx.x; c < CMAX; c += RB) hs[c] = c < ncols ? (float)hprev[c] : 0.f;
   __syncthreads();
   const bool again = NORM || st->reorth != 0;
@@ -748,17 +770,15 @@ __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__r
   float4 *V4 = reinterpret_cast<float4 *>(V);
   float4 *c4 = reinterpret_cast<float4 *>(vcopy);
   float q = 0.f;
-  for(int64_t g = (int64_t)blockIdx.x * RB + threadIdx.x; g < n4; g += (int64_t)gridDim.x * RB) {
-    float4 wv = w4[g];
+  for(int64_t g = g0; g < n4; g += (int64_t)gridDim.x * RB) {
+    const bool have = ahead && g == g0;
+    float4 wv = have ? w0 : w4[g];
     // one batch of eight column loads in flight at a time (unrolled
     // batches would hoist every load and spill)
 #pragma unroll 1
     for(int c0 = 0; c0 < CMAX; c0 += 8) {
       if(c0 < ncols) {
-        float4 v[8];
-#pragma unroll
-        for(int u = 0; u < 8; ++u)
-          v[u] = c0 + u < ncols ? __ldcs(V4 + vidx4(g, c0 + u, m1)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if(c0 || !have) load(g, c0);
 #pragma unroll
         for(int u = 0; u < 8; ++u) {
           const float h = hs[c0 + u];

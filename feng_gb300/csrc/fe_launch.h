@@ -16,7 +16,8 @@
 // may move loads through const __restrict__ ones ahead of the entry.
 // Kovasznay solves 32^2 FP64 51.2 -> 49.2 ms, 97^2 mixed 23.2 -> 21.6, 256^2
 // mixed 61.1 -> 58.0, 256^2 FP64 361 -> 343; cavity 384^2 43.7 -> 42.5 and cube
-// 32^3 44.2 -> 43.0 ms per two steps.  FENG_PDL=0 launches
+// 32^3 44.2 -> 43.0 ms per two steps.  (The Gram-Schmidt passes' first basis
+// columns likewise: 97^2 21.6 -> 21.5, 256^2 58.1 -> 57.6.)  FENG_PDL=0 launches
 // without the attribute (the same kernels, fully serialised).
 #pragma once
 
