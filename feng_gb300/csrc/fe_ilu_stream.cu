@@ -298,6 +298,9 @@ int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t>
   std::vector<Step> steps;
   std::vector<int32_t> stepStart(1, 0), pos, dpos, rowDiag(n), level(n, 0);
   std::vector<uint4> col;
+  pos.reserve(2 * lja.size());
+  dpos.reserve(2 * lja.size());
+  col.reserve(6 * (size_t)n);
   std::vector<int32_t> cnt, ord;
   // a warp of a level: rows ord[first] .. ord[first + rows - 1], `slots` each
   struct Warp {

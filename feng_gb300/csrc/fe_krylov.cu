@@ -1541,8 +1541,7 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
     CK(cudaMemcpy(ilu_.lja, lja.data(), sizeof(int32_t) * ilu_.lnnz, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ilu_.ldiag, ldiag.data(), sizeof(int32_t) * n_, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ilu_.srcPos, src.data(), sizeof(int32_t) * ilu_.lnnz, cudaMemcpyHostToDevice));
-    FE_TRY(build_ilu_levels(lia, lja, ldiag));
-    // diagonal blocks whose vector fits in shared memory (about 20 k rows in FP64)
+    // diagonal blocks whose vector fits in shared memory (about 21 k rows in FP64)
     // are solved there; the level kernels stay for larger ones
     ilus_ = new IluStream();
     FE_TRY(ilus_->build(lia, lja, ldiag, perm, bstart, opt.mixed != 0, s_));
@@ -1550,6 +1549,7 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
       delete ilus_;
       ilus_ = nullptr;
     }
+    FE_TRY(build_ilu_levels(lia, lja, ldiag));
   }
   return FE_OK;
 }
@@ -1607,14 +1607,15 @@ int Krylov::build_ilu_levels(const std::vector<int32_t> &lia, const std::vector<
   };
   std::vector<int32_t> rl, ll, ru, lu;
   ilu_.nLevL = schedule(true, rl, ll, ilu_.segL);
-  ilu_.nLevU = schedule(false, ru, lu, ilu_.segU);
   CK(cudaMalloc(&ilu_.rowsL, sizeof(int32_t) * n));
-  CK(cudaMalloc(&ilu_.rowsU, sizeof(int32_t) * n));
   CK(cudaMalloc(&ilu_.lvlL, sizeof(int32_t) * ll.size()));
-  CK(cudaMalloc(&ilu_.lvlU, sizeof(int32_t) * lu.size()));
   CK(cudaMemcpy(ilu_.rowsL, rl.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ilu_.rowsU, ru.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ilu_.lvlL, ll.data(), sizeof(int32_t) * ll.size(), cudaMemcpyHostToDevice));
+  if(ilus_) return FE_OK;  // U's levels only for the solves by level
+  ilu_.nLevU = schedule(false, ru, lu, ilu_.segU);
+  CK(cudaMalloc(&ilu_.rowsU, sizeof(int32_t) * n));
+  CK(cudaMalloc(&ilu_.lvlU, sizeof(int32_t) * lu.size()));
+  CK(cudaMemcpy(ilu_.rowsU, ru.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ilu_.lvlU, lu.data(), sizeof(int32_t) * lu.size(), cudaMemcpyHostToDevice));
   return FE_OK;
 }
