@@ -114,7 +114,7 @@ __device__ __forceinline__ void givens_warp(GmresState *gs, int j, int lane, dou
     s = b * inv;
   } else {
     r = hypot(a, b);
-    if(r > 0) { c = a / r; s = b / r; }
+    if(r != 0) { c = a / r; s = b / r; }  // not finite: so is the estimate
   }
   gs->cs[j] = c;
   gs->sn[j] = s;

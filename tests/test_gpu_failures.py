@@ -88,6 +88,32 @@ def test_zero_pivot_gives_pc_failed():
     assert r["status"] == PC_FAILED
 
 
+def _overflowing_diffusion(coeff, source, **options):
+    """P2 diffusion whose matrix entries scale with coeff, the right-hand side
+    with source alone (zero state)."""
+    g = load_golden("diffusion_p2_8")
+    _, forms = problem_spaces("diffusion", golden_mesh(g))
+    forms = [fe.createBilinearForm(f.spaces, fe.feSysElm_Diffusion(coeff) if f.sysElm.kind == 2
+                                   else fe.feSysElm_Source(fe.api.SRC_SIN_SIN, (source,))) for f in forms]
+    s = TablesSystem(g, forms, fe.LinearSolverOptions(**options))
+    s.setSolution(np.zeros(s.nDofs))
+    s.setToZero()
+    s.assembleResiduals()
+    s.assembleMatrices()
+    assert 0 < s.getRHSMaxNorm() < np.inf
+    return s
+
+
+@pytest.mark.parametrize("precision,coeff", [("fp64", 1e308), ("mixed", 1e39)])
+def test_nonfinite_krylov_vector_is_not_convergence(precision, coeff):
+    """The matrix overflows to infinities of both signs, so the first product
+    is NaN: no rotation of such a column may leave an estimate of 0."""
+    s = _overflowing_diffusion(coeff, 1.0, krylov="fgmres", precond="none", precision=precision)
+    assert not np.all(np.isfinite(s.getMatrix()))
+    r = s.solve(raise_on_failure=False)
+    assert r["status"] == NONFINITE
+
+
 def test_linear_iteration_limit_gives_not_converged():
     g, sys = _kovasznay()
     sys.setSolution(g["u0"])
