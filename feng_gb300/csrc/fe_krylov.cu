@@ -2415,6 +2415,7 @@ int Krylov::solve_cg64(const double *vals, const double *b, double *x, double to
   CGState init{};
   init.tol = tolAbs;
   init.done = 0;
+  init.rr = st.rnorm0 * st.rnorm0;  // r = b, should the iteration break down at once
   cudaMemcpyAsync(w.cg, &init, sizeof(CGState), cudaMemcpyHostToDevice, s_);
   // z = M r ; rz = r.z ; p = z
   precond64(r_, t_, &w.cg->done);
@@ -2439,7 +2440,7 @@ int Krylov::solve_cg64(const double *vals, const double *b, double *x, double to
   }
   st.iterations = w.hcg->it;
   st.rnorm = sqrt(w.hcg->rr);
-  if(!std::isfinite(st.rnorm)) { set_error("non-finite residual in CG"); return FE_NONFINITE; }
+  if(!std::isfinite(st.rnorm) || !std::isfinite(w.hcg->pq)) { set_error("non-finite residual in CG"); return FE_NONFINITE; }
   return st.rnorm <= tolAbs * 1.0000001 ? FE_OK : FE_NOT_CONVERGED;
 }
 

@@ -114,6 +114,23 @@ def test_nonfinite_krylov_vector_is_not_convergence(precision, coeff):
     assert r["status"] == NONFINITE
 
 
+def test_cg_that_breaks_down_at_once_reports_the_right_hand_side():
+    """p.q not finite (A p overflows: entries of 1e200, a right-hand side of
+    1e120) or zero (the matrix is zeroed and not assembled again) before the
+    first residual: a failure, never the residual 0 of an iteration that was
+    not made."""
+    s = _overflowing_diffusion(1e200, 1e120, krylov="cg", precond="none")
+    assert np.all(np.isfinite(s.getMatrix()))
+    r = s.solve(raise_on_failure=False)
+    assert (r["status"], r["nIter"]) == (NONFINITE, 0)
+    s = _overflowing_diffusion(1.0, 1.0, krylov="cg", precond="none")
+    s.setMatrixToZero()
+    r = s.solve(raise_on_failure=False)
+    assert (r["status"], r["nIter"]) == (NOT_CONVERGED, 0)
+    assert r["normAxb"] == pytest.approx(np.linalg.norm(s.getRHS()), rel=1e-12)
+    assert np.all(s.getDu() == 0.0)
+
+
 def test_linear_iteration_limit_gives_not_converged():
     g, sys = _kovasznay()
     sys.setSolution(g["u0"])
