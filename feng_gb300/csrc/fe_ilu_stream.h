@@ -51,6 +51,7 @@ class IluStream {
   bool usable_ = false, fp32_ = false;
   int64_t nBlocks_ = 0, nEntries_ = 0, nRows_ = 0;
   size_t smem_ = 0;
+  int lateStep_ = -1;
   Step *steps_ = nullptr;          // all blocks' steps
   int32_t *stepStart_ = nullptr;   // [nBlocks + 1]
   int32_t *start_ = nullptr, *perm_ = nullptr;

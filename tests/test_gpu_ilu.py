@@ -9,11 +9,16 @@ FP64, 1e-5 with the FP32 factors of the mixed path.  Cases: the 64 x 64 P2
 diffusion system of the CPU-runnable configuration as one block (254
 levels in its L and in its U part), and a Taylor-Hood Jacobian in
 block-Jacobi form (the blocks of the set-up's partition)."""
+import json
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import feng_gb300 as fe
-from conftest import load_golden
+from conftest import ROOT, load_golden
 from helpers import golden_mesh, problem_spaces
 
 from oracle.oracle import OracleProblem  # noqa: E402
@@ -109,3 +114,39 @@ def test_ilu0_solves_match_serial_over_block_shapes(n, rows, precision):
     r = np.random.default_rng(4).uniform(-1, 1, sys_.nInc)
     z, ref = sys_.applyPreconditioner(r), _ilu_reference(A, r, blocks)
     assert np.max(np.abs(z - ref)) <= (1e-11 if precision == "fp64" else 1e-2) * np.max(np.abs(ref))
+
+
+LATE = r"""
+import json, sys
+import numpy as np
+import feng_gb300 as fe
+sys.path.insert(0, "tests")
+from helpers import problem_spaces
+precision, rows, krylov = sys.argv[1], int(sys.argv[2]), sys.argv[3]
+num, forms = problem_spaces("diffusion", fe.Mesh2DP1.generate_square(20, jitter=0.1, seed=2))
+s = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(
+    krylov=krylov, precond="ilu0" if rows == 0 else "bjacobi-ilu0", pc_block_rows=max(rows, 1), precision=precision))
+s.setToZero()
+s.assembleResiduals()
+s.assembleMatrices()
+z = s.applyPreconditioner(np.random.default_rng(4).uniform(-1, 1, s.nInc))
+st = s.solve(raise_on_failure=False)
+print(json.dumps([int(np.isfinite(z).sum()), len(z), st["status"], bool(np.all(np.isfinite(s.getMatrix())))]))
+"""
+
+
+@pytest.mark.parametrize("krylov,precision,rows,step", [("fgmres", "fp64", 0, k) for k in (0, 1, 2, 3, 4, 5, 60)] +
+                         [("fgmres", "mixed", 0, 7), ("fgmres", "fp64", 256, 0), ("fgmres", "fp64", 256, 6),
+                          ("fgmres", "fp64", 0, 4095), ("cg", "fp64", 0, 1), ("cg", "fp64", 0, 4095)])
+def test_a_late_copy_ends_the_solve_without_a_result(krylov, precision, rows, step):
+    """Where a step's operands do not come in time (FENG_ILU_LATE_STEP: a step
+    that counts as late) the whole of z is NaN, whatever lay in the stage, the
+    solve says that it is not finite, and the GPU goes on working.  Steps
+    among those asked for at the start, behind them and far behind them; one
+    that does not exist changes nothing."""
+    r = subprocess.run([sys.executable, "-c", LATE, precision, str(rows), krylov], cwd=ROOT,
+                       env=dict(os.environ, FENG_ILU_LATE_STEP=str(step)), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    finite, n, status, matrix = json.loads(r.stdout.splitlines()[-1])
+    assert n > 0 and matrix
+    assert (finite, status) == ((n, 0) if step == 4095 else (0, -7))
