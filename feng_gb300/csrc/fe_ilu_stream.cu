@@ -2,7 +2,6 @@
 #include "fe_ilu_stream.h"
 
 #include <algorithm>
-#include <climits>
 #include <cmath>
 #include <cstdlib>
 
@@ -29,7 +28,7 @@ constexpr int STAGES = 3;
 constexpr int WARPS = WORKERS / 32;
 constexpr int LONG_ROW = 8;        // rows with more entries take LONG_SLOTS slots, the others two
 constexpr int LONG_SLOTS = 4;
-constexpr unsigned NO_ROW = 0xffffu;  // above every block's rows
+constexpr unsigned NO_ROW = 0xffffu;
 constexpr int MAX_STEPS = 4096;    // of one block (shared memory)
 constexpr size_t MAX_SMEM = 226 * 1024;
 enum : uint8_t { STEP_FIRST = 1, STEP_LAST = 2, STEP_SCALE = 4 };
@@ -105,10 +104,14 @@ __device__ __forceinline__ void load_if(bool on, const double *p, double &v)
 // writes.
 // Bound: the chain of levels (FP64 products and exchanges, about 700 cycles;
 // gathers, the next step's operands and the barrier, as many).  64 x 64 P2
-// diffusion (16 k rows, 254 levels per triangle): 0.34 ms per application; six
+// diffusion (16 k rows, 254 levels per triangle): 0.33 ms per application; six
 // products in a chain and copies by half of the threads 0.42, a warp per row
 // and the vector in global memory 3.75.
-template <typename V>
+// MANY: more than one block.  The copying warp's lanes then meet after their
+// wait: apart they take issue slots from the SM's other blocks (256 x 256
+// Kovasznay, blocks of 256 rows, FP64 434 -> 360 us, FP32 357 -> 307); alone on
+// its SM a block is faster without (329 against 335, 243 against 257).
+template <typename V, bool MANY>
 __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *__restrict__ steps,
                                                         const int32_t *__restrict__ stepStart,
                                                         const int32_t *__restrict__ start,
@@ -122,20 +125,25 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
   if(done && *done) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const int b = blockIdx.x, tid = threadIdx.x;
-  const int32_t p0 = start[b];
-  const unsigned n = start[b + 1] - p0;
+  const int32_t p0 = start[b], n = start[b + 1] - p0;
   const int32_t s0 = stepStart[b], ns = stepStart[b + 1] - s0;
   Stage<V> *stage = reinterpret_cast<Stage<V> *>(smem);
   V *x = reinterpret_cast<V *>(smem + STAGES * sizeof(Stage<V>));
   IluStream::Step *st = reinterpret_cast<IluStream::Step *>(
       smem + STAGES * sizeof(Stage<V>) + (((size_t)n * sizeof(V) + 15) & ~(size_t)15));
   __shared__ uint64_t full[STAGES];
-  __shared__ int late;  // a copy did not come
+  // A copy did not come.  The solving threads run on (to ask at each step costs 4
+  // to 9% of an application, as a flag or in the barrier): a stage's columns hold
+  // indices of the block at any time, those set here or an earlier step's.
+  __shared__ volatile int late;
   if(tid == 0) {
     late = 0;
     for(int k = 0; k < STAGES; ++k) bar_init(full + k);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for(int i = tid; i < STAGES * WORKERS; i += THREADS)
+    stage[i / WORKERS].col[i % WORKERS] = make_uint4(0, 0, 0, NO_ROW << 16);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies come after
   for(int i = tid; i < ns; i += THREADS) st[i] = steps[s0 + i];
   for(int i0 = tid; i0 < n; i0 += 8 * THREADS) {
     V t[8];
@@ -147,48 +155,44 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
   }
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
-  // the copying warp: lane k < E brings the warps' entries k, lane E the columns
+  // the copying warp: lane k < E brings the warps' entries k, lane E the columns.
+  // Steps below `asked` have been asked for; a copy that did not come ends that.
+  int asked = 0;
   auto copy = [&](int q) {
     if(q >= ns) return;
     const IluStream::Step s = st[q];
+    if(late) return;
+    asked = q + 1;
     Stage<V> &g = stage[q % STAGES];
     const int pre = lane <= E ? lane : E;
     int before = 0, own = 0;  // warps with an entry j < pre, with entry lane
+    const unsigned lanes = s.lanes;
 #pragma unroll
-    for(int w = 0; w < WARPS; ++w) {
-      const int chain = (s.chains >> (4 * w)) & 15;
-      before += min(chain, pre);
-      own += chain > lane;
+    for(int j = 0; j < E; ++j) {
+      // nibbles (at most E) above j
+      const int c = __popc((s.chains + (7u - j) * 0x11111111u) & 0x88888888u);
+      before += j < pre ? c : 0;
+      own = j == lane ? c : own;
     }
-    const void *src = val + s.entry + 32 * before;
+    const void *src = val + s.entry + (int)lanes * before;
     void *dst = &g.val[lane < E ? lane : 0][0];
-    unsigned bytes = lane < E ? 32u * own * (unsigned)sizeof(V) : 0u;
+    unsigned bytes = lane < E ? lanes * own * (unsigned)sizeof(V) : 0u;
     if(lane == E) {
       src = col + s.slot;
       dst = &g.col[0];
-      bytes = 32u * s.warps * 16u;
+      bytes = lanes * s.warps * 16u;
+      bar_expect(full + q % STAGES, bytes + lanes * before * (unsigned)sizeof(V));
     }
-    const unsigned all = __reduce_add_sync(0xffffffffu, bytes);
-    if(lane == 0) bar_expect(full + q % STAGES, all);
     __syncwarp();
     if(bytes) bulk_copy(dst, src, bytes, full + q % STAGES);
   };
   auto phase = [](int q) { return (unsigned)(q / STAGES) & 1u; };
-  // until step q's operands are there; the barrier that follows tells the others.
-  // When they do not come (lateStep: a step that counts as late, to test this),
-  // the copying warp asks for nothing more, and there is no result at the end.
-  int missing = INT_MAX;  // the first step that has not come
+  // until step q's operands are there; the barrier that follows tells the others
+  // (lateStep: a step that counts as late, to test what follows)
   auto arrived = [&](int q) {
-    const bool here = q >= ns || (q != lateStep && bar_wait(full + q % STAGES, phase(q)));
-    if(__all_sync(0xffffffffu, here) || missing != INT_MAX) return;
-    missing = q;
-    if(lane == 0) late = 1;
+    if(q < asked && (q == lateStep || !bar_wait(full + q % STAGES, phase(q)))) late = 1;
+    if constexpr(MANY) __syncwarp();
   };
-  // The solving threads run on without asking whether a step's operands came
-  // (that costs 4 to 9% of an application, as a flag or in the barrier): the
-  // indices that they take from a stage are bounded by the vector's length, so
-  // what lies in a stage that was not filled reads and writes entries of it.
-  const unsigned top = (unsigned)(n - 1) | (unsigned)(n - 1) << 16;
   // the solving threads: the next step's operands, and what the slot starts from
   uint4 c4 = make_uint4(0, 0, 0, 0);
   V v[E], acc = 0, rhs = 0;
@@ -200,14 +204,11 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
     if(warp >= s.warps) return;
     const Stage<V> &g = stage[q % STAGES];
     c4 = g.col[tid];
-    c4.x = __vminu2(c4.x, top);
-    c4.y = __vminu2(c4.y, top);
-    c4.z = __vminu2(c4.z, top);
 #pragma unroll
     for(int k = 0; k < E; ++k) load_if(k < (int)((s.chains >> (4 * warp)) & 15), &g.val[k][tid], v[k]);
     const unsigned row = c4.w >> 16;
     const int last = (s.wide >> warp) & 1 ? LONG_SLOTS - 1 : 1;
-    const V own = x[row < n ? row : 0];
+    const V own = x[row != NO_ROW ? row : 0];
     rhs = (tid & last) == last ? own : (V)0;
   };
   if(warp == WARPS) {
@@ -219,19 +220,15 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
   __syncthreads();
   if(warp < WARPS) fetch(0);
   __syncthreads();
-  int asked = STAGES;
   for(int q = 0; q < ns; ++q) {
     if(warp == WARPS) {
-      if(missing == INT_MAX) {
-        copy(q + STAGES);  // into the stage of this step, whose operands are in registers
-        asked = q + STAGES + 1;
-        arrived(q + 2);
-      }
+      copy(q + STAGES);  // into the stage of this step, whose operands are in registers
+      arrived(q + 2);
     } else if(warp < s.warps) {
       const unsigned cw[4] = {c4.x, c4.y, c4.z, c4.w};
       const unsigned row = c4.w >> 16;
       const int chain = (s.chains >> (4 * warp)) & 15;
-      const bool wide = (s.wide >> warp) & 1, end = s.flags & STEP_LAST;
+      const bool wide = (s.wide >> warp) & 1, end = s.flags & STEP_LAST, stored = lane < s.lanes;
       V xv[E];
 #pragma unroll
       for(int k = 0; k < E; ++k) load_if(k < chain, x + ((cw[k >> 1] >> (16 * (k & 1))) & 0xffffu), xv[k]);
@@ -245,7 +242,7 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
         if(wide)
 #pragma unroll
           for(int o = 2; o < LONG_SLOTS; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if(row < n && !(tid & (wide ? LONG_SLOTS - 1 : 1))) x[row] = acc;
+        if(stored && row != NO_ROW && !(tid & (wide ? LONG_SLOTS - 1 : 1))) x[row] = acc;
       }
     } else {
       if(s.flags & STEP_SCALE) {
@@ -261,27 +258,50 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
   if(late) {  // no result: the caller sees that it is not finite
     for(int i = tid; i < n; i += THREADS) z[perm[p0 + i]] = (V)NAN;
     if(warp == WARPS)  // the copies in flight
-      for(int k = missing; k < min(ns, asked); ++k) bar_wait(full + k % STAGES, phase(k));
+      for(int k = max(0, asked - STAGES); k < asked; ++k) bar_wait(full + k % STAGES, phase(k));
     return;
   }
   for(int i = tid; i < n; i += THREADS) z[perm[p0 + i]] = x[i];
 }
 
 // The packed values: L as it is, U divided by its row's diagonal, and the
-// inverse diagonal by row.
+// inverse diagonal by row.  A warp per step (and warp of the step, grid y),
+// which finds the factor's entries from the rows of its slots.
 template <typename V>
-__global__ void k_ilu_pack(int64_t ne, const int32_t *__restrict__ pos, const int32_t *__restrict__ dpos,
-                           const V *__restrict__ f, V *__restrict__ val, int64_t nrows,
-                           const int32_t *__restrict__ rowDiag, V *__restrict__ scale)
+__global__ void __launch_bounds__(256) k_ilu_pack(int64_t nSteps, const IluStream::Step *__restrict__ steps,
+                                                  const int2 *__restrict__ from, const uint4 *__restrict__ col,
+                                                  const int32_t *__restrict__ perm, const int32_t *__restrict__ lia,
+                                                  const int32_t *__restrict__ ldiag, const V *f,
+                                                  V *__restrict__ val, int64_t nRows, V *__restrict__ scale)
 {
   FE_PDL_ENTRY();
-  for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
-    V v = pos[e] >= 0 ? f[pos[e]] : (V)0;
-    if(pos[e] >= 0 && dpos[e] >= 0) v /= f[dpos[e]];
-    val[e] = v;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if(blockIdx.y == 0)
+    for(int64_t q = t; q < nRows; q += (int64_t)gridDim.x * blockDim.x) scale[q] = (V)1 / f[ldiag[perm[q]]];
+  const int64_t q = t >> 5;
+  if(q >= nSteps) return;
+  const IluStream::Step s = steps[q];
+  const int w = blockIdx.y, lane = (int)(t & 31);
+  if(w >= s.warps || lane >= s.lanes) return;
+  const int2 at = from[q];  // the block's first row, the step's chunk of its rows (odd: of L)
+  const bool lower = at.y & 1;
+  const int slots = (s.wide >> w) & 1 ? LONG_SLOTS : 2;
+  const unsigned row = col[s.slot + 32 * w + lane].w >> 16;
+  int32_t e = 0, end = 0;
+  V inv = 1;
+  if(row != NO_ROW) {
+    const int32_t i = perm[at.x + (int)row], d = ldiag[i];
+    e = (lower ? lia[i] : d + 1) + slots * (at.y >> 1) * E + lane % slots;
+    end = lower ? d : lia[i + 1];
+    if(!lower) inv = f[d];
   }
-  for(int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nrows; q += (int64_t)gridDim.x * blockDim.x)
-    scale[q] = (V)1 / f[rowDiag[q]];
+  int64_t dst = s.entry + 32 * w + lane;
+  for(int k = 0; k < (int)((s.chains >> (4 * w)) & 15); ++k, e += slots) {
+    V v = e < end ? f[e] : (V)0;
+    if(e < end && !lower) v /= inv;
+    val[dst] = v;
+    for(int u = 0; u < WARPS; ++u) dst += ((s.chains >> (4 * u)) & 15) > k ? s.lanes : 0;
+  }
 }
 
 template <typename T>
@@ -292,13 +312,23 @@ int to_device(T **dst, const std::vector<T> &v)
   return FE_OK;
 }
 
+// The steps of some consecutive blocks.
+struct Packed {
+  std::vector<IluStream::Step> steps;
+  std::vector<int2> from;          // k_ilu_pack
+  std::vector<uint4> col;
+  std::vector<int32_t> count;      // steps of each block
+  int64_t entries = 0;
+  size_t smem = 0;
+  bool fits = true;
+};
+
 }  // namespace
 
 IluStream::~IluStream()
 {
-  cudaFree(steps_); cudaFree(stepStart_); cudaFree(start_); cudaFree(perm_);
-  cudaFree(col_); cudaFree(pos_); cudaFree(dpos_); cudaFree(val_);
-  cudaFree(rowDiag_); cudaFree(scale_);
+  cudaFree(steps_); cudaFree(from_); cudaFree(stepStart_); cudaFree(start_); cudaFree(perm_);
+  cudaFree(col_); cudaFree(val_); cudaFree(scale_);
 }
 
 int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t> &lja,
@@ -319,156 +349,172 @@ int IluStream::build(const std::vector<int32_t> &lia, const std::vector<int32_t>
   }
   // the vector's order: a block's rows by levels of L, so that the rows of a
   // warp read neighbouring entries (fewer bank conflicts)
-  std::vector<int32_t> local(n), order(n);
-  std::vector<Step> steps;
-  std::vector<int32_t> stepStart(1, 0), pos, dpos, rowDiag(n), level(n, 0);
-  std::vector<uint4> col;
-  pos.reserve(2 * lja.size());
-  dpos.reserve(2 * lja.size());
-  col.reserve(6 * (size_t)n);
-  std::vector<int32_t> cnt, ord;
-  // a warp of a level: rows ord[first] .. ord[first + rows - 1], `slots` each
-  struct Warp {
-    int32_t first, rows, slots, chain;
-  };
-  std::vector<Warp> warps;
-  for(int64_t b = 0; b < nBlocks_; ++b) {
-    const int32_t p0 = start[b], p1 = start[b + 1];
-    for(int lower = 1; lower >= 0; --lower) {
-      // levels (the block's rows ascend in perm)
-      int32_t nl = 0;
-      for(int32_t k = 0; k < p1 - p0; ++k) {
-        const int32_t i = perm[lower ? p0 + k : p1 - 1 - k];
-        const int32_t kb = lower ? lia[i] : ldiag[i] + 1, ke = lower ? ldiag[i] : lia[i + 1];
-        int32_t m = 0;
-        for(int32_t e = kb; e < ke; ++e) m = std::max(m, level[lja[e]] + 1);
-        level[i] = m;
-        nl = std::max(nl, m + 1);
-      }
-      cnt.assign(nl + 1, 0);
-      for(int32_t q = p0; q < p1; ++q) cnt[level[perm[q]] + 1]++;
-      for(int32_t l = 0; l < nl; ++l) cnt[l + 1] += cnt[l];
-      ord.resize(p1 - p0);
-      {
-        std::vector<int32_t> fill(cnt.begin(), cnt.end() - 1);
-        for(int32_t q = p0; q < p1; ++q) ord[fill[level[perm[q]]]++] = perm[q];
-      }
-      auto len = [&](int32_t i) { return lower ? ldiag[i] - lia[i] : lia[i + 1] - ldiag[i] - 1; };
-      for(int32_t l = 0; l < nl; ++l)  // rows of similar length together
-        std::stable_sort(ord.begin() + cnt[l], ord.begin() + cnt[l + 1],
-                         [&](int32_t x, int32_t y) { return len(x) > len(y); });
-      if(lower)
-        for(int32_t q = 0; q < p1 - p0; ++q) {
-          order[p0 + q] = ord[q];
-          local[ord[q]] = q;
-          rowDiag[p0 + q] = ldiag[ord[q]];
+  std::vector<int32_t> local(n), order(n), level(n, 0);
+  auto pack = [&](int64_t b0, int64_t b1, Packed &P) {
+    std::vector<int32_t> cnt, ord;
+    // a warp of a level: rows ord[first] .. ord[first + rows - 1], `slots` each
+    struct Warp {
+      int32_t first, rows, slots, chain;
+    };
+    std::vector<Warp> warps;
+    for(int64_t b = b0; b < b1 && P.fits; ++b) {
+      const int32_t p0 = start[b], p1 = start[b + 1];
+      const size_t first = P.steps.size();
+      for(int lower = 1; lower >= 0; --lower) {
+        // levels (the block's rows ascend in perm)
+        int32_t nl = 0;
+        for(int32_t k = 0; k < p1 - p0; ++k) {
+          const int32_t i = perm[lower ? p0 + k : p1 - 1 - k];
+          const int32_t kb = lower ? lia[i] : ldiag[i] + 1, ke = lower ? ldiag[i] : lia[i + 1];
+          int32_t m = 0;
+          for(int32_t e = kb; e < ke; ++e) m = std::max(m, level[lja[e]] + 1);
+          level[i] = m;
+          nl = std::max(nl, m + 1);
         }
-      for(int32_t l = 0; l < nl; ++l) {
-        warps.clear();
-        for(int32_t r0 = cnt[l]; r0 < cnt[l + 1];) {
-          const int slots = len(ord[r0]) > LONG_ROW ? LONG_SLOTS : 2;
-          int32_t r1 = r0 + 1;
-          while(r1 < cnt[l + 1] && r1 - r0 < 32 / slots && (slots == 2 || len(ord[r1]) > LONG_ROW)) ++r1;
-          warps.push_back({r0, r1 - r0, slots, (len(ord[r0]) + slots - 1) / slots});
-          r0 = r1;
+        cnt.assign(nl + 1, 0);
+        for(int32_t q = p0; q < p1; ++q) cnt[level[perm[q]] + 1]++;
+        for(int32_t l = 0; l < nl; ++l) cnt[l + 1] += cnt[l];
+        ord.resize(p1 - p0);
+        {
+          std::vector<int32_t> fill(cnt.begin(), cnt.end() - 1);
+          for(int32_t q = p0; q < p1; ++q) ord[fill[level[perm[q]]]++] = perm[q];
         }
-        std::stable_sort(warps.begin(), warps.end(), [](const Warp &x, const Warp &y) { return x.chain > y.chain; });
-        for(size_t w0 = 0; w0 < warps.size(); w0 += WARPS) {
-          const int nw = (int)std::min<size_t>(WARPS, warps.size() - w0);
-          const int chunks = std::max(1, (warps[w0].chain + E - 1) / E);
-          for(int c = 0; c < chunks; ++c) {
-            Step st = {};
-            st.entry = (int32_t)pos.size();
-            st.slot = (int32_t)col.size();
-            st.warps = (uint8_t)nw;
-            st.flags = (uint8_t)((c == 0 ? STEP_FIRST : 0) | (c + 1 == chunks ? STEP_LAST : 0));
-            for(int w = 0; w < nw; ++w)
-              if(warps[w0 + w].slots != 2) st.wide |= (uint8_t)(1u << w);
-            // row, first entry and end of lane t of warp w (row -1: none)
-            auto lane = [&](int w, int t, int32_t &i, int32_t &e, int32_t &end, int &slots) {
-              const Warp &W = warps[w0 + w];
-              slots = W.slots;
-              i = t / slots < W.rows ? ord[W.first + t / slots] : -1;
-              e = i < 0 ? 0 : (lower ? lia[i] : ldiag[i] + 1) + slots * c * E + t % slots;
-              end = i < 0 ? 0 : (lower ? ldiag[i] : lia[i + 1]);
-            };
-            for(int w = 0; w < nw; ++w)
-              st.chains |= (uint32_t)std::max(0, std::min<int>(E, warps[w0 + w].chain - c * E)) << (4 * w);
-            for(int k = 0; k < E; ++k) {
-              int g = 0;
-              while(g < nw && warps[w0 + g].chain > c * E + k) ++g;
-              for(int t = 0; t < 32 * g; ++t) {
-                int32_t i, e, end;
-                int slots;
-                lane(t / 32, t % 32, i, e, end, slots);
-                const bool ok = i >= 0 && e + slots * k < end;
-                pos.push_back(ok ? e + slots * k : -1);
-                dpos.push_back(ok && !lower ? ldiag[i] : -1);
+        auto len = [&](int32_t i) { return lower ? ldiag[i] - lia[i] : lia[i + 1] - ldiag[i] - 1; };
+        for(int32_t l = 0; l < nl; ++l)  // rows of similar length together
+          std::stable_sort(ord.begin() + cnt[l], ord.begin() + cnt[l + 1],
+                           [&](int32_t x, int32_t y) { return len(x) > len(y); });
+        if(lower)
+          for(int32_t q = 0; q < p1 - p0; ++q) {
+            order[p0 + q] = ord[q];
+            local[ord[q]] = q;
+          }
+        for(int32_t l = 0; l < nl; ++l) {
+          warps.clear();
+          for(int32_t r0 = cnt[l]; r0 < cnt[l + 1];) {
+            const int slots = len(ord[r0]) > LONG_ROW ? LONG_SLOTS : 2;
+            int32_t r1 = r0 + 1;
+            while(r1 < cnt[l + 1] && r1 - r0 < 32 / slots && (slots == 2 || len(ord[r1]) > LONG_ROW)) ++r1;
+            warps.push_back({r0, r1 - r0, slots, (len(ord[r0]) + slots - 1) / slots});
+            r0 = r1;
+          }
+          std::stable_sort(warps.begin(), warps.end(), [](const Warp &x, const Warp &y) { return x.chain > y.chain; });
+          for(size_t w0 = 0; w0 < warps.size(); w0 += WARPS) {
+            const int nw = (int)std::min<size_t>(WARPS, warps.size() - w0);
+            const int chunks = std::max(1, (warps[w0].chain + E - 1) / E);
+            // a warp alone keeps the lanes that it uses (copies of 16 bytes)
+            const int pad = 16 / (int)vs - 1, lanes = nw > 1 ? 32 : (warps[w0].rows * warps[w0].slots + pad) & ~pad;
+            for(int c = 0; c < chunks; ++c) {
+              Step st = {};
+              st.entry = (int32_t)P.entries;
+              st.slot = (int32_t)P.col.size();
+              st.warps = (uint8_t)nw;
+              st.lanes = (uint8_t)lanes;
+              st.flags = (uint8_t)((c == 0 ? STEP_FIRST : 0) | (c + 1 == chunks ? STEP_LAST : 0));
+              for(int w = 0; w < nw; ++w) {
+                const Warp &W = warps[w0 + w];
+                const int chain = std::max(0, std::min<int>(E, W.chain - c * E));
+                if(W.slots != 2) st.wide |= (uint8_t)(1u << w);
+                st.chains |= (uint32_t)chain << (4 * w);
+                P.entries += chain * lanes;
+                for(int t = 0; t < lanes; ++t) {
+                  // row, first entry and end of the lane (row -1: none)
+                  const int32_t i = t / W.slots < W.rows ? ord[W.first + t / W.slots] : -1;
+                  const int32_t e = i < 0 ? 0 : (lower ? lia[i] : ldiag[i] + 1) + W.slots * c * E + t % W.slots;
+                  const int32_t end = i < 0 ? 0 : (lower ? ldiag[i] : lia[i + 1]);
+                  uint32_t x[4] = {0, 0, 0, (i >= 0 ? (uint32_t)local[i] : NO_ROW) << 16};
+                  for(int k = 0; k < E && i >= 0; ++k) {
+                    // padding (value 0) reads the row's own entry of the vector
+                    const int32_t j = e + W.slots * k < end ? local[lja[e + W.slots * k]] : local[i];
+                    x[k >> 1] |= (uint32_t)j << (16 * (k & 1));
+                  }
+                  P.col.push_back(make_uint4(x[0], x[1], x[2], x[3]));
+                }
               }
+              P.steps.push_back(st);
+              P.from.push_back(make_int2(p0, 2 * c + lower));
             }
-            for(int t = 0; t < 32 * nw; ++t) {
-              int32_t i, e, end;
-              int slots;
-              lane(t / 32, t % 32, i, e, end, slots);
-              uint32_t w[4] = {0, 0, 0, (i >= 0 ? (uint32_t)local[i] : NO_ROW) << 16};
-              for(int k = 0; k < E && i >= 0; ++k) {
-                // padding (value 0) reads the row's own entry of the vector
-                const int32_t j = e + slots * k < end ? local[lja[e + slots * k]] : local[i];
-                w[k >> 1] |= (uint32_t)j << (16 * (k & 1));
-              }
-              col.push_back(make_uint4(w[0], w[1], w[2], w[3]));
-            }
-            steps.push_back(st);
           }
         }
+        // between the triangles a step without rows, which scales the vector
+        if(lower) {
+          P.steps.push_back(Step{});
+          P.steps.back().flags = STEP_SCALE;
+          P.from.push_back(make_int2(p0, 0));
+        }
       }
-      // between the triangles a step without rows, which scales the vector
-      if(lower) {
-        steps.push_back(Step{});
-        steps.back().flags = STEP_SCALE;
-      }
+      const size_t own = P.steps.size() - first;
+      const size_t need = stages + (((size_t)(p1 - p0) * vs + 15) & ~(size_t)15) + own * sizeof(Step);
+      P.count.push_back((int32_t)own);
+      P.smem = std::max(P.smem, need);
+      P.fits = own <= MAX_STEPS && need <= MAX_SMEM && P.entries <= INT32_MAX / 2;
     }
-    stepStart.push_back((int32_t)steps.size());
-    const int32_t own = stepStart[b + 1] - stepStart[b];
-    const size_t need = stages + (((size_t)(p1 - p0) * vs + 15) & ~(size_t)15) + (size_t)own * sizeof(Step);
-    if(own > MAX_STEPS || need > MAX_SMEM || pos.size() > (size_t)INT32_MAX / 2) return FE_OK;
-    smem_ = std::max(smem_, need);
+  };
+  // blocks are independent: packed by ranges, side by side
+  const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(nBlocks_, 64));
+  std::vector<Packed> P(parts);
+  parallel_for(parts, [&](int64_t q0, int64_t q1) {
+    for(int64_t q = q0; q < q1; ++q) pack(nBlocks_ * q / parts, nBlocks_ * (q + 1) / parts, P[q]);
+  }, 1);
+  size_t nCol = 0;
+  nSteps_ = nEntries_ = 0;
+  maxWarps_ = 1;
+  std::vector<int32_t> stepStart(1, 0);
+  for(Packed &p : P) {
+    for(Step &st : p.steps) {
+      st.entry += (int32_t)nEntries_;
+      st.slot += (int32_t)nCol;
+      maxWarps_ = std::max<int>(maxWarps_, st.warps);
+    }
+    for(int32_t c : p.count) stepStart.push_back(stepStart.back() + c);
+    nSteps_ += (int64_t)p.steps.size();
+    nEntries_ += p.entries;
+    nCol += p.col.size();
+    smem_ = std::max(smem_, p.smem);
+    if(!p.fits || nEntries_ > INT32_MAX / 2) return FE_OK;
   }
-  nEntries_ = (int64_t)pos.size();
   nRows_ = n;
-  FE_TRY(to_device(&steps_, steps));
+  CKI(cudaMalloc(&steps_, sizeof(Step) * std::max<int64_t>(1, nSteps_)));
+  CKI(cudaMalloc(&from_, sizeof(int2) * std::max<int64_t>(1, nSteps_)));
+  CKI(cudaMalloc(&col_, sizeof(uint4) * std::max<size_t>(1, nCol)));
+  size_t s0 = 0, c0 = 0;
+  for(const Packed &p : P) {
+    CKI(cudaMemcpy(steps_ + s0, p.steps.data(), sizeof(Step) * p.steps.size(), cudaMemcpyHostToDevice));
+    CKI(cudaMemcpy(from_ + s0, p.from.data(), sizeof(int2) * p.from.size(), cudaMemcpyHostToDevice));
+    CKI(cudaMemcpy(col_ + c0, p.col.data(), sizeof(uint4) * p.col.size(), cudaMemcpyHostToDevice));
+    s0 += p.steps.size();
+    c0 += p.col.size();
+  }
   FE_TRY(to_device(&stepStart_, stepStart));
   FE_TRY(to_device(&start_, start));
   FE_TRY(to_device(&perm_, order));
-  FE_TRY(to_device(&col_, col));
-  FE_TRY(to_device(&pos_, pos));
-  FE_TRY(to_device(&dpos_, dpos));
-  FE_TRY(to_device(&rowDiag_, rowDiag));
   CKI(cudaMalloc(&val_, vs * std::max<int64_t>(1, nEntries_)));
   CKI(cudaMalloc(&scale_, vs * std::max<int64_t>(1, nRows_)));
   // the copies ran on the legacy stream, with which s is not ordered
   CKI(cudaStreamSynchronize(cudaStreamLegacy));
-  if(fp32) CKI(cudaFuncSetAttribute(k_ilu_stream<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-  else CKI(cudaFuncSetAttribute(k_ilu_stream<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
+  const auto opt_in = [](auto kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM);
+  };
+  if(fp32) CKI(nBlocks_ > 1 ? opt_in(k_ilu_stream<float, true>) : opt_in(k_ilu_stream<float, false>));
+  else CKI(nBlocks_ > 1 ? opt_in(k_ilu_stream<double, true>) : opt_in(k_ilu_stream<double, false>));
   usable_ = true;
   return FE_OK;
 }
 
-void IluStream::gather(const void *f)
+void IluStream::gather(const void *f, const int32_t *lia, const int32_t *ldiag)
 {
-  const int g = (int)std::max<int64_t>(1, std::min<int64_t>((nEntries_ + 255) / 256, 4096));
-  if(fp32_)
-    ::feng::launch_k(k_ilu_pack<float>, g, 256, 0, s_, nEntries_, pos_, dpos_, (const float *)f, (float *)val_, nRows_,
-                     rowDiag_, (float *)scale_);
-  else
-    ::feng::launch_k(k_ilu_pack<double>, g, 256, 0, s_, nEntries_, pos_, dpos_, (const double *)f, (double *)val_,
-                     nRows_, rowDiag_, (double *)scale_);
+  const dim3 g((unsigned)std::max<int64_t>(1, (nSteps_ + 7) / 8), (unsigned)maxWarps_);
+  auto go = [&](auto kernel, auto *v, auto *scale, auto *fv) {
+    ::feng::launch_k(kernel, g, 256, 0, s_, nSteps_, steps_, from_, col_, perm_, lia, ldiag, fv, v, nRows_, scale);
+  };
+  if(fp32_) go(k_ilu_pack<float>, (float *)val_, (float *)scale_, (const float *)f);
+  else go(k_ilu_pack<double>, (double *)val_, (double *)scale_, (const double *)f);
 }
 
 template <typename V>
 void IluStream::launch(const V *r, V *z, const int *done) const
 {
-  ::feng::launch_k(k_ilu_stream<V>, (int)nBlocks_, THREADS, smem_, s_, steps_, stepStart_, start_, perm_, col_,
+  auto kernel = nBlocks_ > 1 ? k_ilu_stream<V, true> : k_ilu_stream<V, false>;
+  ::feng::launch_k(kernel, (int)nBlocks_, THREADS, smem_, s_, steps_, stepStart_, start_, perm_, col_,
                    (const V *)val_, (const V *)scale_, r, z, done, lateStep_);
 }
 

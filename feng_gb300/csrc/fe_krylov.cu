@@ -1541,13 +1541,20 @@ int Krylov::setup(const DeviceCSR &A, const std::vector<int32_t> &blockOfRow, in
     CK(cudaMemcpy(ilu_.lja, lja.data(), sizeof(int32_t) * ilu_.lnnz, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ilu_.ldiag, ldiag.data(), sizeof(int32_t) * n_, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ilu_.srcPos, src.data(), sizeof(int32_t) * ilu_.lnnz, cudaMemcpyHostToDevice));
-    // diagonal blocks whose vector fits in shared memory (about 21 k rows in FP64)
-    // are solved there; the level kernels stay for larger ones
-    ilus_ = new IluStream();
-    FE_TRY(ilus_->build(lia, lja, ldiag, perm, bstart, opt.mixed != 0, s_));
-    if(!ilus_->usable()) {
-      delete ilus_;
-      ilus_ = nullptr;
+    // Diagonal blocks whose vector fits in shared memory (about 21 k rows in FP64)
+    // are solved there, a thread block each; the level kernels, which take a level
+    // of all blocks at once, stay for larger ones and for many small ones.  us per
+    // application, blocks / levels, rows per block on average: Kovasznay 256^2
+    // FP64 16 rows 1258 / 1210, 24 779 / 1221, 256 361 / 1627; FP32 64 rows
+    // 424 / 321, 96 357 / 359, 256 308 / 555; P2 diffusion 256^2 FP64 16 rows
+    // 387 / 373, 24 252 / 386, 256 231 / 747; FP32 64 rows 166 / 157, 96 153 / 194.
+    if(nb == 1 || n_ >= nb * (opt.mixed ? 96 : 24)) {
+      ilus_ = new IluStream();
+      FE_TRY(ilus_->build(lia, lja, ldiag, perm, bstart, opt.mixed != 0, s_));
+      if(!ilus_->usable()) {
+        delete ilus_;
+        ilus_ = nullptr;
+      }
     }
     FE_TRY(build_ilu_levels(lia, lja, ldiag));
   }
@@ -1698,7 +1705,7 @@ int Krylov::factor(const double *values64, const float *values32)
   } else {
     if(opt.mixed) ilu_factor_levels<float>(nullptr, values32);
     else ilu_factor_levels<double>(values64, nullptr);
-    if(ilus_) ilus_->gather(ilu_.vals);
+    if(ilus_) ilus_->gather(ilu_.vals, ilu_.lia, ilu_.ldiag);
   }
   CK(cudaGetLastError());
   int hs = 0;

@@ -150,3 +150,51 @@ def test_a_late_copy_ends_the_solve_without_a_result(krylov, precision, rows, st
     finite, n, status, matrix = json.loads(r.stdout.splitlines()[-1])
     assert n > 0 and matrix
     assert (finite, status) == ((n, 0) if step == 4095 else (0, -7))
+
+
+def _block_entries(s, blocks):
+    ia, ja = s.pattern()
+    return int(np.sum(blocks[np.repeat(np.arange(s.nInc), np.diff(ia))] == blocks[ja]))
+
+
+@pytest.mark.parametrize("rows", [8, 24, 256])
+def test_block_jacobi_memory_stays_near_the_factor(rows):
+    """A system of many diagonal blocks holds, beside the factor (FP64 value,
+    column and position in the matrix: 16 bytes an entry), at most 4 values and
+    1.1 column words (of 16 bytes) an entry packed for the solves, and 64 bytes a
+    row of schedules.  A count of the packing on this mesh gives 3.2 and 3.7
+    values and 1.0 column words an entry with blocks of 24 and 256 rows (blocks
+    of 8 rows are not packed)."""
+    torch = pytest.importorskip("torch")
+    from feng_gb300 import kovasznay
+    _, num, forms = kovasznay.build(128)
+    blocks = num.setup(rows).blocks()
+    used = {}
+    for precond in ("none", "bjacobi-ilu0", "none", "bjacobi-ilu0"):
+        before = torch.cuda.mem_get_info()[0]
+        s = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(precond=precond, pc_block_rows=rows))
+        used[precond] = before - torch.cuda.mem_get_info()[0]
+        entries = _block_entries(s, blocks)
+        del s
+    extra = used["bjacobi-ilu0"] - used["none"]
+    assert 0 < extra <= (16 + 4 * 8 + 1.1 * 16) * entries + 64 * len(blocks)
+
+
+@pytest.mark.parametrize("rows", [8, 24, 96])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_ilu0_solves_match_serial_over_block_sizes(precision, rows):
+    """Blocks of few rows (by levels), of the fewest that are solved in shared
+    memory (24 rows in FP64, 96 in FP32: a warp alone in most steps, stored
+    with the lanes that it uses) and of more.  Tolerance as for the smaller
+    diffusion systems above: rounding, no growth (1e-12 and 1e-5 of max |z|)."""
+    import scipy.sparse as sp
+    num, forms = problem_spaces("diffusion", fe.Mesh2DP1.generate_square(23, jitter=0.1, seed=2), 40.0)
+    s = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(
+        krylov="fgmres", precond="bjacobi-ilu0", pc_block_rows=rows, precision=precision))
+    s.setToZero()
+    s.assembleMatrices()
+    ia, ja = s.pattern()
+    A = sp.csr_matrix((s.getMatrix(), ja, ia))
+    r = np.random.default_rng(4).uniform(-1, 1, s.nInc)
+    z, ref = s.applyPreconditioner(r), _ilu_reference(A, r, num.setup(rows).blocks())
+    assert np.max(np.abs(z - ref)) <= (1e-12 if precision == "fp64" else 1e-5) * np.max(np.abs(ref))
