@@ -198,3 +198,22 @@ def test_ilu0_solves_match_serial_over_block_sizes(precision, rows):
     r = np.random.default_rng(4).uniform(-1, 1, s.nInc)
     z, ref = s.applyPreconditioner(r), _ilu_reference(A, r, num.setup(rows).blocks())
     assert np.max(np.abs(z - ref)) <= (1e-12 if precision == "fp64" else 1e-5) * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("precision,n", [("fp64", 80), ("mixed", 120)])
+def test_ilu0_block_above_shared_memory_matches_serial(precision, n):
+    """One block of more rows than shared memory holds (25,281 in FP64, 57,121
+    in FP32): solved by levels.  Tolerances of the 64 x 64 system."""
+    num, forms = problem_spaces("diffusion", fe.Mesh2DP1.generate_square(n, jitter=0.1, seed=2))
+    s = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(krylov="fgmres", precond="ilu0",
+                                                                         precision=precision))
+    s.setToZero()
+    s.assembleMatrices()
+    st = num.setup()
+    ia, ja = s.pattern()
+    off, el = st.coloring()
+    g = {"tri": num.mesh.arrays()["tri"], "adr": st.elementDofs(), "nInc": s.nInc, "nDofs": s.nDofs,
+         "color_offsets": off, "color_elements": el, "ia": ia, "ja": ja, "quad_degree": 4}
+    r = np.random.default_rng(3).uniform(-1, 1, s.nInc)
+    z, ref = s.applyPreconditioner(r), _oracle_ilu(g, s.getMatrix(), r)
+    assert np.max(np.abs(z - ref)) <= (1e-12 if precision == "fp64" else 1e-5) * np.max(np.abs(ref))
