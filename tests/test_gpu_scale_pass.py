@@ -53,3 +53,23 @@ def test_pass_inside_and_alone_agree(precision, tmp_path):
     for a, b in zip(*got):
         assert np.all(np.isfinite(a))
         assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)
+
+
+COUNTS = SNIPPET.replace("out.append(s.getDu())", "out.append(st['nIter'])").replace(
+    "np.savez(sys.argv[3], *out)", "print(json.dumps(out))")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pass_inside_and_alone_take_the_same_steps(precision):
+    """A wrong basis vector, rotation or scaled right-hand side that restarts
+    from the true residual repair costs steps: the counts agree to rounding
+    (one step, and in mixed precision one per restart)."""
+    got = []
+    for graphs in ("1", "0"):
+        r = subprocess.run([sys.executable, "-c", COUNTS, precision, json.dumps(SIZES)], cwd=ROOT,
+                           env=dict(os.environ, FENG_CUDA_GRAPHS=graphs), capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-2000:]
+        got.append(json.loads(r.stdout.splitlines()[-1]))
+    for (n, restart), a, b in zip(SIZES, *got):
+        assert min(a, b) > restart or min(a, b) > 5
+        assert abs(a - b) <= (1 if precision == "fp64" else 1 + min(a, b) // restart), (n, restart, a, b)
