@@ -178,6 +178,7 @@ SIGNATURES = {
                                            C.POINTER(P)]),
     "fe_cuda_transient_steps": (C.c_int, [P, C.c_int, P]),
     "fe_cuda_apply_preconditioner": (C.c_int, [P, P, P]),
+    "fe_cuda_apply_matrix": (C.c_int, [P, P, P]),
     "fe_setup_set_quadrature": (C.c_int, [P, C.c_int, P]),
     "fe_cuda_system_create_from_tables_rule": (C.c_int, [C.c_int, C.c_int64, P, P, C.c_int64, C.c_int64, C.c_int, P, P,
                                                           P, P, P, P, C.c_int, P, C.c_int, P, P]),

@@ -529,6 +529,13 @@ class feLinearSystemCUDA:
         check(self.lib.fe_cuda_apply_preconditioner(self._h, ptr(r), ptr(z)))
         return z
 
+    def applyMatrix(self, x):
+        """y = A x as the solver's iterations multiply (in FP32 on the mixed path)."""
+        x = np.ascontiguousarray(x, np.float64)
+        y = np.empty(self.nInc)
+        check(self.lib.fe_cuda_apply_matrix(self._h, ptr(x), ptr(y)))
+        return y
+
     def correctSolution(self):
         check(self.lib.fe_cuda_correct_solution(self._h))
 

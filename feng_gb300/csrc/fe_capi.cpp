@@ -861,6 +861,14 @@ int fe_cuda_apply_preconditioner(fe_cuda_system *s, const double *r, double *z)
   GUARD_END
 }
 
+int fe_cuda_apply_matrix(fe_cuda_system *s, const double *x, double *y)
+{
+  GUARD_BEGIN
+  if(!s || !x || !y) { set_error("null argument"); return FE_INVALID_ARG; }
+  return s->sys.applyMatrix(x, y);
+  GUARD_END
+}
+
 int fe_cuda_get_du(const fe_cuda_system *s, double *du)
 {
   if(!s || !du) { set_error("null argument"); return FE_INVALID_ARG; }

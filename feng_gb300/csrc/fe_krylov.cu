@@ -1781,8 +1781,7 @@ int Krylov::spmvHot()
     set_error("no mixed-precision FGMRES");
     return FE_INVALID_ARG;
   }
-  if(bs_) bs_->mul32(Z32_, w32_, nullptr);
-  else if(cur32_) spmv_launch<float, float, float, float, false>(lanes_, n_, A_, cur32_, Z32_, nullptr, w32_, nullptr, s_);
+  if(bs_ || cur32_) mul32(cur32_, Z32_, w32_, nullptr);
   return FE_OK;
 }
 
@@ -1884,6 +1883,31 @@ __global__ void k_f32_to_f64(int64_t n, const float *__restrict__ x, double *__r
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (double)x[i];
+}
+
+// y = A x in FP32, as an Arnoldi step of the mixed path multiplies.
+void Krylov::mul32(const float *vals, const float *x, float *y, const int *done)
+{
+  if(bs_) bs_->mul32(x, y, done);
+  else spmv_launch<float, float, float, float, false>(lanes_, n_, A_, vals, x, nullptr, y, done, s_);
+}
+
+int Krylov::applyMatrix(const double *x, double *y)
+{
+  if(!factoredOk_) {
+    set_error("preconditioner not built");
+    return FE_PC_FAILED;
+  }
+  if(opt.mixed) {
+    const int gv = grid_for(n_, 256, 2048);
+    ::feng::launch_k(k_to_f32, gv, 256, 0, s_, n_, x, v32_, nullptr);
+    mul32(cur32_, v32_, w32_, nullptr);
+    ::feng::launch_k(k_f32_to_f64, gv, 256, 0, s_, n_, w32_, y);
+  } else {
+    mul64(cur64_, x, y, nullptr);
+  }
+  CK(cudaGetLastError());
+  return FE_OK;
 }
 
 int Krylov::applyPrecond(const double *r, double *z)
@@ -2177,10 +2201,7 @@ void Krylov::mixed_part(const float *vals, const double *b, double *x, int j0, i
     float *zj = Z32_ + (int64_t)j * ld32_;
     precond32(vj, zj, &w.gs->done, fuse && j > j0 ? &sc : nullptr);
     double *Hcol = w.gs->H + (int64_t)j * (MAXM + 1);
-    if(bs_)
-      bs_->mul32(zj, w32_, &w.gs->done);
-    else
-      spmv_launch<float, float, float, float, false>(lanes_, n_, A_, vals, zj, nullptr, w32_, &w.gs->done, s_);
+    mul32(vals, zj, w32_, &w.gs->done);
     if(opt.gsPasses == 2) {
       // always twice: dots, fused update + dots, update + norm
       gs32(0, j + 1, nullptr, w.gs->hcur, Hcol, &w.gs->done, 0);

@@ -127,6 +127,9 @@ class Krylov {
   void spmv32(const float *values, const double *x, double *y);
   // One preconditioner application z = M^-1 r (the FP32 path rounds r).
   int applyPrecond(const double *r, double *z);
+  // One product y = A x of the iteration, on the matrix of the last factor()
+  // (the FP32 path rounds x).
+  int applyMatrix(const double *x, double *y);
   double dot(const double *x, const double *y);
   double norm2(const double *x);
   double norminf(const double *x);
@@ -251,6 +254,7 @@ class Krylov {
   // copy when built, else CSR), FP32 vectors (benchmark phase).
   int spmvHot();
   void resid32(const float *vals, const double *x, const double *b, double *r);
+  void mul32(const float *vals, const float *x, float *y, const int *done);
   // The preconditioner application of an Arnoldi step (the mixed path: the
   // FP32 basis column 0 into Z column 0; FP64 otherwise), reps of them
   // captured in one CUDA graph and replayed (after a warm replay) without

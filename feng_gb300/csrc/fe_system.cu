@@ -1710,29 +1710,44 @@ int SystemCUDA::getRHS(double *hostRhs) const
   return FE_OK;
 }
 
-// One application z = M^-1 r of the current preconditioner (built from the
-// current matrix if that changed), host vectors of nInc entries.
-int SystemCUDA::applyPreconditioner(const double *hostR, double *hostZ)
+// One application of a solver operator (built from the current matrix if that
+// changed), host vectors of nInc entries.
+int SystemCUDA::applyHost(int (Krylov::*f)(const double *, double *), const double *hostIn, double *hostOut)
 {
   FE_TRY(ensureMatrixZeroed());
   FE_TRY(factorIfPending());
-  double *r = nullptr, *z = nullptr;
-  CK(cudaMalloc(&r, sizeof(double) * nInc_));
-  if(cudaMalloc(&z, sizeof(double) * nInc_) != cudaSuccess) {
-    cudaFree(r);
+  double *in = nullptr, *out = nullptr;
+  CK(cudaMalloc(&in, sizeof(double) * nInc_));
+  if(cudaMalloc(&out, sizeof(double) * nInc_) != cudaSuccess) {
+    cudaFree(in);
     set_error("device allocation failed");
     return FE_CUDA_FAIL;
   }
   int st = FE_OK;
-  if(cudaMemcpyAsync(r, hostR, sizeof(double) * nInc_, cudaMemcpyHostToDevice, s_) != cudaSuccess) st = FE_CUDA_FAIL;
-  if(st == FE_OK) st = kry_.applyPrecond(r, z);
-  if(st == FE_OK && cudaMemcpyAsync(hostZ, z, sizeof(double) * nInc_, cudaMemcpyDeviceToHost, s_) != cudaSuccess)
+  if(cudaMemcpyAsync(in, hostIn, sizeof(double) * nInc_, cudaMemcpyHostToDevice, s_) != cudaSuccess) st = FE_CUDA_FAIL;
+  if(st == FE_OK) st = (kry_.*f)(in, out);
+  if(st == FE_OK && cudaMemcpyAsync(hostOut, out, sizeof(double) * nInc_, cudaMemcpyDeviceToHost, s_) != cudaSuccess)
     st = FE_CUDA_FAIL;
   if(cudaStreamSynchronize(s_) != cudaSuccess) st = FE_CUDA_FAIL;
-  cudaFree(r);
-  cudaFree(z);
-  if(st == FE_CUDA_FAIL) set_error("preconditioner application failed on the device");
+  cudaFree(in);
+  cudaFree(out);
+  if(st == FE_CUDA_FAIL) set_error("preconditioner or matrix application failed on the device");
   return st;
+}
+
+// z = M^-1 r with the current preconditioner.
+int SystemCUDA::applyPreconditioner(const double *hostR, double *hostZ)
+{
+  return applyHost(&Krylov::applyPrecond, hostR, hostZ);
+}
+
+// y = A x with the current matrix, as the iteration multiplies.
+int SystemCUDA::applyMatrix(const double *hostX, double *hostY)
+{
+  FE_TRY(ensureMatrixZeroed());
+  if(!factorPending_ && zeroedOut_) kry_.refreshMatrix(vals64_, vals32_);  // as in solve()
+  zeroedOut_ = false;
+  return applyHost(&Krylov::applyMatrix, hostX, hostY);
 }
 
 int SystemCUDA::jacobianTimes(const double *x, double *y)

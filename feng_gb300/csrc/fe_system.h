@@ -112,6 +112,7 @@ class SystemCUDA {
   int getRHS(double *hostRhs) const;
   int getDu(double *hostDu) const;
   int applyPreconditioner(const double *hostR, double *hostZ);
+  int applyMatrix(const double *hostX, double *hostY);
   // y = J x with the Jacobian last assembled (device vectors of nInc
   // entries); FE_INVALID_ARG when no assembled Jacobian is held.
   int jacobianTimes(const double *x, double *y);
@@ -153,6 +154,7 @@ class SystemCUDA {
   int timing = 1;  // record CUDA events around the phases
 
  private:
+  int applyHost(int (Krylov::*f)(const double *, double *), const double *hostIn, double *hostOut);
   int64_t nInc_ = 0, nDofs_ = 0;
   int nloc_ = 0;
   double t_ = 0, c0_ = 0;

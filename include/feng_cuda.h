@@ -379,6 +379,9 @@ int fe_cuda_get_du_max_norm(fe_cuda_system *s, double *norm);
 /* One application z = M^-1 r of the preconditioner (PETSc's PCApply),
  * built from the current matrix first if needed; r, z host arrays [n_inc]. */
 int fe_cuda_apply_preconditioner(fe_cuda_system *s, const double *r, double *z);
+/* y = A x as the solver's iterations multiply (the mixed path: x, the products
+ * and y in FP32), A the current matrix; x, y host arrays [n_inc]. */
+int fe_cuda_apply_matrix(fe_cuda_system *s, const double *x, double *y);
 
 /* ---- Newton driver (solveNewtonRaphson, src/feNonLinearSolver.cpp:38-181) */
 int fe_cuda_newton(fe_cuda_system *s, const fe_newton_options *o, fe_newton_stats *st);

@@ -72,3 +72,26 @@ def test_solve_leaves_the_asked_residual(case, precision):
     assert left <= 1.01e-6 * np.linalg.norm(b)
     # the reported residual: the recurrence's (CG) or the one at the end
     assert st["normAxb"] == pytest.approx(left, rel=1e-2)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_product_matches_rows(case, precision):
+    """The iteration's product itself, row by row: a sum of k products of rounded
+    operands is off by at most (k + 2) roundings of the sum of their magnitudes."""
+    num, forms = CASES[case]()
+    s = fe.createLinearSystem(fe.CUDA, forms, num, fe.LinearSolverOptions(precond="none", precision=precision))
+    assert s.nInc >= 75000
+    rng = np.random.default_rng(5)
+    s.setSolution(rng.uniform(-1, 1, s.nDofs))
+    s.setTime(0.0, 150.0)
+    s.setToZero()
+    s.assembleMatrices()
+    ia, ja = s.pattern()
+    A = sp.csr_matrix((s.getMatrix(), ja, ia))
+    x = rng.uniform(-1, 1, s.nInc)
+    y = s.applyMatrix(x)
+    unit = 2.0 ** (-53 if precision == "fp64" else -24)
+    assert np.all(np.abs(y - A @ x) <= (np.diff(ia) + 2) * unit * (abs(A) @ np.abs(x)))
+    s.setMatrixToZero()  # the copy follows the matrix
+    assert np.all(s.applyMatrix(x) == 0.0)
