@@ -1360,7 +1360,7 @@ Krylov::~Krylov()
   cudaFreeHost(h_gmres_); cudaFreeHost(h_cg_); cudaFreeHost(hflag_); cudaFreeHost(htol_); cudaFreeHost(hdone_);
   for(auto e : evs_) cudaEventDestroy(e);
   for(auto &g : graphs_) cudaGraphExecDestroy(g.second);
-  delete mg_;
+  free_mg();
 }
 
 static int grid_for(int64_t n, int threads, int maxBlocks)

@@ -265,6 +265,7 @@ class Krylov {
   // disabled, so that all m Arnoldi steps run: ms per Arnoldi step, the
   // cycle's residual and update included (benchmark phase; x is scratch).
   int cycleGraph(bool mixed, const void *vals, const double *b, double *x, int reps, double *msPerStep);
+  void free_mg();
   int factor_mg(const double *values64, const float *values32);
   template <typename V> void apply_mg(const V *vals, const V *r, V *z, const int *skip, const ScaleStep<V> *sc);
 };

@@ -632,6 +632,12 @@ int up(T **dst, const std::vector<T> &v)
 
 }  // namespace
 
+void Krylov::free_mg()
+{
+  delete mg_;
+  mg_ = nullptr;
+}
+
 int Krylov::setup_mg(const PrecondInfo &pi)
 {
   if(!pi.lap || pi.lap->n <= 0) {
