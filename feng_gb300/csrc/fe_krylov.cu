@@ -636,14 +636,17 @@ __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const
   const float4 *V4 = reinterpret_cast<const float4 *>(V);
   const int64_t g0 = (int64_t)blockIdx.x * RB + tid;
   // one batch of eight loads in flight (clamped columns, the extra products
-  // dropped by selects); the first ahead of the entry: the kernel before wrote
-  // w, not the basis (a second pass, which mostly returns at once, reads none)
+  // dropped by selects); the first ahead of the entry, where its columns are
+  // older than this step (a second pass, which mostly returns at once, reads none)
   float4 v[8];
   auto load = [&](int64_t g, int c0) {
 #pragma unroll
     for(int u = 0; u < 8; ++u) v[u] = __ldcs(V4 + vidx4(g, cb + (c0 + u < cn ? c0 + u : c0), m1));
   };
-  if(!second && g0 < n4) load(g0, 0);
+  const bool ahead = !second && cb + 8 < ncols;
+  if(ahead && g0 < n4)
+#pragma unroll
+    for(int u = 0; u < 8; ++u) v[u] = __ldcg(V4 + vidx4(g0, cb + u, m1));
   FE_PDL_ENTRY();
   if(*done || (second && !st->reorth)) return;
   float acc[CMAX];
@@ -656,7 +659,7 @@ __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const
 #pragma unroll
     for(int c0 = 0; c0 < CMAX; c0 += 8) {
       if(c0 < cn) {
-        if(c0 || second || g != g0) load(g, c0);
+        if(c0 || !ahead || g != g0) load(g, c0);
 #pragma unroll
         for(int u = 0; u < 8; ++u) {
           const float t = fmaf(v[u].x, x.x, fmaf(v[u].y, x.y, fmaf(v[u].z, x.z, v[u].w * x.w)));
@@ -744,9 +747,9 @@ __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__r
   __shared__ float hs[CMAX];
   __shared__ double wred[RB / 32];
   __shared__ bool last;
-  // the first rows' first batch ahead of the entry: the kernel before formed
-  // the coefficients, not w or the basis
-  const bool ahead = NORM && !second;
+  // the first rows' first batch ahead of the entry, where its columns are older
+  // than this step
+  const bool ahead = NORM && !second && ncols > 8;
   const int64_t g0 = (int64_t)blockIdx.x * RB + threadIdx.x;
   float4 v[8];
   auto load = [&](int64_t g, int c0) {
@@ -755,11 +758,9 @@ __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__r
       v[u] = c0 + u < ncols ? __ldcs(reinterpret_cast<const float4 *>(V) + vidx4(g, c0 + u, m1))
                             : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if(ahead && g0 < n4) {
-    w0 = reinterpret_cast<const float4 *>(w)[g0];
-    load(g0, 0);
-  }
+  if(ahead && g0 < n4)
+#pragma unroll
+    for(int u = 0; u < 8; ++u) v[u] = __ldcg(reinterpret_cast<const float4 *>(V) + vidx4(g0, u, m1));
   FE_PDL_ENTRY();
   if(*done || (NORM && second && !st->reorth)) return;
   for(int c = threadIdx.x; c < CMAX; c += RB) hs[c] = c < ncols ? (float)hprev[c] : 0.f;
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__r
   float q = 0.f;
   for(int64_t g = g0; g < n4; g += (int64_t)gridDim.x * RB) {
     const bool have = ahead && g == g0;
-    float4 wv = have ? w0 : w4[g];
+    float4 wv = w4[g];
     // one batch of eight column loads in flight at a time (unrolled
     // batches would hoist every load and spill)
 #pragma unroll 1

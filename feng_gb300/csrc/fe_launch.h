@@ -9,9 +9,11 @@
 // (a V-cycle's coarse levels, the Gram-Schmidt reductions).  Every kernel
 // launched through launch_k starts with FE_PDL_ENTRY(); kernels launched
 // without the attribute keep the plain stream order.  A kernel may read before
-// that entry what its predecessor does not write (the kernels before that one
-// have finished when it starts): the products of an iteration take their
+// that entry what no kernel of the iteration writes: its products take their
 // operator's first entries there, which hides two dependent latencies of each.
+// Of what is written in the iteration only basis columns older than the step are
+// read there (each kernel waits before it lets the next start, so all kernels but
+// the predecessor have finished), through the L2.
 // What the predecessor does write is read through plain pointers: the compiler
 // may move loads through const __restrict__ ones ahead of the entry.
 // Kovasznay solves 32^2 FP64 51.2 -> 49.2 ms, 97^2 mixed 23.2 -> 21.6, 256^2
