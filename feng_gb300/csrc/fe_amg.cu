@@ -61,7 +61,7 @@ __device__ __forceinline__ Vals<V, NV> ldv(const V *__restrict__ p, int64_t i)
 // entry is used once per product), then the gathers of x.
 template <typename V, int LANES, int NV>
 __device__ __forceinline__ void row_dot(int32_t beg, int32_t end, int sub, const int32_t *__restrict__ ja,
-                                        const V *__restrict__ a, const V *__restrict__ x, V (&acc)[NV])
+                                        const V *__restrict__ a, const V *x, V (&acc)[NV])
 {
   constexpr int UNR = LANES >= 8 ? 4 : 2;
 #pragma unroll
@@ -97,7 +97,7 @@ __device__ __forceinline__ void row_dot(int32_t beg, int32_t end, int sub, const
 template <typename V, int LANES, int NV>
 __device__ __forceinline__ void row_dot_w(int32_t beg, int32_t end, int sub, const int32_t *__restrict__ ja,
                                           const V *__restrict__ a, const V *__restrict__ w,
-                                          const V *__restrict__ x, V (&acc)[NV])
+                                          const V *x, V (&acc)[NV])
 {
   constexpr int UNR = LANES >= 8 ? 4 : 2;
 #pragma unroll
@@ -129,7 +129,7 @@ __device__ __forceinline__ void row_dot_w(int32_t beg, int32_t end, int sub, con
 template <typename V, int LANES, int MODE, int NV>
 __device__ __forceinline__ void csr_row(int64_t t, int64_t n, const int32_t *__restrict__ ia,
                                         const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                        const V *__restrict__ x, const V *__restrict__ b, V *__restrict__ y)
+                                        const V *x, const V *b, V *y)
 {
   const int64_t row = t / LANES;
   const int sub = (int)(t % LANES);
@@ -158,8 +158,8 @@ __device__ __forceinline__ void csr_row(int64_t t, int64_t n, const int32_t *__r
 template <typename V, int LANES, int MODE, int NV>
 __global__ void __launch_bounds__(256) k_csr(int64_t n, const int32_t *__restrict__ ia,
                                              const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                             const V *__restrict__ x, const V *__restrict__ b,
-                                             V *__restrict__ y, const int *__restrict__ skip)
+                                             const V *x, const V *b,
+                                             V *y, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -178,8 +178,8 @@ void csr(int lanes, int64_t n, const int32_t *ia, const int32_t *ja, const V *a,
 
 // Chebyshev start (x = 0): r = D^-1 b, d = r / theta, x = 0.
 template <typename V, int NV>
-__global__ void k_cheb_start(int64_t n, const V *__restrict__ dinv, const V *__restrict__ b, V *__restrict__ r,
-                             V *__restrict__ d, V *__restrict__ x, V inv_theta, const int *__restrict__ skip)
+__global__ void k_cheb_start(int64_t n, const V *__restrict__ dinv, const V *b, V *__restrict__ r,
+                             V *__restrict__ d, V *__restrict__ x, V inv_theta, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -195,9 +195,9 @@ __global__ void k_cheb_start(int64_t n, const V *__restrict__ dinv, const V *__r
 template <typename V, int LANES, int NV>
 __global__ void __launch_bounds__(256) k_cheb_restart(int64_t n, const int32_t *__restrict__ ia,
                                                       const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                                      const V *__restrict__ dinv, const V *__restrict__ b,
-                                                      const V *__restrict__ x, V *__restrict__ r,
-                                                      V *__restrict__ d, V inv_theta, const int *__restrict__ skip)
+                                                      const V *__restrict__ dinv, const V *b,
+                                                      const V *x, V *__restrict__ r,
+                                                      V *__restrict__ d, V inv_theta, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -223,9 +223,9 @@ __global__ void __launch_bounds__(256) k_cheb_restart(int64_t n, const int32_t *
 template <typename V, int LANES, int NV>
 __global__ void __launch_bounds__(256) k_cheb_step(int64_t n, const int32_t *__restrict__ ia,
                                                    const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                                   const V *__restrict__ dinv, const V *__restrict__ d,
-                                                   V *__restrict__ dn, V *__restrict__ r,
-                                                   V *__restrict__ x, V c1, V c2, const int *__restrict__ skip)
+                                                   const V *__restrict__ dinv, const V *d,
+                                                   V *__restrict__ dn, V *r,
+                                                   V *x, V c1, V c2, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -257,8 +257,8 @@ __global__ void __launch_bounds__(256) k_cheb_step(int64_t n, const int32_t *__r
 template <typename V, int LANES, int NV>
 __device__ __forceinline__ void cheb_first_row(int64_t t, int64_t n, const int32_t *__restrict__ ia,
                                                const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                               const V *__restrict__ dinv, const V *__restrict__ b,
-                                               V *__restrict__ dn, V *__restrict__ r, V *__restrict__ x,
+                                               const V *__restrict__ dinv, const V *b,
+                                               V *__restrict__ dn, V *r, V *x,
                                                V inv_theta, V c1, V c2)
 {
   const int64_t row = t / LANES;
@@ -290,9 +290,9 @@ __device__ __forceinline__ void cheb_first_row(int64_t t, int64_t n, const int32
 template <typename V, int LANES, int NV>
 __global__ void __launch_bounds__(256) k_cheb_first(int64_t n, const int32_t *__restrict__ ia,
                                                     const int32_t *__restrict__ ja, const V *__restrict__ a,
-                                                    const V *__restrict__ dinv, const V *__restrict__ b,
+                                                    const V *__restrict__ dinv, const V *b,
                                                     V *__restrict__ dn, V *__restrict__ r, V *__restrict__ x,
-                                                    V inv_theta, V c1, V c2, const int *__restrict__ skip)
+                                                    V inv_theta, V c1, V c2, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -363,9 +363,9 @@ __device__ __forceinline__ bool early_entry(const int *skip)
 template <typename V, int NV>
 __global__ void __launch_bounds__(256) k_cheb_first_sell(int64_t n, const int32_t *__restrict__ sp,
                                                          const int32_t *__restrict__ sc, const V *__restrict__ sv,
-                                                         const V *__restrict__ dinv, const V *__restrict__ b,
+                                                         const V *__restrict__ dinv, const V *b,
                                                          V *__restrict__ dn, V *__restrict__ r, V *__restrict__ x,
-                                                         V inv_theta, V c1, V c2, const int *__restrict__ skip)
+                                                         V inv_theta, V c1, V c2, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(256) k_up(int lu, int64_t n, const int32_t *__
 // Last step of a smoothing whose residual is not needed afterwards: x += d
 // only (the step's product with A would be discarded).
 template <typename V>
-__global__ void k_cheb_last(int64_t m, const V *__restrict__ d, V *__restrict__ x, const int *__restrict__ skip)
+__global__ void k_cheb_last(int64_t m, const V *d, V *x, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;

@@ -308,25 +308,33 @@ __global__ void k_fill(BlockSell::Part P, const int32_t *__restrict__ ia, const 
 }
 
 // The values of every entry from the CSR rows (padding: 0), one thread per
-// group.
+// group, the loads of four entries ahead of their stores (32^3 cube, two time
+// steps with an entry at a time 40.2 ms, two 39.1, four 38.9).
 template <int NR, int NC, typename VA>
 __device__ __forceinline__ void gather_steps(const int32_t *__restrict__ off, VA *__restrict__ val, int32_t k0,
-                                             int32_t k1, int lane, const VA *__restrict__ a, const int32_t (&beg)[NR])
+                                             int32_t k1, int lane, const VA *a, const int32_t (&beg)[NR])
 {
-  constexpr int NV = NR * NC, W = vec_width<VA, NV>(), PL = NV / W;
-  for(int32_t k = k0; k < k1; ++k) {
-    const int32_t o = off[((int64_t)k << 5) + lane];
+  constexpr int NV = NR * NC, W = vec_width<VA, NV>(), PL = NV / W, U = 4;
+  for(int32_t k = k0; k < k1; k += U) {
+    int32_t o[U];
+    VA v[U][NV];
 #pragma unroll
-    for(int q = 0; q < NV; ++q) {
-      const VA v = o >= 0 ? a[beg[q / NC] + o + q % NC] : (VA)0;
-      val[((((int64_t)k * PL + q / W) << 5) + lane) * W + q % W] = v;
-    }
+    for(int u = 0; u < U; ++u) o[u] = k + u < k1 ? off[((int64_t)(k + u) << 5) + lane] : -1;
+#pragma unroll
+    for(int u = 0; u < U; ++u)
+#pragma unroll
+      for(int q = 0; q < NV; ++q) v[u][q] = o[u] >= 0 ? a[beg[q / NC] + o[u] + q % NC] : (VA)0;
+#pragma unroll
+    for(int u = 0; u < U; ++u)
+      if(k + u < k1)
+#pragma unroll
+        for(int q = 0; q < NV; ++q) val[((((int64_t)(k + u) * PL + q / W) << 5) + lane) * W + q % W] = v[u][q];
   }
 }
 
 template <int NR, int D, typename VA>
 __global__ void __launch_bounds__(256) k_bgather(BlockSell::Part P, const int32_t *__restrict__ ia,
-                                                 const VA *__restrict__ a)
+                                                 const VA *a)
 {
   FE_PDL_ENTRY();
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -117,9 +117,9 @@ __global__ void __launch_bounds__(THREADS) k_ilu_stream(const IluStream::Step *_
                                                         const int32_t *__restrict__ start,
                                                         const int32_t *__restrict__ perm,
                                                         const uint4 *__restrict__ col, const V *__restrict__ val,
-                                                        const V *__restrict__ scale, const V *__restrict__ r,
+                                                        const V *__restrict__ scale, const V *r,
                                                         V *__restrict__ z,
-                                                        const int *__restrict__ done, int lateStep)
+                                                        const int *done, int lateStep)
 {
   FE_PDL_ENTRY();
   if(done && *done) return;

@@ -163,7 +163,7 @@ __device__ void finish_reduction(const double (&v)[K], double *partials, RedStat
   if(threadIdx.x == 0) st->counter = 0;
 }
 
-__global__ void k_dot(int64_t n, const double *__restrict__ x, const double *__restrict__ y,
+__global__ void k_dot(int64_t n, const double *x, const double *y,
                       double *partials, RedState *st, double *out)
 {
   FE_PDL_ENTRY();
@@ -174,7 +174,7 @@ __global__ void k_dot(int64_t n, const double *__restrict__ x, const double *__r
   finish_reduction<1, false>(v, partials, st, out);
 }
 
-__global__ void k_absmax(int64_t n, const double *__restrict__ x, double *partials, RedState *st,
+__global__ void k_absmax(int64_t n, const double *x, double *partials, RedState *st,
                          double *out)
 {
   FE_PDL_ENTRY();
@@ -186,8 +186,8 @@ __global__ void k_absmax(int64_t n, const double *__restrict__ x, double *partia
 }
 
 // ||w||^2 into st->result[0], 1 / ||w|| (0 for a zero w) into st->result[1].
-__global__ void k_norm_to(int64_t n, const double *__restrict__ w, double *partials, RedState *st,
-                          const int *__restrict__ done)
+__global__ void k_norm_to(int64_t n, const double *w, double *partials, RedState *st,
+                          const int *done)
 {
   FE_PDL_ENTRY();
   if(*done) return;
@@ -200,8 +200,8 @@ __global__ void k_norm_to(int64_t n, const double *__restrict__ w, double *parti
 }
 
 // v = w / ||w|| (st->result as k_norm_to leaves it), *Hsub = ||w||.
-__global__ void k_scale_from(int64_t n, const double *__restrict__ w, double *__restrict__ v,
-                             const RedState *st, double *Hsub, const int *__restrict__ done)
+__global__ void k_scale_from(int64_t n, const double *w, double *__restrict__ v,
+                             const RedState *st, double *Hsub, const int *done)
 {
   FE_PDL_ENTRY();
   if(*done) return;
@@ -213,8 +213,8 @@ __global__ void k_scale_from(int64_t n, const double *__restrict__ w, double *__
 }
 
 template <typename VO>
-__global__ void k_scale_vec(int64_t n, const double *__restrict__ w, VO *__restrict__ v,
-                            const double *__restrict__ s, int invert)
+__global__ void k_scale_vec(int64_t n, const double *w, VO *__restrict__ v,
+                            const double *s, int invert)
 {
   FE_PDL_ENTRY();
   const double f = invert ? (*s > 0 ? 1.0 / *s : 0.0) : *s;
@@ -223,8 +223,8 @@ __global__ void k_scale_vec(int64_t n, const double *__restrict__ w, VO *__restr
     v[i] = (VO)(w[i] * f);
 }
 
-__global__ void k_to_f32(int64_t n, const double *__restrict__ x, float *__restrict__ y,
-                         const int *__restrict__ done)
+__global__ void k_to_f32(int64_t n, const double *x, float *__restrict__ y,
+                         const int *done)
 {
   FE_PDL_ENTRY();
   if(done && *done) return;
@@ -299,8 +299,8 @@ __global__ void k_backsolve(GmresState *gs)
 // FP64 pipe of the GB300 would bound the pass at ~50 us for 50 columns of
 // 588 k rows; double-float keeps it at the bytes), added to x in FP64.
 template <typename VZ>
-__global__ void k_xupdate(int64_t n, int64_t ld, const VZ *__restrict__ Z, const GmresState *gs,
-                          double *__restrict__ x)
+__global__ void k_xupdate(int64_t n, int64_t ld, const VZ *Z, const GmresState *gs,
+                          double *x)
 {
   FE_PDL_ENTRY();
   const int k = gs->k;
@@ -364,10 +364,10 @@ __device__ __forceinline__ float4 ld4_l1(const float4 *p)
 }
 
 template <int CMAX, int MODE>
-__global__ void __launch_bounds__(RB, 3) k_gs32(int64_t n4, int m1, const float *__restrict__ V, int ncols,
-                                             const double *__restrict__ hprev, float *__restrict__ w,
+__global__ void __launch_bounds__(RB, 3) k_gs32(int64_t n4, int m1, const float *V, int ncols,
+                                             const double *hprev, float *w,
                                              double *partials, RedState *st, double *hcur, double *Hcol,
-                                             const int *__restrict__ done, int pass)
+                                             const int *done, int pass)
 {
   FE_PDL_ENTRY();
   // Rows are taken four at a time (16-byte loads); the basis is in row
@@ -487,9 +487,9 @@ __global__ void __launch_bounds__(RB, 3) k_gs32(int64_t n4, int m1, const float 
 // inverse; otherwise st->reorth asks for the second pass.
 // second = 1: the reorthogonalisation pass, run only when it was asked for;
 // its coefficients are added to the Hessenberg column.
-__global__ void __launch_bounds__(RB) k_gs_dots(int64_t n4, int m1, const float *__restrict__ V, int ncols,
-                                                const float *__restrict__ w, double *partials, RedState *st,
-                                                double *hcur, double *Hcol, const int *__restrict__ done,
+__global__ void __launch_bounds__(RB) k_gs_dots(int64_t n4, int m1, const float *V, int ncols,
+                                                const float *w, double *partials, RedState *st,
+                                                double *hcur, double *Hcol, const int *done,
                                                 int second, int pyth)
 {
   FE_PDL_ENTRY();
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(RB) k_gs_dots(int64_t n4, int m1, const float 
 // run only when it was asked for, adds h to Hcol) and st->result[2].
 // gridDim.x <= MAXRED.
 template <int CMAX>
-__global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const float *__restrict__ V,
+__global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const float *V,
                                                       int ncols, const float *w, double *partials,
                                                       RedState *st, double *hcur, double *Hcol,
                                                       const int *done, int second)
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(RB, 4) k_gs_dots_all(int64_t n4, int m1, const
 // (column ncols of the row-blocked basis, and its contiguous copy vcopy, the
 // preconditioner's next input); otherwise it goes back to w.
 template <int CMAX, bool NORM>
-__global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *__restrict__ V, int ncols,
+__global__ void __launch_bounds__(RB, 4) k_gs_upd(int64_t n4, int m1, float *V, int ncols,
                                                   const double *hprev, float *w,
                                                   float *__restrict__ vcopy, RedState *st, double *partials,
                                                   double *Hnext, const int *done, int second)
@@ -903,9 +903,9 @@ __device__ __forceinline__ double lane_sum_n(double (&v)[B], int lane)
 // (DOT only): slices of `slice` columns.
 template <int MODE, int TB, int R, int B>
 __global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
-    int64_t n, int64_t ld, const double *__restrict__ V, int ncols, int slice, const double *hprev,
+    int64_t n, int64_t ld, const double *V, int ncols, int slice, const double *hprev,
     const double *w, double *wo, double *partials, RedState *st, double *hcur, double *Hcol,
-    const int *__restrict__ done, int second)
+    const int *done, int second)
 {
   FE_PDL_ENTRY();
   if(*done) return;
@@ -1051,8 +1051,8 @@ __global__ void __launch_bounds__(TB, TB >= 256 ? 2 : 4) k_gs64(
 
 // V_0 = r / ||r|| rounded to FP32 (start of a mixed cycle; column 0 of the
 // row-blocked basis V and its contiguous copy vcopy), beta = ||r||.
-__global__ void k_scale_r32(int64_t n, const double *__restrict__ r, float *__restrict__ V, int m1,
-                            float *__restrict__ vcopy, const RedState *st, double *beta, const int *__restrict__ done)
+__global__ void k_scale_r32(int64_t n, const double *r, float *__restrict__ V, int m1,
+                            float *__restrict__ vcopy, const RedState *st, double *beta, const int *done)
 {
   FE_PDL_ENTRY();
   if(*done) return;
@@ -1087,8 +1087,8 @@ __global__ void k_gmres_init(GmresState *gs, const RedState *st)
 constexpr int ILU_NARROW_THREADS = 1024;  // one block of 32 warps runs a run of narrow levels
 
 template <typename VF>
-__global__ void k_ilu_copy(int64_t lnnz, const int32_t *__restrict__ srcPos, const double *__restrict__ v64,
-                           const float *__restrict__ v32, VF *__restrict__ f)
+__global__ void k_ilu_copy(int64_t lnnz, const int32_t *__restrict__ srcPos, const double *v64,
+                           const float *v32, VF *__restrict__ f)
 {
   FE_PDL_ENTRY();
   for(int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < lnnz; k += (int64_t)gridDim.x * blockDim.x)
@@ -1101,7 +1101,7 @@ __global__ void k_ilu_copy(int64_t lnnz, const int32_t *__restrict__ srcPos, con
 template <typename VF>
 __device__ __forceinline__ void ilu_factor_row(int32_t i, const int32_t *__restrict__ lia,
                                                const int32_t *__restrict__ lja, const int32_t *__restrict__ ldiag,
-                                               VF *__restrict__ f, int *__restrict__ status)
+                                               VF *f, int *__restrict__ status)
 {
   const int lane = threadIdx.x & 31;
   const int32_t rb = lia[i], re = lia[i + 1], rd = ldiag[i];
@@ -1142,7 +1142,7 @@ __device__ __forceinline__ void ilu_factor_row(int32_t i, const int32_t *__restr
 template <typename VF, typename VV, bool LOWER>
 __device__ __forceinline__ void ilu_solve_row(int32_t i, const int32_t *__restrict__ lia,
                                               const int32_t *__restrict__ lja, const int32_t *__restrict__ ldiag,
-                                              const VF *__restrict__ f, const VV *__restrict__ r, VV *__restrict__ z)
+                                              const VF *__restrict__ f, const VV *r, VV *z)
 {
   const int lane = threadIdx.x & 31;
   const int32_t d = ldiag[i];
@@ -1161,7 +1161,7 @@ template <typename VF>
 __global__ void __launch_bounds__(ILU_NARROW_THREADS) k_ilu_factor_run(
     int32_t lv0, int32_t lv1, const int32_t *__restrict__ lvl, const int32_t *__restrict__ rows,
     const int32_t *__restrict__ lia, const int32_t *__restrict__ lja, const int32_t *__restrict__ ldiag,
-    VF *__restrict__ f, int *__restrict__ status)
+    VF *f, int *__restrict__ status)
 {
   FE_PDL_ENTRY();
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1175,7 +1175,7 @@ __global__ void __launch_bounds__(ILU_NARROW_THREADS) k_ilu_factor_run(
 template <typename VF>
 __global__ void k_ilu_factor_level(int32_t q0, int32_t q1, const int32_t *__restrict__ rows,
                                    const int32_t *__restrict__ lia, const int32_t *__restrict__ lja,
-                                   const int32_t *__restrict__ ldiag, VF *__restrict__ f, int *__restrict__ status)
+                                   const int32_t *__restrict__ ldiag, VF *f, int *__restrict__ status)
 {
   FE_PDL_ENTRY();
   const int64_t q = q0 + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
@@ -1186,7 +1186,7 @@ template <typename VF, typename VV, bool LOWER>
 __global__ void __launch_bounds__(ILU_NARROW_THREADS) k_ilu_solve_run(
     int32_t lv0, int32_t lv1, const int32_t *__restrict__ lvl, const int32_t *__restrict__ rows,
     const int32_t *__restrict__ lia, const int32_t *__restrict__ lja, const int32_t *__restrict__ ldiag,
-    const VF *__restrict__ f, const VV *__restrict__ r, VV *__restrict__ z, const int *__restrict__ done)
+    const VF *__restrict__ f, const VV *r, VV *z, const int *done)
 {
   FE_PDL_ENTRY();
   if(done && *done) return;
@@ -1202,7 +1202,7 @@ template <typename VF, typename VV, bool LOWER>
 __global__ void k_ilu_solve_level(int32_t q0, int32_t q1, const int32_t *__restrict__ rows,
                                   const int32_t *__restrict__ lia, const int32_t *__restrict__ lja,
                                   const int32_t *__restrict__ ldiag, const VF *__restrict__ f,
-                                  const VV *__restrict__ r, VV *__restrict__ z, const int *__restrict__ done)
+                                  const VV *r, VV *z, const int *done)
 {
   FE_PDL_ENTRY();
   if(done && *done) return;
@@ -1211,8 +1211,8 @@ __global__ void k_ilu_solve_level(int32_t q0, int32_t q1, const int32_t *__restr
 }
 
 template <typename VV, typename VD>
-__global__ void k_jacobi(int64_t n, const VD *__restrict__ dinv, const VV *__restrict__ r,
-                         VV *__restrict__ z, const int *__restrict__ done)
+__global__ void k_jacobi(int64_t n, const VD *__restrict__ dinv, const VV *r,
+                         VV *__restrict__ z, const int *done)
 {
   FE_PDL_ENTRY();
   if(done && *done) return;
@@ -1222,7 +1222,7 @@ __global__ void k_jacobi(int64_t n, const VD *__restrict__ dinv, const VV *__res
 }
 
 template <typename VA, typename VD>
-__global__ void k_inv_diag(int64_t n, const int32_t *__restrict__ diag, const VA *__restrict__ a,
+__global__ void k_inv_diag(int64_t n, const int32_t *__restrict__ diag, const VA *a,
                            VD *__restrict__ dinv, int *__restrict__ status)
 {
   FE_PDL_ENTRY();
@@ -1245,7 +1245,7 @@ struct CGState {
 };
 
 // pq = p.q and alpha = rz / pq (done when pq is zero or not finite).
-__global__ void k_cg_pq(int64_t n, const double *__restrict__ p, const double *__restrict__ q, double *partials,
+__global__ void k_cg_pq(int64_t n, const double *p, const double *q, double *partials,
                         RedState *st, CGState *cs)
 {
   FE_PDL_ENTRY();
@@ -1261,19 +1261,35 @@ __global__ void k_cg_pq(int64_t n, const double *__restrict__ p, const double *_
 }
 
 // x += alpha p ; r -= alpha q ; rr = r.r, the convergence test
-__global__ void k_cg_xr(int64_t n, CGState *cs, const double *__restrict__ p,
-                        const double *__restrict__ q, double *__restrict__ x,
-                        double *__restrict__ r, double *partials, RedState *st)
+__global__ void k_cg_xr(int64_t n, CGState *cs, const double *p,
+                        const double *q, double *x,
+                        double *r, double *partials, RedState *st)
 {
   FE_PDL_ENTRY();
   if(cs->done) return;
   double v[1] = {0.};
   const double alpha = cs->alpha;
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * p[i];
-    const double ri = r[i] - alpha * q[i];
-    r[i] = ri;
-    v[0] += ri * ri;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for(int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
+    // four rows' loads ahead of their stores
+    double xv[4], pv[4], rv[4], qv[4];
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int64_t i = i0 + u * step < n ? i0 + u * step : i0;
+      xv[u] = x[i];
+      pv[u] = p[i];
+      rv[u] = r[i];
+      qv[u] = q[i];
+    }
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int64_t i = i0 + u * step;
+      if(i >= n) break;
+      const double ri = rv[u] - alpha * qv[u];
+      x[i] = xv[u] + alpha * pv[u];
+      r[i] = ri;
+      v[0] += ri * ri;
+    }
   }
   finish_reduction<1, false>(v, partials, st, nullptr, [&](double rr) {
     cs->rr = rr;
@@ -1283,7 +1299,7 @@ __global__ void k_cg_xr(int64_t n, CGState *cs, const double *__restrict__ p,
 }
 
 // rz = r.z, beta = rz / previous rz (first: 0)
-__global__ void k_cg_rz(int64_t n, const double *__restrict__ r, const double *__restrict__ z, double *partials,
+__global__ void k_cg_rz(int64_t n, const double *r, const double *z, double *partials,
                         RedState *st, CGState *cs, int first)
 {
   FE_PDL_ENTRY();
@@ -1299,7 +1315,7 @@ __global__ void k_cg_rz(int64_t n, const double *__restrict__ r, const double *_
 
 // p = z + beta p; the first p is z alone: p is not initialised then (0 * NaN
 // is NaN)
-__global__ void k_cg_p(int64_t n, const CGState *cs, const double *__restrict__ z, double *__restrict__ p, int first)
+__global__ void k_cg_p(int64_t n, const CGState *cs, const double *z, double *p, int first)
 {
   FE_PDL_ENTRY();
   if(cs->done) return;
@@ -1316,7 +1332,7 @@ __global__ void k_zero(int64_t n, double *x)
     x[i] = 0.;
 }
 
-__global__ void k_copy(int64_t n, const double *__restrict__ a, double *__restrict__ b)
+__global__ void k_copy(int64_t n, const double *a, double *__restrict__ b)
 {
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -1324,7 +1340,7 @@ __global__ void k_copy(int64_t n, const double *__restrict__ a, double *__restri
     b[i] = a[i];
 }
 
-__global__ void k_axpy(int64_t n, double alpha, const double *__restrict__ x, double *__restrict__ y)
+__global__ void k_axpy(int64_t n, double alpha, const double *x, double *__restrict__ y)
 {
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -1669,7 +1685,7 @@ void Krylov::ilu_solve_levels(const VV *r, VV *z, const int *done)
 
 namespace {
 // x split into two floats, x ~ hi + lo (the operand of BlockSell::resid32_df)
-__global__ void k_split_x(int64_t n, const double *__restrict__ x, float2 *__restrict__ xs)
+__global__ void k_split_x(int64_t n, const double *x, float2 *__restrict__ xs)
 {
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1879,7 +1895,7 @@ void Krylov::resid64(const double *vals, const double *x, const double *b, doubl
   else spmv_launch<double, double, double, double, true>(lanes_, n_, A_, vals, x, b, r, nullptr, s_);
 }
 
-__global__ void k_f32_to_f64(int64_t n, const float *__restrict__ x, double *__restrict__ y)
+__global__ void k_f32_to_f64(int64_t n, const float *x, double *__restrict__ y)
 {
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)

@@ -110,7 +110,7 @@ constexpr int NPART = 512;
 constexpr double SCHUR_FACTOR = 6.0;
 
 template <typename V>
-__global__ void k_dot_part(int64_t n, const V *__restrict__ a, const V *__restrict__ b, double *part)
+__global__ void k_dot_part(int64_t n, const V *a, const V *b, double *part)
 {
   FE_PDL_ENTRY();
   __shared__ double sh[256];
@@ -126,7 +126,7 @@ __global__ void k_dot_part(int64_t n, const V *__restrict__ a, const V *__restri
   if(threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__global__ void k_dot_fin(int nparts, const double *__restrict__ part, double *out)
+__global__ void k_dot_fin(int nparts, const double *part, double *out)
 {
   FE_PDL_ENTRY();
   __shared__ double sh[256];
@@ -144,8 +144,8 @@ __global__ void k_dot_fin(int nparts, const double *__restrict__ part, double *o
 // x += alpha p, r -= alpha q with alpha = rz / pq (device scalars); a zero
 // or non-finite pq leaves x, r unchanged.
 template <typename V>
-__global__ void k_pcg_xr(int64_t n, const double *__restrict__ scal, const V *__restrict__ p,
-                         const V *__restrict__ q, V *__restrict__ x, V *__restrict__ r)
+__global__ void k_pcg_xr(int64_t n, const double *scal, const V *p,
+                         const V *q, V *x, V *r)
 {
   FE_PDL_ENTRY();
   const double pq = scal[1];
@@ -159,7 +159,7 @@ __global__ void k_pcg_xr(int64_t n, const double *__restrict__ scal, const V *__
 // p = z + beta p with beta = rz_new / rz (scal[2] / scal[0]); then rz =
 // rz_new.  The first p is z alone (p is not initialised then: 0 * NaN is NaN).
 template <typename V>
-__global__ void k_pcg_p(int64_t n, const double *__restrict__ scal, const V *__restrict__ z, V *__restrict__ p,
+__global__ void k_pcg_p(int64_t n, const double *scal, const V *z, V *p,
                         int first)
 {
   FE_PDL_ENTRY();
@@ -172,7 +172,7 @@ __global__ void k_pcg_shift(double *scal) {
   FE_PDL_ENTRY(); scal[0] = scal[2]; }
 
 template <typename V>
-__global__ void k_copy_v(int64_t n, const V *__restrict__ a, V *__restrict__ b)
+__global__ void k_copy_v(int64_t n, const V *a, V *__restrict__ b)
 {
   FE_PDL_ENTRY();
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -237,7 +237,7 @@ int grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 25
 // partial sums of the entries a[pos[i]] (the finest velocity diagonal),
 // one per block; k_dot_fin adds them in block order
 template <typename VA>
-__global__ void k_diag_part(int64_t n, const int32_t *__restrict__ pos, const VA *__restrict__ a, double *part)
+__global__ void k_diag_part(int64_t n, const int32_t *__restrict__ pos, const VA *a, double *part)
 {
   FE_PDL_ENTRY();
   __shared__ double sh[256];
@@ -254,8 +254,8 @@ __global__ void k_diag_part(int64_t n, const int32_t *__restrict__ pos, const VA
 }
 
 template <typename V>
-__global__ void k_scale_copy(int64_t n, const V *__restrict__ r, V *__restrict__ z, V f,
-                             const int *__restrict__ skip)
+__global__ void k_scale_copy(int64_t n, const V *r, V *__restrict__ z, V f,
+                             const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -268,9 +268,9 @@ __global__ void k_scale_copy(int64_t n, const V *__restrict__ r, V *__restrict__
 // c = 1 on the pressure unknowns, (c^T r) read from *cr.
 template <typename V, typename S>
 __global__ void k_pressure(int64_t nP, const int32_t *__restrict__ rows, const S *__restrict__ sc,
-                           const double *__restrict__ mass, const double *__restrict__ cr,
-                           const double *__restrict__ consts, const V *__restrict__ r, V *__restrict__ z,
-                           const int *__restrict__ skip)
+                           const double *__restrict__ mass, const double *cr,
+                           const double *__restrict__ consts, const V *r, V *__restrict__ z,
+                           const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -290,7 +290,7 @@ __global__ void k_pressure(int64_t nP, const int32_t *__restrict__ rows, const S
 // of k_vel_rhs_fold).
 template <typename V>
 __device__ __forceinline__ void psum_blocks(int vb, int vg, int64_t nP, const int32_t *__restrict__ rows,
-                                            const V *__restrict__ r, V f, double *part, unsigned *count,
+                                            const V *r, V f, double *part, unsigned *count,
                                             double *out)
 {
   __shared__ double sh[256];
@@ -327,7 +327,7 @@ __device__ __forceinline__ void psum_blocks(int vb, int vg, int64_t nP, const in
 }
 
 template <typename V>
-__global__ void k_psum(int64_t nP, const int32_t *__restrict__ rows, const V *__restrict__ r, double *part,
+__global__ void k_psum(int64_t nP, const int32_t *__restrict__ rows, const V *r, double *part,
                        unsigned *count, double *out)
 {
   FE_PDL_ENTRY();
@@ -335,7 +335,7 @@ __global__ void k_psum(int64_t nP, const int32_t *__restrict__ rows, const V *__
 }
 
 // partial sums of a double array
-__global__ void k_tsum(int64_t n, const double *__restrict__ t, double *part)
+__global__ void k_tsum(int64_t n, const double *t, double *part)
 {
   FE_PDL_ENTRY();
   __shared__ double sh[256];
@@ -354,7 +354,7 @@ __global__ void k_tsum(int64_t n, const double *__restrict__ t, double *part)
 // g = G c: row sums of the G block per velocity slot.
 template <typename V>
 __global__ void k_gsum(int64_t nN, const int32_t *__restrict__ upIa, const int32_t *__restrict__ upPos,
-                       const V *__restrict__ a, V *__restrict__ bx, V *__restrict__ by)
+                       const V *a, V *__restrict__ bx, V *__restrict__ by)
 {
   FE_PDL_ENTRY();
   for(int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nN; k += (int64_t)gridDim.x * blockDim.x)
@@ -370,7 +370,7 @@ __global__ void k_gsum(int64_t nN, const int32_t *__restrict__ upIa, const int32
 template <typename V>
 __global__ void k_dw(int64_t nP, const int32_t *__restrict__ dnIa, const int32_t *__restrict__ dnPos,
                      const int32_t *__restrict__ dnCol, const int32_t *__restrict__ slotOf,
-                     const V *__restrict__ a, const V *__restrict__ wx, const V *__restrict__ wy,
+                     const V *a, const V *wx, const V *wy,
                      double *__restrict__ t)
 {
   FE_PDL_ENTRY();
@@ -390,8 +390,8 @@ template <typename V>
 __global__ void k_vel_rhs(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
                           const int32_t *__restrict__ upIa, const int32_t *__restrict__ upPos,
                           const int32_t *__restrict__ upCol, const V *__restrict__ a,
-                          const V *__restrict__ r, const V *__restrict__ z, V *__restrict__ bx,
-                          V *__restrict__ by, const int *__restrict__ skip)
+                          const V *r, const V *z, V *__restrict__ bx,
+                          V *__restrict__ by, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -409,7 +409,7 @@ __global__ void k_vel_rhs(int64_t nN, const int32_t *__restrict__ dofX, const in
 }
 
 template <typename V>
-__global__ void k_gather_vals(int64_t n, const int32_t *__restrict__ pos, const V *__restrict__ a, V *__restrict__ out)
+__global__ void k_gather_vals(int64_t n, const int32_t *__restrict__ pos, const V *a, V *__restrict__ out)
 {
   FE_PDL_ENTRY();
   for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
@@ -421,8 +421,8 @@ __global__ void k_gather_vals(int64_t n, const int32_t *__restrict__ pos, const 
 // z_p += cc * pz afterwards.
 template <typename V>
 __global__ void k_p_gather(int64_t nP, const int32_t *__restrict__ rows, const double *__restrict__ mass,
-                           const double *__restrict__ cr, const double *__restrict__ consts, const V *__restrict__ r,
-                           V *__restrict__ pr, const int *__restrict__ skip)
+                           const double *cr, const double *__restrict__ consts, const V *r,
+                           V *__restrict__ pr, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -433,8 +433,8 @@ __global__ void k_p_gather(int64_t nP, const int32_t *__restrict__ rows, const d
 }
 
 template <typename V>
-__global__ void k_p_add(int64_t nP, const int32_t *__restrict__ rows, const V *__restrict__ pz,
-                        const double *__restrict__ consts, V *__restrict__ z, const int *__restrict__ skip)
+__global__ void k_p_add(int64_t nP, const int32_t *__restrict__ rows, const V *pz,
+                        const double *__restrict__ consts, V *z, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -448,8 +448,8 @@ template <typename V>
 __global__ void k_vel_rhs_pair(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
                                const int32_t *__restrict__ upIa, const int32_t *__restrict__ upPos,
                                const int32_t *__restrict__ upCol, const V *__restrict__ a,
-                               const V *__restrict__ r, const V *__restrict__ z, V *__restrict__ bxy,
-                               const int *__restrict__ skip)
+                               const V *r, const V *z, V *__restrict__ bxy,
+                               const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -475,9 +475,9 @@ __global__ void k_vel_rhs_pair(int64_t nN, const int32_t *__restrict__ dofX, con
 template <typename V>
 __global__ void k_vel_rhs_fold(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
                                const int32_t *__restrict__ upIa, const int32_t *__restrict__ upCol,
-                               const V *__restrict__ gs, const V *__restrict__ r, V *__restrict__ bxy,
+                               const V *__restrict__ gs, const V *r, V *__restrict__ bxy,
                                int gp, int64_t nP, const int32_t *__restrict__ pRows, double *part,
-                               unsigned *count, double *cr, ScaleStep<V> sc, const int *__restrict__ skip)
+                               unsigned *count, double *cr, ScaleStep<V> sc, const int *skip)
 {
   FE_PDL_ENTRY();
   const V *x = sc.w ? sc.w : r;
@@ -525,7 +525,7 @@ __global__ void k_pressure_scale(int64_t nP, double coef, double den, const doub
 // gu[q] = sum_e G_e u_k(e) on slot q (FP64 sums).
 template <typename V, typename S>
 __global__ void k_fold_prep(int64_t nq, const int32_t *__restrict__ upIa, const int32_t *__restrict__ upColP,
-                            const V *__restrict__ g, const S *__restrict__ sc, const double *__restrict__ u,
+                            const V *g, const S *sc, const double *u,
                             V *__restrict__ gScaled, V *__restrict__ gu)
 {
   FE_PDL_ENTRY();
@@ -542,8 +542,8 @@ __global__ void k_fold_prep(int64_t nq, const int32_t *__restrict__ upIa, const 
 
 template <typename V>
 __global__ void k_vel_out_pair(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
-                               const V *__restrict__ zxy, const double *__restrict__ consts, V *__restrict__ z,
-                               const int *__restrict__ skip)
+                               const V *zxy, const double *__restrict__ consts, V *__restrict__ z,
+                               const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -556,8 +556,8 @@ __global__ void k_vel_out_pair(int64_t nN, const int32_t *__restrict__ dofX, con
 
 template <typename V>
 __global__ void k_vel_out(int64_t nN, const int32_t *__restrict__ dofX, const int32_t *__restrict__ dofY,
-                          const V *__restrict__ zx, const V *__restrict__ zy, const double *__restrict__ consts,
-                          V *__restrict__ z, const int *__restrict__ skip)
+                          const V *zx, const V *zy, const double *__restrict__ consts,
+                          V *__restrict__ z, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -572,8 +572,8 @@ __global__ void k_vel_out(int64_t nN, const int32_t *__restrict__ dofX, const in
 // b[q] = r_u - G z_p on slot q.
 template <typename V>
 __global__ void k_vel_rhs_nc(int64_t nq, const int32_t *__restrict__ dofC, const int32_t *__restrict__ upIa,
-                             const int32_t *__restrict__ upCol, const V *__restrict__ g, const V *__restrict__ r,
-                             const V *__restrict__ z, V *__restrict__ b, const int *__restrict__ skip)
+                             const int32_t *__restrict__ upCol, const V *__restrict__ g, const V *r,
+                             const V *z, V *__restrict__ b, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -585,8 +585,8 @@ __global__ void k_vel_rhs_nc(int64_t nq, const int32_t *__restrict__ dofC, const
 }
 
 template <typename V>
-__global__ void k_vel_out_nc(int64_t nq, const int32_t *__restrict__ dofC, const V *__restrict__ zc,
-                             const double *__restrict__ consts, V *__restrict__ z, const int *__restrict__ skip)
+__global__ void k_vel_out_nc(int64_t nq, const int32_t *__restrict__ dofC, const V *zc,
+                             const double *__restrict__ consts, V *__restrict__ z, const int *skip)
 {
   FE_PDL_ENTRY();
   if(skip && *skip) return;
@@ -598,7 +598,7 @@ __global__ void k_vel_out_nc(int64_t nq, const int32_t *__restrict__ dofC, const
 // g = G c per slot (row sums of the G block).
 template <typename V>
 __global__ void k_gsum_nc(int64_t nq, const int32_t *__restrict__ upIa, const int32_t *__restrict__ upPos,
-                          const V *__restrict__ a, V *__restrict__ b)
+                          const V *a, V *__restrict__ b)
 {
   FE_PDL_ENTRY();
   for(int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += (int64_t)gridDim.x * blockDim.x) {
@@ -612,7 +612,7 @@ __global__ void k_gsum_nc(int64_t nq, const int32_t *__restrict__ upIa, const in
 template <typename V>
 __global__ void k_dw_nc(int64_t nP, const int32_t *__restrict__ dnIa, const int32_t *__restrict__ dnPos,
                         const int32_t *__restrict__ dnCol, const int32_t *__restrict__ slotOf,
-                        const V *__restrict__ a, const V *__restrict__ w, double *__restrict__ t)
+                        const V *a, const V *w, double *__restrict__ t)
 {
   FE_PDL_ENTRY();
   for(int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nP; k += (int64_t)gridDim.x * blockDim.x) {

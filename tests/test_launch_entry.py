@@ -58,3 +58,25 @@ def test_only_operators_and_older_columns_are_read_ahead_of_the_entry():
             assert re.search(r"ahead = [^;]*(cb \+ 8 < ncols|ncols > 8);", ahead), n
             assert "__ldcg(" in ahead and "__ldcs(" not in ahead and "load(" not in ahead, n
             assert "w4[" not in ahead and "(w)[" not in ahead, n
+
+
+# Read-only for as long as a system's set-up or factorisation stands: patterns
+# and maps, and operators where an iteration's kernels read them.
+CONSTANT = set("""ia ja a dinv sp sc sv ria rja ra tia tja ta trow qia qja qa qrow M steps stepStart start perm col from
+lia lja ldiag val scale lvl rows srcPos diag pos upIa upPos upCol upColP dnIa dnPos dnCol slotOf dofX dofY dofC pRows
+mass consts gs f g""".split())
+# ... and where a kernel of the factorisation reads values that one before it wrote.
+FORMED = {"k_bgather": {"a"}, "k_inv_diag": {"a"}, "k_diag_part": {"a"}, "k_gsum": {"a"}, "k_dw": {"a"},
+          "k_gather_vals": {"a"}, "k_gsum_nc": {"a"}, "k_dw_nc": {"a"}, "k_fold_prep": {"g", "sc", "u"},
+          "k_dot_part": {"a", "b"}, "k_copy_v": {"a"}, "k_copy": {"a"}, "k_ilu_pack": {"f"}}
+
+
+def test_what_an_earlier_kernel_writes_is_read_through_plain_pointers():
+    """Loads through const __restrict__ pointers are read-only to the compiler,
+    which may move them ahead of the entry."""
+    found = []
+    for n, params, _ in entered_kernels():
+        for x in re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params):
+            if x not in CONSTANT or x in FORMED.get(n, ()):
+                found.append(f"{n}: {x}")
+    assert found == []
