@@ -176,21 +176,6 @@ void csr(int lanes, int64_t n, const int32_t *ia, const int32_t *ja, const V *a,
   else ::feng::launch_k(k_csr<V, 4, MODE, NV>, g, 256, 0, s, n, ia, ja, a, x, b, y, skip);
 }
 
-// Chebyshev start (x = 0): r = D^-1 b, d = r / theta, x = 0.
-template <typename V, int NV>
-__global__ void k_cheb_start(int64_t n, const V *__restrict__ dinv, const V *b, V *__restrict__ r,
-                             V *__restrict__ d, V *__restrict__ x, V inv_theta, const int *skip)
-{
-  FE_PDL_ENTRY();
-  if(skip && *skip) return;
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * NV; i += (int64_t)gridDim.x * blockDim.x) {
-    const V ri = dinv[i / NV] * b[i];
-    r[i] = ri;
-    d[i] = ri * inv_theta;
-    x[i] = 0;
-  }
-}
-
 // Chebyshev start from a nonzero x: r = D^-1 (b - A x), d = r / theta.
 template <typename V, int LANES, int NV>
 __global__ void __launch_bounds__(256) k_cheb_restart(int64_t n, const int32_t *__restrict__ ia,
@@ -957,7 +942,7 @@ static void chebyshev(int lanes, int64_t n, const int32_t *ia, const int32_t *ja
   const int g = grid(n * lanes);
   int k0 = 0;
   V *d = d0, *dn = d1;
-  if(zeroStart && (needResidual || p.chebyDegree > 1)) {
+  if(zeroStart) {
     // start + first step in one pass
     const double rhoN = 1.0 / (2.0 * sigma - rho);
     const V c1 = (V)(rhoN * rho), c2 = (V)(2.0 * rhoN / delta);
@@ -969,8 +954,6 @@ static void chebyshev(int lanes, int64_t n, const int32_t *ia, const int32_t *ja
     rho = rhoN;
     std::swap(d, dn);
     k0 = 1;
-  } else if(zeroStart) {
-    ::feng::launch_k(k_cheb_start<V, NV>, grid(n * NV), 256, 0, s, n, dinv, b, r, d0, x, (V)(1.0 / theta), skip);
   } else {
     if(lanes == 16) ::feng::launch_k(k_cheb_restart<V, 16, NV>, g, 256, 0, s, n, ia, ja, a, dinv, b, x, r, d0, (V)(1.0 / theta), skip);
     else if(lanes == 8) ::feng::launch_k(k_cheb_restart<V, 8, NV>, g, 256, 0, s, n, ia, ja, a, dinv, b, x, r, d0, (V)(1.0 / theta), skip);

@@ -212,17 +212,6 @@ __global__ void k_scale_from(int64_t n, const double *w, double *__restrict__ v,
     v[i] = w[i] * inv;
 }
 
-template <typename VO>
-__global__ void k_scale_vec(int64_t n, const double *w, VO *__restrict__ v,
-                            const double *s, int invert)
-{
-  FE_PDL_ENTRY();
-  const double f = invert ? (*s > 0 ? 1.0 / *s : 0.0) : *s;
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = (VO)(w[i] * f);
-}
-
 __global__ void k_to_f32(int64_t n, const double *x, float *__restrict__ y,
                          const int *done)
 {
@@ -1338,14 +1327,6 @@ __global__ void k_copy(int64_t n, const double *a, double *__restrict__ b)
   for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (int64_t)gridDim.x * blockDim.x)
     b[i] = a[i];
-}
-
-__global__ void k_axpy(int64_t n, double alpha, const double *x, double *__restrict__ y)
-{
-  FE_PDL_ENTRY();
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (int64_t)gridDim.x * blockDim.x)
-    y[i] += alpha * x[i];
 }
 
 }  // namespace

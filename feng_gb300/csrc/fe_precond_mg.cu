@@ -253,16 +253,6 @@ __global__ void k_diag_part(int64_t n, const int32_t *__restrict__ pos, const VA
   if(threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-template <typename V>
-__global__ void k_scale_copy(int64_t n, const V *r, V *__restrict__ z, V f,
-                             const int *skip)
-{
-  FE_PDL_ENTRY();
-  if(skip && *skip) return;
-  for(int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    z[i] = r[i] * f;
-}
-
 // Pressure block with the constant mode deflated:
 //   z_p = pscale_p (r_p - (c^T r) m_p / c^T M c) + (c^T r) / c^T S c,
 // c = 1 on the pressure unknowns, (c^T r) read from *cr.

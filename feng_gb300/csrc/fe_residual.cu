@@ -545,13 +545,8 @@ void ResidualTH::run(const FormCoeffs &fc, const In *tab, const In *u, const In 
   // tetrahedra: 3 warps a block, 15 an SM within 128 registers; triangles: 4,
   // or 2 while the elements do not give every SM one block
   const int eb = D == 2 && nE >= 152 * 64 ? 64 : 32;
+  // (at most 34 KB: 64 nodes of a tetrahedral rule)
   auto bytes = [](int ns, int e) { return 8 * (size_t)(table_words(D) + own_words(D, ns) + elem_words(D) * e); };
-  static bool set = false;
-  if(!set) {
-    cudaFuncSetAttribute(k_residual_elem<D, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)bytes(RES_MAXQ, 64));
-    set = true;
-  }
   (k_residual_elem<D, A><<<(unsigned)((nE + eb - 1) / eb), dim3(eb, D), bytes(nqs, eb), s_>>>(
        nE, dm_.adr, dm_.geo, dm_.geoPair, dm_.xy, tab, own_, fc, coeffs<typename A::T>(fc), u, ud, nqs, be_),
    ::feng::count_launch());

@@ -12,8 +12,6 @@
 
 namespace feng {
 
-constexpr int RES_MAXQ = 64;  // nodes of a rule
-
 // Tables of a rule on the reference element (D = 2: 3 + 3 functions, D = 3:
 // 4 + 6), in the order in which a block keeps them; l: the barycentric
 // coordinates.
