@@ -1,6 +1,6 @@
 // Device V-cycle of the smoothed-aggregation hierarchy (see fe_amg.h).
 // Smoother degree 1 (damped Jacobi, the default): two kernels per level on
-// the level's combined operators (Lev::downT and below).  Degree 2 to 6:
+// the level's combined operators (AMGDevice::Lev: T, Q, Q^T).  Degree 2 to 6:
 // Chebyshev smoothing on D^-1 A (polynomial, SpMV-only), residual,
 // restriction, coarse correction, prolongation, Chebyshev again.  The
 // coarsest level is a dense inverse applied as a mat-vec.
@@ -781,7 +781,7 @@ AMGDevice::~AMGDevice()
   cudaFree(coarseInv_);
 }
 
-// The combined operators of a level (Lev::downT): with w = D^-1 / theta,
+// The combined operators of a level (AMGDevice::Lev: T, Q, Q^T): with w = D^-1 / theta,
 //   T = 2 w - w A w    (A's pattern),
 //   Q = P - w (A P)    (the pattern of A P, which holds P's: A has a diagonal),
 // so that the damped-Jacobi V-cycle of the level is b_c = Q^T b and

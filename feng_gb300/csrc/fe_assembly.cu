@@ -2,8 +2,8 @@
 // the fused weak forms.
 //
 // Colored kernels (scalar P2 residual and Jacobian; Taylor-Hood residuals:
-// fe_residual.cu): one launch per element color, entries scattered into CSR through the element-to-nonzero map as
-// L2 reductions; no two elements of a color share a DOF, so every entry
+// fe_residual.cu): one launch per element color, entries scattered into CSR
+// through the element-to-nonzero map as L2 reductions; no two elements of a color share a DOF, so every entry
 // receives one contribution per color and the sums are the colored
 // read-modify-write's, in color order.
 //
@@ -376,8 +376,8 @@ __global__ void k_pack_th(DeviceMesh dm, int hasConv, const double *__restrict__
 
 // Both component rows (a, 0) and (a, 1) of velocity function a of an
 // element, from its packed data e (u, G, J): A[m][12] velocity columns and
-// the pressure-column factors Bp[m][3] -- k_matrix_th's arithmetic for one
-// (element, a).
+// the pressure-column factors Bp[m][3], by the contraction described above for
+// one (element, a) (k_jac_th regroups it: the two agree to rounding).
 template <typename V>
 __device__ __forceinline__ void th_rows_pair(const SharedTensors<V> &sT, const FormCoeffs &fc, double c0,
                                              const V *e, int a, V (&A)[2][12], V (&Bp)[2][3])
@@ -468,10 +468,10 @@ __device__ __forceinline__ void th_rows_pair(const SharedTensors<V> &sT, const F
 // Thread = unit (RowAsm): a pair of component rows of one velocity node, or
 // one row.  Entry (p, li): li < 12 is velocity row (a = li / 2, component
 // m = li % 2) of element p, whose 12 velocity and 3 pressure columns are the
-// element-matrix row of k_matrix_th; li >= 12 is pressure row j = li - 12,
+// element matrix's row; li >= 12 is pressure row j = li - 12,
 // whose 12 velocity columns are divu * int psi_j d_m phi_a.  A pair takes
 // the entries of its component-0 row and builds both rows (same columns,
-// same offsets); the arithmetic is k_matrix_th's.
+// same offsets); th_rows_pair.
 template <typename V>
 __global__ void __launch_bounds__(256) k_matrix_th_rows(RowAsm ra, FormCoeffs fc, const RefTensors *__restrict__ gT,
                                                         double c0, V *__restrict__ values, int accumulate)

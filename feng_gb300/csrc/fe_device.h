@@ -113,8 +113,8 @@ struct DeviceMesh {
 // CSR row from the (element, local row) entries whose DOF is that row, in
 // color order of the elements, inside a shared-memory copy of its block's
 // contiguous range of CSR values, which the block then writes once.  No
-// atomics, no element-to-nonzero map; each value is the same sum, in the
-// same order, as the colored scatter.
+// atomics, no element-to-nonzero map; each value sums its elements' terms in
+// the colored scatter's order.
 // Units: a velocity node's two component rows together when they hold the
 // same columns (one thread builds both, sharing the element terms), else one
 // row.

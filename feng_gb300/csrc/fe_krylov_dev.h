@@ -35,8 +35,8 @@ struct GmresState : GmresHead {
 };
 
 // One warp: the column and the previous rotations are staged in shared
-// memory, the (inherently sequential) rotation chain runs on lane 0 out of
-// registers and shared memory, and the column is written back by the warp.
+// memory, the rotation chain runs as a scan over the lanes, and the column is
+// written back by the warp.
 // Applies the previous rotations to Hessenberg column j, forms rotation j,
 // updates g and the residual estimate, sets done (one warp; sh, scs, ssn:
 // shared arrays of MAXM + 1, MAXM, MAXM doubles).

@@ -1,4 +1,5 @@
-// Taylor-Hood residuals, one thread per element (see fe_residual.h).
+// Taylor-Hood residuals, one thread per element and velocity component (see
+// fe_residual.h).
 #include "fe_residual.h"
 
 #include <algorithm>

@@ -51,7 +51,7 @@ def test_assembly_fp32_matrix(name):
 
 
 def test_double_float_residual_with_mass_matches_fp64():
-    """The mixed path's residual (double-float, k_residual_th_df) against the
+    """The mixed path's residual (double-float, k_residual_elem) against the
     FP64 kernel on the lid-driven cavity forms (transient mass with a
     nonzero u-dot, convection, stress, divergence) at a random state."""
     from helpers import cavity_spaces
